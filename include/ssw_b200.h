@@ -268,6 +268,31 @@ int ssw_voxel_grid_build(const int32_t* coords, int64_t n, int32_t batch, const 
                          int32_t* grid, int32_t* err, void* stream);
 int ssw_subm_neighbors(const int32_t* coords, int64_t n, int32_t batch, const int32_t dims[3],
                        const int32_t* grid, int32_t ksize, int32_t* nbr, void* stream);
+/* Whole rulebooks, in two calls each: *_count leaves the sizes to allocate by in the first words of
+ * `workspace` (the caller reads them back), the second call fills the arrays from the same workspace.
+ * Coordinates int32 [n, 4] (b, z, y, x), n > 0.
+ * ssw_subm_rulebook_count: nbr as ssw_subm_neighbors gives it; workspace[0] = error bits
+ *   (SSW_DEV_BAD_COORD / SSW_DEV_DUPLICATE), [1] = pairs of the off-centre tap that has most, [2] = all
+ *   off-centre pairs.
+ * ssw_subm_rulebook_pairs: the off-centre pairs grouped by tap, every tap's run `seg` slots long (seg >=
+ *   workspace[1]): pair_in [(k^3 - 1) * seg] input voxel of every slot (runs in output order, -1 behind
+ *   them), row_start [n + 1] and row_slots [workspace[2]] the slots of every output voxel in tap order.
+ * ssw_strided_rulebook_count (kernel = stride = ksize, out_dims = output grid): workspace[0] = error bits,
+ *   [1] = occupied output cells m.
+ * ssw_strided_rulebook_fill: parent [n] (-1: no output cell) and tap [n] of every voxel, nbr [m, k^3],
+ *   out_coords [m, 4] in ascending cell order. */
+int64_t ssw_subm_rulebook_workspace_ints(int64_t n, int32_t batch, const int32_t dims[3], int32_t ksize);
+int ssw_subm_rulebook_count(const int32_t* coords, int64_t n, int32_t batch, const int32_t dims[3], int32_t ksize,
+                            int32_t* nbr, int32_t* workspace, void* stream);
+int ssw_subm_rulebook_pairs(const int32_t* nbr, int64_t n, int32_t batch, const int32_t dims[3], int32_t ksize,
+                            int64_t seg, const int32_t* workspace, int32_t* pair_in, int32_t* row_start,
+                            int32_t* row_slots, void* stream);
+int64_t ssw_strided_rulebook_workspace_ints(int32_t batch, const int32_t out_dims[3]);
+int ssw_strided_rulebook_count(const int32_t* coords, int64_t n, int32_t batch, const int32_t out_dims[3],
+                               int32_t ksize, int32_t* workspace, void* stream);
+int ssw_strided_rulebook_fill(const int32_t* coords, int64_t n, int32_t batch, const int32_t out_dims[3], int32_t ksize,
+                              const int32_t* workspace, int64_t m, int32_t* parent, int32_t* tap, int32_t* nbr,
+                              int32_t* out_coords, void* stream);
 int ssw_gather_cols(const void* x, int dtype, int64_t n_src, int64_t m_rows, int32_t taps, int32_t cin,
                     const int32_t* nbr, void* cols, void* stream);
 int ssw_gather_slices(const void* z, int dtype, int64_t n_src, int32_t taps, int32_t cout, int64_t n,

@@ -64,6 +64,12 @@ def _load() -> C.CDLL:
         "ssw_attn_fused_multi": (C.c_int, [vp, C.c_int, i32, i32, P(PlanLayout), vp, vp, P(i32), f32, C.c_int, P(vp), i32, vp, vp]),
         "ssw_voxel_grid_build": (C.c_int, [vp, i64, i32, P(i32), vp, vp, vp]),
         "ssw_subm_neighbors": (C.c_int, [vp, i64, i32, P(i32), vp, i32, vp, vp]),
+        "ssw_subm_rulebook_workspace_ints": (i64, [i64, i32, P(i32), i32]),
+        "ssw_subm_rulebook_count": (C.c_int, [vp, i64, i32, P(i32), i32, vp, vp, vp]),
+        "ssw_subm_rulebook_pairs": (C.c_int, [vp, i64, i32, P(i32), i32, i64, vp, vp, vp, vp, vp]),
+        "ssw_strided_rulebook_workspace_ints": (i64, [i32, P(i32)]),
+        "ssw_strided_rulebook_count": (C.c_int, [vp, i64, i32, P(i32), i32, vp, vp]),
+        "ssw_strided_rulebook_fill": (C.c_int, [vp, i64, i32, P(i32), i32, vp, i64, vp, vp, vp, vp, vp]),
         "ssw_gather_cols": (C.c_int, [vp, C.c_int, i64, i64, i32, i32, vp, vp, vp]),
         "ssw_gather_reduce": (C.c_int, [vp, vp, C.c_int, i64, vp, vp, i64, i64, i32, vp, vp]),
         "ssw_gather_slices": (C.c_int, [vp, C.c_int, i64, i32, i32, i64, vp, vp, vp, vp]),

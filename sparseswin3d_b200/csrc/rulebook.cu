@@ -1,0 +1,361 @@
+// Rulebooks of the sparse convolutions (sparse_conv.cu), built on the device in two calls each: a
+// counting call that leaves the sizes the host has to allocate by in a small device array (one
+// read-back), and a filling call.
+//
+// What bounds a build is the random access to the cell tables of the scene.  An occupancy bitmap
+// (1 bit per cell: 3 MB for 400 x 400 x 150, resident in every cache level that matters) answers nine
+// in ten of the 27 look-ups of a voxel on a surface-sparse scene; only occupied neighbours read the
+// 4-byte id table, which therefore needs no clearing (96 MB of stores at that size): a cell whose bit
+// is clear is never read.
+//
+// Submanifold rulebook, pair form.  The existing (input, output) pairs are grouped by tap in output
+// order, so a pair's slot is (pairs of its tap in earlier blocks of output voxels) + (rank inside the
+// block): k_rb_neighbors leaves per-(tap, block) counts, k_rb_scan turns every tap's counts into
+// prefixes (one block per tap), k_rb_pairs ranks inside the block by warp ballots.  Everything is in
+// voxel order, so the result does not depend on scheduling.
+//
+// 150 000-voxel room, 3^3 taps (400 x 400 x 150 cells): 61 us of kernels (28 neighbours, 22 pairs, 5 mark)
+// against 0.59 ms as torch index arithmetic (a [26, N] transposed table, an int32 cumsum along its rows
+// at 0.21 ms, five boolean selections); the residual block + merging + expansion it belongs to took
+// 1 864 us and takes 816 us.
+#include "scan.cuh"
+#include "ssw_common.cuh"
+
+namespace ssw {
+
+struct RbGrid {
+  int batch, D, H, W;
+};
+
+// cell index of a voxel, or -1 when it lies outside the grid
+__device__ __forceinline__ int64_t rb_cell(const RbGrid& g, int4 c) {
+  if ((unsigned)c.x >= (unsigned)g.batch || (unsigned)c.y >= (unsigned)g.D || (unsigned)c.z >= (unsigned)g.H ||
+      (unsigned)c.w >= (unsigned)g.W)
+    return -1;
+  return (((int64_t)c.x * g.D + c.y) * g.H + c.z) * g.W + c.w;
+}
+
+// counts: [0] error bits, [1] longest run of one tap, [2] pairs
+__global__ void k_rb_mark(const int32_t* __restrict__ coords, int64_t n, RbGrid g, uint32_t* __restrict__ bitmap,
+                          int32_t* __restrict__ grid, int32_t* __restrict__ counts) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int64_t cell = rb_cell(g, __ldg(reinterpret_cast<const int4*>(coords) + i));
+  if (cell < 0) {
+    atomicOr(reinterpret_cast<unsigned*>(counts), SSW_DEV_BAD_COORD);
+    return;
+  }
+  const uint32_t bit = 1u << (cell & 31);
+  if (atomicOr(bitmap + (cell >> 5), bit) & bit) atomicOr(reinterpret_cast<unsigned*>(counts), SSW_DEV_DUPLICATE);
+  grid[cell] = (int)i;
+}
+
+constexpr int kRbThreads = 256;
+// Output voxels per block: the ranks of a block's pairs are staged in shared memory, taps x 2 bytes each.
+__host__ __device__ inline int rb_rows(int taps) { return taps <= 27 ? 128 : 32; }
+
+// nbr[i, t] for all taps; per block and off-centre tap the number of existing pairs, per block their sum
+__global__ void __launch_bounds__(kRbThreads) k_rb_neighbors(const int32_t* __restrict__ coords, int64_t n, RbGrid g, int K,
+                                                             const uint32_t* __restrict__ bitmap,
+                                                             const int32_t* __restrict__ grid, int32_t* __restrict__ nbr,
+                                                             int32_t* __restrict__ tap_block, int n_blocks) {
+  extern __shared__ int32_t cnt_s[];  // [taps]
+  __shared__ int4 c_s[128];
+  const int taps = K * K * K, rows = rb_rows(taps), centre = taps / 2, r = K / 2;
+  const int64_t i0 = (int64_t)blockIdx.x * rows;
+  const int live = (int)min((int64_t)rows, n - i0);
+  for (int t = threadIdx.x; t < taps; t += kRbThreads) cnt_s[t] = 0;
+  for (int v = threadIdx.x; v < live; v += kRbThreads) c_s[v] = __ldg(reinterpret_cast<const int4*>(coords) + i0 + v);
+  __syncthreads();
+  for (int idx = threadIdx.x; idx < live * taps; idx += kRbThreads) {
+    const int v = idx / taps, t = idx - v * taps;
+    int4 c = c_s[v];
+    const int tz = t / (K * K), ty = (t - tz * K * K) / K, tx = t - (tz * K + ty) * K;
+    c.y += tz - r;
+    c.z += ty - r;
+    c.w += tx - r;
+    const int64_t cell = rb_cell(g, c);
+    int id = -1;
+    if (cell >= 0 && (__ldg(bitmap + (cell >> 5)) >> (cell & 31)) & 1u) id = __ldg(grid + cell);
+    nbr[i0 * taps + idx] = id;
+    if (id >= 0 && t != centre) atomicAdd(cnt_s + t, 1);
+  }
+  __syncthreads();
+  int sum = 0;
+  for (int t = threadIdx.x; t < taps; t += kRbThreads) {
+    tap_block[(int64_t)t * n_blocks + blockIdx.x] = cnt_s[t];
+    sum += cnt_s[t];
+  }
+  // the block's pairs, for the row lists: kept as one more "tap"
+  sum += __shfl_xor_sync(0xffffffffu, sum, 16);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 8);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 4);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+  __shared__ int ws[kRbThreads / 32];
+  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int s = 0;
+    for (int w = 0; w < kRbThreads / 32; ++w) s += ws[w];
+    tap_block[(int64_t)taps * n_blocks + blockIdx.x] = s;
+  }
+}
+
+// One block per tap (and one for the blocks' sums): exclusive prefix over the blocks, in place; totals.
+__global__ void __launch_bounds__(kScanT) k_rb_scan(int32_t* __restrict__ tap_block, int n_blocks, int taps,
+                                                    int32_t* __restrict__ tap_total, int32_t* __restrict__ counts) {
+  const int t = blockIdx.x;
+  int32_t* p = tap_block + (int64_t)t * n_blocks;
+  long long carry = 0;
+  for (int b0 = 0; b0 < n_blocks; b0 += kScanT) {
+    const int b = b0 + threadIdx.x;
+    const long long v = b < n_blocks ? p[b] : 0;
+    long long tot;
+    const long long ex = block_excl_scan_i64(v, tot) + carry;
+    if (b < n_blocks) p[b] = (int32_t)ex;
+    carry += tot;
+  }
+  if (threadIdx.x == 0) {
+    if (t == taps) {
+      counts[2] = (int32_t)carry;
+    } else {
+      tap_total[t] = (int32_t)carry;
+      if (t != taps / 2) atomicMax(counts + 1, (int32_t)carry);
+    }
+  }
+}
+
+// Blocks [0, n_blocks): the pairs of one block of output voxels.  Blocks beyond: the padding of one tap's run.
+__global__ void __launch_bounds__(kRbThreads) k_rb_pairs(const int32_t* __restrict__ nbr, int64_t n, int taps,
+                                                         const int32_t* __restrict__ tap_block,
+                                                         const int32_t* __restrict__ tap_total, int n_blocks, int64_t seg,
+                                                         int32_t* __restrict__ pair_in, int32_t* __restrict__ row_start,
+                                                         int32_t* __restrict__ row_slots) {
+  extern __shared__ uint16_t rank_s[];  // [rows][taps]: rank of the pair inside its block and tap
+  const int centre = taps / 2;
+  if ((int)blockIdx.x >= n_blocks) {
+    const int tt = blockIdx.x - n_blocks, t = tt < centre ? tt : tt + 1;
+    for (int64_t s = tap_total[t] + threadIdx.x; s < seg; s += kRbThreads) pair_in[tt * seg + s] = -1;
+    return;
+  }
+  const int rows = rb_rows(taps);
+  const int64_t i0 = (int64_t)blockIdx.x * rows;
+  const int live = (int)min((int64_t)rows, n - i0);
+  const int32_t* nb = nbr + i0 * taps;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int t = warp; t < taps; t += kRbThreads / 32) {
+    if (t == centre) continue;
+    const int tt = t < centre ? t : t - 1;
+    int run = 0;
+    const int64_t base = tt * seg + tap_block[(int64_t)t * n_blocks + blockIdx.x];
+    for (int v0 = 0; v0 < rows; v0 += 32) {
+      const int v = v0 + lane;
+      const int id = v < live ? __ldg(nb + v * taps + t) : -1;
+      const unsigned m = __ballot_sync(0xffffffffu, id >= 0);
+      if (id >= 0) {
+        const int rank = run + __popc(m & ((1u << lane) - 1u));
+        pair_in[base + rank] = id;
+        rank_s[v * taps + t] = (uint16_t)rank;
+      }
+      run += __popc(m);
+    }
+  }
+  // row lists: prefix of the rows' pair counts (the first `rows` threads, whole warps)
+  __shared__ int wsum[4];
+  int c = 0;
+  const int v = threadIdx.x;
+  if (v < live)
+    for (int t = 0; t < taps; ++t) c += t != centre && __ldg(nb + v * taps + t) >= 0;
+  int inc = warp_incl_scan(c);
+  if (lane == 31 && warp < 4) wsum[warp] = inc;
+  __syncthreads();
+  if (v < live) {
+    int p = tap_block[(int64_t)taps * n_blocks + blockIdx.x] + inc - c;
+    for (int w = 0; w < warp; ++w) p += wsum[w];
+    row_start[i0 + v] = p;
+    if (i0 + v == n - 1) row_start[n] = p + c;
+    for (int t = 0; t < taps; ++t) {
+      if (t == centre || __ldg(nb + v * taps + t) < 0) continue;
+      const int tt = t < centre ? t : t - 1;
+      row_slots[p++] = (int32_t)(tt * seg) + tap_block[(int64_t)t * n_blocks + blockIdx.x] + rank_s[v * taps + t];
+    }
+  }
+}
+
+// ---- strided convolution (kernel = stride) -------------------------------------------------------
+struct RbStrided {
+  int batch, k;
+  int od[3];
+};
+// output cell of a voxel (-1: none) and the tap through which it feeds it; false: negative coordinate or
+// batch index outside the scene
+__device__ __forceinline__ bool rb_parent(const RbStrided& s, int4 c, int64_t& cell, int& tap) {
+  const int k = s.k;
+  cell = -1;
+  tap = 0;
+  if ((unsigned)c.x >= (unsigned)s.batch || (c.y | c.z | c.w) < 0) return false;
+  const int z = c.y / k, y = c.z / k, x = c.w / k;
+  tap = ((c.y - z * k) * k + (c.z - y * k)) * k + (c.w - x * k);
+  if (z < s.od[0] && y < s.od[1] && x < s.od[2]) cell = (((int64_t)c.x * s.od[0] + z) * s.od[1] + y) * s.od[2] + x;
+  return true;
+}
+// counts: [0] error bits, [1] occupied output cells
+__global__ void k_rb_strided_mark(const int32_t* __restrict__ coords, int64_t n, RbStrided s, uint32_t* __restrict__ bitmap,
+                                  int32_t* __restrict__ counts) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  int64_t cell;
+  int tap;
+  if (!rb_parent(s, __ldg(reinterpret_cast<const int4*>(coords) + i), cell, tap))
+    atomicOr(reinterpret_cast<unsigned*>(counts), SSW_DEV_BAD_COORD);
+  else if (cell >= 0)
+    atomicOr(bitmap + (cell >> 5), 1u << (cell & 31));
+}
+__global__ void k_rb_strided_total(const long long* __restrict__ ws, int32_t* __restrict__ counts) { counts[1] = (int32_t)ws[1]; }
+__global__ void k_rb_strided_fill(const int32_t* __restrict__ coords, int64_t n, RbStrided s, const uint32_t* __restrict__ bitmap,
+                                  const int32_t* __restrict__ prefix, int32_t* __restrict__ parent, int32_t* __restrict__ tap_out,
+                                  int32_t* __restrict__ nbr, int32_t* __restrict__ out_coords) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int4 c = __ldg(reinterpret_cast<const int4*>(coords) + i);
+  int64_t cell;
+  int tap;
+  const bool ok = rb_parent(s, c, cell, tap) && cell >= 0;
+  int rank = -1;
+  if (ok) {
+    rank = __ldg(prefix + (cell >> 5)) + __popc(__ldg(bitmap + (cell >> 5)) & ((1u << (cell & 31)) - 1u));
+    nbr[(int64_t)rank * s.k * s.k * s.k + tap] = (int)i;
+    // every voxel of a cell writes the same row
+    reinterpret_cast<int4*>(out_coords)[rank] = make_int4(c.x, c.y / s.k, c.z / s.k, c.w / s.k);
+  }
+  parent[i] = rank;
+  tap_out[i] = tap;
+}
+
+}  // namespace ssw
+
+using namespace ssw;
+
+static inline int64_t align4_rb(int64_t x) { return (x + 3) & ~int64_t(3); }
+static inline int rb_blocks(int64_t n, int taps) { return (int)ceil_div64(n, rb_rows(taps)); }
+
+// int32 words: [counts 4][bitmap][per-tap totals][(taps + 1) x blocks prefixes][id table, cells]
+extern "C" int64_t ssw_subm_rulebook_workspace_ints(int64_t n, int32_t batch, const int32_t dims[3], int32_t ksize) {
+  if (n < 0 || batch <= 0 || !dims || ksize < 1) return -1;
+  const int64_t cells = (int64_t)batch * dims[0] * dims[1] * dims[2];
+  const int taps = ksize * ksize * ksize;
+  return 4 + align4_rb(ceil_div64(cells, 32)) + align4_rb(taps) + align4_rb((int64_t)(taps + 1) * rb_blocks(n, taps)) + cells;
+}
+
+struct SubmWs {
+  int32_t *counts, *tap_total, *tap_block, *grid;
+  uint32_t* bitmap;
+  int64_t cells;
+};
+static SubmWs subm_ws(int32_t* ws, int64_t n, int32_t batch, const int32_t dims[3], int taps) {
+  SubmWs s;
+  s.cells = (int64_t)batch * dims[0] * dims[1] * dims[2];
+  s.counts = ws;
+  s.bitmap = reinterpret_cast<uint32_t*>(ws + 4);
+  s.tap_total = ws + 4 + align4_rb(ceil_div64(s.cells, 32));
+  s.tap_block = s.tap_total + align4_rb(taps);
+  s.grid = s.tap_block + align4_rb((int64_t)(taps + 1) * rb_blocks(n, taps));
+  return s;
+}
+static int subm_check(int64_t n, int32_t batch, const int32_t dims[3], int32_t ksize) {
+  if (n <= 0 || batch <= 0 || !dims || ksize < 1 || ksize > 7 || !(ksize & 1)) return SSW_E_INVALID;
+  for (int i = 0; i < 3; ++i)
+    if (dims[i] <= 0) return SSW_E_INVALID;
+  if ((int64_t)batch * dims[0] * dims[1] * dims[2] >= ((int64_t)1 << 31) || n * ksize * ksize * ksize >= ((int64_t)1 << 31)) return SSW_E_RANGE;
+  return SSW_OK;
+}
+
+extern "C" int ssw_subm_rulebook_count(const int32_t* coords, int64_t n, int32_t batch, const int32_t dims[3], int32_t ksize,
+                                       int32_t* nbr, int32_t* workspace, void* stream_) {
+  const int rc = subm_check(n, batch, dims, ksize);
+  if (rc) return rc;
+  if (!coords || !nbr || !workspace || (reinterpret_cast<uintptr_t>(coords) & 15)) return SSW_E_INVALID;
+  cudaStream_t st = (cudaStream_t)stream_;
+  const int taps = ksize * ksize * ksize, blocks = rb_blocks(n, taps);
+  const SubmWs w = subm_ws(workspace, n, batch, dims, taps);
+  const RbGrid g{batch, dims[0], dims[1], dims[2]};
+  SSW_CUDA_TRY(cudaMemsetAsync(workspace, 0, sizeof(int32_t) * (size_t)(4 + ceil_div64(w.cells, 32)), st));
+  k_rb_mark<<<(unsigned)ceil_div64(n, 256), 256, 0, st>>>(coords, n, g, w.bitmap, w.grid, w.counts);
+  SSW_LAUNCH_CHECK("k_rb_mark");
+  k_rb_neighbors<<<blocks, kRbThreads, taps * sizeof(int32_t), st>>>(coords, n, g, ksize, w.bitmap, w.grid, nbr, w.tap_block, blocks);
+  SSW_LAUNCH_CHECK("k_rb_neighbors");
+  k_rb_scan<<<taps + 1, kScanT, 0, st>>>(w.tap_block, blocks, taps, w.tap_total, w.counts);
+  SSW_LAUNCH_CHECK("k_rb_scan");
+  return SSW_OK;
+}
+
+extern "C" int ssw_subm_rulebook_pairs(const int32_t* nbr, int64_t n, int32_t batch, const int32_t dims[3], int32_t ksize,
+                                       int64_t seg, const int32_t* workspace, int32_t* pair_in, int32_t* row_start,
+                                       int32_t* row_slots, void* stream_) {
+  const int rc = subm_check(n, batch, dims, ksize);
+  if (rc) return rc;
+  if (!nbr || !workspace || !pair_in || !row_start || !row_slots || seg <= 0 || ksize < 2) return SSW_E_INVALID;
+  cudaStream_t st = (cudaStream_t)stream_;
+  const int taps = ksize * ksize * ksize, blocks = rb_blocks(n, taps);
+  if (seg * (taps - 1) >= ((int64_t)1 << 31)) return SSW_E_RANGE;
+  const SubmWs w = subm_ws(const_cast<int32_t*>(workspace), n, batch, dims, taps);
+  k_rb_pairs<<<blocks + taps - 1, kRbThreads, (size_t)rb_rows(taps) * taps * sizeof(uint16_t), st>>>(
+      nbr, n, taps, w.tap_block, w.tap_total, blocks, seg, pair_in, row_start, row_slots);
+  SSW_LAUNCH_CHECK("k_rb_pairs");
+  return SSW_OK;
+}
+
+// int32 words: [counts 4][scan workspace][bitmap][prefix per bitmap word]
+extern "C" int64_t ssw_strided_rulebook_workspace_ints(int32_t batch, const int32_t out_dims[3]) {
+  if (batch <= 0 || !out_dims) return -1;
+  const int64_t words = ceil_div64((int64_t)batch * out_dims[0] * out_dims[1] * out_dims[2], 32);
+  return 4 + 2 * scan_workspace_i64(words) + 2 * align4_rb(words);
+}
+static int strided_check(int64_t n, int32_t batch, const int32_t od[3], int32_t k) {
+  if (n <= 0 || batch <= 0 || !od || k < 1 || k > 1024 || od[0] <= 0 || od[1] <= 0 || od[2] <= 0) return SSW_E_INVALID;
+  if ((int64_t)batch * od[0] * od[1] * od[2] >= ((int64_t)1 << 31) - 1 || n >= ((int64_t)1 << 31)) return SSW_E_RANGE;
+  return SSW_OK;
+}
+
+extern "C" int ssw_strided_rulebook_count(const int32_t* coords, int64_t n, int32_t batch, const int32_t out_dims[3], int32_t ksize,
+                                          int32_t* workspace, void* stream_) {
+  const int rc = strided_check(n, batch, out_dims, ksize);
+  if (rc) return rc;
+  if (!coords || !workspace || ((reinterpret_cast<uintptr_t>(coords) | reinterpret_cast<uintptr_t>(workspace)) & 15)) return SSW_E_INVALID;
+  cudaStream_t st = (cudaStream_t)stream_;
+  const int64_t words = ceil_div64((int64_t)batch * out_dims[0] * out_dims[1] * out_dims[2], 32);
+  long long* ws = reinterpret_cast<long long*>(workspace + 4);
+  uint32_t* bitmap = reinterpret_cast<uint32_t*>(ws + scan_workspace_i64(words));
+  int32_t* prefix = reinterpret_cast<int32_t*>(bitmap + align4_rb(words));
+  const RbStrided s{batch, ksize, {out_dims[0], out_dims[1], out_dims[2]}};
+  SSW_CUDA_TRY(cudaMemsetAsync(workspace, 0, reinterpret_cast<char*>(bitmap + words) - reinterpret_cast<char*>(workspace), st));
+  k_rb_strided_mark<<<(unsigned)ceil_div64(n, 256), 256, 0, st>>>(coords, n, s, bitmap, workspace);
+  SSW_LAUNCH_CHECK("k_rb_strided_mark");
+  auto f = [bitmap] __device__(int64_t w) -> int { return __popc(bitmap[w]); };
+  auto g = [prefix] __device__(int64_t w, int, long long ex) { prefix[w] = (int32_t)ex; };
+  const int rs = device_scan(f, g, words, ws, st);
+  if (rs) return rs;
+  k_rb_strided_total<<<1, 1, 0, st>>>(ws, workspace);
+  SSW_LAUNCH_CHECK("k_rb_strided_total");
+  return SSW_OK;
+}
+
+extern "C" int ssw_strided_rulebook_fill(const int32_t* coords, int64_t n, int32_t batch, const int32_t out_dims[3], int32_t ksize,
+                                         const int32_t* workspace, int64_t m, int32_t* parent, int32_t* tap, int32_t* nbr,
+                                         int32_t* out_coords, void* stream_) {
+  const int rc = strided_check(n, batch, out_dims, ksize);
+  if (rc) return rc;
+  if (!coords || !workspace || m < 0 || !parent || !tap || (m > 0 && (!nbr || !out_coords || (reinterpret_cast<uintptr_t>(out_coords) & 15))))
+    return SSW_E_INVALID;
+  cudaStream_t st = (cudaStream_t)stream_;
+  const int64_t words = ceil_div64((int64_t)batch * out_dims[0] * out_dims[1] * out_dims[2], 32);
+  const long long* ws = reinterpret_cast<const long long*>(workspace + 4);
+  const uint32_t* bitmap = reinterpret_cast<const uint32_t*>(ws + scan_workspace_i64(words));
+  const int32_t* prefix = reinterpret_cast<const int32_t*>(bitmap + align4_rb(words));
+  const RbStrided s{batch, ksize, {out_dims[0], out_dims[1], out_dims[2]}};
+  if (m > 0) SSW_CUDA_TRY(cudaMemsetAsync(nbr, 0xff, sizeof(int32_t) * (size_t)m * ksize * ksize * ksize, st));
+  k_rb_strided_fill<<<(unsigned)ceil_div64(n, 256), 256, 0, st>>>(coords, n, s, bitmap, prefix, parent, tap, nbr, out_coords);
+  SSW_LAUNCH_CHECK("k_rb_strided_fill");
+  return SSW_OK;
+}

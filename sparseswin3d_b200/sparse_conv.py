@@ -34,7 +34,7 @@ from typing import Optional, Sequence
 import torch
 import torch.nn as nn
 
-from . import _lib, ops
+from . import _lib
 from ._lib import check, dtype_code, lib, ptr, stream_ptr
 from .stage import SparseVoxels
 
@@ -69,8 +69,7 @@ def _dims3(d: Sequence[int]):
 
 def voxel_grid(indices: torch.Tensor, batch_size: int, spatial_shape: Sequence[int], strict: bool = True) -> torch.Tensor:
     """Dense cell -> voxel id table (int32 [B, D, H, W], -1 = empty)."""
-    if not indices.is_cuda or indices.dtype != I32 or indices.dim() != 2 or indices.shape[1] != 4 or not indices.is_contiguous():
-        raise _lib.SswError("indices must be a contiguous CUDA int32 [N, 4] tensor (b, z, y, x)")
+    _coords_i32(indices)
     D, H, W = (int(v) for v in spatial_shape)
     grid = torch.empty((int(batch_size), D, H, W), dtype=I32, device=indices.device)
     err = torch.zeros(1, dtype=I32, device=indices.device)
@@ -85,40 +84,42 @@ def voxel_grid(indices: torch.Tensor, batch_size: int, spatial_shape: Sequence[i
     return grid
 
 
+def _coords_i32(indices: torch.Tensor):
+    if not indices.is_cuda or indices.dtype != I32 or indices.dim() != 2 or indices.shape[1] != 4 or not indices.is_contiguous():
+        raise _lib.SswError("indices must be a contiguous CUDA int32 [N, 4] tensor (b, z, y, x)")
+
+
 def subm_rulebook(x, ksize: int) -> Rulebook:
+    """One host synchronisation: the error bits and the sizes of the pair arrays come back together."""
     if ksize % 2 != 1:
         raise _lib.SswError("a submanifold convolution needs an odd kernel size")
-    grid = voxel_grid(x.indices, x.batch_size, x.spatial_shape)
-    n = x.indices.shape[0]
-    nbr = torch.empty((n, ksize ** 3), dtype=I32, device=x.indices.device)
-    check(lib.ssw_subm_neighbors(ptr(x.indices), n, int(x.batch_size), _dims3(x.spatial_shape), ptr(grid), int(ksize), ptr(nbr),
-                                 stream_ptr(x.indices.device)), "ssw_subm_neighbors")
-    rb = Rulebook("subm", ksize, x.indices, list(x.spatial_shape), x.indices, list(x.spatial_shape), nbr)
+    idx, k, k3 = x.indices, int(ksize), int(ksize) ** 3
+    _coords_i32(idx)
+    n, dev, batch, dims = idx.shape[0], idx.device, int(x.batch_size), _dims3(x.spatial_shape)
+    nbr = torch.empty((n, k3), dtype=I32, device=dev)
+    rb = Rulebook("subm", k, idx, list(x.spatial_shape), idx, list(x.spatial_shape), nbr)
+    if n == 0:
+        return rb
+    ws = torch.empty(int(lib.ssw_subm_rulebook_workspace_ints(n, batch, dims, k)), dtype=I32, device=dev)
+    st = stream_ptr(dev)
+    check(lib.ssw_subm_rulebook_count(ptr(idx), n, batch, dims, k, ptr(nbr), ptr(ws), st), "ssw_subm_rulebook_count")
+    err, longest, pairs = ws[:3].tolist()
+    if err & _lib.DEV_BAD_COORD:
+        raise _lib.SswError("a voxel lies outside the grid")
+    if err & _lib.DEV_DUPLICATE:
+        raise _lib.SswError("two voxels share a cell: coordinates must be unique")
     # Pair form.  On a surface-sparse scene a voxel has a few of its k^3 neighbours, and the gathered
     # operand [N, k^3 Cin] would be mostly zeros.  Group the existing (input, output) pairs by tap
     # instead, pad every off-centre tap's run to the longest one (so that one batched GEMM serves
-    # them all) and let the output side pick its pairs up (`ssw_gather_reduce`).  One read-back.
-    k3 = ksize ** 3
-    if n > 0 and k3 > 1:
-        centre = k3 // 2
-        off = torch.cat([nbr[:, :centre], nbr[:, centre + 1:]], 1).t().contiguous()   # [k^3 - 1, N], tap-major
-        has = off >= 0
-        rank = torch.cumsum(has, 1, dtype=torch.int32) - 1                   # position inside its tap's run
-        seg = int(rank[:, -1].max()) + 1
-        seg = (seg + 7) // 8 * 8
-        if 0 < (k3 - 1) * seg <= PAIR_FORM_MAX_FILL * k3 * n:
-            taps = torch.arange(k3 - 1, dtype=torch.int32, device=nbr.device).unsqueeze(1)
-            slot = taps * seg + rank
-            pair_in = torch.full(((k3 - 1) * seg,), -1, dtype=I32, device=nbr.device)
-            pair_in[slot[has].long()] = off[has]
-            rb.pair_in = pair_in.view(-1, 1)
-            # the same pairs seen from the output side: per output row the list of its slots, in tap order
-            has_rt = has.t().contiguous()                                     # [N, k^3 - 1]
-            rb.row_slots = slot.t()[has_rt].to(I32).contiguous()
-            row_start = torch.zeros(n + 1, dtype=I32, device=nbr.device)
-            row_start[1:] = torch.cumsum(has_rt.sum(1, dtype=torch.int32), 0, dtype=torch.int32)
-            rb.row_start = row_start
-            rb.seg = seg
+    # them all) and let the output side pick its pairs up (`ssw_gather_reduce`).
+    seg = (longest + 7) // 8 * 8
+    if k3 > 1 and 0 < (k3 - 1) * seg <= PAIR_FORM_MAX_FILL * k3 * n:
+        rb.seg = seg
+        rb.pair_in = torch.empty(((k3 - 1) * seg, 1), dtype=I32, device=dev)
+        rb.row_start = torch.empty(n + 1, dtype=I32, device=dev)
+        rb.row_slots = torch.empty(pairs, dtype=I32, device=dev)
+        check(lib.ssw_subm_rulebook_pairs(ptr(nbr), n, batch, dims, k, seg, ptr(ws), ptr(rb.pair_in), ptr(rb.row_start),
+                                          ptr(rb.row_slots), st), "ssw_subm_rulebook_pairs")
     return rb
 
 
@@ -130,32 +131,32 @@ def strided_rulebook(x, ksize: int) -> Rulebook:
     n = idx.shape[0]
     dims = [int(v) for v in x.spatial_shape]
     od = [(d - k) // k + 1 if d >= k else 0 for d in dims]
-    n_cells = int(x.batch_size) * od[0] * od[1] * od[2]
+    batch = int(x.batch_size)
+    n_cells = batch * od[0] * od[1] * od[2]
     if n_cells >= 2 ** 31 - 1:
         raise _lib.SswError("the output grid leaves the int32 domain")
-    b, z, y, xx = idx[:, 0], idx[:, 1], idx[:, 2], idx[:, 3]
-    valid = (z < od[0] * k) & (y < od[1] * k) & (xx < od[2] * k)
-    cell = ((b * od[0] + z // k) * od[1] + y // k) * od[2] + xx // k
-    tap = ((z % k) * k + y % k) * k + xx % k
     if n == 0 or n_cells == 0:
         out_idx = torch.zeros((0, 4), dtype=I32, device=dev)
+        z, y, xx = idx[:, 1], idx[:, 2], idx[:, 3]
+        tap = ((z % k) * k + y % k) * k + xx % k
         return Rulebook("strided", k, idx, dims, out_idx, od, torch.zeros((0, k ** 3), dtype=I32, device=dev),
                         torch.full((n,), -1, dtype=I32, device=dev), tap.to(I32))
-    # rank of every voxel's output cell among the occupied cells (ascending cell id = (b, z, y, x) order);
-    # voxels without an output cell go to one extra bin behind all cells
-    keyed = torch.where(valid, cell, torch.full_like(cell, n_cells)).to(I32).contiguous()
-    rank, count = ops.return_inverse(keyed, n_cells + 1)
-    n_invalid = int((~valid).sum())
-    m = count - (1 if n_invalid else 0)
-    parent = torch.where(valid, rank, torch.full_like(rank, -1))
-    vi = valid.nonzero().squeeze(1)
-    cell_of = torch.empty(m, dtype=torch.int64, device=dev)
-    cell_of[parent[vi].long()] = cell[vi].long()
-    out_idx = torch.stack([cell_of // (od[0] * od[1] * od[2]), (cell_of // (od[1] * od[2])) % od[0], (cell_of // od[2]) % od[1],
-                           cell_of % od[2]], 1).to(I32).contiguous()
-    nbr = torch.full((m, k ** 3), -1, dtype=I32, device=dev)
-    nbr[parent[vi].long(), tap[vi].long()] = vi.to(I32)
-    return Rulebook("strided", k, idx, dims, out_idx, od, nbr, parent.to(I32).contiguous(), tap.to(I32).contiguous())
+    if not idx.is_cuda:
+        raise _lib.SswError("indices must be a CUDA tensor (there is no CPU path)")
+    src = idx.to(I32).contiguous()
+    odc, st = _dims3(od), stream_ptr(dev)
+    ws = torch.empty(int(lib.ssw_strided_rulebook_workspace_ints(batch, odc)), dtype=I32, device=dev)
+    check(lib.ssw_strided_rulebook_count(ptr(src), n, batch, odc, k, ptr(ws), st), "ssw_strided_rulebook_count")
+    err, m = ws[:2].tolist()
+    if err:
+        raise _lib.SswError("a voxel lies outside the grid")
+    parent = torch.empty(n, dtype=I32, device=dev)
+    tap = torch.empty(n, dtype=I32, device=dev)
+    nbr = torch.empty((m, k ** 3), dtype=I32, device=dev)
+    out_idx = torch.empty((m, 4), dtype=I32, device=dev)
+    check(lib.ssw_strided_rulebook_fill(ptr(src), n, batch, odc, k, ptr(ws), m, ptr(parent), ptr(tap), ptr(nbr), ptr(out_idx), st),
+          "ssw_strided_rulebook_fill")
+    return Rulebook("strided", k, idx, dims, out_idx, od, nbr, parent, tap)
 
 
 def gather_cols(x: torch.Tensor, nbr: torch.Tensor) -> torch.Tensor:

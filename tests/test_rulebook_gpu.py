@@ -1,0 +1,80 @@
+"""Rulebook kernels at the edges of their blocks (128 output voxels for 3^3 taps, 32 for larger kernels),
+against a dictionary of the coordinates and against the same arrays as torch index arithmetic: every
+entry is an integer and has to be equal."""
+import pytest
+import torch
+
+from tests.cases import make_case
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ksize,n,dims", [(1, 40, (5, 6, 7)), (3, 1, (4, 4, 4)), (3, 127, (9, 6, 8)), (3, 128, (9, 6, 8)),
+                                          (3, 129, (9, 6, 8)), (3, 5000, (40, 41, 37)), (5, 31, (7, 7, 7)), (5, 33, (7, 7, 7)),
+                                          (5, 700, (20, 9, 31)), (7, 65, (6, 6, 6)), (7, 900, (33, 20, 18))])
+@pytest.mark.parametrize("batch", [1, 3])
+def test_submanifold_rulebook(ksize, n, dims, batch, monkeypatch):
+    from sparseswin3d_b200 import sparse_conv, stage
+
+    monkeypatch.setattr(sparse_conv, "PAIR_FORM_MAX_FILL", 2.0)  # always the pair form
+    dev = torch.device("cuda:0")
+    coords = make_case(n_vox=n, dims=dims, batch=batch, seed=n + ksize)["coords"]
+    N, k3, r = coords.shape[0], ksize ** 3, ksize // 2
+    rb = sparse_conv.subm_rulebook(stage.SparseVoxels(torch.zeros(N, 8, device=dev), coords.to(dev), dims, batch), ksize)
+    table = torch.full((batch, *(d + 2 * r for d in dims)), -1, dtype=torch.int32)
+    b, z, y, x = coords.long().unbind(1)
+    table[b, z + r, y + r, x + r] = torch.arange(N, dtype=torch.int32)
+    want = torch.stack([table[b, z + dz, y + dy, x + dx] for dz in range(ksize) for dy in range(ksize) for dx in range(ksize)], 1)
+    assert torch.equal(rb.nbr.cpu(), want)
+    off = torch.cat([want[:, :k3 // 2], want[:, k3 // 2 + 1:]], 1).t().contiguous()
+    has = off >= 0
+    if not bool(has.any()):
+        assert rb.seg == 0
+        return
+    rank = torch.cumsum(has, 1) - 1
+    seg = (int(rank[:, -1].max()) + 8) // 8 * 8
+    assert rb.seg == seg
+    slot = torch.arange(k3 - 1).unsqueeze(1) * seg + rank
+    pair_in = torch.full(((k3 - 1) * seg,), -1, dtype=torch.int32)
+    pair_in[slot[has]] = off[has]
+    assert torch.equal(rb.pair_in.cpu().view(-1), pair_in)
+    has_rt = has.t().contiguous()
+    assert torch.equal(rb.row_slots.cpu(), slot.t()[has_rt].to(torch.int32))
+    start = torch.cat([torch.zeros(1, dtype=torch.long), torch.cumsum(has_rt.sum(1), 0)])
+    assert torch.equal(rb.row_start.cpu().long(), start)
+
+
+@pytest.mark.parametrize("ksize,n,dims", [(1, 50, (5, 6, 7)), (2, 1, (2, 2, 2)), (2, 300, (9, 12, 7)), (2, 4000, (65, 64, 33)), (3, 500, (20, 9, 31))])
+@pytest.mark.parametrize("batch", [1, 2])
+def test_strided_rulebook(ksize, n, dims, batch):
+    from sparseswin3d_b200 import sparse_conv, stage
+
+    dev = torch.device("cuda:0")
+    coords = make_case(n_vox=min(n, dims[0] * dims[1] * dims[2]), dims=dims, batch=batch, seed=n)["coords"]
+    N, k = coords.shape[0], ksize
+    rb = sparse_conv.strided_rulebook(stage.SparseVoxels(torch.zeros(N, 8, device=dev), coords.to(dev), dims, batch), k)
+    od = [(d - k) // k + 1 for d in dims]
+    c = coords.long()
+    valid = (c[:, 1] < od[0] * k) & (c[:, 2] < od[1] * k) & (c[:, 3] < od[2] * k)
+    tap = ((c[:, 1] % k) * k + c[:, 2] % k) * k + c[:, 3] % k
+    cells, inv = torch.unique(torch.cat([c[valid][:, :1], c[valid][:, 1:] // k], 1), dim=0, return_inverse=True)
+    parent = torch.full((N,), -1, dtype=torch.long)
+    parent[valid] = inv
+    nbr = torch.full((cells.shape[0], k ** 3), -1, dtype=torch.long)
+    nbr[inv, tap[valid]] = torch.arange(N)[valid]
+    assert rb.out_shape == od and torch.equal(rb.out_indices.cpu().long(), cells)
+    assert torch.equal(rb.parent.cpu().long(), parent) and torch.equal(rb.tap.cpu().long(), tap)
+    assert torch.equal(rb.nbr.cpu().long(), nbr)
+
+
+def test_rulebooks_reject_bad_coordinates():
+    from sparseswin3d_b200 import _lib, sparse_conv, stage
+
+    dev = torch.device("cuda:0")
+    for rows, match in (([[0, 1, 1, 1], [0, 1, 1, 1]], "share a cell"), ([[0, 1, 1, 1], [0, 1, 1, 8]], "outside")):
+        x = stage.SparseVoxels(torch.zeros(2, 8, device=dev), torch.tensor(rows, dtype=torch.int32, device=dev), (8, 8, 8), 1)
+        with pytest.raises(_lib.SswError, match=match):
+            sparse_conv.subm_rulebook(x, 3)
+    x = stage.SparseVoxels(torch.zeros(1, 8, device=dev), torch.tensor([[1, 0, 0, 0]], dtype=torch.int32, device=dev), (8, 8, 8), 1)
+    with pytest.raises(_lib.SswError):
+        sparse_conv.strided_rulebook(x, 2)
