@@ -244,6 +244,36 @@ int ssw_peer_buffer_destroy(void* ptr);
 int ssw_add_layernorm(const void* a, const void* b, const float* gamma, const float* beta, float eps,
                       int dtype, int64_t n_rows, int32_t channels, void* sum_out, void* norm_out,
                       void* stream);
+/* The same with gamma and beta in `param_dtype` (a bf16 module's parameters are read as they are). */
+int ssw_add_layernorm_p(const void* a, const void* b, const void* gamma, const void* beta, int param_dtype, float eps,
+                        int dtype, int64_t n_rows, int32_t channels, void* sum_out, void* norm_out, void* stream);
+
+/* The LayerNorms on either side of a kernel = stride convolution (patch merging and expansion,
+ * swin3d_base.py:950-1004), on the rows as the convolution moves them.
+ * _scatter: out [n_out * taps, channels] = 0, then row parent[i] * taps + tap[i] = LayerNorm(x[i]) for every i whose
+ * parent lies in [0, n_out) and whose slot `owner` (= the strided rulebook's nbr [n_out, taps]) names i: the operand
+ * of the merging GEMM.
+ * _slices: out[i] = LayerNorm(row parent[i] * taps + tap[i] of x [n_src * taps, channels]), a row of zeros being
+ * normalised where the parent is not in [0, n_src). */
+int ssw_layernorm_scatter(const void* x, const void* gamma, const void* beta, int param_dtype, float eps, int dtype,
+                          int64_t n_rows, int32_t channels, const int32_t* parent, const int32_t* tap,
+                          const int32_t* owner, int32_t taps, int64_t n_out, void* out, void* stream);
+int ssw_layernorm_slices(const void* x, const void* gamma, const void* beta, int param_dtype, float eps, int dtype,
+                         int64_t n_src, int32_t channels, const int32_t* parent, const int32_t* tap, int32_t taps,
+                         int64_t n_out, void* out, void* stream);
+
+/* Backward of ssw_add_layernorm: x is the normalised sum, dy the gradient of the norm's output, dsum (may be
+ * NULL) the gradient that reaches the sum past the norm: dx = dLayerNorm(dy) + dsum.  dgamma, dbeta in
+ * param_dtype.  n_rows > 0; workspace as sized by the first call. */
+int64_t ssw_layernorm_bwd_workspace_floats(int64_t n_rows, int32_t channels);
+int ssw_layernorm_bwd(const void* x, const void* dy, const void* dsum, const void* gamma, int param_dtype, float eps, int dtype,
+                      int64_t n_rows, int32_t channels, void* dx, void* dgamma, void* dbeta, float* workspace, void* stream);
+
+/* out[c] = sum over the rows of x [n_rows, channels], fp32 accumulation in a fixed order (the bias gradient
+ * of a Linear layer).  n_rows > 0, rows as above. */
+int64_t ssw_col_sum_workspace_floats(int64_t n_rows, int32_t channels);
+int ssw_col_sum(const void* x, int dtype, int64_t n_rows, int32_t channels, void* out, int out_dtype, float* workspace,
+                void* stream);
 
 /* Sparse 3-D convolutions of the layers around the attention stages (upstream takes them from the
  * spconv library: SubMConv3d swin3d_base.py:915-923, 1039-1059; SparseConv3d :932-935, 965-970;

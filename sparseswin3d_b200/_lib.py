@@ -74,6 +74,13 @@ def _load() -> C.CDLL:
         "ssw_gather_reduce": (C.c_int, [vp, vp, C.c_int, i64, vp, vp, i64, i64, i32, vp, vp]),
         "ssw_gather_slices": (C.c_int, [vp, C.c_int, i64, i32, i32, i64, vp, vp, vp, vp]),
         "ssw_add_layernorm": (C.c_int, [vp, vp, vp, vp, f32, C.c_int, i64, i32, vp, vp, vp]),
+        "ssw_add_layernorm_p": (C.c_int, [vp, vp, vp, vp, C.c_int, f32, C.c_int, i64, i32, vp, vp, vp]),
+        "ssw_layernorm_scatter": (C.c_int, [vp, vp, vp, C.c_int, f32, C.c_int, i64, i32, vp, vp, vp, i32, i64, vp, vp]),
+        "ssw_layernorm_slices": (C.c_int, [vp, vp, vp, C.c_int, f32, C.c_int, i64, i32, vp, vp, i32, i64, vp, vp]),
+        "ssw_layernorm_bwd_workspace_floats": (i64, [i64, i32]),
+        "ssw_layernorm_bwd": (C.c_int, [vp, vp, vp, vp, C.c_int, f32, C.c_int, i64, i32, vp, vp, vp, vp, vp]),
+        "ssw_col_sum_workspace_floats": (i64, [i64, i32]),
+        "ssw_col_sum": (C.c_int, [vp, C.c_int, i64, i32, vp, C.c_int, vp, vp]),
         "ssw_enable_peer_access": (C.c_int, [i32]),
         "ssw_peer_buffer_create": (C.c_int, [i64, P(vp), C.c_char_p]),
         "ssw_peer_buffer_open": (C.c_int, [C.c_char_p, P(vp)]),

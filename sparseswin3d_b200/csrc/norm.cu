@@ -7,10 +7,22 @@
 // does both in one pass over the rows: sum = a (+ b), norm = LayerNorm(sum) * gamma + beta, either
 // output optional.  HBM bound: each row is read once per input and written once per output.
 //
-// A row of C elements is handled by a group of 8, 16 or 32 lanes, 16 bytes per lane and step, values
+// A row of C elements is handled by a group of 4 to 32 lanes, 16 bytes per lane and step, values
 // kept in registers between the statistics and the normalisation (C * elt <= 32 lanes * 16 B * 4
 // steps).  Statistics in fp32, two passes over the registers (mean, then the centred second
 // moment), biased variance and eps as torch.nn.LayerNorm has them.
+//
+// The same row loop with an index in front serves patch merging and expansion (swin3d_base.py:950-1004): the
+// norm that precedes the strided convolution writes straight into the GEMM operand, the one that follows the
+// inverse convolution reads the GEMM's result by (parent, tap).  150 000 x 48 channels of bf16: merging 383 us
+// for the pair as torch LayerNorms beside 20 us of gathers, 45 + 13 us with the norm done once per operand
+// slot (three in four are empty), 14 us and a
+// 15 us clear + 13 us when it is scattered from the voxel side.  The backward
+// (ssw_layernorm_bwd) recomputes the statistics from the saved row instead of storing them, adds the
+// gradient that reaches the sum past the norm, and keeps the parameter gradients of a lane's channels
+// in registers over all its rows.
+#include <initializer_list>
+
 #include "ssw_common.cuh"
 
 namespace ssw {
@@ -82,121 +94,417 @@ struct Vec16<__half> {
   }
 };
 
+// Affine parameters and their gradients come in the module's own type (no conversion pass per call).
+enum ParamType { kParamF32 = SSW_F32, kParamBF16 = SSW_BF16, kParamF16 = SSW_F16 };
+__device__ __forceinline__ float load_param(const void* p, int type, int i) {
+  if (type == kParamBF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(p)[i]);
+  if (type == kParamF16) return __half2float(reinterpret_cast<const __half*>(p)[i]);
+  return reinterpret_cast<const float*>(p)[i];
+}
+__device__ __forceinline__ void store_param(void* p, int type, int i, float v) {
+  if (type == kParamBF16) reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
+  else if (type == kParamF16) reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
+  else reinterpret_cast<float*>(p)[i] = v;
+}
+
+// Where rows come from and go to.  Dense: row i to row i.  Slice: row idx[i] * taps + sub[i] of the source to
+// row i, an invalid parent giving a row of zeros to be normalised (a voxel without a parent).  Scatter: row i
+// to row idx[i] * taps + sub[i] of the result, which the caller has cleared; nowhere if that is outside the
+// result or if `owner` (the input row of every result row) names another row - of two voxels in one cell
+// exactly one is written, whole.
+enum RowMode { kRowDense, kRowScatter, kRowSlice };
+struct RowIndex {
+  const int32_t* idx;
+  const int32_t* sub;
+  const int32_t* owner;
+  int taps;
+  int64_t n;  // valid range of idx
+};
+
+template <int GL>
+__device__ __forceinline__ float group_sum(float x) {
+#pragma unroll
+  for (int o = GL / 2; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  return x;
+}
+
+// mean and 1 / sqrt(var + eps) of a row held as v[STEPS][V] by GL lanes
+template <int GL, int STEPS, int V>
+__device__ __forceinline__ void row_stats(const float (&v)[STEPS][V], int gl, int chunks, float inv_c, float eps, float& mean,
+                                          float& rstd) {
+  float part = 0.f;
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s)
+#pragma unroll
+    for (int i = 0; i < V; ++i) part += v[s][i];
+  mean = group_sum<GL>(part) * inv_c;
+  float sq = 0.f;
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s) {
+    if (s * GL + gl < chunks) {
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        const float d = v[s][i] - mean;
+        sq += d * d;
+      }
+    }
+  }
+  rstd = rsqrtf(group_sum<GL>(sq) * inv_c + eps);
+}
+
 // GL lanes per row, STEPS 16-byte chunks per lane; chunk k of a lane is chunk k * GL + lane-in-group
-// of the row, so a group's loads of one step are contiguous.
-template <typename T, int GL, int STEPS>
-__global__ void __launch_bounds__(256) k_add_layernorm(const T* a, const T* b,
-                                                       const float* __restrict__ gamma, const float* __restrict__ beta,
-                                                       float eps, int64_t n_rows, int C, T* sum_out, T* norm_out) {
-  constexpr int V = Vec16<T>::N;
+// of the row, so a group's loads of one step are contiguous.  R rows per group and iteration.
+//
+// HBM bound, so what counts is bytes in flight: all of an iteration's loads (R rows, both inputs) are issued
+// before anything is stored - the outputs may alias the inputs, so the compiler cannot move a load above a
+// store.  A group spans the whole row where 32 lanes can: with 96 channels of bf16 (12 chunks) 16 lanes x 1
+// chunk against 4 lanes x 3 chunks, whose 64-byte pieces of eight rows per load cost more than the idle
+// quarter of the lanes saves (150 000 rows, five calls of a stage: 109 against 122 us; the bytes take 75).
+// 10 000 x 192 of fp32: 7.6 -> 6.1 us a call.
+constexpr int kNormBlocksPerSm = 4;  // resident: the grid is no larger, blocks stride over the rows
+template <int STEPS>
+__host__ __device__ constexpr int rows_per_iter() { return STEPS == 1 ? 2 : 1; }
+
+template <typename T, int GL, int STEPS, int MODE>
+__global__ void __launch_bounds__(256, kNormBlocksPerSm) k_add_layernorm(const T* a, const T* b, const void* __restrict__ gamma,
+                                                       const void* __restrict__ beta, int ptype, float eps, int64_t n_rows, int C,
+                                                       RowIndex ix, T* sum_out, T* norm_out) {
+  constexpr int V = Vec16<T>::N, R = rows_per_iter<STEPS>();
   grid_dependency_wait();
-  const int lane = threadIdx.x & 31;
-  const int gl = lane % GL;
+  const int gl = (threadIdx.x & 31) % GL;
   const int chunks = C / V;
   const int64_t groups_per_block = blockDim.x / GL;
   const int64_t g0 = (int64_t)blockIdx.x * groups_per_block + threadIdx.x / GL;
   const int64_t g_step = (int64_t)gridDim.x * groups_per_block;
-  // the affine parameters of this lane's channels stay in registers for all its rows
-  float gm[STEPS][V], bt[STEPS][V];
+  // the affine parameters in shared memory, as fp32: registers are better spent on rows in flight
+  extern __shared__ __align__(16) float par_s[];  // [gamma C][beta C]
+  if (norm_out) {
+    for (int i = threadIdx.x; i < C; i += blockDim.x) {
+      par_s[i] = load_param(gamma, ptype, i);
+      par_s[C + i] = load_param(beta, ptype, i);
+    }
+    __syncthreads();
+  }
+  const float inv_c = 1.0f / (float)C;
+  // every lane of a warp runs the same number of iterations, so the group shuffles are convergent
+  const int64_t n_iter = (n_rows + g_step * R - 1) / (g_step * R);
+  for (int64_t it = 0; it < n_iter; ++it) {
+    float v[R][STEPS][V];
+    bool live[R], have[R];
+    int64_t row[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      row[r] = g0 + (it * R + r) * g_step;
+      live[r] = have[r] = row[r] < n_rows;
+    }
+    int64_t src[R], dst[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      src[r] = dst[r] = row[r];
+      if constexpr (MODE != kRowDense) {
+        const int j = live[r] ? __ldg(ix.idx + row[r]) : -1, t = live[r] ? __ldg(ix.sub + row[r]) : -1;
+        have[r] = (unsigned)j < (unsigned)ix.n && (unsigned)t < (unsigned)ix.taps;
+        const int64_t slot = (int64_t)j * ix.taps + t;
+        if constexpr (MODE == kRowSlice) {
+          src[r] = slot;
+        } else {
+          have[r] = live[r] = have[r] && __ldg(ix.owner + slot) == (int)row[r];
+          dst[r] = slot;
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) {
+        const int ch = s * GL + gl;
+#pragma unroll
+        for (int i = 0; i < V; ++i) v[r][s][i] = 0.f;
+        if (have[r] && ch < chunks) Vec16<T>::load(a + src[r] * C + ch * V, v[r][s]);
+      }
+    if constexpr (MODE == kRowDense) {
+      if (b) {
+        float w[R][STEPS][V];
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int s = 0; s < STEPS; ++s) {
+            const int ch = s * GL + gl;
+#pragma unroll
+            for (int i = 0; i < V; ++i) w[r][s][i] = 0.f;
+            if (live[r] && ch < chunks) Vec16<T>::load(b + row[r] * C + ch * V, w[r][s]);
+          }
+        // With 16-bit rows the sum that is normalised is the rounded sum the caller sees in sum_out
+        // (what a separate add followed by LayerNorm would read), not the fp32 value.
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int s = 0; s < STEPS; ++s)
+#pragma unroll
+            for (int i = 0; i < V; ++i) v[r][s][i] = round_to<T>(v[r][s][i] + w[r][s][i]);
+      }
+      if (sum_out) {
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int s = 0; s < STEPS; ++s)
+            if (live[r] && s * GL + gl < chunks) Vec16<T>::store(sum_out + row[r] * C + (s * GL + gl) * V, v[r][s]);
+      }
+      if (!norm_out) continue;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float mean, rstd;
+      row_stats<GL, STEPS, V>(v[r], gl, chunks, inv_c, eps, mean, rstd);
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) {
+        const int ch = s * GL + gl;
+        if (live[r] && ch < chunks) {
+          float y[V];
+#pragma unroll
+          for (int i = 0; i < V; i += 4) {
+            const float4 g = *reinterpret_cast<const float4*>(par_s + ch * V + i);
+            const float4 t = *reinterpret_cast<const float4*>(par_s + C + ch * V + i);
+            const float gv[4] = {g.x, g.y, g.z, g.w}, tv[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              y[i + k] = (v[r][s][i + k] - mean) * rstd * gv[k] + tv[k];
+          }
+          Vec16<T>::store(norm_out + dst[r] * C + ch * V, y);
+        }
+      }
+    }
+  }
+}
+
+// dx = rstd (dy g - mean(dy g) - xhat mean(dy g xhat)) (+ dsum), dgamma = sum dy xhat, dbeta = sum dy.
+// One pass: x, dy (and dsum) are read once, dx is written once; statistics are recomputed from x (in
+// registers anyway).  A lane sums its channels' parameter gradients over all its rows, the block adds its
+// groups up in shared memory and leaves one row of partials [2 C]; k_param_grad adds the blocks' rows in
+// block order, so the result does not depend on scheduling.  A lane holds one chunk where the row allows: with three a
+// lane (4 lanes a row) the block's sum over 64 groups took longer than its rows.  40 000 x 96 of bf16: 15 us with
+// the reduction against 222 us in torch's two kernels; the bytes take 5.
+template <typename T, int GL, int STEPS>
+__global__ void __launch_bounds__(256) k_layernorm_bwd(const T* __restrict__ x, const T* __restrict__ dy,
+                                                       const T* __restrict__ dsum, const void* __restrict__ gamma, int ptype,
+                                                       float eps, int64_t n_rows, int C, T* __restrict__ dx,
+                                                       float* __restrict__ partial) {
+  constexpr int V = Vec16<T>::N, R = STEPS == 1 ? 2 : 1;
+  extern __shared__ float acc_s[];  // [4 warps][2 C]
+  const int gl = (threadIdx.x & 31) % GL;
+  const int chunks = C / V;
+  const int64_t groups_per_block = blockDim.x / GL;
+  const int64_t g0 = (int64_t)blockIdx.x * groups_per_block + threadIdx.x / GL;
+  const int64_t g_step = (int64_t)gridDim.x * groups_per_block;
+  float gm[STEPS][V], dg[STEPS][V], db[STEPS][V];
 #pragma unroll
   for (int s = 0; s < STEPS; ++s) {
     const int ch = s * GL + gl;
 #pragma unroll
     for (int i = 0; i < V; ++i) {
-      gm[s][i] = (norm_out && ch < chunks) ? __ldg(gamma + ch * V + i) : 0.f;
-      bt[s][i] = (norm_out && ch < chunks) ? __ldg(beta + ch * V + i) : 0.f;
+      gm[s][i] = ch < chunks ? load_param(gamma, ptype, ch * V + i) : 0.f;
+      dg[s][i] = db[s][i] = 0.f;
     }
   }
   const float inv_c = 1.0f / (float)C;
-  // every lane of a warp runs the same number of iterations, so the group shuffles are convergent
-  const int64_t n_iter = (n_rows + g_step - 1) / g_step;
+  const int64_t n_iter = (n_rows + g_step * R - 1) / (g_step * R);
   for (int64_t it = 0; it < n_iter; ++it) {
-    const int64_t row = g0 + it * g_step;
-    const bool live = row < n_rows;
-    float v[STEPS][V];
-    float part = 0.f;
+    float v[R][STEPS][V], d[R][STEPS][V], w[R][STEPS][V];
+    bool live[R];
 #pragma unroll
-    for (int s = 0; s < STEPS; ++s) {
-      const int ch = s * GL + gl;
-      const bool on = live && ch < chunks;
+    for (int r = 0; r < R; ++r) {
+      const int64_t row = g0 + (it * R + r) * g_step;
+      live[r] = row < n_rows;
 #pragma unroll
-      for (int i = 0; i < V; ++i) v[s][i] = 0.f;
-      if (on) {
-        Vec16<T>::load(a + row * C + ch * V, v[s]);
-        if (b) {
-          float w[V];
-          Vec16<T>::load(b + row * C + ch * V, w);
+      for (int s = 0; s < STEPS; ++s) {
+        const int ch = s * GL + gl;
 #pragma unroll
-          for (int i = 0; i < V; ++i) v[s][i] += w[i];
+        for (int i = 0; i < V; ++i) v[r][s][i] = d[r][s][i] = w[r][s][i] = 0.f;
+        if (live[r] && ch < chunks) {
+          Vec16<T>::load(x + row * C + ch * V, v[r][s]);
+          Vec16<T>::load(dy + row * C + ch * V, d[r][s]);
+          if (dsum) Vec16<T>::load(dsum + row * C + ch * V, w[r][s]);
         }
-        // With 16-bit rows the sum that is normalised is the rounded sum the caller sees in sum_out
-        // (what a separate add followed by LayerNorm would read), not the fp32 value.
-        if (b) {
-#pragma unroll
-          for (int i = 0; i < V; ++i) v[s][i] = round_to<T>(v[s][i]);
-        }
-        if (sum_out) Vec16<T>::store(sum_out + row * C + ch * V, v[s]);
       }
     }
-    if (!norm_out) continue;
 #pragma unroll
-    for (int s = 0; s < STEPS; ++s)
+    for (int r = 0; r < R; ++r) {
+      float mean, rstd;
+      row_stats<GL, STEPS, V>(v[r], gl, chunks, inv_c, eps, mean, rstd);
+      float c1 = 0.f, c2 = 0.f;
 #pragma unroll
-      for (int i = 0; i < V; ++i) part += v[s][i];
-#pragma unroll
-    for (int o = GL / 2; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    const float mean = part * inv_c;
-    float sq = 0.f;
-#pragma unroll
-    for (int s = 0; s < STEPS; ++s) {
-      const int ch = s * GL + gl;
-      if (ch < chunks) {
+      for (int s = 0; s < STEPS; ++s) {
 #pragma unroll
         for (int i = 0; i < V; ++i) {
-          const float d = v[s][i] - mean;
-          sq += d * d;
+          const float xh = (v[r][s][i] - mean) * rstd;
+          v[r][s][i] = xh;
+          dg[s][i] = fmaf(d[r][s][i], xh, dg[s][i]);  // channels and rows beyond the end: d is zero
+          db[s][i] += d[r][s][i];
+          d[r][s][i] *= gm[s][i];
+          c1 += d[r][s][i];
+          c2 = fmaf(d[r][s][i], xh, c2);
         }
       }
-    }
+      c1 = group_sum<GL>(c1) * inv_c;
+      c2 = group_sum<GL>(c2) * inv_c;
+      const int64_t row = g0 + (it * R + r) * g_step;
 #pragma unroll
-    for (int o = GL / 2; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    const float rstd = rsqrtf(sq * inv_c + eps);
+      for (int s = 0; s < STEPS; ++s) {
+        const int ch = s * GL + gl;
+        if (live[r] && ch < chunks) {
+          float y[V];
 #pragma unroll
-    for (int s = 0; s < STEPS; ++s) {
-      const int ch = s * GL + gl;
-      if (live && ch < chunks) {
-        float y[V];
-#pragma unroll
-        for (int i = 0; i < V; ++i) y[i] = (v[s][i] - mean) * rstd * gm[s][i] + bt[s][i];
-        Vec16<T>::store(norm_out + row * C + ch * V, y);
+          for (int i = 0; i < V; ++i) y[i] = rstd * (d[r][s][i] - c1 - v[r][s][i] * c2) + w[r][s][i];
+          Vec16<T>::store(dx + row * C + ch * V, y);
+        }
       }
     }
   }
+  // groups of a warp first (the lanes that hold the same channels), then the block's warps, four at a time
+#pragma unroll
+  for (int s = 0; s < STEPS; ++s)
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+#pragma unroll
+      for (int o = GL; o < 32; o <<= 1) {
+        dg[s][i] += __shfl_xor_sync(0xffffffffu, dg[s][i], o);
+        db[s][i] += __shfl_xor_sync(0xffffffffu, db[s][i], o);
+      }
+  const int warp = threadIdx.x >> 5;
+  float* acc = acc_s + (warp & 3) * 2 * C;
+  for (int half = 0; half < 2; ++half) {
+    if ((warp >> 2) == half && (threadIdx.x & 31) < GL) {
+#pragma unroll
+      for (int s = 0; s < STEPS; ++s) {
+        const int ch = s * GL + gl;
+        if (ch < chunks) {
+#pragma unroll
+          for (int i = 0; i < V; ++i) {
+            const int c = ch * V + i;
+            acc[c] = (half ? acc[c] : 0.f) + dg[s][i];
+            acc[C + c] = (half ? acc[C + c] : 0.f) + db[s][i];
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int i = threadIdx.x; i < 2 * C; i += blockDim.x)
+    partial[(int64_t)blockIdx.x * 2 * C + i] = (acc_s[i] + acc_s[2 * C + i]) + (acc_s[4 * C + i] + acc_s[6 * C + i]);
 }
 
+// Sum of `rows` rows of partials [rows][width] into out0 (columns below `split`) and out1 (the others).
+// One block per 32 columns, 32 row lanes each: coalesced 128-byte reads, rows added in a fixed order.
+__global__ void __launch_bounds__(1024) k_param_grad(const float* __restrict__ partial, int rows, int width, int split, void* out0,
+                                                     void* out1, int ptype) {
+  __shared__ float t[32][33];
+  grid_dependency_wait();
+  const int col = blockIdx.x * 32 + threadIdx.x;
+  float s = 0.f;
+  if (col < width)
+    for (int r = threadIdx.y; r < rows; r += 32) s += partial[(int64_t)r * width + col];
+  t[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  s = group_sum<32>(t[threadIdx.x][threadIdx.y]);
+  const int c = blockIdx.x * 32 + threadIdx.y;
+  if (threadIdx.x == 0 && c < width) {
+    if (c < split) store_param(out0, ptype, c, s);
+    else store_param(out1, ptype, c - split, s);
+  }
+}
+
+// Column sums of a [n, C] matrix (the bias gradient of a Linear layer), one pass, HBM bound: a thread owns
+// one 16-byte chunk of columns and strides over the rows, four rows in flight; the block's row lanes are
+// added up in shared memory and one row of partials per block goes to k_param_grad.  150 000 x (288 + 96) of fp32: 47 us against 214
+// us as torch sums; the bytes take 35.
+constexpr int kColThreads = 256;
+template <typename T>
+__global__ void __launch_bounds__(kColThreads) k_col_sum(const T* __restrict__ x, int64_t n, int C, int64_t rows_per_block,
+                                                         float* __restrict__ partial) {
+  constexpr int V = Vec16<T>::N, U = 4;
+  extern __shared__ float red_s[];  // [row lanes][chunks of this block * V]
+  const int chunks = C / V;
+  const int cpb = min(chunks, kColThreads);         // chunks a block looks after
+  const int lanes = kColThreads / cpb;              // rows in step
+  const int ch0 = blockIdx.y * cpb;
+  const int rl = threadIdx.x / cpb, cl = threadIdx.x - rl * cpb, ch = ch0 + cl;
+  const bool on = rl < lanes && ch < chunks;
+  const int64_t r0 = (int64_t)blockIdx.x * rows_per_block, r1 = min(n, r0 + rows_per_block);
+  float acc[V];
+#pragma unroll
+  for (int i = 0; i < V; ++i) acc[i] = 0.f;
+  if (on) {
+    for (int64_t r = r0 + rl; r < r1; r += (int64_t)lanes * U) {
+      float v[U][V];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) v[u][i] = 0.f;
+        if (r + (int64_t)u * lanes < r1) Vec16<T>::load(x + (r + (int64_t)u * lanes) * C + ch * V, v[u]);
+      }
+#pragma unroll
+      for (int i = 0; i < V; ++i) acc[i] += (v[0][i] + v[1][i]) + (v[2][i] + v[3][i]);
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) red_s[(rl * cpb + cl) * V + i] = acc[i];
+  }
+  __syncthreads();
+  for (int c = threadIdx.x; c < cpb * V; c += kColThreads) {
+    if (ch0 * V + c >= C) continue;
+    float s = 0.f;
+    for (int l = 0; l < lanes; ++l) s += red_s[l * cpb * V + c];
+    partial[(int64_t)blockIdx.x * C + ch0 * V + c] = s;
+  }
+}
+
+struct NormArgs {
+  const void *a, *b, *gamma, *beta;
+  int ptype;
+  float eps;
+  int64_t n;
+  int C;
+  void *sum_out, *norm_out;
+  // indexed forms
+  int mode;
+  RowIndex ix;
+  // backward
+  const void* dsum;
+  float* partial;
+  int blocks;
+};
+constexpr int kNormBwdBlocksPerSm = 2;
+
 template <typename T, int GL, int STEPS>
-static int launch_norm(const void* a, const void* b, const float* gamma, const float* beta, float eps, int64_t n, int C,
-                       void* sum_out, void* norm_out, cudaStream_t stream) {
+static int launch_norm(const NormArgs& p, bool bwd, cudaStream_t stream) {
   int dev = 0, sms = 0;
   SSW_CUDA_TRY(cudaGetDevice(&dev));
   SSW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  if (bwd) {
+    k_layernorm_bwd<T, GL, STEPS><<<p.blocks, 256, 8 * p.C * sizeof(float), stream>>>(
+        reinterpret_cast<const T*>(p.a), reinterpret_cast<const T*>(p.b), reinterpret_cast<const T*>(p.dsum), p.gamma, p.ptype, p.eps,
+        p.n, p.C, reinterpret_cast<T*>(p.norm_out), p.partial);
+    SSW_LAUNCH_CHECK("k_layernorm_bwd");
+    return SSW_OK;
+  }
   const int64_t groups_per_block = 256 / GL;
-  int64_t blocks = ceil_div64(n, groups_per_block);
-  const int64_t cap = (int64_t)sms * 8;  // eight resident blocks per SM, rows beyond that by striding
+  int64_t blocks = ceil_div64(p.n, groups_per_block * rows_per_iter<STEPS>());
+  const int64_t cap = (int64_t)sms * kNormBlocksPerSm;
   if (blocks > cap) blocks = cap;
-  SSW_CUDA_TRY(launch_chained(k_add_layernorm<T, GL, STEPS>, dim3((unsigned)blocks), dim3(256), 0, stream,
-                              reinterpret_cast<const T*>(a), reinterpret_cast<const T*>(b), gamma, beta, eps, n, C,
-                              reinterpret_cast<T*>(sum_out), reinterpret_cast<T*>(norm_out)));
+  auto kern = p.mode == kRowDense ? k_add_layernorm<T, GL, STEPS, kRowDense>
+              : p.mode == kRowScatter ? k_add_layernorm<T, GL, STEPS, kRowScatter> : k_add_layernorm<T, GL, STEPS, kRowSlice>;
+  SSW_CUDA_TRY(launch_chained(kern, dim3((unsigned)blocks), dim3(256), 2 * p.C * sizeof(float), stream, reinterpret_cast<const T*>(p.a),
+                              reinterpret_cast<const T*>(p.b), p.gamma, p.beta, p.ptype, p.eps, p.n, p.C, p.ix,
+                              reinterpret_cast<T*>(p.sum_out), reinterpret_cast<T*>(p.norm_out)));
   SSW_LAUNCH_CHECK("k_add_layernorm");
   return SSW_OK;
 }
 
 template <typename T>
-static int dispatch_norm(const void* a, const void* b, const float* gamma, const float* beta, float eps, int64_t n, int C,
-                         void* sum_out, void* norm_out, cudaStream_t stream) {
-  const int chunks = C / Vec16<T>::N;
+static int dispatch_norm_t(const NormArgs& p, bool bwd, cudaStream_t stream) {
+  const int chunks = p.C / Vec16<T>::N;
 #define SSW_NORM_CASE(GL, STEPS) \
-  if (chunks <= GL * STEPS) return launch_norm<T, GL, STEPS>(a, b, gamma, beta, eps, n, C, sum_out, norm_out, stream)
+  if (chunks <= GL * STEPS) return launch_norm<T, GL, STEPS>(p, bwd, stream)
+  SSW_NORM_CASE(4, 1);
   SSW_NORM_CASE(8, 1);
   SSW_NORM_CASE(16, 1);
   SSW_NORM_CASE(32, 1);
@@ -206,30 +514,141 @@ static int dispatch_norm(const void* a, const void* b, const float* gamma, const
 #undef SSW_NORM_CASE
   return SSW_E_UNSUPPORTED;
 }
+static int dispatch_norm(const NormArgs& p, int dtype, bool bwd, cudaStream_t stream) {
+  switch (dtype) {
+    case SSW_F32: return dispatch_norm_t<float>(p, bwd, stream);
+    case SSW_BF16: return dispatch_norm_t<__nv_bfloat16>(p, bwd, stream);
+    case SSW_F16: return dispatch_norm_t<__half>(p, bwd, stream);
+  }
+  return SSW_E_INVALID;
+}
+static int norm_elt(int dtype) { return dtype == SSW_F32 ? 4 : (dtype == SSW_BF16 || dtype == SSW_F16) ? 2 : 0; }
 
 }  // namespace ssw
 
 using namespace ssw;
 
-extern "C" int ssw_add_layernorm(const void* a, const void* b, const float* gamma, const float* beta, float eps,
-                                 int dtype, int64_t n_rows, int32_t channels, void* sum_out, void* norm_out,
-                                 void* stream_) {
-  if (n_rows < 0 || channels <= 0) return SSW_E_INVALID;
-  if (n_rows == 0) return SSW_OK;
-  if (!a || (!sum_out && !norm_out) || (norm_out && (!gamma || !beta))) return SSW_E_INVALID;
-  if (!b && sum_out && !norm_out) return SSW_E_INVALID;  // a plain copy is not this call's business
-  const int elt = dtype == SSW_F32 ? 4 : (dtype == SSW_BF16 || dtype == SSW_F16) ? 2 : 0;
+// what every entry point here asks of its rows: a known type, 16-byte multiples, aligned bases
+static int norm_check(int dtype, int64_t n_rows, int32_t channels, std::initializer_list<const void*> ptrs) {
+  const int elt = norm_elt(dtype);
   if (!elt) return SSW_E_INVALID;
-  if ((channels * elt) % 16) return SSW_E_UNSUPPORTED;
-  const void* ptrs[4] = {a, b, sum_out, norm_out};
+  if (((int64_t)channels * elt) % 16) return SSW_E_UNSUPPORTED;
   for (const void* q : ptrs)
     if (q && (reinterpret_cast<uintptr_t>(q) & 15)) return SSW_E_INVALID;
   if (n_rows * (int64_t)channels >= (int64_t)1 << 40) return SSW_E_RANGE;
+  return SSW_OK;
+}
+
+extern "C" int ssw_add_layernorm_p(const void* a, const void* b, const void* gamma, const void* beta, int param_dtype, float eps,
+                                   int dtype, int64_t n_rows, int32_t channels, void* sum_out, void* norm_out, void* stream) {
+  if (n_rows < 0 || channels <= 0) return SSW_E_INVALID;
+  if (n_rows == 0) return SSW_OK;
+  if (!a || (!sum_out && !norm_out) || (norm_out && (!gamma || !beta || !norm_elt(param_dtype)))) return SSW_E_INVALID;
+  if (!b && sum_out && !norm_out) return SSW_E_INVALID;  // a plain copy is not this call's business
+  const int rc = norm_check(dtype, n_rows, channels, {a, b, sum_out, norm_out});
+  if (rc != SSW_OK) return rc;
+  NormArgs p = {};
+  p.a = a; p.b = b; p.gamma = gamma; p.beta = beta; p.ptype = param_dtype; p.eps = eps; p.n = n_rows; p.C = channels;
+  p.sum_out = sum_out; p.norm_out = norm_out; p.mode = kRowDense;
+  return dispatch_norm(p, dtype, false, (cudaStream_t)stream);
+}
+
+extern "C" int ssw_add_layernorm(const void* a, const void* b, const float* gamma, const float* beta, float eps,
+                                 int dtype, int64_t n_rows, int32_t channels, void* sum_out, void* norm_out,
+                                 void* stream_) {
+  return ssw_add_layernorm_p(a, b, gamma, beta, SSW_F32, eps, dtype, n_rows, channels, sum_out, norm_out, stream_);
+}
+
+static int layernorm_indexed(int mode, const void* x, const void* gamma, const void* beta, int param_dtype, float eps, int dtype,
+                             int32_t channels, RowIndex ix, int64_t n_rows, void* out, cudaStream_t stream) {
+  NormArgs p = {};
+  p.a = x; p.gamma = gamma; p.beta = beta; p.ptype = param_dtype; p.eps = eps; p.n = n_rows; p.C = channels; p.norm_out = out;
+  p.mode = mode;
+  p.ix = ix;
+  return dispatch_norm(p, dtype, false, stream);
+}
+
+extern "C" int ssw_layernorm_slices(const void* x, const void* gamma, const void* beta, int param_dtype, float eps, int dtype,
+                                    int64_t n_src, int32_t channels, const int32_t* parent, const int32_t* tap, int32_t taps,
+                                    int64_t n_out, void* out, void* stream) {
+  if (n_out < 0 || n_src < 0 || n_src >= ((int64_t)1 << 31) || channels <= 0 || taps <= 0) return SSW_E_INVALID;
+  if (n_out == 0) return SSW_OK;
+  if (!parent || !tap || !out || !gamma || !beta || !norm_elt(param_dtype) || (n_src > 0 && !x)) return SSW_E_INVALID;
+  const int rc = norm_check(dtype, n_out, channels, {x, out});
+  if (rc != SSW_OK) return rc;
+  return layernorm_indexed(kRowSlice, x, gamma, beta, param_dtype, eps, dtype, channels, RowIndex{parent, tap, nullptr, taps, n_src}, n_out,
+                           out, (cudaStream_t)stream);
+}
+
+extern "C" int ssw_layernorm_scatter(const void* x, const void* gamma, const void* beta, int param_dtype, float eps, int dtype,
+                                     int64_t n_rows, int32_t channels, const int32_t* parent, const int32_t* tap,
+                                     const int32_t* owner, int32_t taps, int64_t n_out, void* out, void* stream_) {
+  if (n_rows < 0 || n_rows >= ((int64_t)1 << 31) || n_out < 0 || n_out >= ((int64_t)1 << 31) || channels <= 0 || taps <= 0)
+    return SSW_E_INVALID;
+  if (n_out == 0) return SSW_OK;
+  if (!owner || !out || !gamma || !beta || !norm_elt(param_dtype) || (n_rows > 0 && (!x || !parent || !tap))) return SSW_E_INVALID;
+  const int rc = norm_check(dtype, n_out * taps, channels, {x, out});
+  if (rc != SSW_OK) return rc;
   cudaStream_t stream = (cudaStream_t)stream_;
-  switch (dtype) {
-    case SSW_F32: return dispatch_norm<float>(a, b, gamma, beta, eps, n_rows, channels, sum_out, norm_out, stream);
-    case SSW_BF16: return dispatch_norm<__nv_bfloat16>(a, b, gamma, beta, eps, n_rows, channels, sum_out, norm_out, stream);
-    case SSW_F16: return dispatch_norm<__half>(a, b, gamma, beta, eps, n_rows, channels, sum_out, norm_out, stream);
-  }
-  return SSW_E_INVALID;
+  SSW_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)n_out * taps * channels * norm_elt(dtype), stream));
+  if (n_rows == 0) return SSW_OK;
+  return layernorm_indexed(kRowScatter, x, gamma, beta, param_dtype, eps, dtype, channels, RowIndex{parent, tap, owner, taps, n_out}, n_rows,
+                           out, stream);
+}
+
+// Blocks of a reduction pass over n rows: two per SM (the register budget of the widest rows), fewer for few rows.
+static int reduce_blocks(int64_t n_rows) {
+  const int64_t want = ceil_div64(n_rows, 32);
+  return (int)(want < 148 * kNormBwdBlocksPerSm ? (want > 0 ? want : 1) : 148 * kNormBwdBlocksPerSm);
+}
+extern "C" int64_t ssw_layernorm_bwd_workspace_floats(int64_t n_rows, int32_t channels) {
+  return (int64_t)reduce_blocks(n_rows) * 2 * channels;
+}
+extern "C" int64_t ssw_col_sum_workspace_floats(int64_t n_rows, int32_t channels) {
+  return (int64_t)reduce_blocks(n_rows) * channels;
+}
+
+static int launch_param_grad(const float* partial, int rows, int width, int split, void* out0, void* out1, int ptype,
+                             cudaStream_t stream) {
+  SSW_CUDA_TRY(launch_chained(k_param_grad, dim3((width + 31) / 32), dim3(32, 32), 0, stream, partial, rows, width, split, out0, out1,
+                              ptype));
+  return SSW_OK;
+}
+
+extern "C" int ssw_layernorm_bwd(const void* x, const void* dy, const void* dsum, const void* gamma, int param_dtype, float eps,
+                                 int dtype, int64_t n_rows, int32_t channels, void* dx, void* dgamma, void* dbeta,
+                                 float* workspace, void* stream_) {
+  if (n_rows <= 0 || channels <= 0) return SSW_E_INVALID;
+  if (!x || !dy || !gamma || !norm_elt(param_dtype) || !dx || !dgamma || !dbeta || !workspace) return SSW_E_INVALID;
+  const int rc = norm_check(dtype, n_rows, channels, {x, dy, dsum, dx});
+  if (rc != SSW_OK) return rc;
+  cudaStream_t stream = (cudaStream_t)stream_;
+  NormArgs p = {};
+  p.a = x; p.b = dy; p.dsum = dsum; p.gamma = gamma; p.ptype = param_dtype; p.eps = eps; p.n = n_rows; p.C = channels;
+  p.norm_out = dx; p.partial = workspace; p.blocks = reduce_blocks(n_rows);
+  const int st = dispatch_norm(p, dtype, true, stream);
+  if (st != SSW_OK) return st;
+  return launch_param_grad(workspace, p.blocks, 2 * channels, channels, dgamma, dbeta, param_dtype, stream);
+}
+
+extern "C" int ssw_col_sum(const void* x, int dtype, int64_t n_rows, int32_t channels, void* out, int out_dtype, float* workspace,
+                           void* stream_) {
+  if (n_rows <= 0 || channels <= 0) return SSW_E_INVALID;
+  if (!x || !out || !norm_elt(out_dtype) || !workspace) return SSW_E_INVALID;
+  const int rc = norm_check(dtype, n_rows, channels, {x});
+  if (rc != SSW_OK) return rc;
+  cudaStream_t stream = (cudaStream_t)stream_;
+  const int blocks = reduce_blocks(n_rows), V = 16 / norm_elt(dtype), chunks = channels / V;
+  const int cpb = chunks < kColThreads ? chunks : kColThreads;
+  const dim3 grid(blocks, (chunks + cpb - 1) / cpb);
+  const size_t smem = (size_t)(kColThreads / cpb) * cpb * V * sizeof(float);  // at most 8 KB
+  const int64_t rpb = ceil_div64(n_rows, blocks);
+  if (dtype == SSW_F32)
+    k_col_sum<float><<<grid, kColThreads, smem, stream>>>(reinterpret_cast<const float*>(x), n_rows, channels, rpb, workspace);
+  else if (dtype == SSW_BF16)
+    k_col_sum<__nv_bfloat16><<<grid, kColThreads, smem, stream>>>(reinterpret_cast<const __nv_bfloat16*>(x), n_rows, channels, rpb, workspace);
+  else
+    k_col_sum<__half><<<grid, kColThreads, smem, stream>>>(reinterpret_cast<const __half*>(x), n_rows, channels, rpb, workspace);
+  SSW_LAUNCH_CHECK("k_col_sum");
+  return launch_param_grad(workspace, blocks, channels, channels, out, out, out_dtype, stream);
 }

@@ -1,0 +1,166 @@
+"""Row passes around the GEMMs of a block with autograd recording: residual add + LayerNorm, and the
+bias gradient of a Linear layer, each forward and backward one pass over the voxel rows (csrc/norm.cu).
+
+torch's own kernels stay for everything these do not cover: other dtypes, mixed dtypes, rows that are not
+16-byte multiples, autocast, module hooks, function transforms, forward-mode differentiation, tracing.
+Under create_graph the backward is written in differentiable torch operations."""
+from __future__ import annotations
+
+from typing import Optional
+
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+from ._lib import check, dtype_code, lib, ptr, stream_ptr
+
+_DTYPES = (torch.float32, torch.bfloat16, torch.float16)
+
+
+def unhooked(*modules: nn.Module) -> bool:
+    """Calling the module and using its parameters directly are the same thing."""
+    g = nn.modules.module
+    return not (g._global_forward_hooks or g._global_forward_pre_hooks or g._global_backward_hooks or g._global_backward_pre_hooks
+                or any(m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks for m in modules))
+
+
+def _ordinary_mode() -> bool:
+    return not (torch.is_autocast_enabled("cuda") or torch._C._are_functorch_transforms_active()
+                or torch.autograd.forward_ad._current_level >= 0 or torch.jit.is_tracing() or torch.compiler.is_compiling())
+
+
+def aligned_rows(*tensors: torch.Tensor) -> bool:
+    """[n, C] CUDA rows the kernels take: contiguous, 16-byte aligned, n > 0, C * element size a multiple of 16."""
+    return all(type(t) in (torch.Tensor, nn.Parameter) and t.is_cuda and t.dim() == 2 and t.dtype in _DTYPES and t.is_contiguous() and t.shape[0] > 0
+               and (t.shape[1] * t.element_size()) % 16 == 0 and t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def plain_norm(norm, x: torch.Tensor) -> bool:
+    """`norm` is an affine LayerNorm over the rows of `x`, in their dtype, that the kernels reproduce."""
+    return (type(norm) is nn.LayerNorm and tuple(norm.normalized_shape) == (x.shape[-1],) and norm.weight is not None
+            and norm.bias is not None and norm.weight.dtype == x.dtype and norm.bias.dtype == x.dtype
+            and norm.weight.device == x.device and norm.bias.device == x.device
+            and norm.weight.is_contiguous() and norm.bias.is_contiguous()
+            and x.shape[-1] * x.element_size() <= 2048 and unhooked(norm) and _ordinary_mode())
+
+
+def norm_params(norm: nn.LayerNorm):
+    """(weight, bias, dtype code) as the kernels read them: in place where the module's type allows."""
+    w, b = norm.weight.detach(), norm.bias.detach()
+    if w.dtype != b.dtype or w.dtype not in _DTYPES:
+        w, b = w.float(), b.float()
+    return w.contiguous(), b.contiguous(), dtype_code(w.dtype)
+
+
+class _AddLayerNorm(torch.autograd.Function):
+    """(a + b, LayerNorm(a + b)); b None: (a, LayerNorm(a))."""
+
+    @staticmethod
+    def forward(ctx, a, b, weight, bias, eps):
+        n, c = a.shape
+        s = torch.empty_like(a) if b is not None else a.view_as(a)
+        y = torch.empty_like(a)
+        code = dtype_code(a.dtype)
+        check(lib.ssw_add_layernorm_p(ptr(a), ptr(b), ptr(weight), ptr(bias), code, float(eps), code, n, c,
+                                      ptr(s) if b is not None else 0, ptr(y), stream_ptr(a.device)), "ssw_add_layernorm")
+        ctx.set_materialize_grads(False)
+        ctx.eps, ctx.pair = float(eps), b is not None
+        ctx.save_for_backward(s if b is not None else a, weight)
+        return s, y
+
+    @staticmethod
+    def backward(ctx, ds, dy):
+        x, weight = ctx.saved_tensors
+        if dy is None:
+            return ds, ds if ctx.pair else None, None, None, None
+        if torch.is_grad_enabled():  # create_graph: differentiable operations
+            xf, g = x.float(), dy.float()
+            xc = xf - xf.mean(1, keepdim=True)
+            rstd = (xc.square().mean(1, keepdim=True) + ctx.eps).rsqrt()
+            xh, wg = xc * rstd, g * weight.float()
+            dx = (rstd * (wg - wg.mean(1, keepdim=True) - xh * (wg * xh).mean(1, keepdim=True))).to(x.dtype)
+            if ds is not None:
+                dx = dx + ds
+            return dx, dx if ctx.pair else None, (g * xh).sum(0).to(weight.dtype), g.sum(0).to(weight.dtype), None
+        n, c = x.shape
+        dy = _rows(dy)
+        ds = None if ds is None else _rows(ds)
+        dx = torch.empty_like(x)
+        dw, db = torch.empty_like(weight), torch.empty_like(weight)
+        ws = torch.empty(int(lib.ssw_layernorm_bwd_workspace_floats(n, c)), dtype=torch.float32, device=x.device)
+        code = dtype_code(x.dtype)
+        check(lib.ssw_layernorm_bwd(ptr(x), ptr(dy), ptr(ds), ptr(weight), code, ctx.eps, code, n, c, ptr(dx), ptr(dw), ptr(db), ptr(ws),
+                                    stream_ptr(x.device)), "ssw_layernorm_bwd")
+        return dx, dx if ctx.pair else None, dw, db, None
+
+
+def _rows(g: torch.Tensor) -> torch.Tensor:
+    g = g.contiguous()
+    return g if g.data_ptr() % 16 == 0 else g.clone()
+
+
+def add_layer_norm(a: torch.Tensor, b: Optional[torch.Tensor], norm: nn.LayerNorm):
+    """(a + b, norm(a + b)) with autograd; the caller has checked `aligned_rows` and `plain_norm`."""
+    return _AddLayerNorm.apply(a, b, norm.weight, norm.bias, norm.eps)
+
+
+def col_sum(g: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """Sum over the rows of g [n, C] (fp32 accumulation), in `dtype`."""
+    n, c = g.shape
+    out = torch.empty(c, dtype=dtype, device=g.device)
+    ws = torch.empty(int(lib.ssw_col_sum_workspace_floats(n, c)), dtype=torch.float32, device=g.device)
+    check(lib.ssw_col_sum(ptr(g), dtype_code(g.dtype), n, c, ptr(out), dtype_code(dtype), ptr(ws), stream_ptr(g.device)), "ssw_col_sum")
+    return out
+
+
+class _Linear(torch.autograd.Function):
+    """F.linear whose backward sums the bias gradient in one pass over the rows."""
+
+    @staticmethod
+    def forward(ctx, x, weight, bias):
+        ctx.save_for_backward(x, weight)
+        return F.linear(x, weight, bias)
+
+    @staticmethod
+    def backward(ctx, g):
+        x, weight = ctx.saved_tensors
+        need = ctx.needs_input_grad
+        gx = g @ weight if need[0] else None
+        gw = g.t() @ x if need[1] else None
+        gb = None
+        if need[2]:
+            gb = g.sum(0) if torch.is_grad_enabled() else col_sum(_rows(g), g.dtype)
+        return gx, gw, gb
+
+
+def linear(module: nn.Linear, x: torch.Tensor) -> torch.Tensor:
+    """module(x), through `_Linear` where a bias gradient will be wanted."""
+    if (torch.is_grad_enabled() and type(module) is nn.Linear and module.bias is not None and module.bias.requires_grad
+            and x.dim() == 2 and x.is_cuda and x.shape[0] > 0 and x.dtype in _DTYPES and type(x) is torch.Tensor
+            and type(module.weight) is nn.Parameter and type(module.bias) is nn.Parameter
+            and module.weight.dtype == x.dtype and module.bias.dtype == x.dtype
+            and (module.out_features * x.element_size()) % 16 == 0 and unhooked(module) and _ordinary_mode()):
+        return _Linear.apply(x, module.weight, module.bias)
+    return module(x)
+
+
+def layernorm_scatter(x: torch.Tensor, norm: nn.LayerNorm, parent: torch.Tensor, tap: torch.Tensor, owner: torch.Tensor) -> torch.Tensor:
+    """cols [M, taps * C] with norm(x[i]) in slot (parent[i], tap[i]) and zeros elsewhere; owner [M, taps] is the
+    input row of every slot (-1: none)."""
+    w, b, code = norm_params(norm)
+    n, c = x.shape
+    m, taps = owner.shape
+    out = torch.empty((m, taps * c), dtype=x.dtype, device=x.device)
+    check(lib.ssw_layernorm_scatter(ptr(x), ptr(w), ptr(b), code, float(norm.eps), dtype_code(x.dtype), n, c, ptr(parent), ptr(tap),
+                                    ptr(owner), taps, m, ptr(out), stream_ptr(x.device)), "ssw_layernorm_scatter")
+    return out
+
+
+def layernorm_slices(z: torch.Tensor, norm: nn.LayerNorm, parent: torch.Tensor, tap: torch.Tensor, taps: int) -> torch.Tensor:
+    """out[i] = norm(z[parent[i], tap[i] * C : (tap[i] + 1) * C]), a zero row being normalised where parent[i] < 0."""
+    w, b, code = norm_params(norm)
+    n, c = parent.shape[0], norm.normalized_shape[0]
+    out = torch.empty((n, c), dtype=z.dtype, device=z.device)
+    check(lib.ssw_layernorm_slices(ptr(z), ptr(w), ptr(b), code, float(norm.eps), dtype_code(z.dtype), z.shape[0], c, ptr(parent),
+                                   ptr(tap), taps, n, ptr(out), stream_ptr(z.device)), "ssw_layernorm_slices")
+    return out

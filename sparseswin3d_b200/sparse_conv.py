@@ -34,7 +34,7 @@ from typing import Optional, Sequence
 import torch
 import torch.nn as nn
 
-from . import _lib
+from . import _lib, rows
 from ._lib import check, dtype_code, lib, ptr, stream_ptr
 from .stage import SparseVoxels
 
@@ -187,6 +187,10 @@ def gather_slices(z: torch.Tensor, parent: torch.Tensor, tap: torch.Tensor, taps
     return out
 
 
+def _no_grad(f: torch.Tensor, module: nn.Module) -> bool:
+    return not (torch.is_grad_enabled() and (f.requires_grad or any(p.requires_grad for p in module.parameters())))
+
+
 def weight_from_dense(w: torch.Tensor) -> torch.Tensor:
     """A dense convolution kernel [Cout, Cin, k, k, k] in this module's [k^3, Cin, Cout] layout."""
     co, ci, k = w.shape[0], w.shape[1], w.shape[2]
@@ -277,8 +281,15 @@ class SparseConv3d(_ConvBase):
             raise ValueError("only padding 0 is built")
 
     def forward(self, x):
+        return self._convolve(x, None)
+
+    def _convolve(self, x, norm):
+        """The convolution of norm(x) (norm None: of x); the norm writes the GEMM operand itself."""
         rb = self._rulebook(x, "strided", strided_rulebook)
-        cols = gather_cols(x.features, rb.nbr)
+        if norm is None:
+            cols = gather_cols(x.features, rb.nbr)
+        else:
+            cols = rows.layernorm_scatter(x.features, norm, rb.parent, rb.tap, rb.nbr)
         out = self._affine(cols, self.weight.reshape(-1, self.out_channels))
         y = SparseVoxels(out, rb.out_indices, rb.out_shape, x.batch_size)
         y.indice_dict = x.indice_dict
@@ -293,6 +304,10 @@ class SparseInverseConv3d(_ConvBase):
         super().__init__(in_channels, out_channels, kernel_size, bias, indice_key)
 
     def forward(self, x):
+        return self._expand(x, None)
+
+    def _expand(self, x, norm):
+        """The inverse convolution, then norm (None: none); the norm rides on the gather."""
         rb = getattr(x, "indice_dict", {}).get(self.indice_key)
         if rb is None or rb.kind != "strided" or rb.ksize != self.kernel_size:
             raise _lib.SswError(f"no strided convolution has registered indice_key {self.indice_key!r} on this tensor")
@@ -302,7 +317,10 @@ class SparseInverseConv3d(_ConvBase):
         # all taps of every coarse voxel in one GEMM: z[m, t * Cout + o] = sum_c y[m, c] W[t, c, o]
         w2d = self.weight.permute(1, 0, 2).reshape(self.in_channels, k3 * self.out_channels)
         z = x.features @ w2d.to(x.features.dtype)
-        out = gather_slices(z, rb.parent, rb.tap, k3)
+        if norm is not None:
+            out = rows.layernorm_slices(z, norm, rb.parent, rb.tap, k3)
+        else:
+            out = gather_slices(z, rb.parent, rb.tap, k3)
         if self.bias is not None:
             out = out + self.bias.to(out.dtype)
         y = SparseVoxels(out, rb.in_indices, rb.in_shape, x.batch_size)
@@ -337,7 +355,11 @@ class PatchMerging(SparseModule):
         self.norm = norm_layer(dim)
 
     def forward(self, x):
-        return self.reduction(x.replace_feature(self.norm(x.features)))
+        f = x.features
+        if (type(self.reduction) is SparseConv3d and f.shape[-1] == self.reduction.in_channels and rows.unhooked(self.reduction)
+                and rows.aligned_rows(f) and rows.plain_norm(self.norm, f) and _no_grad(f, self)):
+            return self.reduction._convolve(x, self.norm)
+        return self.reduction(x.replace_feature(self.norm(f)))
 
 
 class PatchExpand(SparseModule):
@@ -349,5 +371,10 @@ class PatchExpand(SparseModule):
         self.norm = norm_layer(dim // 2)
 
     def forward(self, x):
-        y = self.expansion(x)
+        f, e = x.features, self.expansion
+        if (type(e) is SparseInverseConv3d and e.bias is None and e.weight.dtype == f.dtype and rows.unhooked(e) and f.dim() == 2
+                and f.is_cuda and (e.out_channels * f.element_size()) % 16 == 0
+                and rows.plain_norm(self.norm, f.new_empty((0, e.out_channels))) and _no_grad(f, self)):
+            return e._expand(x, self.norm)
+        y = e(x)
         return y.replace_feature(self.norm(y.features))

@@ -14,8 +14,9 @@ The GEMMs themselves (qkv, proj, the two MLP Linears) are library calls (torch /
 
 `SparseVoxels` carries the four fields of an spconv SparseConvTensor that upstream's blocks read
 (`features`, `indices` [N,4] int32 (b,z,y,x), `spatial_shape`, `batch_size`) and `replace_feature`.
-Autograd: with gradients recording, the element-wise shell runs as torch operations (the attention
-core keeps its fused forward and backward); the fused shell is the inference path."""
+Autograd: with gradients recording, the residual add + LayerNorm pairs run as one pass each way
+(`rows.add_layer_norm`), as do the bias gradients of the Linears; the attention core keeps its fused
+forward and backward, and the rest of the shell is torch operations."""
 from __future__ import annotations
 
 import copy
@@ -25,7 +26,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import _lib
+from . import _lib, rows
 from ._lib import check, dtype_code, lib, ptr, stream_ptr
 from .attention import WindowAttentionSparse, plan_params
 from .window import WindowPlan, bucket_windows, resolve_geometry
@@ -61,13 +62,13 @@ def add_layernorm(a: torch.Tensor, b: Optional[torch.Tensor], norm: Optional[nn.
         s = sum_out if sum_out is not None else torch.empty_like(a)
     y = torch.empty_like(a) if norm is not None else None
     gamma = beta = None
-    eps = 0.0
+    eps, code = 0.0, _lib.SSW_F32
     if norm is not None:
         if tuple(norm.normalized_shape) != (c,) or norm.weight is None or norm.bias is None:
             raise _lib.SswError("add_layernorm wants an affine LayerNorm over the channel dimension")
-        gamma, beta, eps = norm.weight.detach().float().contiguous(), norm.bias.detach().float().contiguous(), norm.eps
-    check(lib.ssw_add_layernorm(ptr(a), ptr(b), ptr(gamma), ptr(beta), float(eps), dtype_code(a.dtype), n, c, ptr(s), ptr(y),
-                                stream_ptr(a.device)), "ssw_add_layernorm")
+        (gamma, beta, code), eps = rows.norm_params(norm), norm.eps
+    check(lib.ssw_add_layernorm_p(ptr(a), ptr(b), ptr(gamma), ptr(beta), code, float(eps), dtype_code(a.dtype), n, c, ptr(s), ptr(y),
+                                  stream_ptr(a.device)), "ssw_add_layernorm")
     return (a if b is None else s), y
 
 
@@ -108,7 +109,7 @@ class MLP(nn.Module):
         self.drop2 = self.drop1
 
     def forward(self, x):
-        return self.drop2(self.linear2(self.drop1(self.fn(self.linear1(x)))))
+        return self.drop2(rows.linear(self.linear2, self.drop1(self.fn(rows.linear(self.linear1, x)))))
 
 
 class SwinTransformerBlock(nn.Module):
@@ -167,6 +168,16 @@ class SwinTransformerBlock(nn.Module):
             m = self.mlp(h2)
             out, _ = add_layernorm(x1, m, None, sum_out=x1)
             return x.replace_feature(out)
+        if (fuse_shell and torch.is_grad_enabled() and rows.aligned_rows(feats) and rows.plain_norm(self.norm1, feats)
+                and rows.plain_norm(self.norm2, feats)):
+            x0, h = rows.add_layer_norm(feats, None, self.norm1)
+            a = self.drop_path(self.attention_branch(h, plan, use_mask))
+            if rows.aligned_rows(a) and a.dtype == feats.dtype:
+                x1, h2 = rows.add_layer_norm(x0, a, self.norm2)
+            else:
+                x1 = x0 + a
+                h2 = self.norm2(x1)
+            return x.replace_feature(x1 + self.drop_path(self.mlp(h2)))
         a = self.attention_branch(self.norm1(feats), plan, use_mask)
         x1 = feats + self.drop_path(a)
         return x.replace_feature(x1 + self.drop_path(self.mlp(self.norm2(x1))))

@@ -1,0 +1,101 @@
+"""Row passes of a training step and of patch merging / expansion against float64: LayerNorm backward with
+the residual gradient, column sums, LayerNorm of gathered rows."""
+import pytest
+import torch
+import torch.nn as nn
+import torch.nn.functional as F
+
+from tests.cases import rel_err
+
+pytestmark = pytest.mark.gpu
+
+# one rounding of the result to its type (2^-24, 2^-11, 2^-8 at most, uniform: a third of it in the 2-norm); 32-bit
+# results also carry their sums' roundings
+TOL = {torch.float32: 3e-6, torch.float16: 5e-4, torch.bfloat16: 4e-3}
+DTYPES = [torch.float32, torch.bfloat16, torch.float16]
+
+
+# channels: every (lanes, steps) form of the kernel and its edges; rows: one, a partial group, several blocks
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n,C", [(1, 8), (3, 16), (37, 24), (1000, 48), (5003, 96), (777, 104), (4099, 192), (65, 264), (999, 384), (50, 512)])
+def test_add_layernorm_backward(dtype, n, C):
+    from sparseswin3d_b200 import rows
+
+    g = torch.Generator().manual_seed(n + C)
+    a, b, dy, ds = (torch.randn(n, C, generator=g).to(dtype).cuda() for _ in range(4))
+    ln = nn.LayerNorm(C).cuda().to(dtype)
+    with torch.no_grad():
+        ln.weight.copy_(1 + 0.3 * torch.randn(C, generator=g))
+        ln.bias.copy_(0.3 * torch.randn(C, generator=g))
+    a.requires_grad_(True), b.requires_grad_(True)
+    assert rows.aligned_rows(a, b) and rows.plain_norm(ln, a)
+    for pair in (True, False):
+        s, y = rows.add_layer_norm(a, b if pair else None, ln)
+        leaves = [a, b, ln.weight, ln.bias] if pair else [a, ln.weight, ln.bias]
+        got = torch.autograd.grad((s, y), leaves, (ds, dy))
+        s64 = s.detach().double().requires_grad_(True)
+        w64, b64 = (p.detach().double().requires_grad_(True) for p in (ln.weight, ln.bias))
+        y64 = F.layer_norm(s64, (C,), w64, b64, ln.eps)
+        gs, gw, gb = torch.autograd.grad(y64, (s64, w64, b64), dy.double())
+        ref = [gs + ds.double()] * (2 if pair else 1) + [gw, gb]
+        assert rel_err(y.detach().double().cpu(), y64.detach().cpu()) <= TOL[dtype]
+        for x, r in zip(got, ref):
+            assert x.dtype == dtype and rel_err(x.double().cpu(), r.cpu()) <= TOL[dtype]
+
+
+def test_add_layernorm_second_derivative():
+    from sparseswin3d_b200 import rows
+
+    a = torch.randn(17, 32, device="cuda", requires_grad=True)
+    ln = nn.LayerNorm(32).cuda()
+
+    def penalty(y):
+        return torch.autograd.grad(torch.autograd.grad(y.tanh().sum(), a, create_graph=True)[0].square().sum(), a)[0]
+
+    assert rel_err(penalty(rows.add_layer_norm(a, None, ln)[1]).cpu(), penalty(ln(a)).cpu()) <= 1e-5
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n,C", [(1, 8), (31, 16), (5003, 96), (40001, 288), (123, 1536), (7, 2056)])
+def test_column_sums(dtype, n, C):
+    from sparseswin3d_b200 import rows
+
+    x = torch.randn(n, C, device="cuda").to(dtype)
+    ref = x.double().sum(0)
+    # against the size of what is summed: a sum may cancel
+    scale = x.double().abs().sum(0)
+    err = (rows.col_sum(x, dtype).double() - ref).abs()
+    half_ulp = {torch.float32: 2.0 ** -24, torch.bfloat16: 2.0 ** -9, torch.float16: 2.0 ** -12}[dtype]
+    assert bool((err <= scale * 2e-6 + ref.abs() * 2 * half_ulp).all())
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("n,C", [(5, 16), (1003, 48), (4001, 96), (300, 192)])
+def test_layernorm_on_moved_rows(dtype, n, C):
+    """Scattered into (parent, tap) slots, and of rows read by (parent, tap); parents outside the range."""
+    from sparseswin3d_b200 import rows
+
+    m, taps = n // 2 + 1, 8
+    ln = nn.LayerNorm(C).cuda().to(dtype)
+    x, z = torch.randn(n, C, device="cuda").to(dtype), torch.randn(m, taps * C, device="cuda").to(dtype)
+    slot = torch.randperm(m * taps, device="cuda")[:n]
+    parent, tap = (slot // taps).int(), (slot % taps).int()
+    parent[::7] = -1
+    parent[3::11] = m + 5
+    ok = (parent >= 0) & (parent < m)
+    owner = torch.full((m, taps), -1, dtype=torch.int32, device="cuda")
+    owner[parent[ok].long(), tap[ok].long()] = torch.arange(n, device="cuda", dtype=torch.int32)[ok]
+    with torch.no_grad():
+        ln.weight.add_(torch.randn(C, device="cuda") * 0.2)
+        ln.bias.add_(torch.randn(C, device="cuda") * 0.2)
+        norm64 = lambda r: F.layer_norm(r, (C,), ln.weight.double(), ln.bias.double(), ln.eps)
+        want = torch.zeros(m, taps, C, dtype=torch.float64, device="cuda")
+        want[parent[ok].long(), tap[ok].long()] = norm64(x.double())[ok]
+        got = rows.layernorm_scatter(x, ln, parent, tap, owner)
+        assert rel_err(got.double().cpu(), want.view(m, -1).cpu()) <= TOL[dtype] and not got.view(m, taps, C)[owner < 0].any()
+        # a slot that belongs to another voxel is left to it
+        owner2 = torch.where(owner >= 0, n - 1 - owner, owner)
+        mine = owner2 == owner
+        assert not rows.layernorm_scatter(x, ln, parent, tap, owner2).view(m, taps, C)[~mine].any()
+        src = z.view(m, taps, C).double()[parent.clamp(0, m - 1).long(), tap.long()] * ok[:, None]
+        assert rel_err(rows.layernorm_slices(z, ln, parent, tap, taps).double().cpu(), norm64(src).cpu()) <= TOL[dtype]
