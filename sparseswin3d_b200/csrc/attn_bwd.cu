@@ -11,14 +11,27 @@
 //   dq_i = scale * sum_j dS_ij k_j,  dk_j = scale * sum_i dS_ij q_i,  dv_j = sum_i p_ij dO_i,
 //   dbias[rel_i - rel_j, h] += dS_ij
 //
-// Two kernels over the plan's work items, one thread per (row, head), rows read straight from
-// global memory (the rows of a window are re-read by its own threads only, so they stay in L1/L2):
-//   k_attn_bwd_q : per query row one sweep over the window's keys with an online maximum: the row
-//                  statistics and dq (as (A - D B)/(l+1e-8) with A = sum e dP k, B = sum e k);
-//                  leaves (m_i, 1/(l_i+1e-8), D_i) per (row, head) for
-//   k_attn_bwd_kv: per key row one sweep over the window's queries -> dk, dv and the bias gradient.
-// No atomics on the row gradients; the bias gradient is accumulated in a shared-memory copy of the
-// table per CTA (when it fits) and flushed with global atomics.
+// A unit of work is (work item of the plan, head): the q, k, v and dO slices of its rows are staged in shared
+// memory as fp32 and the c x c matrices s and dP are formed there once, so that every product of the
+// backward reads shared memory only:
+//   scores    : W x parts threads (W = 32 or 64 rows, the row's keys dealt to the parts): s_ij, dP_ij, and the
+//               part's own maximum, denominator and sum e dP, combined over the parts once
+//   elementwise: P and dS in place; dbias into a shared-memory copy of the head's table column
+//   products  : dq (dS, k), dk (dS^T, q), dv (P^T, dO), 16-byte channel chunks dealt to four quarters of the block
+// All of it is packed fp32 FMAs (fma.rn.f32x2); probabilities and gradients are never rounded to 16 bits.
+//   k_attn_bwd_pack: packs of windows (c <= tile), all of the above in one pass
+//   k_attn_bwd_q   : a tile of query rows of a larger window against all its key tiles with an online maximum:
+//                    dq as (A - D B) / (l + 1e-8) with A = sum e dP k, B = sum e k; leaves
+//                    (m_i, 1 / (l_i + 1e-8), D_i) per (row, head) for
+//   k_attn_bwd_kv  : a tile of key rows of a larger window against all its query tiles: dk, dv, dbias.
+// No atomics on the row gradients; the bias gradient of a block is flushed with global atomics at its end.
+//
+// What bounds it: instruction issue (about 160 fp32 multiply-adds per (query, key, head) in 80 packed ones, and
+// 40 16-byte shared-memory reads that broadcast within a window).  Reading the rows from global memory per
+// (query, key), one thread per row, it was bound by the latency of those reads at a tenth of the issue rate.
+// 150 000 voxels x 3 heads of fp32 (10 voxels a window): 585 -> 310 us; 40 000 x 3 of bf16 (33 to 46 a window, one in
+// five beyond a pack): 483 -> 229 us a block.  Measured on the former: 36 % of the issue slots, eight warps a scheduler
+// pair; the 70 KB of rows and matrices leave room for two blocks per SM.
 //
 // The plan may be stale (the backward runs long after the forward that built it, possibly after
 // the caller rebuilt another plan in the same buffer): item counts, descriptors, voxel ids and
@@ -42,210 +55,505 @@ struct BwdParams {
   const int32_t* pack_meta;
   const float* table;
   int rel_off, H, C, tile;
+  int n_per_window;
   int n_vox, pack_cap;  // bounds the kernels hold the plan's voxel ids and item counts to
   float scale;
   int use_mask;
-  int table_floats;  // > 0: the bias gradient is accumulated in shared memory first
+  int table_rows;
+  int table_smem;  // the head's column of the table and of its gradient fit in shared memory
 };
 
+constexpr int kBwdThreads = 256;
+constexpr int kBwdRows = 64;             // rows of a tile at most
+constexpr int kBwdMat = kBwdRows + 1;    // pitch of the score matrices: odd, so rows and columns are conflict free
+// a staged row: q | k | v | dO, then {relative-position code, region}, 8 B unused: an odd number of 16-byte
+// units, so the same chunk of consecutive rows lies in different banks
+template <int HD>
+constexpr int kBwdPitch = 4 * HD + 4;
+
+template <int HD>
+struct BwdSmem {
+  static constexpr int kRows = 0;
+  static constexpr int kS = kRows + kBwdRows * kBwdPitch<HD>;
+  static constexpr int kDP = kS + kBwdRows * kBwdMat;
+  static constexpr int kRed = kDP + kBwdRows * kBwdMat;       // [3][kBwdThreads]
+  static constexpr int kPlan = kRed + 3 * kBwdThreads;        // [2][2 * kBwdRows] voxel ids and metadata, double buffered
+  static constexpr int kTable = kPlan + 4 * kBwdRows;         // head's bias column, then its gradient
+};
+
+// One 16-byte piece of a 16-bit row -> eight floats in shared memory.
+template <typename T>
+__device__ __forceinline__ void store_wide(float* dst, const uint4& u) {
+  float4 a, b;
+  widen8<T>(u, a, b);
+  reinterpret_cast<float4*>(dst)[0] = a;
+  reinterpret_cast<float4*>(dst)[1] = b;
+}
+
+// Slices [slot0, slot0 + NS) (0 q, 1 k, 2 v, 3 dO) of `n` rows into the staged rows; vox: their voxel ids
+// (shared memory).  fp32 goes by asynchronous copies, 16 bits through registers, four loads in flight.
 template <typename T, int HD>
-__device__ __forceinline__ void load_row(const T* src, float (&x)[HD]) {
+__device__ __forceinline__ void stage_slices(float* rows, const BwdParams& p, int h, const int* vox, int n, int mask) {
+  constexpr int E = 16 / (int)sizeof(T), CH = HD / E;
+  const T* qkv = reinterpret_cast<const T*>(p.qkv);
+  const T* go = reinterpret_cast<const T*>(p.grad_out);
+  const int total = n * 4 * CH;
+  auto source = [&](int idx, int& row, int& slot, int& ch) -> const uint4* {
+    row = idx / (4 * CH);
+    const int rem = idx - row * 4 * CH;
+    slot = rem / CH;
+    ch = rem - slot * CH;
+    const int64_t v = vox[row];
+    const T* src = slot == 3 ? go + v * p.C + h * HD : qkv + (v * 3 + slot) * p.C + h * HD;
+    return reinterpret_cast<const uint4*>(src) + ch;
+  };
   if constexpr (sizeof(T) == 4) {
-#pragma unroll
-    for (int e = 0; e < HD / 4; ++e) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(src) + e);
-      x[4 * e] = v.x; x[4 * e + 1] = v.y; x[4 * e + 2] = v.z; x[4 * e + 3] = v.w;
+    for (int idx = threadIdx.x; idx < total; idx += kBwdThreads) {
+      int row, slot, ch;
+      const uint4* src = source(idx, row, slot, ch);
+      if (mask >> slot & 1) cp_async16(rows + row * kBwdPitch<HD> + slot * HD + ch * E, src);
     }
+    cp_async_commit();
+    cp_async_wait<0>();
   } else {
+    for (int base = threadIdx.x; base < total; base += 4 * kBwdThreads) {
+      uint4 u[4];
+      int off[4];
 #pragma unroll
-    for (int e = 0; e < HD / 8; ++e) {
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(src) + e);
-      float4 a, b;
-      widen8<T>(u, a, b);
-      x[8 * e] = a.x; x[8 * e + 1] = a.y; x[8 * e + 2] = a.z; x[8 * e + 3] = a.w;
-      x[8 * e + 4] = b.x; x[8 * e + 5] = b.y; x[8 * e + 6] = b.z; x[8 * e + 7] = b.w;
+      for (int x = 0; x < 4; ++x) {
+        const int idx = base + x * kBwdThreads;
+        off[x] = -1;
+        if (idx < total) {
+          int row, slot, ch;
+          const uint4* src = source(idx, row, slot, ch);
+          if (mask >> slot & 1) {
+            off[x] = row * kBwdPitch<HD> + slot * HD + ch * E;
+            u[x] = __ldg(src);
+          }
+        }
+      }
+#pragma unroll
+      for (int x = 0; x < 4; ++x)
+        if (off[x] >= 0) store_wide<T>(rows + off[x], u[x]);
     }
   }
 }
 
-template <typename T, int HD>
-__device__ __forceinline__ void store_row(T* dst, const float (&x)[HD], float f) {
-  if constexpr (sizeof(T) == 4) {
-#pragma unroll
-    for (int e = 0; e < HD / 4; ++e)
-      reinterpret_cast<float4*>(dst)[e] = make_float4(x[4 * e] * f, x[4 * e + 1] * f, x[4 * e + 2] * f, x[4 * e + 3] * f);
-  } else {
-#pragma unroll
-    for (int e = 0; e < HD / 8; ++e) {
-      uint4 u;
-      u.x = pack2<T>(x[8 * e] * f, x[8 * e + 1] * f);
-      u.y = pack2<T>(x[8 * e + 2] * f, x[8 * e + 3] * f);
-      u.z = pack2<T>(x[8 * e + 4] * f, x[8 * e + 5] * f);
-      u.w = pack2<T>(x[8 * e + 6] * f, x[8 * e + 7] * f);
-      reinterpret_cast<uint4*>(dst)[e] = u;
-    }
+// Row metadata of the staged rows, from plan metadata words in shared memory.
+template <int HD>
+__device__ __forceinline__ void stage_meta(float* rows, const int* meta, int n) {
+  for (int r = threadIdx.x; r < n; r += kBwdThreads) {
+    const int m = meta[r];
+    *reinterpret_cast<int2*>(rows + r * kBwdPitch<HD> + 4 * HD) = make_int2(meta_rel(m), meta_region(m));
   }
 }
 
 template <int HD>
-__device__ __forceinline__ float dot(const float (&a)[HD], const float (&b)[HD]) {
-  float s0 = 0.f, s1 = 0.f;
+__device__ __forceinline__ void load_regs(const float* src, float2 (&x)[HD / 2]) {
 #pragma unroll
-  for (int e = 0; e < HD; e += 2) {
-    s0 = fmaf(a[e], b[e], s0);
-    s1 = fmaf(a[e + 1], b[e + 1], s1);
+  for (int e = 0; e < HD / 4; ++e) {
+    const float4 v = reinterpret_cast<const float4*>(src)[e];
+    x[2 * e] = make_float2(v.x, v.y);
+    x[2 * e + 1] = make_float2(v.z, v.w);
   }
-  return s0 + s1;
 }
-
-// The rows of work item d this thread's local row t belongs with: its own pack row and the first
-// row and length of its window's run.  False when t is beyond the item.
-__device__ __forceinline__ bool item_row(const int4& d, int tile, int t, int& row, int& first, int& count) {
-  const int c = d.y;
-  if (d.z >= 0) {  // pack of d.z windows with c voxels each
-    if (t >= d.z * c) return false;
-    const int wl = t / c;
-    row = d.x + t;
-    first = d.x + wl * c;
-  } else {  // one tile of rows of a large window
-    const int r0 = (-d.z - 1) * tile;
-    if (r0 + t >= c || t >= tile) return false;
-    row = d.x + r0 + t;
-    first = d.x;
+template <int HD>
+__device__ __forceinline__ float dot_smem(const float2 (&x)[HD / 2], const float* y) {
+  float2 a = make_float2(0.f, 0.f), b = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int e = 0; e < HD / 4; ++e) {
+    const float4 v = reinterpret_cast<const float4*>(y)[e];
+    a = __ffma2_rn(x[2 * e], make_float2(v.x, v.y), a);
+    b = __ffma2_rn(x[2 * e + 1], make_float2(v.z, v.w), b);
   }
-  count = c;
-  return true;
-}
-__device__ __forceinline__ int item_rows(const int4& d, int tile) {
-  if (d.z >= 0) return d.z * d.y;
-  return min(tile, d.y - (-d.z - 1) * tile);
+  return (a.x + b.x) + (a.y + b.y);
 }
 
-// log2-domain score of (query i, key j) from the raw dot product
-__device__ __forceinline__ float score2(float qk, float qs, const float* table, int rel_i_off, int meta_i, int meta_j,
-                                        int H, int h, bool use_mask) {
-  const float b = __ldg(table + (rel_i_off - meta_rel(meta_j)) * H + h);
-  const float madd = (use_mask && meta_region(meta_i) != meta_region(meta_j)) ? -100.0f : 0.f;
-  return fmaf(qk, qs, (b + madd) * kLog2e);
+// acc[k] += sum over x in [0, n) of w[x * w_step] * (chunk c0 + k of row x at `src`)
+template <int NCH>
+__device__ __forceinline__ void weighted_sum(float4 (&acc)[NCH], const float* w, int w_step, const float* src, int pitch, int n) {
+  float2 a[2 * NCH];
+#pragma unroll
+  for (int k = 0; k < NCH; ++k) {
+    a[2 * k] = make_float2(acc[k].x, acc[k].y);
+    a[2 * k + 1] = make_float2(acc[k].z, acc[k].w);
+  }
+#pragma unroll 4
+  for (int x = 0; x < n; ++x) {
+    const float f = w[x * w_step];
+    const float2 f2 = make_float2(f, f);
+    const float4* r = reinterpret_cast<const float4*>(src + x * pitch);
+#pragma unroll
+    for (int k = 0; k < NCH; ++k) {
+      const float4 v = r[k];
+      a[2 * k] = __ffma2_rn(f2, make_float2(v.x, v.y), a[2 * k]);
+      a[2 * k + 1] = __ffma2_rn(f2, make_float2(v.z, v.w), a[2 * k + 1]);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < NCH; ++k) acc[k] = make_float4(a[2 * k].x, a[2 * k].y, a[2 * k + 1].x, a[2 * k + 1].y);
+}
+template <int NCH>
+__device__ __forceinline__ void put_chunks(float* dst, const float4 (&v)[NCH], float f) {
+#pragma unroll
+  for (int k = 0; k < NCH; ++k)
+    reinterpret_cast<float4*>(dst)[k] = make_float4(v[k].x * f, v[k].y * f, v[k].z * f, v[k].w * f);
 }
 
+// Slices of the staged rows out to dqkv: slot s of a row is part s of its q | k | v gradient.
 template <typename T, int HD>
-__global__ void __launch_bounds__(128) k_attn_bwd_q(BwdParams p) {
-  const int H = p.H, C = p.C;
-  const int n_items = checked_count(p.header[SSW_H_PACKS], p);
-  const int n_small = min(checked_count(p.header[SSW_H_PACKS_SMALL], p), n_items);
-  const float qs = p.scale * kLog2e;
-  const T* qkv = reinterpret_cast<const T*>(p.qkv);
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int4 d = checked_desc(__ldg(p.pack_desc + item), p, item < n_small);
-    const int nrows = item_rows(d, p.tile);
-    for (int idx = threadIdx.x; idx < nrows * H; idx += blockDim.x) {
-      const int h = idx / nrows, t = idx - h * nrows;
-      int row, first, c;
-      if (!item_row(d, p.tile, t, row, first, c)) continue;
-      const int vi = checked_voxel(__ldg(p.pack_perm + row), p), mi = checked_meta(__ldg(p.pack_meta + row), p);
-      const int rel_i_off = meta_rel(mi) + p.rel_off;
-      float q[HD], go[HD];
-      load_row<T, HD>(qkv + (int64_t)vi * 3 * C + h * HD, q);
-      load_row<T, HD>(reinterpret_cast<const T*>(p.grad_out) + (int64_t)vi * C + h * HD, go);
-      // One sweep over the window's keys with the running maximum (from 0): denominator l,
-      // dn = sum_j e_ij dP_ij, A = sum_j e_ij dP_ij k_j and B = sum_j e_ij k_j, from which
-      // D = dn / (l + 1e-8) and dq = (A - D B) / (l + 1e-8).
-      float m = 0.f, l = 0.f, dn = 0.f;
-      float dq[HD], kb[HD];
-#pragma unroll
-      for (int e = 0; e < HD; ++e) dq[e] = kb[e] = 0.f;
-      for (int j = 0; j < c; ++j) {
-        const int vj = checked_voxel(__ldg(p.pack_perm + first + j), p);
-        const int mj = checked_meta(__ldg(p.pack_meta + first + j), p);
-        float k[HD], v[HD];
-        load_row<T, HD>(qkv + (int64_t)vj * 3 * C + C + h * HD, k);
-        load_row<T, HD>(qkv + (int64_t)vj * 3 * C + 2 * C + h * HD, v);
-        const float s2 = score2(dot<HD>(q, k), qs, p.table, rel_i_off, mi, mj, H, h, p.use_mask != 0);
-        const float dp = dot<HD>(go, v);
-        if (s2 > m) {
-          const float corr = fast_exp2(m - s2);
-          l *= corr;
-          dn *= corr;
-#pragma unroll
-          for (int e = 0; e < HD; ++e) { dq[e] *= corr; kb[e] *= corr; }
-          m = s2;
-        }
-        const float ex = fast_exp2(s2 - m);
-        const float edp = ex * dp;
-        l += ex;
-        dn += edp;
-#pragma unroll
-        for (int e = 0; e < HD; ++e) {
-          dq[e] = fmaf(edp, k[e], dq[e]);
-          kb[e] = fmaf(ex, k[e], kb[e]);
-        }
-      }
-      const float inv = 1.0f / (l + 1e-8f);
-      const float D = dn * inv;
-      reinterpret_cast<float4*>(p.stats)[(int64_t)row * H + h] = make_float4(m, inv, D, 0.f);
-#pragma unroll
-      for (int e = 0; e < HD; ++e) dq[e] = (dq[e] - D * kb[e]) * inv;
-      store_row<T, HD>(reinterpret_cast<T*>(p.dqkv) + (int64_t)vi * 3 * C + h * HD, dq, p.scale);
+__device__ __forceinline__ void flush_slices(const float* rows, const BwdParams& p, int h, const int* vox, int n, int slot0, int n_slots) {
+  constexpr int E = 16 / (int)sizeof(T), CH = HD / E;
+  for (int idx = threadIdx.x; idx < n * n_slots * CH; idx += kBwdThreads) {
+    const int row = idx / (n_slots * CH), rem = idx - row * n_slots * CH;
+    const int slot = slot0 + rem / CH, ch = rem % CH;
+    const float* src = rows + row * kBwdPitch<HD> + slot * HD + ch * E;
+    T* dst = reinterpret_cast<T*>(p.dqkv) + ((int64_t)vox[row] * 3 + slot) * p.C + h * HD + ch * E;
+    const float4 a = reinterpret_cast<const float4*>(src)[0];
+    if constexpr (sizeof(T) == 4) {
+      *reinterpret_cast<float4*>(dst) = a;
+    } else {
+      const float4 b = reinterpret_cast<const float4*>(src)[1];
+      *reinterpret_cast<uint4*>(dst) = make_uint4(pack2<T>(a.x, a.y), pack2<T>(a.z, a.w), pack2<T>(b.x, b.y), pack2<T>(b.z, b.w));
     }
   }
 }
 
-template <typename T, int HD>
-__global__ void __launch_bounds__(128) k_attn_bwd_kv(BwdParams p) {
-  extern __shared__ float dtab_s[];
-  const int H = p.H, C = p.C;
-  for (int i = threadIdx.x; i < p.table_floats; i += blockDim.x) dtab_s[i] = 0.f;
+// Voxel ids and metadata of `n` plan rows from `row0`, bounds checked, as {ids, metadata} at dst.
+__device__ __forceinline__ void stage_plan(int* dst, const BwdParams& p, int row0, int n) {
+  for (int r = threadIdx.x; r < n; r += kBwdThreads) {
+    dst[r] = checked_voxel(__ldg(p.pack_perm + row0 + r), p);
+    dst[kBwdRows + r] = checked_meta(__ldg(p.pack_meta + row0 + r), p);
+  }
+}
+
+// The head's bias column (pre-multiplied by log2 e) and a cleared gradient column, or pointers to the tables
+// in global memory.
+struct BwdTable {
+  const float* bias;
+  float* grad;
+  int step;
+  float mul;
+};
+__device__ __forceinline__ BwdTable open_table(float* t, const BwdParams& p, int h) {
+  if (!p.table_smem) return BwdTable{p.table + h, p.dtable + h, p.H, kLog2e};
+  for (int i = threadIdx.x; i < p.table_rows; i += kBwdThreads) {
+    t[i] = __ldg(p.table + (int64_t)i * p.H + h) * kLog2e;
+    t[p.table_rows + i] = 0.f;
+  }
+  return BwdTable{t, t + p.table_rows, 1, 1.0f};
+}
+__device__ __forceinline__ void close_table(const BwdTable& t, const BwdParams& p, int h) {
+  if (!p.table_smem) return;
   __syncthreads();
+  for (int i = threadIdx.x; i < p.table_rows; i += kBwdThreads) {
+    const float g = t.grad[i];
+    if (g != 0.f) atomicAdd(p.dtable + (int64_t)i * p.H + h, g);
+  }
+}
+
+// log2-domain score of a (query, key) pair from its raw dot product
+__device__ __forceinline__ float pair_score(float qk, float qs, const BwdTable& t, int rel_i_off, int region_i, int2 mj, bool use_mask) {
+  float s = fmaf(qk, qs, t.bias[(rel_i_off - mj.x) * t.step] * t.mul);
+  if (use_mask && region_i != mj.y) s += -100.0f * kLog2e;
+  return s;
+}
+
+// Scores of query row r (staged, q and dO in registers) against staged key rows [j0, j1) of the window that
+// starts at row `first`: s and dP to the matrices (column = key - col0), returns their maximum.
+template <int HD>
+__device__ __forceinline__ float score_keys(const float* rows, float* S, float* DP, int r, int first, int j0, int j1, const float2 (&q)[HD / 2],
+                                            const float2 (&go)[HD / 2], int2 mi, float qs, int rel_off, const BwdTable& tab, bool use_mask) {
+  float mx = -INFINITY;
+#pragma unroll 2
+  for (int j = j0; j < j1; ++j) {
+    const float* kr = rows + (first + j) * kBwdPitch<HD>;
+    const int2 mj = *reinterpret_cast<const int2*>(kr + 4 * HD);
+    const float s = pair_score(dot_smem<HD>(q, kr + HD), qs, tab, mi.x + rel_off, mi.y, mj, use_mask);
+    S[r * kBwdMat + j] = s;
+    DP[r * kBwdMat + j] = dot_smem<HD>(go, kr + 2 * HD);
+    mx = fmaxf(mx, s);
+  }
+  return mx;
+}
+
+template <typename T, int HD>
+__global__ void __launch_bounds__(kBwdThreads, 2) k_attn_bwd_pack(BwdParams p) {
+  extern __shared__ __align__(16) float sm[];
+  using L = BwdSmem<HD>;
+  float *rows = sm + L::kRows, *S = sm + L::kS, *DP = sm + L::kDP, *red = sm + L::kRed;
+  int* plan = reinterpret_cast<int*>(sm + L::kPlan);
+  grid_dependency_wait();
+  const int n_items = checked_count(p.header[SSW_H_PACKS], p);
+  const int n_small = min(checked_count(p.header[SSW_H_PACKS_SMALL], p), n_items);
+  const int h = (int)blockIdx.x % p.H, g = (int)blockIdx.x / p.H, step = (int)gridDim.x / p.H;
+  if (g >= n_small) return;
+  const BwdTable tab = open_table(sm + L::kTable, p, h);
+  const float qs = p.scale * kLog2e;
+  const bool use_mask = p.use_mask != 0;
+  // the list ascends in occupancy: heavy items first
+  int4 d = checked_desc(__ldg(p.pack_desc + n_small - 1 - g), p, true);
+  stage_plan(plan, p, d.x, d.z * d.y);
+  int4 d_next = make_int4(0, 1, 0, 0);
+  if (g + step < n_small) d_next = checked_desc(__ldg(p.pack_desc + n_small - 1 - (g + step)), p, true);
+  int buf = 0;
+  for (int k = g; k < n_small; k += step, buf ^= 1) {
+    const int* vox = plan + buf * 2 * kBwdRows;
+    const int c = d.y, n = d.z * c;
+    __syncthreads();  // ids and metadata are in shared memory; the rows of the item before have left it
+    stage_slices<T, HD>(rows, p, h, vox, n, 15);
+    stage_meta<HD>(rows, vox + kBwdRows, n);
+    __syncthreads();
+    // ids of the next item and the descriptor of the one after it, while this one is computed
+    if (k + step < n_small) stage_plan(plan + (buf ^ 1) * 2 * kBwdRows, p, d_next.x, d_next.z * d_next.y);
+    int4 d_after = make_int4(0, 1, 0, 0);
+    if (k + 2 * step < n_small) d_after = checked_desc(__ldg(p.pack_desc + n_small - 1 - (k + 2 * step)), p, true);
+    const int W = n <= 32 ? 32 : 64, parts = kBwdThreads / W;
+    const int r = threadIdx.x & (W - 1), part = threadIdx.x / W;
+    const bool on = r < n;
+    const int first = on ? r / c * c : 0;
+    const int per = (c + parts - 1) >> (W == 32 ? 3 : 2), j0 = min(part * per, c), j1 = min(j0 + per, c);
+    float m = 0.f, l = 0.f, dn = 0.f;  // this part's maximum (from 0), denominator, sum of e dP
+    const int2 mi = *reinterpret_cast<const int2*>(rows + (on ? r : 0) * kBwdPitch<HD> + 4 * HD);
+    if (on) {
+      float2 q[HD / 2], go[HD / 2];
+      load_regs<HD>(rows + r * kBwdPitch<HD>, q);
+      load_regs<HD>(rows + r * kBwdPitch<HD> + 3 * HD, go);
+      m = fmaxf(m, score_keys<HD>(rows, S, DP, r, first, j0, j1, q, go, mi, qs, p.rel_off, tab, use_mask));
+      for (int j = j0; j < j1; ++j) {
+        const float e = fast_exp2(S[r * kBwdMat + j] - m);
+        S[r * kBwdMat + j] = e;
+        l += e;
+        dn = fmaf(e, DP[r * kBwdMat + j], dn);
+      }
+    }
+    red[threadIdx.x] = m;
+    red[kBwdThreads + threadIdx.x] = l;
+    red[2 * kBwdThreads + threadIdx.x] = dn;
+    __syncthreads();
+    if (on) {
+      float mt = 0.f, lt = 0.f, dt = 0.f;
+      for (int x = 0; x < parts; ++x) mt = fmaxf(mt, red[x * W + r]);
+      for (int x = 0; x < parts; ++x) {
+        const float f = fast_exp2(red[x * W + r] - mt);
+        lt = fmaf(f, red[kBwdThreads + x * W + r], lt);
+        dt = fmaf(f, red[2 * kBwdThreads + x * W + r], dt);
+      }
+      const float inv = 1.0f / (lt + 1e-8f);
+      const float D = dt * inv, f = fast_exp2(m - mt) * inv;
+      for (int j = j0; j < j1; ++j) {
+        const float pij = S[r * kBwdMat + j] * f;
+        const float ds = pij * (DP[r * kBwdMat + j] - D);
+        S[r * kBwdMat + j] = pij;
+        DP[r * kBwdMat + j] = ds;
+        const int relj = *reinterpret_cast<const int*>(rows + (first + j) * kBwdPitch<HD> + 4 * HD);
+        atomicAdd(tab.grad + (mi.x + p.rel_off - relj) * tab.step, ds);
+      }
+    }
+    __syncthreads();
+    // three products of HD / 4 chunks each, dealt to four quarters (with W = 32 the upper half of the block is idle)
+    constexpr int Q = HD / 4, NA = 3 * Q / 4, NB = Q - NA, NC = Q / 2;
+    const float* ds_row = DP + r * kBwdMat;                          // dS[r][j]
+    const float* ds_col = DP + first * kBwdMat + (r - first);        // dS[first + i][r]
+    const float* p_col = S + first * kBwdMat + (r - first);
+    const float* win = rows + first * kBwdPitch<HD>;
+    float4 big[NA] = {}, half_[NC] = {}, small[NB] = {};
+    const int P = kBwdPitch<HD>;
+    if (on) {
+      if (part == 0) {
+        weighted_sum<NA>(big, ds_row, 1, win + HD, P, c);
+      } else if (part == 1) {
+        weighted_sum<NB>(small, ds_row, 1, win + HD + 4 * NA, P, c);
+        weighted_sum<NC>(half_, ds_col, kBwdMat, win, P, c);
+      } else if (part == 2) {
+        weighted_sum<NC>(half_, ds_col, kBwdMat, win + 4 * NC, P, c);
+        weighted_sum<NB>(small, p_col, kBwdMat, win + 3 * HD, P, c);
+      } else if (part == 3) {
+        weighted_sum<NA>(big, p_col, kBwdMat, win + 3 * HD + 4 * NB, P, c);
+      }
+    }
+    __syncthreads();
+    // results take the place of the rows they were made from: q <- dq, k <- dk, v <- dv
+    if (on) {
+      float* o = rows + r * P;
+      if (part == 0) {
+        put_chunks<NA>(o, big, p.scale);
+      } else if (part == 1) {
+        put_chunks<NB>(o + 4 * NA, small, p.scale);
+        put_chunks<NC>(o + HD, half_, p.scale);
+      } else if (part == 2) {
+        put_chunks<NC>(o + HD + 4 * NC, half_, p.scale);
+        put_chunks<NB>(o + 2 * HD, small, 1.0f);
+      } else if (part == 3) {
+        put_chunks<NA>(o + 2 * HD + 4 * NB, big, 1.0f);
+      }
+    }
+    __syncthreads();
+    flush_slices<T, HD>(rows, p, h, vox, n, 0, 3);
+    d = d_next;
+    d_next = d_after;
+  }
+  close_table(tab, p, h);
+}
+
+// Query tiles of windows beyond a pack.
+template <typename T, int HD>
+__global__ void __launch_bounds__(kBwdThreads, 2) k_attn_bwd_q(BwdParams p) {
+  extern __shared__ __align__(16) float sm[];
+  using L = BwdSmem<HD>;
+  float *rows = sm + L::kRows, *S = sm + L::kS, *DP = sm + L::kDP, *red = sm + L::kRed;
+  int* plan = reinterpret_cast<int*>(sm + L::kPlan);
+  grid_dependency_wait();
+  const int n_items = checked_count(p.header[SSW_H_PACKS], p);
+  const int n_small = min(checked_count(p.header[SSW_H_PACKS_SMALL], p), n_items);
+  const int h = (int)blockIdx.x % p.H, g = (int)blockIdx.x / p.H, step = (int)gridDim.x / p.H;
+  if (g >= n_items - n_small) return;
+  const BwdTable tab = open_table(sm + L::kTable, p, h);
+  const float qs = p.scale * kLog2e;
+  const bool use_mask = p.use_mask != 0;
+  const int P = kBwdPitch<HD>;
+  constexpr int NC = HD / 8;
+  for (int k = g; k < n_items - n_small; k += step) {
+    const int4 d = checked_desc(__ldg(p.pack_desc + n_items - 1 - k), p, false);
+    const int c = d.y, r0 = (-d.z - 1) * p.tile, n = min(p.tile, c - r0);
+    const int r = threadIdx.x & 63, part = threadIdx.x >> 6;
+    const bool on = r < n;
+    __syncthreads();
+    stage_plan(plan, p, d.x + r0, n);
+    __syncthreads();
+    stage_slices<T, HD>(rows, p, h, plan, n, 1 | 8);
+    stage_meta<HD>(rows, plan + kBwdRows, n);
+    __syncthreads();
+    const int2 mi = *reinterpret_cast<const int2*>(rows + (on ? r : 0) * P + 4 * HD);
+    float2 q[HD / 2], go[HD / 2];
+    load_regs<HD>(rows + (on ? r : 0) * P, q);
+    load_regs<HD>(rows + (on ? r : 0) * P + 3 * HD, go);
+    float m = 0.f, l = 0.f, dn = 0.f;  // of the whole row, kept by all its threads
+    float4 acc[NC] = {};               // parts 0, 1: chunks of A; 2, 3: chunks of B
+    for (int k0 = 0; k0 < c; k0 += p.tile) {
+      const int nk = min(p.tile, c - k0);
+      __syncthreads();  // everyone is done with the key tile before
+      stage_plan(plan + 2 * kBwdRows, p, d.x + k0, nk);
+      __syncthreads();
+      stage_slices<T, HD>(rows, p, h, plan + 2 * kBwdRows, nk, 2 | 4);
+      stage_meta<HD>(rows, plan + 3 * kBwdRows, nk);
+      __syncthreads();
+      const int per = (nk + 3) / 4, j0 = min(part * per, nk), j1 = min(j0 + per, nk);
+      float mx = m;
+      if (on) mx = fmaxf(mx, score_keys<HD>(rows, S, DP, r, 0, j0, j1, q, go, mi, qs, p.rel_off, tab, use_mask));
+      red[threadIdx.x] = mx;
+      __syncthreads();
+      const float m_new = fmaxf(fmaxf(red[r], red[64 + r]), fmaxf(red[128 + r], red[192 + r]));
+      const float corr = fast_exp2(m - m_new);
+      float lp = 0.f, dp = 0.f;
+      if (on) {
+        for (int j = j0; j < j1; ++j) {
+          const float e = fast_exp2(S[r * kBwdMat + j] - m_new);
+          const float edp = e * DP[r * kBwdMat + j];
+          S[r * kBwdMat + j] = e;
+          DP[r * kBwdMat + j] = edp;
+          lp += e;
+          dp += edp;
+        }
+      }
+      red[kBwdThreads + threadIdx.x] = lp;
+      red[2 * kBwdThreads + threadIdx.x] = dp;
+      __syncthreads();
+      const float *rl = red + kBwdThreads + r, *rd = red + 2 * kBwdThreads + r;
+      l = fmaf(l, corr, (rl[0] + rl[64]) + (rl[128] + rl[192]));
+      dn = fmaf(dn, corr, (rd[0] + rd[64]) + (rd[128] + rd[192]));
+      m = m_new;
+#pragma unroll
+      for (int x = 0; x < NC; ++x) acc[x] = make_float4(acc[x].x * corr, acc[x].y * corr, acc[x].z * corr, acc[x].w * corr);
+      if (on) weighted_sum<NC>(acc, (part < 2 ? DP : S) + r * kBwdMat, 1, rows + HD + (part & 1) * 4 * NC, P, nk);
+    }
+    const float inv = 1.0f / (l + 1e-8f), D = dn * inv;
+    // dq = (A - D B) / (l + 1e-8): B through the k slot, the result in the q slot
+    __syncthreads();
+    if (on && part >= 2) put_chunks<NC>(rows + r * P + HD + (part & 1) * 4 * NC, acc, D);
+    __syncthreads();
+    if (on && part < 2) {
+      const float* db = rows + r * P + HD + part * 4 * NC;
+#pragma unroll
+      for (int x = 0; x < NC; ++x) {
+        const float4 v = reinterpret_cast<const float4*>(db)[x];
+        acc[x] = make_float4(acc[x].x - v.x, acc[x].y - v.y, acc[x].z - v.z, acc[x].w - v.w);
+      }
+      put_chunks<NC>(rows + r * P + part * 4 * NC, acc, inv * p.scale);
+      if (part == 0) reinterpret_cast<float4*>(p.stats)[(int64_t)(d.x + r0 + r) * p.H + h] = make_float4(m, inv, D, 0.f);
+    }
+    __syncthreads();
+    flush_slices<T, HD>(rows, p, h, plan, n, 0, 1);
+  }
+}
+
+// Key tiles of windows beyond a pack.
+template <typename T, int HD>
+__global__ void __launch_bounds__(kBwdThreads, 2) k_attn_bwd_kv(BwdParams p) {
+  extern __shared__ __align__(16) float sm[];
+  using L = BwdSmem<HD>;
+  float *rows = sm + L::kRows, *S = sm + L::kS, *DP = sm + L::kDP, *red = sm + L::kRed;
+  int* plan = reinterpret_cast<int*>(sm + L::kPlan);
   grid_dependency_wait();  // the row statistics come from the kernel this one is chained behind
   const int n_items = checked_count(p.header[SSW_H_PACKS], p);
   const int n_small = min(checked_count(p.header[SSW_H_PACKS_SMALL], p), n_items);
+  const int h = (int)blockIdx.x % p.H, g = (int)blockIdx.x / p.H, step = (int)gridDim.x / p.H;
+  if (g >= n_items - n_small) return;
+  const BwdTable tab = open_table(sm + L::kTable, p, h);
   const float qs = p.scale * kLog2e;
-  const T* qkv = reinterpret_cast<const T*>(p.qkv);
-  for (int item = blockIdx.x; item < n_items; item += gridDim.x) {
-    const int4 d = checked_desc(__ldg(p.pack_desc + item), p, item < n_small);
-    const int nrows = item_rows(d, p.tile);
-    for (int idx = threadIdx.x; idx < nrows * H; idx += blockDim.x) {
-      const int h = idx / nrows, t = idx - h * nrows;
-      int row, first, c;
-      if (!item_row(d, p.tile, t, row, first, c)) continue;
-      const int vj = checked_voxel(__ldg(p.pack_perm + row), p), mj = checked_meta(__ldg(p.pack_meta + row), p);
-      float k[HD], v[HD], dk[HD], dv[HD];
-      load_row<T, HD>(qkv + (int64_t)vj * 3 * C + C + h * HD, k);
-      load_row<T, HD>(qkv + (int64_t)vj * 3 * C + 2 * C + h * HD, v);
-#pragma unroll
-      for (int e = 0; e < HD; ++e) dk[e] = dv[e] = 0.f;
-      for (int i = 0; i < c; ++i) {
-        const int vi = checked_voxel(__ldg(p.pack_perm + first + i), p);
-        const int mi = checked_meta(__ldg(p.pack_meta + first + i), p);
-        float q[HD], go[HD];
-        load_row<T, HD>(qkv + (int64_t)vi * 3 * C + h * HD, q);
-        load_row<T, HD>(reinterpret_cast<const T*>(p.grad_out) + (int64_t)vi * C + h * HD, go);
-        const float4 st = reinterpret_cast<const float4*>(p.stats)[(int64_t)(first + i) * H + h];
-        const float s2 = score2(dot<HD>(q, k), qs, p.table, meta_rel(mi) + p.rel_off, mi, mj, H, h, p.use_mask != 0);
-        const float pij = fast_exp2(s2 - st.x) * st.y;
-        const float ds = pij * (dot<HD>(go, v) - st.z);
-#pragma unroll
-        for (int e = 0; e < HD; ++e) {
-          dk[e] = fmaf(ds, q[e], dk[e]);
-          dv[e] = fmaf(pij, go[e], dv[e]);
-        }
-        const int ti = (meta_rel(mi) + p.rel_off - meta_rel(mj)) * H + h;
-        if (p.table_floats > 0) atomicAdd(dtab_s + ti, ds);
-        else atomicAdd(p.dtable + ti, ds);
-      }
-      T* dst = reinterpret_cast<T*>(p.dqkv) + (int64_t)vj * 3 * C + h * HD;
-      store_row<T, HD>(dst + C, dk, p.scale);
-      store_row<T, HD>(dst + 2 * C, dv, 1.0f);
-    }
-  }
-  if (p.table_floats > 0) {
+  const bool use_mask = p.use_mask != 0;
+  const int P = kBwdPitch<HD>;
+  constexpr int NC = HD / 8;
+  for (int k = g; k < n_items - n_small; k += step) {
+    const int4 d = checked_desc(__ldg(p.pack_desc + n_items - 1 - k), p, false);
+    const int c = d.y, r0 = (-d.z - 1) * p.tile, n = min(p.tile, c - r0);
+    const int r = threadIdx.x & 63, part = threadIdx.x >> 6;
+    const bool on = r < n;
     __syncthreads();
-    for (int i = threadIdx.x; i < p.table_floats; i += blockDim.x) {
-      const float g = dtab_s[i];
-      if (g != 0.f) atomicAdd(p.dtable + i, g);
+    stage_plan(plan, p, d.x + r0, n);
+    __syncthreads();
+    stage_slices<T, HD>(rows, p, h, plan, n, 2 | 4);
+    stage_meta<HD>(rows, plan + kBwdRows, n);
+    __syncthreads();
+    const int2 mj = *reinterpret_cast<const int2*>(rows + (on ? r : 0) * P + 4 * HD);
+    float2 kr[HD / 2], vr[HD / 2];
+    load_regs<HD>(rows + (on ? r : 0) * P + HD, kr);
+    load_regs<HD>(rows + (on ? r : 0) * P + 2 * HD, vr);
+    float4 acc[NC] = {};  // parts 0, 1: chunks of dk; 2, 3: chunks of dv
+    for (int q0 = 0; q0 < c; q0 += p.tile) {
+      const int nq = min(p.tile, c - q0);
+      __syncthreads();  // everyone is done with the query tile before
+      stage_plan(plan + 2 * kBwdRows, p, d.x + q0, nq);
+      float4* st = reinterpret_cast<float4*>(red);  // [64] row statistics
+      if (threadIdx.x < nq) st[threadIdx.x] = reinterpret_cast<const float4*>(p.stats)[(int64_t)(d.x + q0 + threadIdx.x) * p.H + h];
+      __syncthreads();
+      stage_slices<T, HD>(rows, p, h, plan + 2 * kBwdRows, nq, 1 | 8);
+      stage_meta<HD>(rows, plan + 3 * kBwdRows, nq);
+      __syncthreads();
+      const int per = (nq + 3) / 4, i0 = min(part * per, nq), i1 = min(i0 + per, nq);
+      if (on) {
+#pragma unroll 2
+        for (int i = i0; i < i1; ++i) {
+          const float* qr = rows + i * P;
+          const int2 mi = *reinterpret_cast<const int2*>(qr + 4 * HD);
+          const float4 t = st[i];
+          const float s = pair_score(dot_smem<HD>(kr, qr), qs, tab, mi.x + p.rel_off, mi.y, mj, use_mask);
+          const float pij = fast_exp2(s - t.x) * t.y;
+          const float ds = pij * (dot_smem<HD>(vr, qr + 3 * HD) - t.z);
+          S[i * kBwdMat + r] = pij;
+          DP[i * kBwdMat + r] = ds;
+          atomicAdd(tab.grad + (mi.x + p.rel_off - mj.x) * tab.step, ds);
+        }
+      }
+      __syncthreads();
+      if (on) weighted_sum<NC>(acc, (part < 2 ? DP : S) + r, kBwdMat, rows + (part < 2 ? 0 : 3 * HD) + (part & 1) * 4 * NC, P, nq);
     }
+    __syncthreads();
+    if (on) put_chunks<NC>(rows + r * P + (part < 2 ? HD : 2 * HD) + (part & 1) * 4 * NC, acc, part < 2 ? p.scale : 1.0f);
+    __syncthreads();
+    flush_slices<T, HD>(rows, p, h, plan, n, 1, 2);
   }
+  close_table(tab, p, h);
 }
 
 template <typename T, int HD>
@@ -253,12 +561,14 @@ static int launch_bwd(const BwdParams& p, cudaStream_t stream) {
   int dev = 0, sms = 0;
   SSW_CUDA_TRY(cudaGetDevice(&dev));
   SSW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const size_t smem = (size_t)p.table_floats * 4;
-  auto kkv = k_attn_bwd_kv<T, HD>;
-  if (smem > 48 * 1024) SSW_CUDA_TRY(cudaFuncSetAttribute(kkv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  k_attn_bwd_q<T, HD><<<sms * 8, 128, 0, stream>>>(p);
-  SSW_LAUNCH_CHECK("k_attn_bwd_q");
-  SSW_CUDA_TRY(launch_chained(kkv, dim3(sms * 8), dim3(128), smem, stream, p));
+  const size_t smem = sizeof(float) * ((size_t)BwdSmem<HD>::kTable + (p.table_smem ? 2 * (size_t)p.table_rows : 0));
+  void (*kerns[3])(BwdParams) = {k_attn_bwd_pack<T, HD>, k_attn_bwd_q<T, HD>, k_attn_bwd_kv<T, HD>};
+  // two blocks per SM, every block on one head throughout (it keeps that head's table column)
+  const unsigned grid = (unsigned)(p.H * (2 * sms > p.H ? 2 * sms / p.H : 1));
+  for (int k = 0; k < (p.n_per_window > p.tile ? 3 : 1); ++k) {
+    SSW_CUDA_TRY(cudaFuncSetAttribute(kerns[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SSW_CUDA_TRY(launch_chained(kerns[k], dim3(grid), dim3(kBwdThreads), smem, stream, p));
+  }
   return SSW_OK;
 }
 
@@ -301,8 +611,11 @@ extern "C" int ssw_attn_fused_bwd(const void* qkv, const void* grad_out, int dty
   p.tile = L->tile_rows;
   p.scale = scale;
   p.use_mask = use_mask;
-  const int64_t tf = (int64_t)(2 * rpb_window[0] - 1) * (2 * rpb_window[1] - 1) * (2 * rpb_window[2] - 1) * heads;
-  p.table_floats = tf * 4 <= 96 * 1024 ? (int)tf : 0;
+  p.n_per_window = L->n_per_window;
+  p.table_rows = (2 * rpb_window[0] - 1) * (2 * rpb_window[1] - 1) * (2 * rpb_window[2] - 1);
+  // two blocks per SM with both columns: 113 KB a block, 70 of them rows and matrices
+  p.table_smem = p.table_rows <= 5000;
+  if (p.tile > kBwdRows) return SSW_E_INVALID;
   cudaStream_t stream = (cudaStream_t)stream_;
   if (dtype == SSW_F32) {
     if (head_dim == 16) return launch_bwd<float, 16>(p, stream);
