@@ -233,6 +233,9 @@ int ssw_peer_buffer_open(const unsigned char* handle, void** ptr);
 int ssw_peer_buffer_close(void* ptr);
 int ssw_peer_buffer_destroy(void* ptr);
 
+/* Waits for `stream` and reads a plan's error word (SSW_DEV_* bits, header entry SSW_H_ERROR).  Not under capture. */
+int ssw_plan_error_word(const int32_t* plan_header, int32_t* error, void* stream);
+
 /* The element-wise shell of a Swin block between its GEMMs (swin3d_base.py:741-782: norm1, the
  * residual add after attention, norm2, the residual add after the MLP) in one pass over the voxel
  * rows: sum = a + b (b may be NULL: sum = a), norm = LayerNorm(sum) * gamma + beta over the

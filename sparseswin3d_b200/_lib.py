@@ -60,6 +60,7 @@ def _load() -> C.CDLL:
         "ssw_bucket_windows": (C.c_int, [vp, P(Geometry), vp, vp, i32, P(i32), P(PlanLayout), vp, vp, vp]),
         "ssw_bucket_windows_static_capacity": (i64, []),
         "ssw_bucket_windows_static": (C.c_int, [vp, P(Geometry), vp, vp, i32, P(i32), P(PlanLayout), vp, vp]),
+        "ssw_plan_error_word": (C.c_int, [vp, P(i32), vp]),
         "ssw_attn_fused": (C.c_int, [vp, C.c_int, i32, i32, P(PlanLayout), vp, vp, P(i32), f32, C.c_int, vp, vp, vp]),
         "ssw_attn_fused_multi": (C.c_int, [vp, C.c_int, i32, i32, P(PlanLayout), vp, vp, P(i32), f32, C.c_int, P(vp), i32, vp, vp]),
         "ssw_voxel_grid_build": (C.c_int, [vp, i64, i32, P(i32), vp, vp, vp]),
@@ -144,9 +145,11 @@ def ptr(t) -> int:
 
 
 def stream_ptr(device=None) -> int:
+    """Handle of the device's current stream (without building a torch.cuda.Stream: 9 us a call, ten calls a block)."""
     import torch
 
-    return torch.cuda.current_stream(device).cuda_stream
+    index = None if device is None else device.index
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def graph_edges(graph) -> dict:

@@ -2,6 +2,7 @@
 (sparse_swin/swin3d_base.py:589-677)."""
 from __future__ import annotations
 
+import functools
 from typing import Optional, Sequence
 
 import torch
@@ -61,8 +62,12 @@ class FusedWindowAttention(torch.autograd.Function):
 
 def default_tile_rows(num_heads: int, head_dim: int, dtype: torch.dtype, rpb_window: Sequence[int] = (7, 7, 7)) -> int:
     """Rows per work item the fused kernel wants for this configuration (pass it to bucket_windows)."""
-    rw = (_lib.i32 * 3)(*[int(x) for x in rpb_window])
-    return int(lib.ssw_default_tile_rows(num_heads, head_dim, dtype_code(dtype), rw))
+    return _default_tile_rows(num_heads, head_dim, dtype_code(dtype), tuple(int(x) for x in rpb_window))
+
+
+@functools.lru_cache(maxsize=1024)
+def _default_tile_rows(num_heads: int, head_dim: int, code: int, rpb_window: tuple) -> int:
+    return int(lib.ssw_default_tile_rows(num_heads, head_dim, code, (_lib.i32 * 3)(*rpb_window)))
 
 
 def window_attention_fused(qkv: torch.Tensor, plan: WindowPlan, table: torch.Tensor, scale: float,

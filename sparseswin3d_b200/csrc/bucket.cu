@@ -551,6 +551,14 @@ extern "C" int ssw_bucket_windows_range(const int32_t* coords, const ssw_geometr
   return SSW_OK;
 }
 
+extern "C" int ssw_plan_error_word(const int32_t* plan_header, int32_t* error, void* stream_) {
+  if (!plan_header || !error) return SSW_E_INVALID;
+  cudaStream_t stream = (cudaStream_t)stream_;
+  SSW_CUDA_TRY(cudaMemcpyAsync(error, plan_header + SSW_H_ERROR, sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+  SSW_CUDA_TRY(cudaStreamSynchronize(stream));
+  return SSW_OK;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Bucketing without a caller-provided scratch buffer
 // ---------------------------------------------------------------------------------------------

@@ -46,10 +46,10 @@ def plain_norm(norm, x: torch.Tensor) -> bool:
 
 def norm_params(norm: nn.LayerNorm):
     """(weight, bias, dtype code) as the kernels read them: in place where the module's type allows."""
-    w, b = norm.weight.detach(), norm.bias.detach()
-    if w.dtype != b.dtype or w.dtype not in _DTYPES:
-        w, b = w.float(), b.float()
-    return w.contiguous(), b.contiguous(), dtype_code(w.dtype)
+    w, b = norm.weight, norm.bias
+    if w.dtype != b.dtype or w.dtype not in _DTYPES or not (w.is_contiguous() and b.is_contiguous()):
+        w, b = w.detach().float().contiguous(), b.detach().float().contiguous()
+    return w, b, dtype_code(w.dtype)
 
 
 class _AddLayerNorm(torch.autograd.Function):

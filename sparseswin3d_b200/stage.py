@@ -20,6 +20,7 @@ forward and backward, and the rest of the shell is torch operations."""
 from __future__ import annotations
 
 import copy
+import functools
 from typing import Optional, Sequence
 
 import torch
@@ -30,6 +31,11 @@ from . import _lib, rows
 from ._lib import check, dtype_code, lib, ptr, stream_ptr
 from .attention import WindowAttentionSparse, plan_params
 from .window import WindowPlan, bucket_windows, resolve_geometry
+
+
+@functools.lru_cache(maxsize=1024)
+def _shifted(batch: int, dims: tuple, window: tuple, shift: tuple) -> bool:
+    return bool(resolve_geometry(batch, dims, window, shift).shifted)
 
 
 class SparseVoxels:
@@ -133,6 +139,9 @@ class SwinTransformerBlock(nn.Module):
     def geometry(self, x):
         return resolve_geometry(int(x.batch_size), tuple(int(v) for v in x.spatial_shape), self.window_size, self.shift_size)
 
+    def shifted(self, x) -> bool:
+        return _shifted(int(x.batch_size), tuple(int(v) for v in x.spatial_shape), self.window_size, self.shift_size)
+
     def build_plan(self, x, dtype: torch.dtype, scratch=None, plan_buffer=None) -> WindowPlan:
         """Pad, cyclic shift, partition and sort (swin3d_base.py:744-761) as one bucketing call."""
         return bucket_windows(coords=x.indices, geom=self.geometry(x), scratch=scratch, plan_buffer=plan_buffer,
@@ -156,11 +165,10 @@ class SwinTransformerBlock(nn.Module):
         accepted for signature compatibility: region ids come from the geometry in closed form, and
         the mask applies exactly when the resolved shift is non-zero (swin3d_base.py:755-760)."""
         feats = x.features
-        geom = self.geometry(x)
         if plan is None:
             with torch.no_grad():
                 plan = self.build_plan(x, feats.dtype)
-        use_mask = bool(geom.shifted)
+        use_mask = self.shifted(x)
         if fuse_shell and self.fusable(feats):
             _, h = add_layernorm(feats, None, self.norm1)
             a = self.attention_branch(h, plan, use_mask)
@@ -250,7 +258,7 @@ class BasicLayer(nn.Module):
             # running features `cur`, pending branch output `pend` (added by the next one-pass call)
             cur, pend = feats, None
             for i, blk in enumerate(self.blocks):
-                use_mask = bool(blk.geometry(x).shifted)
+                use_mask = blk.shifted(x)
                 cur, h = add_layernorm(cur, pend, blk.norm1)           # ends block i-1, opens block i
                 a = blk.attention_branch(h, plans[i % 2], use_mask)
                 cur, h2 = add_layernorm(cur, a, blk.norm2)

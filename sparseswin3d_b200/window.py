@@ -106,7 +106,11 @@ class WindowPlan:
     def raise_on_error(self):
         """Synchronises.  Upstream silently mis-computes on duplicate or out-of-range voxels;
         this raises instead."""
-        e = int(self.header[_lib.H_ERROR])
+        word = _lib.i32()
+        with torch.cuda.device(self.plan.device):  # the default stream's handle is the current device's
+            check(lib.ssw_plan_error_word(ptr(self.plan) + 4 * self.layout.off_header, word, stream_ptr(self.plan.device)),
+                  "ssw_plan_error_word")
+        e = word.value
         if e & _lib.DEV_BAD_COORD:
             raise _lib.SswError("a voxel lies outside the grid / window table")
         if e & _lib.DEV_DUPLICATE:
