@@ -37,10 +37,10 @@ UNIT = "voxels/s"
 N_VOX = 150_000
 HEADS, HEAD_DIM, WINDOW, SHIFT = 3, 32, (7, 7, 7), (3, 3, 3)
 C = HEADS * HEAD_DIM
-# kernels of this library per pass: k_count, k_reduce, k_compact, k_order, k_scatter, then k_attn_fused
+# kernels of this library per pass: k_clear, k_count, k_compact, k_scatter, then k_attn_fused
 # (fp32) or k_attn_mma followed by k_attn_dense (bf16; the latter finds no window beyond a pack on the
 # room and returns at once)
-KERNELS_PER_PASS = {"f32": 6, "bf16": 7}
+KERNELS_PER_PASS = {"f32": 5, "bf16": 6}
 DOMINANT_KERNEL = {"f32": "k_attn_fused", "bf16": "k_attn_mma"}
 # DRAM bytes one launch of the dominant kernel moves on this workload (dram__bytes_read.sum +
 # dram__bytes_write.sum of the ncu captures summarised under profiles/).  Part of the output is still

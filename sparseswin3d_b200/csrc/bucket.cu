@@ -4,14 +4,19 @@
 // a device value.
 //
 // Pipeline (all on the caller's stream):
-//   zero scratch + header + bin tables
+//   k_clear    : header, bin tables, counters, bitmaps and block states to zero
 //   k_count    : per voxel, count[w]++ and set bit `pos` of window w's occupancy bitmap
-//   k_reduce   : per 2048-window block, totals of (non-empty, c, c^2); last block scans them
-//   k_compact  : exclusive scan -> compact window list, row starts, c^2 starts, histogram of c;
-//                last block turns the histogram into per-occupancy starts and the item count
-//   k_order    : window -> slot inside its occupancy bin; work-item descriptors
-//   k_scatter  : per voxel, rank inside its window = popcount of lower bitmap bits -> perm,
-//                inverse perm, pack-order perm and per-row metadata
+//   k_compact  : exclusive scan of the dense window array -> compact window list, row starts, c^2 starts;
+//                histogram of c, and every window's slot within its occupancy bin.  One pass: a block
+//                publishes its sums and adds up those of the blocks before it
+//   k_scatter  : every block turns the histogram into per-occupancy starts for itself; then per voxel, rank
+//                inside its window = popcount of lower bitmap bits -> perm, inverse perm, pack-order perm and
+//                per-row metadata; per window, its first row in pack order; per work item, its descriptor
+//
+// What bounds a build is the length of this chain, not its 9 MB of traffic at 150 000 voxels: each launch is
+// 2 to 9 us of latency.  With the block sums, the starts of the bins and the two clears as launches or serial
+// tails of their own it was seven launches and 33 us; these four, each resident before the one
+// before it has drained, take 20.
 #include <stdio.h>
 
 #include "ssw_common.cuh"
@@ -78,6 +83,7 @@ __global__ void k_window_keys(KeySrc s, int64_t n, int32_t* __restrict__ indices
 __global__ void k_count(KeySrc s, int64_t n, int words, int32_t* __restrict__ count, uint32_t* __restrict__ bitmap,
                         int32_t* __restrict__ header) {
   grid_dependency_wait();
+  grid_launch_dependents();
   int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= n) return;
   int w, pos, r;
@@ -95,9 +101,10 @@ __global__ void k_count(KeySrc s, int64_t n, int words, int32_t* __restrict__ co
   atomicAdd(count + w, 1);
 }
 
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
+constexpr int kScanThreads = 512;
+constexpr int kScanItems = 4;
 constexpr int kScanBlock = kScanThreads * kScanItems;
+constexpr int kFillThreads = 256;
 
 struct Tri {
   int flags;
@@ -106,10 +113,10 @@ struct Tri {
 };
 __device__ __forceinline__ Tri tri_add(Tri a, Tri b) { return Tri{a.flags + b.flags, a.rows + b.rows, a.sq + b.sq}; }
 
-// Block-wide exclusive scan of one Tri per thread (256 threads); returns the exclusive prefix,
-// `total` gets the block total.
+// Block-wide exclusive scan of one Tri per thread; returns the exclusive prefix, `total` gets the block total.
+template <int THREADS>
 __device__ Tri block_excl_scan(Tri v, Tri& total) {
-  __shared__ Tri warp_tot[kScanThreads / 32];
+  __shared__ Tri warp_tot[THREADS / 32];
   int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   Tri inc = v;
 #pragma unroll
@@ -124,7 +131,7 @@ __device__ Tri block_excl_scan(Tri v, Tri& total) {
   Tri base{0, 0, 0ull};
   Tri tot{0, 0, 0ull};
 #pragma unroll
-  for (int i = 0; i < kScanThreads / 32; ++i) {
+  for (int i = 0; i < THREADS / 32; ++i) {
     if (i < wid) base = tri_add(base, warp_tot[i]);
     tot = tri_add(tot, warp_tot[i]);
   }
@@ -133,74 +140,43 @@ __device__ Tri block_excl_scan(Tri v, Tri& total) {
   return Tri{base.flags + inc.flags - v.flags, base.rows + inc.rows - v.rows, base.sq + inc.sq - v.sq};
 }
 
-// partials: 4 ints per block {flags, rows, sq_lo, sq_hi}; after the last block's pass they hold
-// the exclusive prefix over blocks.
-__global__ void __launch_bounds__(kScanThreads) k_reduce(const int32_t* __restrict__ count, int n_windows,
-                                                         int32_t* __restrict__ partials, int32_t* __restrict__ header,
-                                                         int n_blocks) {
-  grid_dependency_wait();
-  int base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
-  Tri t{0, 0, 0ull};
-#pragma unroll
-  for (int i = 0; i < kScanItems; ++i) {
-    int w = base + i;
-    int c = w < n_windows ? count[w] : 0;
-    t.flags += c > 0;
-    t.rows += c;
-    t.sq += (unsigned long long)c * (unsigned long long)c;
-  }
-  Tri tot;
-  block_excl_scan(t, tot);
-  __shared__ bool last;
-  if (threadIdx.x == 0) {
-    int4 p = make_int4(tot.flags, tot.rows, (int)(tot.sq & 0xffffffffull), (int)(tot.sq >> 32));
-    reinterpret_cast<int4*>(partials)[blockIdx.x] = p;
-    __threadfence();
-    int ticket = atomicAdd(header + SSW_H_TICKET_A, 1);
-    last = ticket == n_blocks - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // exclusive scan of the block totals, 256 at a time with a running carry
-  Tri carry{0, 0, 0ull};
-  for (int b0 = 0; b0 < n_blocks; b0 += kScanThreads) {
-    int b = b0 + threadIdx.x;
-    Tri v{0, 0, 0ull};
-    if (b < n_blocks) {
-      int4 p = __ldcg(reinterpret_cast<const int4*>(partials) + b);
-      v = Tri{p.x, p.y, ((unsigned long long)(unsigned)p.w << 32) | (unsigned)p.z};
-    }
-    Tri tot2;
-    Tri ex = block_excl_scan(v, tot2);
-    ex = tri_add(ex, carry);
-    if (b < n_blocks) {
-      reinterpret_cast<int4*>(partials)[b] =
-          make_int4(ex.flags, ex.rows, (int)(ex.sq & 0xffffffffull), (int)(ex.sq >> 32));
-    }
-    carry = tri_add(carry, tot2);
-  }
-  if (threadIdx.x == 0) {
-    header[SSW_H_W] = carry.flags;
-    header[SSW_H_N] = carry.rows;
-    header[SSW_H_SUMC2_LO] = (int)(carry.sq & 0xffffffffull);
-    header[SSW_H_SUMC2_HI] = (int)(carry.sq >> 32);
-  }
+__global__ void __launch_bounds__(256) k_clear(int4* __restrict__ a, int64_t na, int4* __restrict__ b, int64_t nb) {
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < na + nb; i += step)
+    (i < na ? a + i : b + (i - na))[0] = make_int4(0, 0, 0, 0);
 }
 
+// A block's sums as two 64-bit words, each readable on its own: bit 62 says that the word has been written.
+// flags and rows take 31 bits each; the sum of c^2 stays below 2^31 * 1023.
+constexpr unsigned long long kPublished = 1ull << 62;
+constexpr uint32_t kPollLimit = 1u << 22;
+__device__ __forceinline__ unsigned long long poll_word(const unsigned long long* p, bool& ok) {
+  unsigned long long v = __ldcg(p);
+  for (uint32_t i = 0; !(v & kPublished); v = *reinterpret_cast<const volatile unsigned long long*>(p))
+    if (++i > kPollLimit) {
+      ok = false;
+      return 0;
+    }
+  return v & ~kPublished;
+}
+
+// Blocks number themselves by a ticket, so a block only ever waits for blocks that are already running, and
+// every block publishes its own sums before it waits: the waits end.
 __global__ void __launch_bounds__(kScanThreads) k_compact(int32_t* __restrict__ count, int n_windows,
-                                                          const int32_t* __restrict__ partials,
-                                                          int32_t* __restrict__ header, int32_t* __restrict__ win_id,
-                                                          int32_t* __restrict__ win_start,
-                                                          int32_t* __restrict__ coo_start, int32_t* __restrict__ bins_base,
-                                                          int n_per_window, int tile, int padded, int n_blocks,
-                                                          int pack_cap) {
+                                                          unsigned long long* state, int32_t* __restrict__ header,
+                                                          int32_t* __restrict__ win_id, int32_t* __restrict__ win_start,
+                                                          int32_t* __restrict__ coo_start, int32_t* __restrict__ win_pstart,
+                                                          int32_t* __restrict__ bins_base, int n_per_window, int n_blocks) {
   extern __shared__ int32_t hist[];  // n_per_window + 2
+  __shared__ int ticket;
   BinTables bins(bins_base, n_per_window);
   for (int i = threadIdx.x; i < n_per_window + 2; i += blockDim.x) hist[i] = 0;
   grid_dependency_wait();
+  grid_launch_dependents();
+  if (threadIdx.x == 0) ticket = atomicAdd(header + SSW_H_TICKET_A, 1);
   __syncthreads();
-  int base = blockIdx.x * kScanBlock + threadIdx.x * kScanItems;
+  const int block = ticket;
+  const int base = block * kScanBlock + threadIdx.x * kScanItems;
   int c[kScanItems];
   Tri t{0, 0, 0ull};
 #pragma unroll
@@ -212,10 +188,37 @@ __global__ void __launch_bounds__(kScanThreads) k_compact(int32_t* __restrict__ 
     t.sq += (unsigned long long)c[i] * (unsigned long long)c[i];
   }
   Tri tot;
-  Tri ex = block_excl_scan(t, tot);
-  int4 p = __ldcg(reinterpret_cast<const int4*>(partials) + blockIdx.x);
-  ex = tri_add(ex, Tri{p.x, p.y, ((unsigned long long)(unsigned)p.w << 32) | (unsigned)p.z});
-  int cmax = 0;
+  Tri ex = block_excl_scan<kScanThreads>(t, tot);
+  if (threadIdx.x == 0) {
+    volatile unsigned long long* st = state + 2 * block;
+    st[0] = (unsigned long long)tot.flags | ((unsigned long long)tot.rows << 31) | kPublished;
+    st[1] = tot.sq | kPublished;
+  }
+  // ranks of this block's windows within their occupancies, while the sums travel
+  int rank[kScanItems], cmax = 0;
+#pragma unroll
+  for (int i = 0; i < kScanItems; ++i) {
+    rank[i] = 0;
+    if (c[i] > 0) rank[i] = atomicAdd(&hist[c[i] <= n_per_window ? c[i] : n_per_window + 1], 1);
+    cmax = max(cmax, c[i]);
+  }
+  cmax = __reduce_max_sync(0xffffffffu, cmax);
+  if ((threadIdx.x & 31) == 0 && cmax > 0) atomicMax(header + SSW_H_CMAX, cmax);
+  // the blocks before this one
+  Tri before{0, 0, 0ull};
+  bool ok = true;
+  for (int b = threadIdx.x; b < block; b += kScanThreads) {
+    const unsigned long long w0 = poll_word(state + 2 * b, ok), w1 = poll_word(state + 2 * b + 1, ok);
+    before = tri_add(before, Tri{(int)(w0 & 0x7fffffffull), (int)(w0 >> 31), w1});
+  }
+  if (!ok) atomicOr(reinterpret_cast<unsigned*>(header + SSW_H_ERROR), SSW_DEV_TIMEOUT);
+  Tri prefix;
+  block_excl_scan<kScanThreads>(before, prefix);
+  ex = tri_add(ex, prefix);
+  // the histogram entry becomes the first slot of this block's windows in the bin
+  for (int i = threadIdx.x; i < n_per_window + 2; i += blockDim.x)
+    if (hist[i]) hist[i] = atomicAdd(bins.cnt + i, hist[i]);
+  __syncthreads();
 #pragma unroll
   for (int i = 0; i < kScanItems; ++i) {
     int w = base + i;
@@ -224,9 +227,9 @@ __global__ void __launch_bounds__(kScanThreads) k_compact(int32_t* __restrict__ 
         win_id[ex.flags] = w;
         win_start[ex.flags] = ex.rows;
         coo_start[ex.flags] = (int)ex.sq;
+        // complement of the slot: k_scatter tells it from the row it replaces it with by its sign
+        win_pstart[ex.flags] = ~(hist[c[i] <= n_per_window ? c[i] : n_per_window + 1] + rank[i]);
         count[w] = ex.flags;
-        atomicAdd(&hist[c[i] <= n_per_window ? c[i] : n_per_window + 1], 1);
-        cmax = max(cmax, c[i]);
         ex.flags += 1;
         ex.rows += c[i];
         ex.sq += (unsigned long long)c[i] * (unsigned long long)c[i];
@@ -235,133 +238,144 @@ __global__ void __launch_bounds__(kScanThreads) k_compact(int32_t* __restrict__ 
       }
     }
   }
-  cmax = max(cmax, __shfl_xor_sync(0xffffffffu, cmax, 16));
-  cmax = max(cmax, __shfl_xor_sync(0xffffffffu, cmax, 8));
-  cmax = max(cmax, __shfl_xor_sync(0xffffffffu, cmax, 4));
-  cmax = max(cmax, __shfl_xor_sync(0xffffffffu, cmax, 2));
-  cmax = max(cmax, __shfl_xor_sync(0xffffffffu, cmax, 1));
-  if ((threadIdx.x & 31) == 0 && cmax > 0) atomicMax(header + SSW_H_CMAX, cmax);
-  __syncthreads();
-  for (int i = threadIdx.x; i < n_per_window + 2; i += blockDim.x)
-    if (hist[i]) atomicAdd(bins.cnt + i, hist[i]);
-  __shared__ bool last;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    __threadfence();
-    int ticket = atomicAdd(header + SSW_H_TICKET_B, 1);
-    last = ticket == n_blocks - 1;
-  }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // Per-occupancy starts: exclusive scans over c = 0..n_per_window of (windows, rows, items).
-  int W = __ldcg(header + SSW_H_W);
-  int N = __ldcg(header + SSW_H_N);
-  unsigned long long sq = ((unsigned long long)(unsigned)__ldcg(header + SSW_H_SUMC2_HI) << 32) |
-                          (unsigned)__ldcg(header + SSW_H_SUMC2_LO);
-  Tri carry{0, 0, 0ull};  // flags = windows, rows = rows, sq = work items
-  for (int c0 = 0; c0 < n_per_window + 2; c0 += kScanThreads) {
-    int cc = c0 + threadIdx.x;
-    int cnt = cc < n_per_window + 2 ? __ldcg(bins.cnt + cc) : 0;
-    Tri v{cnt, cnt * cc, (unsigned long long)packs_of_bin(cc, cnt, tile, padded)};
-    Tri tot2;
-    Tri e2 = block_excl_scan(v, tot2);
-    e2 = tri_add(e2, carry);
-    if (cc < n_per_window + 2) {
-      bins.wstart[cc] = e2.flags;
-      bins.rowstart[cc] = e2.rows;
-      bins.packstart[cc] = (int)e2.sq;
-      bins.fill[cc] = 0;
-      if (cc == tile + 1) header[SSW_H_PACKS_SMALL] = (int)e2.sq;
-    }
-    carry = tri_add(carry, tot2);
-  }
-  __syncthreads();  // PACKS_SMALL (written by whichever thread owns c = tile + 1) before thread 0 may clear it
-  if (threadIdx.x == 0) {
-    win_start[W] = N;
-    coo_start[W] = (int)sq;
-    // The descriptor array holds pack_cap items (an upper bound for every occupancy histogram the
-    // layout call could foresee).  Should a count ever exceed it, the plan is declared empty and
-    // flagged rather than written past its end.
-    const bool fits = carry.sq <= (unsigned long long)pack_cap;
-    if (!fits) atomicOr(reinterpret_cast<unsigned*>(header + SSW_H_ERROR), SSW_DEV_BAD_PLAN);
-    header[SSW_H_PACKS] = fits ? (int)carry.sq : 0;
-    if (!fits) header[SSW_H_PACKS_SMALL] = 0;
-    else if (tile + 1 > n_per_window + 1) header[SSW_H_PACKS_SMALL] = (int)carry.sq;
-    header[SSW_H_TILE] = tile;
-    header[SSW_H_PADDED] = padded;
-    if (sq >= (1ull << 31)) atomicOr(reinterpret_cast<unsigned*>(header + SSW_H_ERROR), SSW_DEV_COO_RANGE);
+  if (block == n_blocks - 1 && threadIdx.x == 0) {
+    const Tri all = tri_add(prefix, tot);
+    header[SSW_H_W] = all.flags;
+    header[SSW_H_N] = all.rows;
+    header[SSW_H_SUMC2_LO] = (int)(all.sq & 0xffffffffull);
+    header[SSW_H_SUMC2_HI] = (int)(all.sq >> 32);
+    win_start[all.flags] = all.rows;
+    coo_start[all.flags] = (int)all.sq;
+    if (all.sq >= (1ull << 31)) atomicOr(reinterpret_cast<unsigned*>(header + SSW_H_ERROR), SSW_DEV_COO_RANGE);
   }
 }
 
-// Blocks [0, w_blocks): one thread per non-empty window, claims a slot in its occupancy bin.
-// Blocks [w_blocks, ...): one thread per work item, locates its bin and writes the descriptor.
-__global__ void k_order(const int32_t* __restrict__ header, const int32_t* __restrict__ win_start,
-                        int32_t* __restrict__ win_pstart, int32_t* __restrict__ pack_win,
-                        int32_t* __restrict__ pack_desc, int32_t* __restrict__ bins_base, int n_per_window, int tile,
-                        int padded, int w_blocks, int pack_cap) {
-  BinTables bins(bins_base, n_per_window);
-  grid_dependency_wait();
-  if ((int)blockIdx.x < w_blocks) {
-    int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= header[SSW_H_W]) return;
-    int c = win_start[k + 1] - win_start[k];
-    int slot = atomicAdd(bins.fill + c, 1);
-    win_pstart[k] = bins.rowstart[c] + slot * c;
-    pack_win[bins.wstart[c] + slot] = k;
-    return;
-  }
-  int p = (blockIdx.x - w_blocks) * blockDim.x + threadIdx.x;
-  if (p >= header[SSW_H_PACKS] || p >= pack_cap) return;
-  // largest c with packstart[c] <= p and a non-empty bin: binary search on the monotone table
-  int lo = 1, hi = n_per_window;
-  while (lo < hi) {
-    int mid = (lo + hi + 1) >> 1;
-    if (bins.packstart[mid] <= p) lo = mid; else hi = mid - 1;
-  }
-  int c = lo;
-  int q = p - bins.packstart[c];
-  int cnt = bins.cnt[c];
-  int4 d;
-  if (c <= tile) {
-    int wpp = windows_per_pack(c, tile, padded);
-    int first = q * wpp;
-    d = make_int4(bins.rowstart[c] + first * c, c, min(wpp, cnt - first), bins.wstart[c] + first);
-  } else {
-    int tiles = (c + tile - 1) / tile;
-    int wl = q / tiles, qt = q - wl * tiles;
-    d = make_int4(bins.rowstart[c] + wl * c, c, -(qt + 1), bins.wstart[c] + wl);
-  }
-  reinterpret_cast<int4*>(pack_desc)[p] = d;
-}
+// Blocks [0, v_blocks): `vpt` voxels per thread.  Then w_blocks: one thread per non-empty window.  Then one
+// thread per work item.
+struct FillArgs {
+  int64_t n;
+  int words, vpt, v_blocks, w_blocks, n_per_window, tile, padded, pack_cap, w_cap;
+  const int32_t* compact;
+  const uint32_t* bitmap;
+  int32_t* header;
+  const int32_t* win_start;
+  int32_t* win_pstart;   // complement of the slot on entry, first row in pack order on exit
+  int32_t* bins_base;
+  int32_t *perm, *inv_perm, *pack_perm, *pack_meta, *pack_win, *pack_desc;
+};
+constexpr int kMaxBinsPerThread = (kMaxPerWindow + 2 + kFillThreads - 1) / kFillThreads;
 
-__global__ void k_scatter(KeySrc s, int64_t n, int words, const int32_t* __restrict__ compact,
-                          const uint32_t* __restrict__ bitmap, const int32_t* __restrict__ win_start,
-                          const int32_t* __restrict__ win_pstart, int32_t* __restrict__ perm,
-                          int32_t* __restrict__ inv_perm, int32_t* __restrict__ pack_perm,
-                          int32_t* __restrict__ pack_meta) {
-  int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(kFillThreads) k_scatter(KeySrc s, FillArgs a) {
+  extern __shared__ int32_t tab[];  // [4][n_per_window + 2]: windows, first window slot, first row, first item of every occupancy
+  const int nb = a.n_per_window + 2;
+  int32_t *cnt = tab, *wstart = tab + nb, *rowstart = tab + 2 * nb, *packstart = tab + 3 * nb;
+  BinTables bins(a.bins_base, a.n_per_window);
+  const bool voxels = (int)blockIdx.x < a.v_blocks;
+  int64_t v = (int64_t)blockIdx.x * kFillThreads * a.vpt + threadIdx.x;
   int w = 0, pos = 0, r = 0;
-  const bool ok = v < n && load_key(s, v, w, pos, r);  // coordinates are an input, not a product of the chain
+  // coordinates are an input, not a product of the chain
+  bool ok = voxels && v < a.n && load_key(s, v, w, pos, r) && w >= s.win_lo && w < s.win_hi;
   grid_dependency_wait();
-  if (!ok || w < s.win_lo || w >= s.win_hi) return;
-  int k = compact[w];
-  if (k < 0) return;
-  const uint32_t* bm = bitmap + (int64_t)w * words;
-  int rank = 0;
-  int full = pos >> 5;
-  for (int i = 0; i < full; ++i) rank += __popc(__ldg(bm + i));
-  rank += __popc(__ldg(bm + full) & ((1u << (pos & 31)) - 1u));
-  int dst = win_start[k] + rank;
-  perm[dst] = (int)v;
-  inv_perm[v] = dst;
-  int pdst = win_pstart[k] + rank;
-  pack_perm[pdst] = (int)v;
-  int wyx = s.rpbw[1] * s.rpbw[2];
-  int pz = pos / wyx, rem = pos - pz * wyx;
-  int py = rem / s.rpbw[2], px = rem - py * s.rpbw[2];
-  int rel = (pz * (2 * s.rpbw[1] - 1) + py) * (2 * s.rpbw[2] - 1) + px;
-  pack_meta[pdst] = pos | (r << kMetaRegionShift) | (rel << kMetaRelShift);
+  grid_launch_dependents();
+  int k = ok ? a.compact[w] : -1;  // on its way while the starts are formed
+  // per-occupancy starts: exclusive scans over c = 0..n_per_window + 1 of (windows, rows, items); every thread
+  // takes a run of consecutive occupancies
+  const int per = (nb + kFillThreads - 1) / kFillThreads, c0 = threadIdx.x * per;
+  Tri v3[kMaxBinsPerThread], sum{0, 0, 0ull};  // flags = windows, rows = rows, sq = work items
+#pragma unroll
+  for (int i = 0; i < kMaxBinsPerThread; ++i) {
+    const int cc = c0 + i;
+    const int m = i < per && cc < nb ? bins.cnt[cc] : 0;
+    v3[i] = Tri{m, m * cc, (unsigned long long)packs_of_bin(cc, m, a.tile, a.padded)};
+    sum = tri_add(sum, v3[i]);
+  }
+  Tri all;
+  Tri e = block_excl_scan<kFillThreads>(sum, all);
+#pragma unroll
+  for (int i = 0; i < kMaxBinsPerThread; ++i) {
+    const int cc = c0 + i;
+    if (i < per && cc < nb) {
+      cnt[cc] = v3[i].flags;
+      wstart[cc] = e.flags;
+      rowstart[cc] = e.rows;
+      packstart[cc] = (int)e.sq;
+    }
+    e = tri_add(e, v3[i]);
+  }
+  __syncthreads();
+  // The descriptor array holds pack_cap items (an upper bound for every occupancy histogram the
+  // layout call could foresee).  Should a count ever exceed it, the plan is declared empty and
+  // flagged rather than written past its end.
+  const bool fits = all.sq <= (unsigned long long)a.pack_cap;
+  const int packs = fits ? (int)all.sq : 0;
+  if (blockIdx.x == 0) {
+    for (int i = threadIdx.x; i < nb; i += kFillThreads) {
+      bins.wstart[i] = wstart[i];
+      bins.rowstart[i] = rowstart[i];
+      bins.packstart[i] = packstart[i];
+    }
+    if (threadIdx.x == 0) {
+      if (!fits) atomicOr(reinterpret_cast<unsigned*>(a.header + SSW_H_ERROR), SSW_DEV_BAD_PLAN);
+      a.header[SSW_H_PACKS] = packs;
+      a.header[SSW_H_PACKS_SMALL] = !fits ? 0 : a.tile + 1 < nb ? packstart[a.tile + 1] : packs;
+      a.header[SSW_H_TILE] = a.tile;
+      a.header[SSW_H_PADDED] = a.padded;
+    }
+  }
+  if (voxels) {
+    const int wyx = s.rpbw[1] * s.rpbw[2];
+    for (int i = 0;;) {
+      if (k >= 0) {
+        const uint32_t* bm = a.bitmap + (int64_t)w * a.words;
+        int rank = 0;
+        const int full = pos >> 5;
+        const int start = a.win_start[k], c = a.win_start[k + 1] - start;
+        const int slot = *reinterpret_cast<volatile int32_t*>(a.win_pstart + k);  // its thread may have replaced it
+        for (int x = 0; x < full; ++x) rank += __popc(__ldg(bm + x));
+        rank += __popc(__ldg(bm + full) & ((1u << (pos & 31)) - 1u));
+        const int dst = start + rank;
+        a.perm[dst] = (int)v;
+        a.inv_perm[v] = dst;
+        const int pdst = (slot < 0 ? rowstart[c] + ~slot * c : slot) + rank;
+        a.pack_perm[pdst] = (int)v;
+        int pz = pos / wyx, rem = pos - pz * wyx;
+        int py = rem / s.rpbw[2], px = rem - py * s.rpbw[2];
+        int rel = (pz * (2 * s.rpbw[1] - 1) + py) * (2 * s.rpbw[2] - 1) + px;
+        a.pack_meta[pdst] = pos | (r << kMetaRegionShift) | (rel << kMetaRelShift);
+      }
+      if (++i >= a.vpt) break;
+      v += kFillThreads;
+      ok = v < a.n && load_key(s, v, w, pos, r) && w >= s.win_lo && w < s.win_hi;
+      k = ok ? a.compact[w] : -1;
+    }
+  } else if ((int)blockIdx.x < a.v_blocks + a.w_blocks) {
+    const int x = ((int)blockIdx.x - a.v_blocks) * kFillThreads + threadIdx.x;
+    if (x >= all.flags || x >= a.w_cap) return;
+    const int c = a.win_start[x + 1] - a.win_start[x];
+    const int slot = ~a.win_pstart[x];
+    a.pack_win[wstart[c] + slot] = x;
+    *reinterpret_cast<volatile int32_t*>(a.win_pstart + x) = rowstart[c] + slot * c;
+  } else {
+    const int p = ((int)blockIdx.x - a.v_blocks - a.w_blocks) * kFillThreads + threadIdx.x;
+    if (p >= packs) return;
+    // largest c with packstart[c] <= p and a non-empty bin: binary search on the monotone table
+    int lo = 1, hi = a.n_per_window;
+    while (lo < hi) {
+      int mid = (lo + hi + 1) >> 1;
+      if (packstart[mid] <= p) lo = mid; else hi = mid - 1;
+    }
+    const int c = lo, q = p - packstart[c];
+    int4 d;
+    if (c <= a.tile) {
+      const int wpp = windows_per_pack(c, a.tile, a.padded), first = q * wpp;
+      d = make_int4(rowstart[c] + first * c, c, min(wpp, cnt[c] - first), wstart[c] + first);
+    } else {
+      const int tiles = (c + a.tile - 1) / a.tile;
+      const int wl = q / tiles, qt = q - wl * tiles;
+      d = make_int4(rowstart[c] + wl * c, c, -(qt + 1), wstart[c] + wl);
+    }
+    reinterpret_cast<int4*>(a.pack_desc)[p] = d;
+  }
 }
 
 static void fill_keysrc(KeySrc& s, const int32_t* coords, const ssw_geometry* g, const int32_t* indices,
@@ -516,38 +530,57 @@ extern "C" int ssw_bucket_windows_range(const int32_t* coords, const ssw_geometr
   const int64_t N = L->n_vox;
   const int n = L->n_per_window;
   int32_t* header = plan + L->off_header;
-  // header and the bin tables are adjacent: one clear covers both
-  SSW_CUDA_TRY(cudaMemsetAsync(plan, 0, sizeof(int32_t) * (size_t)(L->off_perm), stream));
-  if (N == 0) return SSW_OK;
-  SSW_CUDA_TRY(cudaMemsetAsync(scratch, 0, sizeof(int32_t) * (size_t)L->off_partials, stream));
+  if (N == 0) {
+    SSW_CUDA_TRY(cudaMemsetAsync(plan, 0, sizeof(int32_t) * (size_t)(L->off_perm), stream));
+    return SSW_OK;
+  }
   KeySrc s;
   fill_keysrc(s, coords, geom, indices, mask, mask_windows, rpb_window, L->n_windows, n);
   s.win_lo = win_lo;
   s.win_hi = win_hi;
   int32_t* count = scratch + L->off_count;
   uint32_t* bitmap = reinterpret_cast<uint32_t*>(scratch + L->off_bitmap);
-  int32_t* partials = scratch + L->off_partials;
   const unsigned vox_blocks = (unsigned)ceil_div64(N, 256);
-  // first of the chain: ordinary launch, fully ordered behind the clears and the caller's earlier work
+  // Header and bin tables are adjacent, and so is all of the scratch; both are cleared in 16-byte pieces.
+  const int64_t na = L->off_perm / 4, nb = L->scratch_ints / 4;
+  k_clear<<<(unsigned)(ceil_div64(na + nb, 1024) < 1184 ? ceil_div64(na + nb, 1024) : 1184), 256, 0, stream>>>(
+      reinterpret_cast<int4*>(plan), na, reinterpret_cast<int4*>(scratch), nb);
+  SSW_LAUNCH_CHECK("k_clear");
+  // ordinary launches, fully ordered behind the caller's earlier work
   k_count<<<vox_blocks, 256, 0, stream>>>(s, N, L->bitmap_words, count, bitmap, header);
   SSW_LAUNCH_CHECK("k_count");
   const int blocks = (int)ceil_div64(L->n_windows, kScanBlock);
-  SSW_CUDA_TRY(launch_chained(k_reduce, dim3(blocks), dim3(kScanThreads), 0, stream, (const int32_t*)count,
-                              (int)L->n_windows, partials, header, blocks));
   SSW_CUDA_TRY(launch_chained(k_compact, dim3(blocks), dim3(kScanThreads), sizeof(int32_t) * (n + 2), stream, count,
-                              (int)L->n_windows, (const int32_t*)partials, header, plan + L->off_win_id,
-                              plan + L->off_win_start, plan + L->off_coo_start, plan + L->off_bins, n,
-                              (int)L->tile_rows, (int)L->padded, blocks, (int)L->pack_cap));
-  const int w_blocks = (int)ceil_div64(L->w_cap, 256);
-  const int p_blocks = (int)ceil_div64(L->pack_cap, 256);
-  SSW_CUDA_TRY(launch_chained(k_order, dim3(w_blocks + p_blocks), dim3(256), 0, stream, (const int32_t*)header,
-                              (const int32_t*)(plan + L->off_win_start), plan + L->off_win_pstart,
-                              plan + L->off_pack_win, plan + L->off_pack_desc, plan + L->off_bins, n,
-                              (int)L->tile_rows, (int)L->padded, w_blocks, (int)L->pack_cap));
-  SSW_CUDA_TRY(launch_chained(k_scatter, dim3(vox_blocks), dim3(256), 0, stream, s, N, (int)L->bitmap_words,
-                              (const int32_t*)count, (const uint32_t*)bitmap, (const int32_t*)(plan + L->off_win_start),
-                              (const int32_t*)(plan + L->off_win_pstart), plan + L->off_perm, plan + L->off_inv_perm,
-                              plan + L->off_pack_perm, plan + L->off_pack_meta));
+                              (int)L->n_windows, reinterpret_cast<unsigned long long*>(scratch + L->off_partials), header,
+                              plan + L->off_win_id, plan + L->off_win_start, plan + L->off_coo_start, plan + L->off_win_pstart,
+                              plan + L->off_bins, n, blocks));
+  FillArgs a;
+  a.n = N;
+  a.words = (int)L->bitmap_words;
+  // one wave of blocks: each forms the starts of the occupancies for itself
+  a.vpt = (int)ceil_div64(N, (int64_t)kFillThreads * 148 * 8);
+  a.v_blocks = (int)ceil_div64(N, (int64_t)kFillThreads * a.vpt);
+  a.w_blocks = (int)ceil_div64(L->w_cap, kFillThreads);
+  a.n_per_window = n;
+  a.tile = (int)L->tile_rows;
+  a.padded = (int)L->padded;
+  a.pack_cap = (int)L->pack_cap;
+  a.w_cap = (int)L->w_cap;
+  a.compact = count;
+  a.bitmap = bitmap;
+  a.header = header;
+  a.win_start = plan + L->off_win_start;
+  a.win_pstart = plan + L->off_win_pstart;
+  a.bins_base = plan + L->off_bins;
+  a.perm = plan + L->off_perm;
+  a.inv_perm = plan + L->off_inv_perm;
+  a.pack_perm = plan + L->off_pack_perm;
+  a.pack_meta = plan + L->off_pack_meta;
+  a.pack_win = plan + L->off_pack_win;
+  a.pack_desc = plan + L->off_pack_desc;
+  const unsigned p_blocks = (unsigned)ceil_div64(L->pack_cap, kFillThreads);
+  SSW_CUDA_TRY(launch_chained(k_scatter, dim3(a.v_blocks + a.w_blocks + p_blocks), dim3(kFillThreads), 4 * sizeof(int32_t) * (n + 2), stream,
+                              s, a));
   return SSW_OK;
 }
 
