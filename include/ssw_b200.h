@@ -272,6 +272,15 @@ int64_t ssw_layernorm_bwd_workspace_floats(int64_t n_rows, int32_t channels);
 int ssw_layernorm_bwd(const void* x, const void* dy, const void* dsum, const void* gamma, int param_dtype, float eps, int dtype,
                       int64_t n_rows, int32_t channels, void* dx, void* dgamma, void* dbeta, float* workspace, void* stream);
 
+/* out [M, N] = a [M, K] w [N, K]^T (+ bias [N], may be NULL), all fp32, row-major, 16-byte aligned, N and K multiples of
+ * four: fp32 accuracy on the tensor cores (three bf16 terms per operand, see csrc/gemm_f32.cu). */
+int ssw_gemm_f32(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, void* stream);
+
+/* Weight gradient with the same arithmetic: out [N, K] = g [M, N]^T x [M, K], M > 0.  The workspace size is asked for with
+ * the device the call will run on current. */
+int64_t ssw_gemm_f32_tn_workspace_floats(int64_t M, int32_t N, int32_t K);
+int ssw_gemm_f32_tn(const float* g, const float* x, float* out, int64_t M, int32_t N, int32_t K, float* workspace, void* stream);
+
 /* out[c] = sum over the rows of x [n_rows, channels], fp32 accumulation in a fixed order (the bias gradient
  * of a Linear layer).  n_rows > 0, rows as above. */
 int64_t ssw_col_sum_workspace_floats(int64_t n_rows, int32_t channels);

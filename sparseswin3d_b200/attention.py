@@ -194,7 +194,7 @@ class WindowAttentionSparse(nn.Module):
         n = x.spatial_shape[0]
         b = x.batch_size
         c = x.features.shape[-1]
-        qkv = self.qkv(x.features).reshape(-1, 3, self.num_heads, c // self.num_heads)
+        qkv = rows.linear(self.qkv, x.features).reshape(-1, 3, self.num_heads, c // self.num_heads)
         q, k_t, v = qkv_sparse_cuda(qkv, x.indices, b, n)
         q = q * self.scale
         attn = spspmm_block_naive(q, k_t, "q_k")
@@ -207,7 +207,7 @@ class WindowAttentionSparse(nn.Module):
         x_ = spspmm_block_naive(attn, v, "qk_v").permute((0, 2, 1, 3))
         arg_sort = ops.return_inverse(ops.flatten_indices(x.indices.T.contiguous(), [b, n]), -1)[0]
         x = x.replace_feature(x_.values.reshape(x.features.shape).index_select(0, arg_sort))
-        return x.replace_feature(self.proj_drop(self.proj(x.features)))
+        return x.replace_feature(self.proj_drop(rows.linear(self.proj, x.features)))
 
     def forward(self, x, mask, plan: Optional[WindowPlan] = None, fused: Optional[bool] = None,
                 strict: Optional[bool] = None):

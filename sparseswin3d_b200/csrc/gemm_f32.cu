@@ -1,0 +1,528 @@
+// fp32 GEMM of the Linear layers: out[M, N] = a[M, K] w[N, K]^T (+ bias), on the fifth-generation tensor cores
+// with the operands split into three bf16 terms each.
+//
+// x = h + m + l with h = bf16(x), m = bf16(x - h), l = bf16(x - h - m) holds all 24 bits of x.  Six of the nine
+// products are formed (h h, h m, m h, m m, h l, l h); the three left out are below 2^-25 of a term.  The tensor
+// cores add up in fp32 but cut off instead of rounding, so the sums are kept short: the h h products of 64 steps
+// of K go into a tensor-memory accumulator of their own, which the epilogue threads add up in registers, rounding
+// to nearest; the five small products (2^-8 and below) share one accumulator for the whole of K.
+// Against 64 bits (2-norm, normal operands): 7e-8 at K = 96, 8e-8 at 192, 1.0e-7 at 768, where the library's fp32 GEMM is
+// at 1.8e-7, 2.5e-7 and 5.0e-7; all-positive operands 8.2e-8, 9.5e-8, 1.0e-7 against 1.5e-7, 2.1e-7, 4.1e-7.  Weight
+// gradients of 150 000 rows: 2.0e-7 against 1.3e-6, all-positive 6e-8 against 2.1e-7 (with 64 steps a chunk 2.0e-7 against
+// the library's 1.5e-7 at 96 x 96, hence one stage a chunk there).
+//
+//
+// The same kernel forms weight gradients, out[N, K] = g[M, N]^T x[M, K] (TN): the operands' rows are then the steps of the
+// sum, so a producer thread takes four columns of eight consecutive rows and turns them in registers, and the sum
+// over M is split over blocks (partial results, added up in order by k_gemm_reduce).
+//
+// An Inf operand has no finite remainder (Inf - Inf), so a result that is not finite is formed again from the
+// operands as they are, by plain fp32 multiply-adds.
+//
+// Persistent, one block per SM, 17 warps: eight bring fp32 pieces in three stages ahead, split them and store the
+// six 64-byte-swizzled operand tiles of a stage (32 of K); one issues the MMAs; eight drain accumulators (a warp
+// may read the 32 tensor-memory lanes warp_id % 4 selects; two warps share them, half the columns each).
+// What bounds it: the issue slots of the split (4.5 instructions per element of both operands) about level with
+// the six MMAs per product.  Against the library's fp32 GEMM with bias:
+// 150 000 x 288 x 96 448 -> 103 us, 150 000 x 96 x 288 270 -> 79, 10 000 x 768 x 192 98 -> 39, 10 000 x 192 x 768
+// 75 -> 46, 128 x 96 x 96 22 -> 12.  Weight gradients: 150 000 rows 288 x 96 358 -> 150, 96 x 96 208 -> 71, 10 000 rows
+// 576 x 192 111 -> 46.  With the raw pieces in registers, two stages ahead, the latter took 226, 97 and 49: they wait for
+// memory, not for the split.
+#include <math.h>
+
+#include "attn_common.cuh"
+#include "tcgen05.cuh"
+
+namespace ssw {
+
+constexpr int kGM = 128;                 // rows of a tile
+constexpr int kGNMax = 96;              // columns of a tile at most (48 sums a drain thread: with 64 they spill)
+constexpr int kGK = 32;                  // K of a stage
+constexpr int kGRowB = kGK * 2;          // bytes of an operand row: one 64-byte swizzle row
+// Stages whose h h products share an accumulator: two, and one for the long sums of a weight gradient.
+template <bool TN>
+struct GemmChunk { static constexpr int kStages = TN ? 1 : 2; };
+constexpr int kGStages = 2;              // of split operands
+constexpr int kGRaw = 3;                 // of fp32 pieces on their way, each read by the thread that asked for it
+constexpr int kGProd = 8, kGEpi = 8;     // warps
+constexpr int kGThreads = 32 * (kGProd + 1 + kGEpi);
+constexpr int kGOpB = kGM * kGRowB;      // bytes of one split tile
+constexpr int kGStageB = 6 * kGOpB;      // A: h, m, l; B: h, m, l
+constexpr int kGTmemLow = 2 * kGNMax;    // two h h accumulators, then two of small products
+constexpr int kGOutCols = 16, kGOutPitch = kGOutCols + 4;   // a warp's output piece, skewed across the banks
+constexpr int kGRawB = kGProd * 32 * 8 * 16;                  // bytes of one raw stage
+constexpr int kGPiece = 1024 + kGStages * kGStageB, kGRawOff = kGPiece + kGEpi * 32 * kGOutPitch * 4;
+constexpr int kGSmem = kGRawOff + kGRaw * kGRawB + 1024;
+
+struct GemmParams {
+  const float *a, *w, *bias;
+  float* out;
+  int64_t M;
+  int N, K;
+  int bn, n_tiles;        // columns of a tile (a multiple of 16), tiles across N
+  int tiles;
+  // TN: a is g [rows, M], w is x [rows, N]; out holds `splits` partial results [M, N] of rows_per_split rows each
+  int64_t rows;
+  int rows_per_split, mn_tiles;
+};
+
+__device__ unsigned g_gemm_timeout = 0;
+
+__device__ __forceinline__ float2 bf16x2_to_f32(uint32_t u) {
+  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+}
+// four fp32 values -> their three bf16 terms, packed
+__device__ __forceinline__ void split4(const float4& x, uint2& h, uint2& m, uint2& l) {
+  const float2 neg = make_float2(-1.f, -1.f);
+  float2 p = make_float2(x.x, x.y), q = make_float2(x.z, x.w);
+  h = make_uint2(pack2<__nv_bfloat16>(p.x, p.y), pack2<__nv_bfloat16>(q.x, q.y));
+  p = __ffma2_rn(bf16x2_to_f32(h.x), neg, p);
+  q = __ffma2_rn(bf16x2_to_f32(h.y), neg, q);
+  m = make_uint2(pack2<__nv_bfloat16>(p.x, p.y), pack2<__nv_bfloat16>(q.x, q.y));
+  p = __ffma2_rn(bf16x2_to_f32(m.x), neg, p);
+  q = __ffma2_rn(bf16x2_to_f32(m.y), neg, q);
+  l = make_uint2(pack2<__nv_bfloat16>(p.x, p.y), pack2<__nv_bfloat16>(q.x, q.y));
+}
+// x[0..7] -> the three terms of each, eight bf16 per 16 bytes
+__device__ __forceinline__ void split8(const float (&x)[8], uint4& h, uint4& m, uint4& l) {
+  uint2 h0, m0, l0, h1, m1, l1;
+  split4(make_float4(x[0], x[1], x[2], x[3]), h0, m0, l0);
+  split4(make_float4(x[4], x[5], x[6], x[7]), h1, m1, l1);
+  h = make_uint4(h0.x, h0.y, h1.x, h1.y);
+  m = make_uint4(m0.x, m0.y, m1.x, m1.y);
+  l = make_uint4(l0.x, l0.y, l1.x, l1.y);
+}
+__device__ __forceinline__ void sts_u4(uint32_t a, const uint4& v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+// 16 bytes from global to shared memory, asynchronously; zeros instead when !on
+__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool on) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
+__device__ __forceinline__ void sts_v2(uint32_t a, uint2 v) {
+  asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(v.x), "r"(v.y) : "memory");
+}
+
+template <bool TN>
+__global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+  uint64_t* full = bars;                     // [kGStages] operands of a stage are in shared memory
+  uint64_t* empty = full + kGStages;         // [kGStages] the stage's MMAs are done
+  uint64_t* hh_full = empty + kGStages;      // [2] a chunk's h h accumulator is complete
+  uint64_t* hh_empty = hh_full + 2;          // [2] ... has been read
+  uint64_t* lo_full = hh_empty + 2;          // [2] a tile's small-product accumulator is complete
+  uint64_t* lo_empty = lo_full + 2;          // [2]
+  uint64_t* drain_bar = lo_empty + 2;        // [1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
+  const uint32_t stage0 = smem_u32(smem + 1024);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kGStages; ++s) {
+      mbar_init(full + s, kGProd);
+      mbar_init(empty + s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(hh_full + b, 1);
+      mbar_init(hh_empty + b, kGEpi);
+      mbar_init(lo_full + b, 1);
+      mbar_init(lo_empty + b, kGEpi);
+    }
+    mbar_init(drain_bar, 1);
+    mbar_fence_init();
+  }
+  if (warp == kGProd) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  grid_dependency_wait();
+  const int n_stages = ((TN ? p.rows_per_split : p.K) + kGK - 1) / kGK;       // of one tile
+  const int bn = p.bn;
+  constexpr int kChunk = GemmChunk<TN>::kStages;
+  bool timed_out = false;
+
+  if (warp < kGProd) {
+    // =========================================== producers ====================================
+    const uint32_t raw = smem_u32(smem + kGRawOff) + threadIdx.x * 16u;   // this thread's pieces: [kGRaw][8], 4 KB apart
+    const int my_tiles = p.tiles > (int)blockIdx.x ? (p.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const int64_t total = (int64_t)my_tiles * n_stages;
+    int lt = blockIdx.x, ls = 0;   // tile and stage the next load belongs to
+    // NT: a thread looks after 16-byte piece f4 of rows r0, r0 + 32, ... of both operands (eight lanes read one row's
+    // 128 bytes).  TN: warps 0-3 take g, 4-7 take x; a thread, columns 4 quad .. 4 quad + 3 of rows 8 oct .. 8 oct + 7 of
+    // a stage (eight lanes read 128 bytes of one row).
+    const int f4 = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+    const bool is_w = threadIdx.x >= 128;
+    const int oct = threadIdx.x & 3, quad = (threadIdx.x & 127) >> 2;
+    const float *pa, *pw = nullptr;   // this thread's piece of the tile's next stage
+    int rows_a, rows_w = 0;           // NT: rows of the tile from r0 on that exist; TN: rows of the split from oct on, and whether the columns do
+    auto open_tile = [&]() {
+      if constexpr (TN) {
+        const int sp = lt / p.mn_tiles, mn = lt - sp * p.mn_tiles, mt = mn / p.n_tiles;
+        const int col = (is_w ? (mn - mt * p.n_tiles) * bn : mt * kGM) + quad * 4, ld = is_w ? p.N : (int)p.M;
+        const int64_t k0 = (int64_t)sp * p.rows_per_split + oct * 8;
+        rows_a = (int)max((int64_t)0, min((int64_t)p.rows_per_split - oct * 8, p.rows - k0));
+        if (col >= ld || (is_w && quad * 4 >= bn)) rows_a = 0;   // M and N are multiples of four
+        pa = (is_w ? p.w : p.a) + k0 * ld + col;
+      } else {
+        const int mt = lt / p.n_tiles, n0 = (lt - mt * p.n_tiles) * bn;
+        const int64_t m0 = (int64_t)mt * kGM;
+        rows_a = (int)min((int64_t)kGM, p.M - m0) - r0;
+        rows_w = min(bn, p.N - n0) - r0;
+        pa = p.a + (m0 + r0) * p.K + f4 * 4;
+        pw = p.w + (int64_t)(n0 + r0) * p.K + f4 * 4;
+      }
+    };
+    open_tile();
+    const int64_t step_rows = TN ? (is_w ? (int64_t)p.N : p.M) : (int64_t)p.K * 32;
+    int lslot = 0;
+    int64_t loaded = 0;
+    auto load = [&]() {   // one commit group per stage, empty beyond the last one
+      if (loaded < total) {
+        const uint32_t dst = raw + (uint32_t)lslot * kGRawB;
+        if constexpr (TN) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const bool on = ls * kGK + i < rows_a;
+            cp_async16_or_zero(dst + i * 4096u, on ? pa + i * step_rows : p.a, on);
+          }
+          pa += kGK * step_rows;
+        } else {
+          const bool kin = ls * kGK + f4 * 4 < p.K;   // K is a multiple of four
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const bool ona = kin && 32 * i < rows_a, onw = kin && 32 * i < rows_w;
+            cp_async16_or_zero(dst + i * 4096u, ona ? pa + i * step_rows : p.a, ona);
+            cp_async16_or_zero(dst + (4 + i) * 4096u, onw ? pw + i * step_rows : p.a, onw);
+          }
+          pa += kGK;
+          pw += kGK;
+        }
+        lslot = lslot + 1 == kGRaw ? 0 : lslot + 1;
+        ++loaded;
+        if (++ls == n_stages) {
+          ls = 0;
+          lt += gridDim.x;
+          if (lt < p.tiles) open_tile();
+        }
+      }
+      cp_async_commit();
+    };
+    for (int x = 0; x < kGRaw; ++x) load();
+    const uint32_t off = (uint32_t)(r0 * kGRowB + (((f4 >> 1) ^ ((r0 >> 1) & 3)) << 4) + (f4 & 1) * 8);
+    int slot = 0;
+    auto step = [&](int64_t i) -> bool {
+      cp_async_wait<kGRaw - 1>();   // this stage's pieces have landed; each thread reads its own
+      const uint32_t src = raw + (uint32_t)slot * kGRawB;
+      slot = slot + 1 == kGRaw ? 0 : slot + 1;
+      float4 v[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const int4 u = lds_v4(src + x * 4096u);
+        v[x] = make_float4(__int_as_float(u.x), __int_as_float(u.y), __int_as_float(u.z), __int_as_float(u.w));
+      }
+      const int s = (int)(i % kGStages);
+      const int64_t use = i / kGStages;
+      if (use > 0 && !mbar_wait_bounded(empty + s, (uint32_t)(use - 1) & 1)) return false;
+      if constexpr (TN) {
+        const uint32_t base = stage0 + (uint32_t)s * kGStageB + (is_w ? 3u * kGOpB : 0u);
+        if (!is_w || quad * 4 < bn) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float x[8];
+#pragma unroll
+            for (int i8 = 0; i8 < 8; ++i8) x[i8] = j == 0 ? v[i8].x : j == 1 ? v[i8].y : j == 2 ? v[i8].z : v[i8].w;
+            uint4 h, m, l;
+            split8(x, h, m, l);
+            const int row = quad * 4 + j;
+            const uint32_t d = base + (uint32_t)(row * kGRowB + ((oct ^ ((row >> 1) & 3)) << 4));
+            sts_u4(d, h);
+            sts_u4(d + kGOpB, m);
+            sts_u4(d + 2 * kGOpB, l);
+          }
+        }
+      } else {
+        const uint32_t base = stage0 + (uint32_t)s * kGStageB + off;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+          if (x >= 4 && r0 + 32 * (x - 4) >= bn) continue;
+          uint2 h, m, l;
+          split4(v[x], h, m, l);
+          const uint32_t d = base + (x >= 4 ? 3u * kGOpB : 0u) + (uint32_t)(x & 3) * (32u * kGRowB);
+          sts_v2(d, h);
+          sts_v2(d + kGOpB, m);
+          sts_v2(d + 2 * kGOpB, l);
+        }
+      }
+      fence_async_smem();  // the tensor cores read shared memory through the async proxy
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + s);
+      load();   // into the slot just read
+      return true;
+    };
+    for (int64_t i = 0; i < total; ++i) {
+      if (!step(i)) {
+        timed_out = true;
+        break;
+      }
+    }
+    cp_async_wait<0>();   // nothing of this block's may still be on its way into shared memory
+  } else if (warp == kGProd) {
+    // =========================================== MMA issuer ===================================
+    const uint32_t idesc = instr_desc(1, 1, 0, bn);
+    uint32_t st = 0, ch = 0, tn = 0;   // stages, chunks, tiles so far
+    for (int t = blockIdx.x; t < p.tiles && !timed_out; t += gridDim.x, ++tn) {
+      const uint32_t lb = tn & 1;
+      if (tn >= 2 && !mbar_wait_bounded(lo_empty + lb, ((tn >> 1) - 1) & 1)) { timed_out = true; break; }
+      for (int ks = 0; ks < n_stages; ++ks, ++st) {
+        const uint32_t s = st % kGStages, hb = ch & 1;
+        const bool first = ks % kChunk == 0, last = ks % kChunk == kChunk - 1 || ks == n_stages - 1;
+        if (first && ch >= 2 && !mbar_wait_bounded(hh_empty + hb, ((ch >> 1) - 1) & 1)) { timed_out = true; break; }
+        if (!mbar_wait_bounded(full + s, (st / kGStages) & 1)) { timed_out = true; break; }
+        tc_fence_after();
+        if (lane == 0) {
+          const uint32_t A = stage0 + s * kGStageB, B = A + 3 * kGOpB;
+#pragma unroll
+          for (int k16 = 0; k16 < kGK / 16; ++k16) {
+            uint64_t da[3], db[3];
+#pragma unroll
+            for (int x = 0; x < 3; ++x) {
+              da[x] = smem_desc(A + x * kGOpB + k16 * 32, 512, 4);
+              db[x] = smem_desc(B + x * kGOpB + k16 * 32, 512, 4);
+            }
+            const uint32_t hh = tmem + hb * kGNMax, lo = tmem + kGTmemLow + lb * kGNMax;
+            umma_ss(hh, da[0], db[0], idesc, !(first && k16 == 0));
+            umma_ss(lo, da[0], db[2], idesc, ks > 0 || k16 > 0);   // smallest first
+            umma_ss(lo, da[2], db[0], idesc, 1);
+            umma_ss(lo, da[1], db[1], idesc, 1);
+            umma_ss(lo, da[0], db[1], idesc, 1);
+            umma_ss(lo, da[1], db[0], idesc, 1);
+          }
+          umma_commit(empty + s);
+          if (last) umma_commit(hh_full + hb);
+          if (ks == n_stages - 1) umma_commit(lo_full + lb);
+        }
+        __syncwarp();
+        if (last) ++ch;
+      }
+    }
+    // let the tensor cores finish whatever was issued before the tensor memory is given back
+    if (lane == 0) umma_commit(drain_bar);
+    __syncwarp();
+    mbar_wait_bounded(drain_bar, 0);
+  } else {
+    // =========================================== epilogue =====================================
+    const int ew = warp - kGProd - 1, half = ew >> 2, sub = warp & 3;
+    const uint32_t t_lane = (uint32_t)(sub * 32) << 16;
+    const int hc = bn / 2, c0 = half * hc;   // this thread's columns [c0, c0 + hc), hc a multiple of eight
+    const int n_chunks = (n_stages + kChunk - 1) / kChunk;
+    uint32_t ch = 0, tn = 0;
+    for (int t = blockIdx.x; t < p.tiles && !timed_out; t += gridDim.x, ++tn) {
+      float acc[kGNMax / 2];
+#pragma unroll
+      for (int e = 0; e < kGNMax / 2; ++e) acc[e] = 0.f;
+      auto add_columns = [&](uint32_t col) {
+#pragma unroll
+        for (int e = 0; e < kGNMax / 2; e += 16) {
+          if (e < hc) {   // (the last eight columns of an odd multiple of eight: read, not used)
+            uint32_t r[16];
+            tmem_ld16(tmem + t_lane + col + c0 + e, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int x = 0; x < 16; ++x) acc[e + x] += __uint_as_float(r[x]);
+          }
+        }
+      };
+      for (int c = 0; c < n_chunks; ++c, ++ch) {
+        const uint32_t hb = ch & 1;
+        if (!mbar_wait_bounded(hh_full + hb, (ch >> 1) & 1)) { timed_out = true; break; }
+        tc_fence_after();
+        add_columns(hb * kGNMax);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(hh_empty + hb);
+      }
+      const uint32_t lb = tn & 1;
+      if (!timed_out && !mbar_wait_bounded(lo_full + lb, (tn >> 1) & 1)) timed_out = true;
+      if (!timed_out) {
+        tc_fence_after();
+        add_columns(kGTmemLow + lb * kGNMax);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(lo_empty + lb);
+      }
+      // Out through shared memory, 16 columns at a time, so that four lanes store 64 bytes of one row.
+      const int sp = TN ? t / p.mn_tiles : 0, mn = t - sp * (TN ? p.mn_tiles : 0), mt = mn / p.n_tiles;
+      const int64_t m0 = (int64_t)mt * kGM + sub * 32;
+      const int n0 = (mn - mt * p.n_tiles) * bn + c0;
+      float* out = p.out + (TN ? (int64_t)sp * p.M * p.N : 0);
+      float* piece = reinterpret_cast<float*>(smem + kGPiece) + ew * 32 * kGOutPitch;
+      const int pr = lane >> 2, pc = (lane & 3) * 4;
+      bool odd = false;   // a result that is not finite (or a sum of four that is not: looked at once more in vain)
+#pragma unroll
+      for (int e = 0; e < kGNMax / 2; e += kGOutCols) {
+        if (e < hc) {
+          __syncwarp();
+#pragma unroll
+          for (int x = 0; x < kGOutCols; x += 4)
+            *reinterpret_cast<float4*>(piece + lane * kGOutPitch + x) = make_float4(acc[e + x], acc[e + x + 1], acc[e + x + 2], acc[e + x + 3]);
+          __syncwarp();
+          const int n = n0 + e + pc;
+          const bool on = e + pc < hc && n < p.N;   // hc and N are multiples of four
+          float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (on && p.bias) b = __ldg(reinterpret_cast<const float4*>(p.bias + n));
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            const int64_t m = m0 + pr + 8 * x;
+            float4 v = *reinterpret_cast<const float4*>(piece + (pr + 8 * x) * kGOutPitch + pc);
+            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+            if (timed_out) v = make_float4(NAN, NAN, NAN, NAN);  // never a plausible result
+            if (on && m < p.M) {
+              odd = odd || not_finite((v.x + v.y) + (v.z + v.w));
+              *reinterpret_cast<float4*>(out + m * p.N + n) = v;
+            }
+          }
+        }
+      }
+      if (!TN && odd && !timed_out) {  // this lane's results once more, those that are not finite from the operands
+        for (int e = 0; e < hc; e += kGOutCols) {
+          const int n = n0 + e + pc;
+          if (e + pc >= hc || n >= p.N) continue;
+          for (int x = 0; x < 4; ++x) {
+            const int64_t m = m0 + pr + 8 * x;
+            if (m >= p.M) continue;
+            for (int c = 0; c < 4; ++c) {
+              if (!not_finite(out[m * p.N + n + c])) continue;
+              float v = 0.f;
+              for (int k = 0; k < p.K; ++k) v = fmaf(__ldg(p.a + m * p.K + k), __ldg(p.w + (int64_t)(n + c) * p.K + k), v);
+              out[m * p.N + n + c] = p.bias ? v + __ldg(p.bias + n + c) : v;
+            }
+          }
+        }
+      }
+    }
+  }
+  if (timed_out) atomicOr(&g_gemm_timeout, 1u);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kGProd) tmem_dealloc(tmem, 512);
+}
+
+// Partial results of a weight gradient added up in order; a sum that is not finite is formed again from g and x.
+__global__ void __launch_bounds__(256) k_gemm_reduce(const float* __restrict__ partial, int splits, const float* __restrict__ g,
+                                                     const float* __restrict__ x, int64_t rows, int N, int K, float* __restrict__ out) {
+  grid_dependency_wait();
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, width = (int64_t)N * K;
+  if (i >= width) return;
+  float s4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+  for (int k = 0; k < splits; k += 4)
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (k + x < splits) s4[x] += __ldcg(partial + (k + x) * width + i);
+  float s = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+  if (not_finite(s)) {
+    const int n = (int)(i / K), c = (int)(i - (int64_t)n * K);
+    s = 0.f;
+    for (int64_t m = 0; m < rows; ++m) s = fmaf(__ldg(g + m * N + n), __ldg(x + m * K + c), s);
+  }
+  out[i] = s;
+}
+
+}  // namespace ssw
+
+using namespace ssw;
+
+// Columns of a tile: the split of N into equal tiles whose waves over the SMs cost least, a tile's cost being
+// its columns plus the rows of A it splits (in the same units: both are rows of operands).
+static int gemm_columns(int64_t m_tiles, int N, int sms, int* n_tiles) {
+  int best = 0;
+  int64_t best_cost = 0;
+  for (int nt = (N + kGNMax - 1) / kGNMax; nt <= (N + 15) / 16; ++nt) {
+    const int bn = ((N + nt - 1) / nt + 15) / 16 * 16;
+    const int used = (N + bn - 1) / bn;
+    const int64_t cost = ((m_tiles * used + sms - 1) / sms) * (bn + kGM);
+    if (!best || cost < best_cost) {
+      best = bn;
+      best_cost = cost;
+      *n_tiles = used;
+    }
+  }
+  return best;
+}
+
+extern "C" int ssw_gemm_f32(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, void* stream_) {
+  if (M < 0 || N <= 0 || K <= 0) return SSW_E_INVALID;
+  if (M == 0) return SSW_OK;
+  if (!a || !w || !out) return SSW_E_INVALID;
+  if ((N | K) & 3) return SSW_E_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(bias) |
+       reinterpret_cast<uintptr_t>(out)) & 15)
+    return SSW_E_INVALID;
+  int dev = 0, sms = 0;
+  SSW_CUDA_TRY(cudaGetDevice(&dev));
+  SSW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  GemmParams p = {};
+  p.a = a; p.w = w; p.bias = bias; p.out = out; p.M = M; p.N = N; p.K = K;
+  const int64_t m_tiles = ceil_div64(M, kGM);
+  p.bn = gemm_columns(m_tiles, N, sms, &p.n_tiles);
+  if (m_tiles * p.n_tiles >= ((int64_t)1 << 30)) return SSW_E_RANGE;
+  p.tiles = (int)(m_tiles * p.n_tiles);
+  SSW_CUDA_TRY(cudaFuncSetAttribute(k_gemm_f32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
+  SSW_CUDA_TRY(launch_chained(k_gemm_f32<false>, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kGThreads), kGSmem,
+                              (cudaStream_t)stream_, p));
+  SSW_LAUNCH_CHECK("k_gemm_f32");
+  return SSW_OK;
+}
+
+// Weight gradient [N, K] of M rows: equal splits of M, as many as give every SM a tile, of two chunks at least.
+static void wgrad_shape(int64_t M, int32_t N, int32_t K, int sms, GemmParams& p, int& splits) {
+  p.n_tiles = (K + kGNMax - 1) / kGNMax;
+  p.bn = ((K + p.n_tiles - 1) / p.n_tiles + 15) / 16 * 16;
+  p.n_tiles = (K + p.bn - 1) / p.bn;
+  p.mn_tiles = (int)ceil_div64(N, kGM) * p.n_tiles;
+  const int unit = 4 * kGK;
+  int64_t want = sms / p.mn_tiles > 0 ? sms / p.mn_tiles : 1;
+  const int64_t per = ceil_div64(ceil_div64(M, want), unit) * unit;
+  p.rows_per_split = (int)(per < (1 << 30) ? per : (1 << 30));
+  splits = (int)ceil_div64(M, p.rows_per_split);
+}
+static int wgrad_sms(int* sms) {
+  int dev = 0;
+  SSW_CUDA_TRY(cudaGetDevice(&dev));
+  SSW_CUDA_TRY(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
+  return SSW_OK;
+}
+
+extern "C" int64_t ssw_gemm_f32_tn_workspace_floats(int64_t M, int32_t N, int32_t K) {
+  if (M <= 0 || N <= 0 || K <= 0) return -1;
+  GemmParams p = {};
+  int sms = 0, splits = 0;
+  if (wgrad_sms(&sms) != SSW_OK) return -1;
+  wgrad_shape(M, N, K, sms, p, splits);
+  return (int64_t)splits * N * K;
+}
+
+extern "C" int ssw_gemm_f32_tn(const float* g, const float* x, float* out, int64_t M, int32_t N, int32_t K, float* workspace, void* stream_) {
+  if (M <= 0 || N <= 0 || K <= 0 || !g || !x || !out || !workspace) return SSW_E_INVALID;
+  if ((N | K) & 3) return SSW_E_UNSUPPORTED;
+  if ((reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) |
+       reinterpret_cast<uintptr_t>(workspace)) & 15)
+    return SSW_E_INVALID;
+  GemmParams p = {};
+  int sms = 0, splits = 0;
+  const int rc = wgrad_sms(&sms);
+  if (rc != SSW_OK) return rc;
+  wgrad_shape(M, N, K, sms, p, splits);
+  p.a = g; p.w = x; p.out = workspace; p.M = N; p.N = K; p.rows = M;
+  if ((int64_t)p.mn_tiles * splits >= ((int64_t)1 << 30)) return SSW_E_RANGE;
+  p.tiles = p.mn_tiles * splits;
+  SSW_CUDA_TRY(cudaFuncSetAttribute(k_gemm_f32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
+  SSW_CUDA_TRY(launch_chained(k_gemm_f32<true>, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kGThreads), kGSmem,
+                              (cudaStream_t)stream_, p));
+  SSW_CUDA_TRY(launch_chained(k_gemm_reduce, dim3((unsigned)ceil_div64((int64_t)N * K, 256)), dim3(256), 0, (cudaStream_t)stream_,
+                              (const float*)workspace, splits, g, x, M, (int)N, (int)K, out));
+  return SSW_OK;
+}

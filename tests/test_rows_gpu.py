@@ -99,3 +99,46 @@ def test_layernorm_on_moved_rows(dtype, n, C):
         assert not rows.layernorm_scatter(x, ln, parent, tap, owner2).view(m, taps, C)[~mine].any()
         src = z.view(m, taps, C).double()[parent.clamp(0, m - 1).long(), tap.long()] * ok[:, None]
         assert rel_err(rows.layernorm_slices(z, ln, parent, tap, taps).double().cpu(), norm64(src).cpu()) <= TOL[dtype]
+
+
+# sizes: below and at the edges of a tile (128 rows, 16 to 128 columns, 32 of K), two chunks of K and a remainder, more
+# tiles than blocks
+@pytest.mark.parametrize("M,N,K", [(1, 4, 4), (127, 16, 32), (128, 96, 96), (129, 100, 36), (1000, 288, 100), (300, 132, 192), (20011, 192, 52),
+                                   (2500, 48, 768)])
+def test_fp32_linear_is_at_least_as_accurate_as_the_library(M, N, K):
+    from sparseswin3d_b200 import rows
+
+    g = torch.Generator().manual_seed(M + N)
+    lin = nn.Linear(K, N).cuda()
+    x = torch.randn(M, K, generator=g).cuda().requires_grad_(True)
+    go = torch.randn(M, N, generator=g).cuda()
+    got = rows.linear(lin, x)
+    grads = torch.autograd.grad(got, (x, lin.weight, lin.bias), go)
+    y64 = x.detach().double() @ lin.weight.detach().double().t()
+    lib32 = F.linear(x.detach(), lin.weight.detach(), lin.bias.detach()).double()
+    ref = y64 + lin.bias.detach().double()
+    err = lambda a, b: float((a.double() - b).norm() / b.norm())
+    # one rounding of every result (2^-24) is the floor of both
+    assert err(got.detach(), ref) <= max(err(lib32, ref), 2.0 ** -24)
+    assert torch.equal(rows._gemm(x.detach(), lin.weight.detach(), None), rows._gemm(x.detach(), lin.weight.detach(), torch.zeros(N, device="cuda")))
+    refs = (go.double() @ lin.weight.detach().double(), go.double().t() @ x.detach().double())
+    libs = (go @ lin.weight.detach(), go.t() @ x.detach())   # (the bias gradient: test_column_sums)
+    for a, r, b in zip(grads, refs, libs):
+        assert err(a, r) <= max(err(b, r), 2.0 ** -24)
+    with torch.no_grad():
+        assert torch.equal(rows.linear(lin, x), got)
+
+
+def test_fp32_products_that_are_not_finite():
+    """Inf and NaN give what plain multiply-adds give, in their own row or column only; so does a value that rounds to Inf
+    in 16 bits."""
+    from sparseswin3d_b200 import rows
+
+    x, w = torch.randn(200, 64, device="cuda"), torch.randn(48, 64, device="cuda").bfloat16().float()
+    x[7, 3], x[130, 0], w[5, 9], x[20, 1] = float("inf"), float("nan"), float("-inf"), 3.4e38
+    w[:, 1] *= 1e-3
+    for got, ref in ((rows._gemm(x, w, None), x.double() @ w.double().t()), (rows._gemm_tn(x, x), x.double().t() @ x.double())):
+        ref = ref.float()
+        assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf() & (got > 0), ref.isinf() & (ref > 0))
+        ok = ref.isfinite()
+        assert rel_err(got[ok].cpu(), ref[ok].cpu()) <= 1e-5
