@@ -8,22 +8,35 @@
 // the tensor cores' operand layout and stay there while the window's query rows pass in tiles of
 // 128:
 //
-//   S[128 x 64]  = Q_tile K_tile^T       tcgen05.mma, operands from shared memory, S in tensor memory
-//   P            = exp2(S*scale + bias + mask - m)   one thread per query row (tcgen05.ld gives a
-//                  thread its row of S), running maximum from 0 and +1e-8 as upstream (ops.cu:137,
-//                  164); P goes back to shared memory in the input type.  bf16 keeps 8 bits of a
-//                  probability, and a row that averages hundreds of keys loses more than the
+//   S[128 x 128] = Q_tile K_tile^T       tcgen05.mma, operands from shared memory, S in tensor memory
+//   P            = exp2(S*scale + bias + mask - m)   two threads per query row (tcgen05.ld gives a
+//                  thread its part of the row of S), running maximum from 0 and +1e-8 as upstream (ops.cu:137,
+//                  164); P goes back to tensor memory in the input type, as the A operand of the next product.
+//                  bf16 keeps 8 bits of a probability, and a row that averages hundreds of keys loses more than the
 //                  tolerance with that, so for bf16 the rounding residual is stored beside P and
 //                  multiplied with the same V tile (A and B of an MMA must have the same 16-bit
 //                  type: an fp16 P against a bf16 V is an illegal instruction)
 //   O_part[128 x 32] = P V_tile          tcgen05.mma, added into fp32 registers by the row's thread
 //                  with the correction factor of the running maximum
 //
+// Two forms of the softmax.  A tile's scores are bounded by |q| |k| scale + bias, the largest of each over the tile (the
+// producers find them while they gather).  While that bound lies below kFastLimit the exponentials need no maximum:
+// upstream's own starts at 0, so with 0 as the reference nothing overflows, the result is the same quotient (the
+// denominator is at least 1 wherever a maximum above 0 would have been subtracted, and there 1e-8 is below its
+// rounding), no row statistics pass between threads, and the P V products of all key tiles add up in one
+// tensor-memory accumulator.  From the first key tile beyond the bound on, the query tile goes on with the
+// running maximum and an O_part per key tile.
+//
+// What bounds it is the hand-over between the roles, once per key tile: with the arithmetic, the row loads and all but two
+// MMAs taken out, more than half of the time stays.  So a tile is 128 keys.  A million voxels, half of the 9^3
+// windows full, six heads of bf16: 5.49 ms with 64-key tiles, P through shared memory and a running maximum throughout;
+// 5.09 with the bound and P in tensor memory; 4.53 with 128 keys a tile.  Four threads a row instead of two: no change.
+//
 // Warp roles (384 threads, one CTA per SM): warp 0 issues the MMAs (one elected lane) and owns the
 // tensor-memory allocation; warps 1-3 gather rows (plain 16-byte loads by voxel id, stored with the
 // 64-byte swizzle the operand descriptors name); warps 4-11 are the softmax rows: a warp may touch
 // the 32 tensor-memory lanes warp_id % 4 selects, so two warps share each quarter of the query
-// rows, one for the first 32 keys of a tile and the first 16 output channels, one for the rest
+// rows, one for the first 64 keys of a tile and the first 16 output channels, one for the rest
 // (they exchange their partial row maxima per tile and their row sums per query tile through shared
 // memory): two warps per scheduler instead of one.  Everything is handed over through mbarriers
 // with bounded waits; on expiry the kernel sets SSW_DEV_TIMEOUT, lets the tensor cores drain and
@@ -36,10 +49,10 @@
 namespace ssw {
 
 constexpr int kDQ = 128;       // query rows per tile = MMA M
-constexpr int kDK = 64;        // keys per tile
+constexpr int kDK = 128;       // keys per tile
 constexpr int kDHD = 32;       // head_dim
 constexpr int kDRowB = 64;     // bytes of one q / k / v head slice (32 x 16 bit)
-constexpr int kDMaxKT = 16;    // key tiles per window at most (1024 keys)
+constexpr int kDMaxKT = 8;     // key tiles per window at most (1024 keys)
 constexpr int kDProd = 3;      // producer warps
 constexpr int kDParts = 2;     // softmax threads per query row, in different warps (2 or 4; measured equal)
 constexpr int kDSoftWarps = 4 * kDParts;
@@ -47,8 +60,18 @@ constexpr int kDThreads = 128 + 32 * kDSoftWarps;
 constexpr int kDHalf = kDK / kDParts;  // keys of a tile one softmax thread looks after
 constexpr int kDCpt = kDHD / kDParts;  // output channels one softmax thread accumulates
 constexpr int kDOutPitch = kDRowB + 16;  // bytes between rows of the output staging tile (skewed across banks)
-constexpr int kTmemCols = 256; // S: 2 x 64 columns, O_part: 2 x 32 columns
-constexpr int kTmemS = 0, kTmemO = 128;
+constexpr int kDSub = 32;       // keys a softmax thread takes at a time
+constexpr int kDSBuf = 2;      // S tiles in tensor memory: the scores run up to three tiles ahead of the softmax
+constexpr int kTmemCols = 512; // S: 2 x 128 columns, O_part: 2 x 32, O_acc: 32, P: 64 + 64 of rounding residuals
+constexpr int kTmemS = 0, kTmemO = 256, kTmemOAcc = 320, kTmemP = 352;
+// Scores (log2 domain) up to which probabilities relative to 0 are formed: exp2 of it times 1024 keys times a v below
+// 2^60 stays far inside fp32, and inside the 16-bit type of P.
+template <typename T>
+struct DenseFast;
+template <>
+struct DenseFast<__nv_bfloat16> { static constexpr float kLimit = 40.f; static constexpr uint32_t kMaxV = (127u + 60u) << 7; };
+template <>
+struct DenseFast<__half> { static constexpr float kLimit = 15.f; static constexpr uint32_t kMaxV = 0x7c00u; };
 
 struct DenseParams {
   const void* qkv;
@@ -68,20 +91,15 @@ struct DenseParams {
   int use_mask;
 };
 
-__device__ __forceinline__ uint32_t f2h2(float a, float b) {  // two floats -> packed fp16 pair
-  __half2 v = __floats2half2_rn(a, b);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-
 // Shared memory (byte offsets from a 1024-byte aligned base):
 //   [0, 1024)        mbarriers and the tensor-memory address
 //   [1024, 1024 + 2 * kDParts * 512)  partial row maxima / sums the softmax threads of a row exchange
-//   K  c_cap x 64    V  c_cap x 64    (64-byte swizzle; key tile j = rows [64 j, 64 j + 64))
-//   Q  2 x 128 x 64  (64-byte swizzle)          P  128 x 128 (128-byte swizzle) twice: P and its bf16 residual
+//   K  c_cap x 64    V  c_cap x 64    (64-byte swizzle; key tile j = rows [128 j, 128 j + 128))
+//   Q  2 x 128 x 64  (64-byte swizzle)
 //   per unit (double buffered): the bias slice of its head, (2Wz-1)(2Wy-1)(2Wx-1) floats
 //   pre-multiplied by log2 e; per row of its window the voxel id, 4 x relative-position code, region
 struct DenseSmem {
-  uint32_t k, v, q, p, bias, bias_floats, vox, rel4, reg, ostage, total;
+  uint32_t k, v, q, bias, bias_floats, vox, rel4, reg, ostage, total;
 };
 __host__ __device__ inline DenseSmem dense_smem(int c_cap, int table_rows) {
   DenseSmem s;
@@ -89,7 +107,6 @@ __host__ __device__ inline DenseSmem dense_smem(int c_cap, int table_rows) {
   s.k = o; o += (uint32_t)c_cap * kDRowB;
   s.v = o; o += (uint32_t)c_cap * kDRowB;
   s.q = o; o += 2u * kDQ * kDRowB;
-  s.p = o; o += 2u * kDQ * 128u;
   s.bias_floats = ((uint32_t)table_rows + 3u) & ~3u;
   s.bias = o; o += 2u * s.bias_floats * 4u;
   s.vox = o; o += 2u * (uint32_t)c_cap * 4u;
@@ -111,9 +128,9 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
   uint64_t* kv_empty = bars + kDMaxKT;         // [kDMaxKT] the unit's last MMA on key tile j is done
   uint64_t* q_full = bars + 2 * kDMaxKT;       // [2]
   uint64_t* q_empty = q_full + 2;              // [2]
-  uint64_t* s_full = q_empty + 2;              // [2] S tile in tensor memory
-  uint64_t* s_empty = s_full + 2;              // [2] S tile read out
-  uint64_t* p_full = s_empty + 2;              // [2] P tile in shared memory
+  uint64_t* s_full = q_empty + 2;              // [kDSBuf] S tile in tensor memory
+  uint64_t* s_empty = s_full + kDSBuf;         // [kDSBuf] S tile read out
+  uint64_t* p_full = s_empty + kDSBuf;         // [2] P tile in tensor memory
   uint64_t* pv_done = p_full + 2;              // [2] P V of the tile done: O_part ready, P buffer free
   uint64_t* o_empty = pv_done + 2;             // [2] O_part read out
   uint64_t* meta_full = o_empty + 2;           // [2] a unit's header: voxel ids, metadata, bias slice of its head
@@ -121,7 +138,14 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
   uint64_t* drain_bar = meta_empty + 2;        // [1]
   uint64_t* xbar = drain_bar + 1;              // [4] the two warps of a row quarter have posted their partial values
   uint64_t* obar = xbar + 4;                   // [1] output staging tile: written by all / read by all
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(obar + 1);
+  uint64_t* oacc_empty = obar + 1;             // [1] a query tile's O_acc has been read (one phase per query tile)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(oacc_empty + 1);
+  int* unit_c = reinterpret_cast<int*>(tmem_slot + 1);      // [2] voxels of the unit's window, with its metadata
+  int* fast_flag = unit_c + 2;                              // [2] the P tile is relative to 0: P V goes to O_acc
+  // largest squared norms of a tile's rows, one word per producer warp (the fourth unused)
+  float4* k_norm = reinterpret_cast<float4*>(smem + 512);   // [kDMaxKT]; infinite where a v is too large for O_acc
+  float4* q_norm = k_norm + kDMaxKT;                        // [4] by query tile number
+  float4* b_max = q_norm + 4;                               // [2] largest entry (or 0) of the unit's bias slice
   float* xch = reinterpret_cast<float*>(smem + 1024);  // [2 buffers][kDParts][128 rows] partial maxima / sums
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int H = p.H, C = p.C;
@@ -143,16 +167,19 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
     for (int b = 0; b < 2; ++b) {
       mbar_init(q_full + b, kDProd);
       mbar_init(q_empty + b, 1);
-      mbar_init(s_full + b, 1);
-      mbar_init(s_empty + b, kDSoftWarps);
       mbar_init(p_full + b, kDSoftWarps);
       mbar_init(pv_done + b, 1);
       mbar_init(o_empty + b, kDSoftWarps);
       mbar_init(meta_full + b, kDProd);
       mbar_init(meta_empty + b, kDSoftWarps);
     }
+    for (int b = 0; b < kDSBuf; ++b) {
+      mbar_init(s_full + b, 1);
+      mbar_init(s_empty + b, kDSoftWarps);
+    }
     for (int x = 0; x < 4; ++x) mbar_init(xbar + x, kDParts);
     mbar_init(obar, kDSoftWarps);
+    mbar_init(oacc_empty, kDSoftWarps);
     mbar_init(drain_bar, 1);
     mbar_fence_init();
   }
@@ -178,8 +205,8 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
     const bool ok = c > p.tile && c <= p.c_cap && first >= 0 && first <= p.n_vox - c;
     if (!ok) {
       atomicOr(reinterpret_cast<unsigned*>(p.header + SSW_H_ERROR), SSW_DEV_BAD_PLAN);
-      first = 0;
-      c = 0;
+      first = 0;   // a one-row window instead: the result is flagged, and every role still finds work
+      c = 1;
     }
   };
   const int a_fmt_qk = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
@@ -187,66 +214,88 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
 
   if (warp == 0) {
     // =========================================== MMA issuer ===================================
-    const uint32_t sK = smem_u32(smem + L.k), sV = smem_u32(smem + L.v), sQ = smem_u32(smem + L.q), sP = smem_u32(smem + L.p);
-    uint32_t g = 0;          // key tiles issued so far (S / P / O_part buffer = g & 1)
-    uint32_t qn = 0;         // query tiles so far (Q buffer = qn & 1)
-    int un = 0;              // units so far
-    for (int u = blockIdx.x; u < n_units && !timed_out; u += gridDim.x, ++un) {
-      int first, c, h;
-      unit_window(u, first, c, h);
-      const int nkt = (c + kDK - 1) / kDK, nqt = (c + kDQ - 1) / kDQ;
-      for (int t = 0; t < nqt && !timed_out; ++t, ++qn) {
-        const uint32_t qb = qn & 1;
-        if (!mbar_wait_bounded(q_full + qb, (qn >> 1) & 1)) { timed_out = true; break; }
-        // software pipeline: S of tile j is issued before P V of tile j - 1, so the tensor cores
-        // work on the next scores while the softmax rows are busy with the current ones
-        for (int j = 0; j <= nkt && !timed_out; ++j) {
-          if (j < nkt) {
-            const uint32_t b = g & 1;
-            const int nk16 = (min(kDK, c - j * kDK) + 15) & ~15;
-            if (t == 0 && !mbar_wait_bounded(kv_full + j, un & 1)) { timed_out = true; break; }
-            if (g >= 2 && !mbar_wait_bounded(s_empty + b, ((g >> 1) - 1) & 1)) { timed_out = true; break; }
-            tc_fence_after();
-            if (lane == 0) {
-              const uint32_t idesc = instr_desc(a_fmt_qk, a_fmt_qk, 0, nk16);
-#pragma unroll
-              for (int ks = 0; ks < kDHD / 16; ++ks)
-                umma_ss(tmem + kTmemS + b * kDK, smem_desc(sQ + qb * (kDQ * kDRowB) + ks * 32, 512, 4),
-                        smem_desc(sK + j * (kDK * kDRowB) + ks * 32, 512, 4), idesc, ks > 0);
-              umma_commit(s_full + b);
-            }
-            __syncwarp();
-            ++g;
+    // One lane, two positions in the same sequence of key tiles: `sp`, the next tile whose scores are formed, runs up to
+    // kDSBuf - 1 tiles ahead of `pp`, the next one whose P V is (also across query tiles and units).  It takes whichever
+    // can go: if the scores waited in turn for the P V before them, the softmax would wait for both.
+    struct Pos {
+      uint32_t g, qn;              // key tiles / query tiles before it
+      int u, un, t, j, c;          // unit, units before it, query tile, key tile, the window's voxels (0: not yet read)
+      uint32_t kv;                 // bit j: parity of the uses of key tile j by earlier units
+    };
+    auto advance = [&](Pos& x) {
+      ++x.g;
+      if (++x.j * kDK < x.c) return;
+      x.j = 0;
+      ++x.qn;
+      if (++x.t * kDQ < x.c) return;
+      x.t = 0;
+      x.kv ^= (1u << ((x.c + kDK - 1) / kDK)) - 1u;
+      x.c = 0;
+      ++x.un;
+      x.u += gridDim.x;
+    };
+    if (lane == 0) {
+      const uint32_t sK = smem_u32(smem + L.k), sV = smem_u32(smem + L.v), sQ = smem_u32(smem + L.q);
+      Pos sp = {0, 0, (int)blockIdx.x, 0, 0, 0, 0, 0u}, pp = sp;
+      uint32_t idle = 0;
+      while (pp.u < n_units) {
+        bool moved = false;
+        // ---- scores of the next tile
+        if (sp.u < n_units && sp.g - pp.g < (uint32_t)kDSBuf) {
+          if (sp.c == 0 && mbar_test(meta_full + (sp.un & 1), (sp.un >> 1) & 1)) {
+            sp.c = *reinterpret_cast<volatile int*>(unit_c + (sp.un & 1));
           }
-          if (j > 0) {
-            const uint32_t gp = g - (j < nkt ? 2 : 1);  // the tile whose P is multiplied now
-            const uint32_t b = gp & 1;
-            const int jp = j - 1;
-            const int nk16 = (min(kDK, c - jp * kDK) + 15) & ~15;
-            if (!mbar_wait_bounded(p_full + b, (gp >> 1) & 1)) { timed_out = true; break; }
-            if (gp >= 2 && !mbar_wait_bounded(o_empty + b, ((gp >> 1) - 1) & 1)) { timed_out = true; break; }
+          const uint32_t b = sp.g % kDSBuf, qb = sp.qn & 1;
+          if (sp.c > 0 && (sp.j > 0 || mbar_test(q_full + qb, (sp.qn >> 1) & 1)) &&
+              (sp.t > 0 || mbar_test(kv_full + sp.j, (sp.kv >> sp.j) & 1)) &&
+              (sp.g < (uint32_t)kDSBuf || mbar_test(s_empty + b, (sp.g / kDSBuf - 1) & 1))) {
             tc_fence_after();
-            if (lane == 0) {
-              const uint32_t idesc = instr_desc(a_fmt_qk, a_fmt_qk, 1, kDHD);  // A = P, B = V (MN-major)
-              for (int part = 0; part < (kSplitP ? 2 : 1); ++part)   // P, then its rounding residual
-                for (int ks = 0; ks < nk16 / 16; ++ks)
-                  umma_ss(tmem + kTmemO + b * kDHD, smem_desc(sP + part * (kDQ * 128) + ks * 32, 1024, 2),
-                          smem_desc(sV + jp * (kDK * kDRowB) + ks * (16 * kDRowB), 512, 4), idesc, (part | ks) > 0);
-              umma_commit(pv_done + b);
-              if (t == nqt - 1) umma_commit(kv_empty + jp);  // the window's last use of key tile jp
-            }
-            __syncwarp();
+            const int nk16 = (min(kDK, sp.c - sp.j * kDK) + 15) & ~15;
+            const uint32_t idesc = instr_desc(a_fmt_qk, a_fmt_qk, 0, nk16);
+#pragma unroll
+            for (int ks = 0; ks < kDHD / 16; ++ks)
+              umma_ss(tmem + kTmemS + b * kDK, smem_desc(sQ + qb * (kDQ * kDRowB) + ks * 32, 512, 4),
+                      smem_desc(sK + sp.j * (kDK * kDRowB) + ks * 32, 512, 4), idesc, ks > 0);
+            umma_commit(s_full + b);
+            if ((sp.j + 1) * kDK >= sp.c) umma_commit(q_empty + qb);  // every S of this query tile has been issued
+            advance(sp);
+            moved = true;
           }
         }
-        if (lane == 0) umma_commit(q_empty + qb);  // every S of this query tile has been computed
-        __syncwarp();
+        // ---- P V of the oldest tile whose scores have been formed
+        if (pp.g != sp.g) {
+          if (pp.c == 0) pp.c = *reinterpret_cast<volatile int*>(unit_c + (pp.un & 1));  // (sp has seen its meta_full)
+          const uint32_t b = pp.g & 1;
+          if (mbar_test(p_full + b, (pp.g >> 1) & 1)) {
+            const bool fast = *reinterpret_cast<volatile int*>(fast_flag + b) != 0;
+            // O_acc starts over with the query tile: the one before must have been read.  O_part: the tile two before.
+            const bool go = fast ? pp.j > 0 || pp.qn == 0 || mbar_test(oacc_empty, (pp.qn - 1) & 1)
+                                 : pp.g < 2 || mbar_test(o_empty + b, ((pp.g >> 1) - 1) & 1);
+            if (go) {
+              tc_fence_after();
+              const int nk16 = (min(kDK, pp.c - pp.j * kDK) + 15) & ~15;
+              const uint32_t idesc = instr_desc(a_fmt_qk, a_fmt_qk, 1, kDHD);  // A = P, B = V (MN-major)
+              const uint32_t dst = fast ? tmem + kTmemOAcc : tmem + kTmemO + b * kDHD;
+              for (int part = 0; part < (kSplitP ? 2 : 1); ++part)   // P, then its rounding residual
+                for (int ks = 0; ks < nk16 / 16; ++ks)
+                  umma_ts(dst, tmem + kTmemP + part * (kDK / 2) + ks * 8,
+                          smem_desc(sV + pp.j * (kDK * kDRowB) + ks * (16 * kDRowB), 512, 4), idesc,
+                          (part | ks) > 0 || (fast && pp.j > 0));
+              umma_commit(pv_done + b);
+              if ((pp.t + 1) * kDQ >= pp.c) umma_commit(kv_empty + pp.j);  // the window's last use of the key tile
+              advance(pp);
+              moved = true;
+            }
+          }
+        }
+        idle = moved ? 0 : idle + 1;
+        if (idle > (1u << 24)) {
+          timed_out = true;
+          break;
+        }
       }
-      // Key tiles this window does not have: their barriers advance one phase per unit all the
-      // same, so that a unit's number gives every barrier's phase whatever the windows' sizes.
-      if (lane == 0)
-        for (int j = nkt; j < kDMaxKT; ++j) umma_commit(kv_empty + j);
-      __syncwarp();
     }
+    __syncwarp();
     // let the tensor cores finish whatever was issued before the tensor memory is given back
     if (lane == 0) umma_commit(drain_bar);
     __syncwarp();
@@ -257,8 +306,11 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
     const int chunk = lane & 3, rsub = lane >> 2;
     const T* qkv = reinterpret_cast<const T*>(p.qkv);
     // rows [r0, r0 + n_rows) of the window -> tile at `dst` (64-byte rows, 64-byte swizzle); rows
-    // from `c` on are zero.  `part`: 0 q, 1 k, 2 v.  Row groups of eight are dealt to the warps.
-    auto gather = [&](unsigned char* dst, const int* wvox, int r0, int n_rows, int c, int part, int h) {
+    // from `c` on are zero.  `part`: 0 q, 1 k, 2 v.  Row groups of eight are dealt to the warps.  Returns the largest
+    // squared norm of this warp's rows (q, k; infinite if one is not finite), or 0 / infinity (v: within kMaxV or not).
+    auto gather = [&](unsigned char* dst, const int* wvox, int r0, int n_rows, int c, int part, int h) -> float {
+      float top = 0.f;
+      uint32_t vm = 0;
       const int n_groups = (n_rows + 7) >> 3;
       for (int g0 = pw; g0 < n_groups; g0 += kDProd * 4) {
         uint4 val[4];
@@ -276,10 +328,27 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
           const int gi = g0 + x * kDProd, rl = gi * 8 + rsub;
           if (gi < n_groups && rl < n_rows)
             *reinterpret_cast<uint4*>(dst + (size_t)rl * kDRowB + ((chunk ^ ((rl >> 1) & 3)) << 4)) = val[x];
+          if (part == 2) {
+            vm = __vmaxu2(__vmaxu2(vm, __vmaxu2(val[x].x & 0x7fff7fffu, val[x].y & 0x7fff7fffu)),
+                          __vmaxu2(val[x].z & 0x7fff7fffu, val[x].w & 0x7fff7fffu));
+          } else {
+            float4 a, b;
+            widen8<T>(val[x], a, b);
+            float n2 = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, a.w * a.w))) + fmaf(b.x, b.x, fmaf(b.y, b.y, fmaf(b.z, b.z, b.w * b.w)));
+            n2 += __shfl_xor_sync(0xffffffffu, n2, 1);  // the four lanes of a row
+            n2 += __shfl_xor_sync(0xffffffffu, n2, 2);
+            top = n2 <= 3.0e38f ? fmaxf(top, n2) : INFINITY;  // (NaN as well)
+          }
         }
       }
+      if (part == 2) {
+        const uint32_t m16 = __reduce_max_sync(0xffffffffu, max(vm & 0xffffu, vm >> 16));
+        return m16 < DenseFast<T>::kMaxV ? 0.f : INFINITY;
+      }
+      return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(top)));  // not negative: ordered as integers
     };
     uint32_t qn = 0;
+    uint32_t kv_used = 0, kv_par = 0;   // bit j: key tile j has been filled before / how often, modulo two
     int un = 0;
     for (int u = blockIdx.x; u < n_units && !timed_out; u += gridDim.x, ++un) {
       int first, c, h;
@@ -291,6 +360,7 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
       int* wreg = reinterpret_cast<int*>(smem + L.reg) + mb * p.c_cap;
       // ---- the window's voxel ids and metadata
       if (un >= 2 && !mbar_wait_bounded(meta_empty + mb, ((un >> 1) - 1) & 1)) { timed_out = true; break; }
+      if (pw == 0 && lane == 0) unit_c[mb] = c;
       for (int r = pw * 32 + lane; r < nkt * kDK; r += kDProd * 32) {  // (rows from c on: neutral entries)
         int vx = 0, m = 0;
         if (r < c) {
@@ -306,7 +376,14 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
       // ---- the head's bias slice (rows of the table are [code][head])
       {
         float* bs = reinterpret_cast<float*>(smem + L.bias) + (size_t)mb * L.bias_floats;
-        for (int i = pw * 32 + lane; i < p.table_rows; i += kDProd * 32) bs[i] = __ldg(p.table + (int64_t)i * H + h) * kLog2e;
+        float bm = 0.f;
+        for (int i = pw * 32 + lane; i < p.table_rows; i += kDProd * 32) {
+          const float b = __ldg(p.table + (int64_t)i * H + h) * kLog2e;
+          bs[i] = b;
+          bm = b <= 3.0e38f ? fmaxf(bm, b) : INFINITY;
+        }
+        const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bm)));
+        if (lane == 0) reinterpret_cast<float*>(b_max + mb)[pw] = top;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(meta_full + mb);
@@ -314,10 +391,11 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
       if (!mbar_wait_bounded(meta_full + mb, (un >> 1) & 1)) { timed_out = true; break; }
       // ---- key tiles (k and v), the first query tile in between so that the MMAs can start early
       for (int j = 0; j < nkt && !timed_out; ++j) {
-        if (un >= 1 && !mbar_wait_bounded(kv_empty + j, (un - 1) & 1)) { timed_out = true; break; }
+        if ((kv_used >> j & 1) && !mbar_wait_bounded(kv_empty + j, (kv_par >> j & 1) ^ 1)) { timed_out = true; break; }
         const int n_rows = (min(kDK, c - j * kDK) + 15) & ~15;
-        gather(smem + L.k + (size_t)j * kDK * kDRowB, wvox, j * kDK, n_rows, c, 1, h);
-        gather(smem + L.v + (size_t)j * kDK * kDRowB, wvox, j * kDK, n_rows, c, 2, h);
+        const float kn = gather(smem + L.k + (size_t)j * kDK * kDRowB, wvox, j * kDK, n_rows, c, 1, h);
+        const float vn = gather(smem + L.v + (size_t)j * kDK * kDRowB, wvox, j * kDK, n_rows, c, 2, h);
+        if (lane == 0) reinterpret_cast<float*>(k_norm + j)[pw] = fmaxf(kn, vn);
         fence_async_smem();  // the tensor cores read shared memory through the async proxy
         __syncwarp();
         if (lane == 0) mbar_arrive(kv_full + j);
@@ -327,18 +405,16 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
           for (int t = (nkt == 1 ? 0 : t_lo); t < (nkt == 1 ? nqt : t_hi) && !timed_out; ++t) {
             const uint32_t qi = qn + t, qb = qi & 1;
             if (qi >= 2 && !mbar_wait_bounded(q_empty + qb, ((qi >> 1) - 1) & 1)) { timed_out = true; break; }
-            gather(smem + L.q + (size_t)qb * kDQ * kDRowB, wvox, t * kDQ, kDQ, c, 0, h);
+            const float qm = gather(smem + L.q + (size_t)qb * kDQ * kDRowB, wvox, t * kDQ, kDQ, c, 0, h);
+            if (lane == 0) reinterpret_cast<float*>(q_norm + (qi & 3))[pw] = qm;
             fence_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(q_full + qb);
           }
         }
       }
-      // key tiles this window does not have (see the MMA warp)
-      for (int j = nkt; j < kDMaxKT && !timed_out; ++j) {
-        if (un >= 1 && !mbar_wait_bounded(kv_empty + j, (un - 1) & 1)) { timed_out = true; break; }
-        if (lane == 0) mbar_arrive(kv_full + j);
-      }
+      kv_used |= (1u << nkt) - 1u;
+      kv_par ^= (1u << nkt) - 1u;
       qn += nqt;
     }
   } else {
@@ -370,6 +446,7 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
       return ok;
     };
     uint32_t on = 0;  // query tiles this thread has put through the output staging tile
+    uint32_t qt = 0;  // query tiles begun
     for (int u = blockIdx.x; u < n_units && !timed_out; u += gridDim.x, ++un) {
       int first, c, h;
       unit_window(u, first, c, h);
@@ -388,6 +465,8 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
         const uint32_t my_bias = bias_a + (uint32_t)(live ? wrel4[qrow] : 0) + (uint32_t)p.rel_off * 4u;
         const int my_region = live ? wreg[qrow] : 0;
         float m = 0.f, l = 0.f, corr_prev = 1.f;   // the maximum starts from 0 (ops.cu:137)
+        bool fast = true;       // every key tile so far was within the bound
+        float k_limit = 0.f;    // largest squared key norm the bound allows for this query tile
         float o[kDCpt];
 #pragma unroll
         for (int e = 0; e < kDCpt; ++e) o[e] = 0.f;
@@ -395,34 +474,122 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
           const uint32_t gp = g - 1, bp = gp & 1;
           if (j < nkt) {
             const uint32_t b = g & 1;
-            const int nk = min(kDK, c - j * kDK) - half * kDHalf;  // valid keys among this thread's 32
-            if (!mbar_wait_bounded(s_full + b, (g >> 1) & 1)) { timed_out = true; break; }
+            const int nk = min(kDK, c - j * kDK) - half * kDHalf;  // valid keys among this thread's 64
+            const uint32_t sb = g % kDSBuf;
+            if (!mbar_wait_bounded(s_full + sb, (g / kDSBuf) & 1)) { timed_out = true; break; }
             tc_fence_after();
-            uint32_t sr[kDHalf];
-            tmem_ldn(tmem + t_lane + kTmemS + b * kDK + half * kDHalf, sr);
-            tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(s_empty + b);
+            const uint32_t s_src = tmem + t_lane + kTmemS + sb * kDK + half * kDHalf;
+            const uint32_t p_dst = tmem + t_lane + kTmemP + half * (kDHalf / 2);  // two keys a column
+            if (j == 0) {
+              const float4 q4 = q_norm[qt & 3], b4 = b_max[mb];
+              const float lim = (DenseFast<T>::kLimit - fmaxf(fmaxf(b4.x, b4.y), b4.z)) / fabsf(qscale);
+              const float q2 = fmaxf(fmaxf(q4.x, q4.y), q4.z);
+              k_limit = lim > 0.f && q2 <= 3.0e38f ? lim * lim / fmaxf(q2, 1e-30f) : -1.f;
+            }
+            const float4 k4 = k_norm[j];
+            const bool was_fast = fast;
+            fast = fast && fmaxf(fmaxf(k4.x, k4.y), k4.z) <= k_limit;   // the same in every softmax thread
+            if (fast) {
+              // Packed arithmetic, two keys at a time; nothing here depends on the tile before until P is stored.
+              float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+              const float2 qs2 = make_float2(qscale, qscale), neg = make_float2(-1.f, -1.f);
+#pragma unroll
+              for (int sub = 0; sub < kDHalf / kDSub; ++sub) {
+                uint32_t sr[kDSub], hi[kDSub / 2], lo[kDSub / 2];
+                tmem_ldn(s_src + sub * kDSub, sr);
+                tmem_ld_wait();
+                if (sub == kDHalf / kDSub - 1) {
+                  tc_fence_before();
+                  __syncwarp();
+                  if (lane == 0) mbar_arrive(s_empty + sb);
+                }
+                const int nks = nk - sub * kDSub;
+#pragma unroll
+                for (int q4 = 0; q4 < kDSub / 4; ++q4) {
+                  const uint32_t key4 = (uint32_t)(j * kDK + sub * kDSub + q4 * 4) * 4u;
+                  const int4 kr = lds_v4(rel4_a + key4);
+                  float2 bias[2] = {make_float2(lds_f32(my_bias - (uint32_t)kr.x), lds_f32(my_bias - (uint32_t)kr.y)),
+                                    make_float2(lds_f32(my_bias - (uint32_t)kr.z), lds_f32(my_bias - (uint32_t)kr.w))};
+                  if constexpr (kMask) {
+                    const int4 kg = lds_v4(reg_a + key4);
+                    if (kg.x != my_region) bias[0].x += -100.0f * kLog2e;
+                    if (kg.y != my_region) bias[0].y += -100.0f * kLog2e;
+                    if (kg.z != my_region) bias[1].x += -100.0f * kLog2e;
+                    if (kg.w != my_region) bias[1].y += -100.0f * kLog2e;
+                  }
+#pragma unroll
+                  for (int x = 0; x < 2; ++x) {
+                    const int jj = q4 * 4 + x * 2;
+                    const float2 v = __ffma2_rn(make_float2(__uint_as_float(sr[jj]), __uint_as_float(sr[jj + 1])), qs2, bias[x]);
+                    float2 pv = make_float2(fast_exp2(v.x), fast_exp2(v.y));
+                    if (nks < kDSub) {  // the window's last key tile: nothing beyond its last voxel
+                      if (jj >= nks) pv.x = 0.f;
+                      if (jj + 1 >= nks) pv.y = 0.f;
+                    }
+                    sum2[x] = __fadd2_rn(sum2[x], pv);
+                    hi[jj / 2] = pack2<T>(pv.x, pv.y);
+                    if constexpr (kSplitP) {
+                      const float2 res = __ffma2_rn(make_float2(__uint_as_float(hi[jj / 2] << 16), __uint_as_float(hi[jj / 2] & 0xffff0000u)), neg, pv);
+                      lo[jj / 2] = pack2<T>(res.x, res.y);
+                    }
+                  }
+                }
+                // the P buffer is free once the P V of the tile before is done
+                if (sub == 0 && g >= 1 && !mbar_wait_bounded(pv_done + bp, (gp >> 1) & 1)) timed_out = true;
+                tmem_stn(p_dst + sub * (kDSub / 2), hi);
+                if constexpr (kSplitP) tmem_stn(p_dst + kDK / 2 + sub * (kDSub / 2), lo);
+              }
+              if (timed_out) break;
+              l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
+              if (threadIdx.x == 128) fast_flag[b] = 1;
+              tmem_st_wait();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) {
+                mbar_arrive(p_full + b);
+                if (j > 0) mbar_arrive(o_empty + bp);  // O_part of the tile before was not used: its phase goes on
+              }
+              ++g;
+              continue;
+            }
+            if (was_fast && j > 0) {  // from here on with a running maximum: what has been added up so far is relative to 0
+              if (!mbar_wait_bounded(pv_done + bp, (gp >> 1) & 1)) { timed_out = true; break; }
+              tc_fence_after();
+              uint32_t orr[kDCpt];
+              tmem_ldn(tmem + t_lane + kTmemOAcc + half * kDCpt, orr);
+              tmem_ld_wait();
+              tc_fence_before();
+#pragma unroll
+              for (int e = 0; e < kDCpt; ++e) o[e] = __uint_as_float(orr[e]);
+            }
             // scores in the log2 domain: bias from the head's slice, -100 across regions, -inf beyond c
             float s[kDHalf];
 #pragma unroll
-            for (int q4 = 0; q4 < kDHalf / 4; ++q4) {
-              const int4 kr = lds_v4(rel4_a + (uint32_t)(j * kDK + q4 * 4) * 4u);
-              const int krv[4] = {kr.x, kr.y, kr.z, kr.w};
-              int kgv[4] = {0, 0, 0, 0};
-              if constexpr (kMask) {
-                const int4 kg = lds_v4(reg_a + (uint32_t)(j * kDK + q4 * 4) * 4u);
-                kgv[0] = kg.x; kgv[1] = kg.y; kgv[2] = kg.z; kgv[3] = kg.w;
-              }
+            for (int sub = 0; sub < kDHalf / kDSub; ++sub) {
+              uint32_t sr[kDSub];
+              tmem_ldn(s_src + sub * kDSub, sr);
+              tmem_ld_wait();
 #pragma unroll
-              for (int x = 0; x < 4; ++x) {
-                const int jj = q4 * 4 + x;
-                float v = fmaf(__uint_as_float(sr[jj]), qscale, lds_f32(my_bias - (uint32_t)krv[x]));
-                if (kMask && kgv[x] != my_region) v += -100.0f * kLog2e;
-                s[jj] = v;
+              for (int q4 = 0; q4 < kDSub / 4; ++q4) {
+                const uint32_t key4 = (uint32_t)(j * kDK + sub * kDSub + q4 * 4) * 4u;
+                const int4 kr = lds_v4(rel4_a + key4);
+                const int krv[4] = {kr.x, kr.y, kr.z, kr.w};
+                int kgv[4] = {0, 0, 0, 0};
+                if constexpr (kMask) {
+                  const int4 kg = lds_v4(reg_a + key4);
+                  kgv[0] = kg.x; kgv[1] = kg.y; kgv[2] = kg.z; kgv[3] = kg.w;
+                }
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                  float v = fmaf(__uint_as_float(sr[q4 * 4 + x]), qscale, lds_f32(my_bias - (uint32_t)krv[x]));
+                  if (kMask && kgv[x] != my_region) v += -100.0f * kLog2e;
+                  s[sub * kDSub + q4 * 4 + x] = v;
+                }
               }
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(s_empty + sb);
             if (nk < kDHalf) {  // the window's last key tile: nothing beyond its last voxel
 #pragma unroll
               for (int jj = 0; jj < kDHalf; ++jj) s[jj] = jj < nk ? s[jj] : -INFINITY;
@@ -439,41 +606,46 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
             const float m_new = fmaxf(m, fmaxf(mx, mx_other));
             const float corr = fast_exp2(m - m_new);
             m = m_new;
-            // The one P buffer was last read by the P V of the tile before; the same completion says
-            // that tile's O_part is in tensor memory.
+            // O_part of the tile before is in tensor memory (and so the P buffer, last read by the tile before that, is free)
             if (g >= 1 && !mbar_wait_bounded(pv_done + bp, (gp >> 1) & 1)) { timed_out = true; break; }
-            const uint32_t prow = smem_u32(smem + L.p) + (uint32_t)row_in_tile * 128u;
             float sum4[4] = {0.f, 0.f, 0.f, 0.f};  // partial row sums, one per pair position
 #pragma unroll
-            for (int ch = 0; ch < kDHalf / 8; ++ch) {
-              uint32_t hi[4], lo[4];
+            for (int sub = 0; sub < kDHalf / kDSub; ++sub) {
+              uint32_t hi[kDSub / 2], lo[kDSub / 2];
 #pragma unroll
-              for (int x = 0; x < 4; ++x) {
-                const float p0 = fast_exp2(s[8 * ch + 2 * x] - m), p1 = fast_exp2(s[8 * ch + 2 * x + 1] - m);
-                sum4[x] += p0 + p1;
+              for (int x = 0; x < kDSub / 2; ++x) {
+                const float p0 = fast_exp2(s[sub * kDSub + 2 * x] - m), p1 = fast_exp2(s[sub * kDSub + 2 * x + 1] - m);
+                sum4[x & 3] += p0 + p1;
                 hi[x] = pack2<T>(p0, p1);
                 if constexpr (kSplitP)
                   lo[x] = pack2<T>(p0 - __uint_as_float(hi[x] << 16), p1 - __uint_as_float(hi[x] & 0xffff0000u));
               }
-              const int chg = half * (kDHalf / 8) + ch;  // 16-byte chunk of the tile's 128-byte row
-              sts_v4(prow + ((chg ^ (row_in_tile & 7)) << 4), hi[0], hi[1], hi[2], hi[3]);
-              if constexpr (kSplitP) sts_v4(prow + kDQ * 128 + ((chg ^ (row_in_tile & 7)) << 4), lo[0], lo[1], lo[2], lo[3]);
+              tmem_stn(p_dst + sub * (kDSub / 2), hi);
+              if constexpr (kSplitP) tmem_stn(p_dst + kDK / 2 + sub * (kDSub / 2), lo);
             }
             l = l * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-            fence_async_smem();
+            if (threadIdx.x == 128) fast_flag[b] = 0;
+            tmem_st_wait();
+            tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(p_full + b);
             // fold the previous tile's O_part in with the factor its maximum update gave
             if (j > 0) {
-              tc_fence_after();
-              uint32_t orr[kDCpt];
-              tmem_ldn(tmem + t_lane + kTmemO + bp * kDHD + half * kDCpt, orr);
-              tmem_ld_wait();
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(o_empty + bp);
+              if (was_fast) {
+                // O_acc was taken over above; it is scaled like a previous O_part whose own factor is 1
+                __syncwarp();
+                if (lane == 0) mbar_arrive(o_empty + bp);
+              } else {
+                tc_fence_after();
+                uint32_t orr[kDCpt];
+                tmem_ldn(tmem + t_lane + kTmemO + bp * kDHD + half * kDCpt, orr);
+                tmem_ld_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(o_empty + bp);
 #pragma unroll
-              for (int e = 0; e < kDCpt; ++e) o[e] = fmaf(o[e], corr_prev, __uint_as_float(orr[e]));
+                for (int e = 0; e < kDCpt; ++e) o[e] = fmaf(o[e], corr_prev, __uint_as_float(orr[e]));
+              }
             }
             corr_prev = corr;
             ++g;
@@ -481,13 +653,16 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
             if (!mbar_wait_bounded(pv_done + bp, (gp >> 1) & 1)) { timed_out = true; break; }
             tc_fence_after();
             uint32_t orr[kDCpt];
-            tmem_ldn(tmem + t_lane + kTmemO + bp * kDHD + half * kDCpt, orr);
+            tmem_ldn(tmem + t_lane + (fast ? kTmemOAcc : kTmemO + bp * kDHD) + half * kDCpt, orr);
             tmem_ld_wait();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(o_empty + bp);
+            if (lane == 0) {
+              mbar_arrive(o_empty + bp);
+              mbar_arrive(oacc_empty);
+            }
 #pragma unroll
-            for (int e = 0; e < kDCpt; ++e) o[e] = fmaf(o[e], corr_prev, __uint_as_float(orr[e]));
+            for (int e = 0; e < kDCpt; ++e) o[e] = fast ? __uint_as_float(orr[e]) : fmaf(o[e], corr_prev, __uint_as_float(orr[e]));
           }
         }
         // the row's sum is the two halves' sums (both were kept relative to the same running maximum)
@@ -529,6 +704,7 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
         __syncwarp();
         if (lane == 0) mbar_arrive(obar);
         ++on;
+        ++qt;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(meta_empty + mb);

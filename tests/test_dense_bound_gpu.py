@@ -1,0 +1,69 @@
+"""Windows beyond a pack, 16-bit: query tiles whose scores stay within the bound, exceed it from some key tile on, or
+from the first, against the dense restatement in float64."""
+import pytest
+import torch
+
+from oracle import ssw_oracle as O
+from tests.cases import rel_err
+from tests.test_backward_tiles_gpu import _windows
+
+pytestmark = pytest.mark.gpu
+
+def _bound(dtype, v, ref):
+    """One rounding of the output (half an ulp: at most 2^-8 / 2^-11 of it) and that of the probabilities, which weigh values
+    up to max |v| (fp16: 2^-11; bf16 keeps the rounding residual as well: 2^-17), over the rms the error is measured by."""
+    p, out = (2.0 ** -17, 2.0 ** -8) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -11)
+    return out + p * float(v.double().abs().max() / ref.pow(2).mean().sqrt())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("loud", ["nothing", "late keys", "one query tile", "bias", "values", "all"])
+def test_bound_and_running_maximum(dtype, loud):
+    from sparseswin3d_b200 import attention, window
+
+    w, heads, hd = 9, 2, 32
+    counts = [65, 128, 129, 200, 729, 3, 70]   # (the window of three goes to the other kernel: not looked at)
+    coords, dims = _windows(counts, w, seed=5)
+    n = len(coords)
+    g = torch.Generator().manual_seed(11)
+    qkv = torch.randn(n, 3, heads, hd, generator=g)
+    table = torch.randn((2 * w - 1) ** 3, heads, generator=g) * 0.5
+    if dtype == torch.float16:
+        qkv[:, 0] *= 0.5                  # within 15 where nothing else is done to it
+    idx = O.window_keys(coords, 1, dims, (w,) * 3, (0, 0, 0))[0]
+    pos = idx[:, 1].long()
+    if loud == "late keys":               # the key tiles of the upper half of every window
+        qkv[pos > 400, 1] *= 12
+    elif loud == "one query tile":
+        qkv[(pos > 250) & (pos < 300), 0] *= 12
+    elif loud == "bias":
+        table[::7] += 60
+    elif loud == "values":
+        qkv[:, 2] *= 1e4 if dtype == torch.float16 else 1e25
+    elif loud == "all":
+        qkv[:, :2] *= 6
+    qkv = qkv.to(dtype)
+    geom = window.resolve_geometry(1, dims, (w,) * 3)
+    plan = window.bucket_windows(coords=coords.cuda(), geom=geom, **attention.plan_params(heads, hd, dtype, (w,) * 3))
+    out = attention.window_attention_fused(qkv.cuda(), plan, table.cuda(), hd ** -0.5)
+    plan.raise_on_error()
+    ref = O.dense_window_attention(qkv.double(), idx, hd ** -0.5, table.double(), O.relative_position_index((w,) * 3))
+    scale = 1e25 if loud == "values" and dtype == torch.bfloat16 else 1.0
+    here = idx[:, 0] != 5
+    assert rel_err(out.double().cpu()[here] / scale, ref[here] / scale) <= _bound(dtype, qkv[:, 2], ref)
+
+
+def test_values_that_are_not_finite_stay_in_their_window():
+    from sparseswin3d_b200 import attention, window
+
+    w, heads, hd = 9, 1, 32
+    coords, dims = _windows([300, 300, 300], w, seed=6)
+    qkv = torch.randn(900, 3, heads, hd).bfloat16()
+    win = O.window_keys(coords, 1, dims, (w,) * 3, (0, 0, 0))[0][:, 0]
+    hit = int((win == 1).nonzero()[5])
+    qkv[hit, 2, 0, 4], qkv[hit, 1, 0, 3] = float("nan"), float("inf")
+    geom = window.resolve_geometry(1, dims, (w,) * 3)
+    plan = window.bucket_windows(coords=coords.cuda(), geom=geom, **attention.plan_params(heads, hd, torch.bfloat16, (w,) * 3))
+    out = attention.window_attention_fused(qkv.cuda(), plan, torch.zeros((2 * w - 1) ** 3, heads, device="cuda"), hd ** -0.5).cpu()
+    plan.raise_on_error()
+    assert bool(out[win != 1].isfinite().all()) and not bool(out[win == 1][:, 4].isfinite().any())
