@@ -276,6 +276,12 @@ int ssw_layernorm_bwd(const void* x, const void* dy, const void* dsum, const voi
  * four: fp32 accuracy on the tensor cores (three bf16 terms per operand, see csrc/gemm_f32.cu). */
 int ssw_gemm_f32(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, void* stream);
 
+/* gelu(a w^T + bias), erf form, as one kernel: in fp32 with the arithmetic above, and in bf16 / fp16 with fp32
+ * accumulation and the activation taken before the one rounding (N and K multiples of eight; bias in `dtype` or NULL). */
+int ssw_gemm_f32_gelu(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, void* stream);
+int ssw_gemm_gelu(const void* a, const void* w, const void* bias, int dtype, void* out, int64_t M, int32_t N, int32_t K,
+                  void* stream);
+
 /* Weight gradient with the same arithmetic: out [N, K] = g [M, N]^T x [M, K], M > 0.  The workspace size is asked for with
  * the device the call will run on current. */
 int64_t ssw_gemm_f32_tn_workspace_floats(int64_t M, int32_t N, int32_t K);

@@ -57,6 +57,7 @@ constexpr int kGSmem = kGRawOff + kGRaw * kGRawB + 1024;
 struct GemmParams {
   const float *a, *w, *bias;
   float* out;
+  int gelu;               // the results go through GELU (erf form)
   int64_t M;
   int N, K;
   int bn, n_tiles;        // columns of a tile (a multiple of 16), tiles across N
@@ -95,10 +96,7 @@ __device__ __forceinline__ void split8(const float (&x)[8], uint4& h, uint4& m, 
 __device__ __forceinline__ void sts_u4(uint32_t a, const uint4& v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
-// 16 bytes from global to shared memory, asynchronously; zeros instead when !on
-__device__ __forceinline__ void cp_async16_or_zero(uint32_t dst, const void* src, bool on) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(on ? 16 : 0) : "memory");
-}
+__device__ __forceinline__ float gelu_erf(float x) { return x * 0.5f * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
 __device__ __forceinline__ void sts_v2(uint32_t a, uint2 v) {
   asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(v.x), "r"(v.y) : "memory");
@@ -381,6 +379,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
             if (timed_out) v = make_float4(NAN, NAN, NAN, NAN);  // never a plausible result
             if (on && m < p.M) {
               odd = odd || not_finite((v.x + v.y) + (v.z + v.w));
+              if (!TN && p.gelu) v = make_float4(gelu_erf(v.x), gelu_erf(v.y), gelu_erf(v.z), gelu_erf(v.w));
               *reinterpret_cast<float4*>(out + m * p.N + n) = v;
             }
           }
@@ -397,7 +396,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
               if (!not_finite(out[m * p.N + n + c])) continue;
               float v = 0.f;
               for (int k = 0; k < p.K; ++k) v = fmaf(__ldg(p.a + m * p.K + k), __ldg(p.w + (int64_t)(n + c) * p.K + k), v);
-              out[m * p.N + n + c] = p.bias ? v + __ldg(p.bias + n + c) : v;
+              if (p.bias) v += __ldg(p.bias + n + c);
+              out[m * p.N + n + c] = p.gelu ? gelu_erf(v) : v;
             }
           }
         }
@@ -453,7 +453,7 @@ static int gemm_columns(int64_t m_tiles, int N, int sms, int* n_tiles) {
   return best;
 }
 
-extern "C" int ssw_gemm_f32(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, void* stream_) {
+static int gemm_nt(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, int gelu, void* stream_) {
   if (M < 0 || N <= 0 || K <= 0) return SSW_E_INVALID;
   if (M == 0) return SSW_OK;
   if (!a || !w || !out) return SSW_E_INVALID;
@@ -465,7 +465,7 @@ extern "C" int ssw_gemm_f32(const float* a, const float* w, const float* bias, f
   SSW_CUDA_TRY(cudaGetDevice(&dev));
   SSW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   GemmParams p = {};
-  p.a = a; p.w = w; p.bias = bias; p.out = out; p.M = M; p.N = N; p.K = K;
+  p.a = a; p.w = w; p.bias = bias; p.out = out; p.M = M; p.N = N; p.K = K; p.gelu = gelu;
   const int64_t m_tiles = ceil_div64(M, kGM);
   p.bn = gemm_columns(m_tiles, N, sms, &p.n_tiles);
   if (m_tiles * p.n_tiles >= ((int64_t)1 << 30)) return SSW_E_RANGE;
@@ -475,6 +475,13 @@ extern "C" int ssw_gemm_f32(const float* a, const float* w, const float* bias, f
                               (cudaStream_t)stream_, p));
   SSW_LAUNCH_CHECK("k_gemm_f32");
   return SSW_OK;
+}
+
+extern "C" int ssw_gemm_f32(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, void* stream) {
+  return gemm_nt(a, w, bias, out, M, N, K, 0, stream);
+}
+extern "C" int ssw_gemm_f32_gelu(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, void* stream) {
+  return gemm_nt(a, w, bias, out, M, N, K, 1, stream);
 }
 
 // Weight gradient [N, K] of M rows: equal splits of M, as many as give every SM a tile, of two chunks at least.

@@ -174,18 +174,47 @@ class _Linear(torch.autograd.Function):
         return gx, gw, gb
 
 
-def linear(module: nn.Linear, x: torch.Tensor) -> torch.Tensor:
-    """module(x), through the passes above where they apply."""
+def _own_linear(module: nn.Linear, x: torch.Tensor) -> bool:
     w, b = module.weight, module.bias
-    if not (type(module) is nn.Linear and type(x) is torch.Tensor and x.dim() == 2 and x.is_cuda and x.shape[0] > 0 and x.dtype in _DTYPES
+    return (type(module) is nn.Linear and type(x) is torch.Tensor and x.dim() == 2 and x.is_cuda and x.shape[0] > 0 and x.dtype in _DTYPES
             and x.shape[1] == w.shape[1] and type(w) is nn.Parameter and w.dtype == x.dtype and w.device == x.device
             and x.device.index == torch.cuda.current_device()
             and (b is None or (type(b) is nn.Parameter and b.dtype == x.dtype and b.device == x.device))
-            and (w.shape[0] * x.element_size()) % 16 == 0 and unhooked(module) and _ordinary_mode()):
+            and (w.shape[0] * x.element_size()) % 16 == 0 and unhooked(module) and _ordinary_mode())
+
+
+def linear(module: nn.Linear, x: torch.Tensor) -> torch.Tensor:
+    """module(x), through the passes above where they apply."""
+    if not _own_linear(module, x):
         return module(x)
+    w, b = module.weight, module.bias
     if not torch.is_grad_enabled() or not (x.requires_grad or w.requires_grad or (b is not None and b.requires_grad)):
         return _affine(x, w, b)
     return _Linear.apply(x, w, b)
+
+
+def linear_gelu(module: nn.Linear, act: nn.Module, x: torch.Tensor) -> Optional[torch.Tensor]:
+    """act(module(x)) in one kernel; None where that is not to be had (autograd recording, another activation, shapes)."""
+    w, b = module.weight, module.bias
+    if not (type(act) is nn.GELU and act.approximate == "none" and unhooked(act) and _own_linear(module, x)) or (
+            torch.is_grad_enabled() and (x.requires_grad or w.requires_grad or (b is not None and b.requires_grad))):
+        return None
+    (m, k), n = x.shape, w.shape[0]
+    if x.dtype == torch.float32:
+        if not (_gemm_ready(x, w) and (b is None or b.data_ptr() % 16 == 0)):
+            return None
+        fn, args = lib.ssw_gemm_f32_gelu, ()
+    else:
+        # K up to 256: beyond it the library's GEMM gains more than the pass over the hidden rows costs (10 000 rows of 384:
+        # 35 us against 41; of 192: 25 against 20)
+        if not (k <= 256 and x.is_contiguous() and w.is_contiguous() and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
+                and n % 8 == 0 and k % 8 == 0
+                and (b is None or b.is_contiguous())):
+            return None
+        fn, args = lib.ssw_gemm_gelu, (dtype_code(x.dtype),)
+    out = torch.empty((m, n), dtype=x.dtype, device=x.device)
+    check(fn(ptr(x), ptr(w), ptr(b), *args, ptr(out), m, n, k, stream_ptr(x.device)), "ssw_gemm_gelu")
+    return out
 
 
 def layernorm_scatter(x: torch.Tensor, norm: nn.LayerNorm, parent: torch.Tensor, tap: torch.Tensor, owner: torch.Tensor) -> torch.Tensor:

@@ -115,7 +115,10 @@ class MLP(nn.Module):
         self.drop2 = self.drop1
 
     def forward(self, x):
-        return self.drop2(rows.linear(self.linear2, self.drop1(self.fn(rows.linear(self.linear1, x)))))
+        h = rows.linear_gelu(self.linear1, self.fn, x)
+        if h is None:
+            h = self.fn(rows.linear(self.linear1, x))
+        return self.drop2(rows.linear(self.linear2, self.drop1(h)))
 
 
 class SwinTransformerBlock(nn.Module):

@@ -142,3 +142,41 @@ def test_fp32_products_that_are_not_finite():
         assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf() & (got > 0), ref.isinf() & (ref > 0))
         ok = ref.isfinite()
         assert rel_err(got[ok].cpu(), ref[ok].cpu()) <= 1e-5
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_gelu_values(dtype):
+    """Identity weights: the activation alone, over its whole range, against float64."""
+    from sparseswin3d_b200 import rows
+
+    lin = nn.Linear(16, 16, bias=False).cuda().to(dtype)
+    with torch.no_grad():
+        lin.weight.copy_(torch.eye(16))
+        x = torch.linspace(-13, 13, 4096, device="cuda").reshape(-1, 16).to(dtype)
+        x[3, 2], x[5, 1], x[7, 0] = float("inf"), float("-inf"), float("nan")
+        got, xd = rows.linear_gelu(lin, nn.GELU(), x).double(), x.double()
+    ref = xd * 0.5 * torch.erfc(-xd / 2 ** 0.5)
+    row = torch.ones(256, dtype=torch.bool, device="cuda")
+    row[[3, 5, 7]] = False           # Inf and NaN times the zeros of the identity: NaN in the whole row, as in any product
+    half_ulp, tiny = {torch.float32: (2.0 ** -24, 0), torch.bfloat16: (2.0 ** -8, 0), torch.float16: (2.0 ** -11, 2.0 ** -24)}[dtype]
+    # fp32: erff has an absolute error of an ulp near -1, the 16-bit form a relative one of a few 1e-6
+    slack = xd.abs() * 2.0 ** -23 if dtype == torch.float32 else ref.abs() * 5e-6
+    assert bool(((got - ref).abs() <= ref.abs() * half_ulp + slack + tiny)[row].all())
+    assert torch.equal(got[~row].isnan(), F.gelu(x @ lin.weight.t())[~row].isnan())
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("M,N,K", [(1, 16, 16), (127, 64, 32), (129, 192, 48), (1000, 384, 96), (300, 136, 40), (20011, 192, 48), (2500, 1024, 256)])
+def test_linear_gelu(dtype, M, N, K):
+    from sparseswin3d_b200 import rows
+
+    lin = nn.Linear(K, N).cuda().to(dtype)
+    x = torch.randn(M, K, device="cuda").to(dtype)
+    with torch.no_grad():
+        got = rows.linear_gelu(lin, nn.GELU(), x)
+    assert got is not None
+    pre = x.double() @ lin.weight.detach().double().t() + lin.bias.detach().double()
+    assert rel_err(got.double().cpu(), F.gelu(pre).cpu()) <= {torch.float32: 3e-6, torch.float16: 1e-3, torch.bfloat16: 8e-3}[dtype]
+    assert rows.linear_gelu(lin, nn.GELU(), x) is None            # autograd recording: not here
+    with torch.no_grad():
+        assert rows.linear_gelu(lin, nn.GELU("tanh"), x) is None
