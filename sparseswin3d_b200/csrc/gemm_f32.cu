@@ -19,15 +19,15 @@
 // An Inf operand has no finite remainder (Inf - Inf), so a result that is not finite is formed again from the
 // operands as they are, by plain fp32 multiply-adds.
 //
-// Persistent, one block per SM, 17 warps: eight bring fp32 pieces in three stages ahead, split them and store the
+// Persistent, one block per SM, 17 warps: eight bring fp32 pieces in two stages ahead, split them and store the
 // six 64-byte-swizzled operand tiles of a stage (32 of K); one issues the MMAs; eight drain accumulators (a warp
 // may read the 32 tensor-memory lanes warp_id % 4 selects; two warps share them, half the columns each).
 // What bounds it: the issue slots of the split (4.5 instructions per element of both operands) about level with
 // the six MMAs per product.  Against the library's fp32 GEMM with bias:
-// 150 000 x 288 x 96 448 -> 103 us, 150 000 x 96 x 288 270 -> 79, 10 000 x 768 x 192 98 -> 39, 10 000 x 192 x 768
-// 75 -> 46, 128 x 96 x 96 22 -> 12.  Weight gradients: 150 000 rows 288 x 96 358 -> 150, 96 x 96 208 -> 71, 10 000 rows
-// 576 x 192 111 -> 46.  With the raw pieces in registers, two stages ahead, the latter took 226, 97 and 49: they wait for
-// memory, not for the split.
+// 150 000 x 288 x 96 448 -> 101 us, 150 000 x 96 x 288 270 -> 76, 10 000 x 768 x 192 98 -> 37, 10 000 x 192 x 768
+// 75 -> 46, 128 x 96 x 96 22 -> 12.  Weight gradients: 150 000 rows 288 x 96 358 -> 146, 96 x 96 208 -> 72, 10 000 rows
+// 576 x 192 111 -> 45.  With the raw pieces in registers the latter took 226, 97 and 49: they wait for memory, not for
+// the split.  Two split and three raw stages instead of three and two: 103, 79, 39 and 150.
 #include <math.h>
 
 #include "attn_common.cuh"
@@ -42,12 +42,13 @@ constexpr int kGRowB = kGK * 2;          // bytes of an operand row: one 64-byte
 // Stages whose h h products share an accumulator: two, and one for the long sums of a weight gradient.
 template <bool TN>
 struct GemmChunk { static constexpr int kStages = TN ? 1 : 2; };
-constexpr int kGStages = 2;              // of split operands
-constexpr int kGRaw = 3;                 // of fp32 pieces on their way, each read by the thread that asked for it
+constexpr int kGStages = 3;              // of split operands
+constexpr int kGRaw = 2;                 // of fp32 pieces on their way, each read by the thread that asked for it
 constexpr int kGProd = 8, kGEpi = 8;     // warps
 constexpr int kGThreads = 32 * (kGProd + 1 + kGEpi);
 constexpr int kGOpB = kGM * kGRowB;      // bytes of one split tile
-constexpr int kGStageB = 6 * kGOpB;      // A: h, m, l; B: h, m, l
+constexpr int kGOpWB = kGNMax * kGRowB;  // ... of w
+constexpr int kGStageB = 3 * kGOpB + 3 * kGOpWB;   // A: h, m, l; B: h, m, l
 constexpr int kGTmemLow = 2 * kGNMax;    // two h h accumulators, then two of small products
 constexpr int kGOutCols = 16, kGOutPitch = kGOutCols + 4;   // a warp's output piece, skewed across the banks
 constexpr int kGRawB = kGProd * 32 * 8 * 16;                  // bytes of one raw stage
@@ -236,9 +237,10 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
             split8(x, h, m, l);
             const int row = quad * 4 + j;
             const uint32_t d = base + (uint32_t)(row * kGRowB + ((oct ^ ((row >> 1) & 3)) << 4));
+            const uint32_t op = is_w ? kGOpWB : kGOpB;
             sts_u4(d, h);
-            sts_u4(d + kGOpB, m);
-            sts_u4(d + 2 * kGOpB, l);
+            sts_u4(d + op, m);
+            sts_u4(d + 2 * op, l);
           }
         }
       } else {
@@ -249,9 +251,10 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
           uint2 h, m, l;
           split4(v[x], h, m, l);
           const uint32_t d = base + (x >= 4 ? 3u * kGOpB : 0u) + (uint32_t)(x & 3) * (32u * kGRowB);
+          const uint32_t op = x >= 4 ? kGOpWB : kGOpB;
           sts_v2(d, h);
-          sts_v2(d + kGOpB, m);
-          sts_v2(d + 2 * kGOpB, l);
+          sts_v2(d + op, m);
+          sts_v2(d + 2 * op, l);
         }
       }
       fence_async_smem();  // the tensor cores read shared memory through the async proxy
@@ -288,7 +291,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
 #pragma unroll
             for (int x = 0; x < 3; ++x) {
               da[x] = smem_desc(A + x * kGOpB + k16 * 32, 512, 4);
-              db[x] = smem_desc(B + x * kGOpB + k16 * 32, 512, 4);
+              db[x] = smem_desc(B + x * kGOpWB + k16 * 32, 512, 4);
             }
             const uint32_t hh = tmem + hb * kGNMax, lo = tmem + kGTmemLow + lb * kGNMax;
             umma_ss(hh, da[0], db[0], idesc, !(first && k16 == 0));
