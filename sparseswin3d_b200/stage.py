@@ -179,7 +179,7 @@ class SwinTransformerBlock(nn.Module):
             m = self.mlp(h2)
             out, _ = add_layernorm(x1, m, None, sum_out=x1)
             return x.replace_feature(out)
-        if (fuse_shell and torch.is_grad_enabled() and rows.aligned_rows(feats) and rows.plain_norm(self.norm1, feats)
+        if (fuse_shell and torch.is_grad_enabled() and feats.shape[0] >= rows.ADD_NORM_ROWS and rows.aligned_rows(feats) and rows.plain_norm(self.norm1, feats)
                 and rows.plain_norm(self.norm2, feats)):
             x0, h = rows.add_layer_norm(feats, None, self.norm1)
             a = self.drop_path(self.attention_branch(h, plan, use_mask))
