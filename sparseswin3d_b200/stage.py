@@ -10,7 +10,8 @@ for reuse across the blocks of a stage:
   running features and normalises the sum for the next branch in one pass, also across the block
   boundary (the residual add that ends block i and norm1 of block i+1).
 
-The GEMMs themselves (qkv, proj, the two MLP Linears) are library calls (torch / cuBLAS).
+The GEMMs (qkv, proj, the two MLP Linears) are this library's in fp32 and, with its GELU, for the first MLP Linear in
+16-bit inference (`rows.py`); the other 16-bit ones are library calls (torch / cuBLAS).
 
 `SparseVoxels` carries the four fields of an spconv SparseConvTensor that upstream's blocks read
 (`features`, `indices` [N,4] int32 (b,z,y,x), `spatial_shape`, `batch_size`) and `replace_feature`.
