@@ -8,7 +8,7 @@
 // the tensor cores' operand layout and stay there while the window's query rows pass in tiles of
 // 128:
 //
-//   S[128 x 128] = Q_tile K_tile^T       tcgen05.mma, operands from shared memory, S in tensor memory
+//   S[128 x 96]  = Q_tile K_tile^T       tcgen05.mma, operands from shared memory, S in tensor memory
 //   P            = exp2(S*scale + bias + mask - m)   two threads per query row (tcgen05.ld gives a
 //                  thread its part of the row of S), running maximum from 0 and +1e-8 as upstream (ops.cu:137,
 //                  164); P goes back to tensor memory in the input type, as the A operand of the next product.
@@ -16,32 +16,34 @@
 //                  rounding of the output with that, so the rounding residual is stored beside P and
 //                  multiplied with the same V tile (A and B of an MMA must have the same 16-bit
 //                  type: an fp16 P against a bf16 V is an illegal instruction)
-//   O_part[128 x 32] = P V_tile          tcgen05.mma, added into fp32 registers by the row's thread
-//                  with the correction factor of the running maximum
+//   O[128 x 32] += P V_tile              tcgen05.mma, over all key tiles of a query tile; where a running maximum grows, the
+//                  row's threads scale what has been added up
 //
 // Two forms of the softmax.  A tile's scores are bounded by |q| |k| scale + bias, the largest of each over the tile (the
 // producers find them while they gather).  While that bound lies below kLimit the exponentials need no maximum:
 // upstream's own starts at 0, so with 0 as the reference (fp16: kRef, see there) nothing overflows, the
 // result is the same quotient (the denominator relative to 0 is at least 1 wherever a maximum above 0 would have been
-// subtracted, and there 1e-8 is below its rounding), no row statistics pass between threads, and the P V products
+// subtracted, and there 1e-8 is below its rounding), no row statistics pass between threads.  The P V products
 // of all key tiles (up to 1024 keys, 128 MMAs) add up in one tensor-memory accumulator; the tensor cores cut off where an fp32
 // add rounds, some 1e-6 of the sum, two hundred times less than the rounding of the output.  From the first key tile beyond the bound on, the query tile
-// goes on with the running maximum and an O_part per key tile.
+// goes on with the running maximum, which takes a pass over the scores of its own.
 //
-// What bounds it is the hand-over between the roles, once per key tile: with the arithmetic, the row loads and all but two
-// MMAs taken out, more than half of the time stays.  So a tile is 128 keys.  A million voxels, half of the 9^3
-// windows full, six heads of bf16: 5.49 ms with 64-key tiles, P through shared memory and a running maximum throughout;
-// 5.09 with the bound and P in tensor memory; 4.53 with 128 keys a tile.  Four threads a row instead of two: no change.
+// Two query tiles are in flight, each a stream of its own: its own issuing warp, scores, P, sums and eight softmax warps, over key tiles that
+// both share.  While one stream waits for a hand-over the other has the SM.  Nothing but key tiles and the units' headers
+// ties them to one another.  A million voxels, half of the 9^3 windows full, six heads of bf16, in ms: 4.53 with one stream, 128-key tiles and
+// MMAs issued from a branch of one lane (there every operand is looked for among the lanes: see the issuer); 2.99 two streams of four
+// softmax warps; 2.82 eight softmax warps each (two threads a row); 2.30 MMAs issued from uniform registers; 2.27 the residual
+// of P in one mixed-precision instruction.  Bound by issue slots and their latencies: 66 % of them used (13 warp instructions a key, 7.5 of them
+// the look-up of the bias, the exponential and the split of P), exponential unit 46 %, shared memory 35 to 60 %; without exponentials
+// the time is the same within 3 %.  Floor of the exponential unit: 0.97 ms.
 //
-// Warp roles (384 threads, one CTA per SM): warp 0 issues the MMAs (one elected lane) and owns the
-// tensor-memory allocation; warps 1-3 gather rows (plain 16-byte loads by voxel id, stored with the
-// 64-byte swizzle the operand descriptors name); warps 4-11 are the softmax rows: a warp may touch
-// the 32 tensor-memory lanes warp_id % 4 selects, so two warps share each quarter of the query
-// rows, one for the first 64 keys of a tile and the first 16 output channels, one for the rest
-// (they exchange their partial row maxima per tile and their row sums per query tile through shared
-// memory): two warps per scheduler instead of one.  Everything is handed over through mbarriers
-// with bounded waits; on expiry the kernel sets SSW_DEV_TIMEOUT, lets the tensor cores drain and
-// frees its tensor memory before it returns.
+// Warp roles (768 threads, one CTA per SM): warps 0-1 issue the MMAs of a stream (one elected lane); warps 2-7 gather rows (plain 16-byte loads by
+// voxel id, stored with the 64-byte swizzle the operand descriptors name); warps 8-23 are the softmax rows, eight warps a stream: a
+// warp may touch the 32 tensor-memory lanes warp_id % 4 selects, so two warps share each quarter of the query rows and take
+// sixteens of keys in turn (they exchange row maxima per key tile beyond the bound and row sums per query tile through shared memory).
+// P takes the place of the scores it comes from: of sixteen columns of scores the first eight become P and the others its residual.
+// Everything is handed over through mbarriers with bounded waits; on expiry the kernel sets SSW_DEV_TIMEOUT, lets the tensor
+// cores drain and frees its tensor memory before it returns.
 #include <math.h>
 
 #include "attn_common.cuh"
@@ -50,30 +52,33 @@
 namespace ssw {
 
 template <typename T>
-__device__ __forceinline__ float2 widen2(uint32_t u);
-template <>
-__device__ __forceinline__ float2 widen2<__nv_bfloat16>(uint32_t u) {
-  return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+__device__ __forceinline__ float residual(float p, uint32_t h) {   // p less a 16-bit value
+  float r;
+  if constexpr (std::is_same<T, __nv_bfloat16>::value)
+    asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(r) : "h"((uint16_t)h), "h"((uint16_t)0xbf80), "f"(p));
+  else
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(r) : "h"((uint16_t)h), "h"((uint16_t)0xbc00), "f"(p));
+  return r;
 }
-template <>
-__device__ __forceinline__ float2 widen2<__half>(uint32_t u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); }
 
 constexpr int kDQ = 128;       // query rows per tile = MMA M
-constexpr int kDK = 128;       // keys per tile
+constexpr int kDK = 96;        // keys per tile
 constexpr int kDHD = 32;       // head_dim
 constexpr int kDRowB = 64;     // bytes of one q / k / v head slice (32 x 16 bit)
-constexpr int kDMaxKT = 8;     // key tiles per window at most (1024 keys)
-constexpr int kDProd = 3;      // producer warps
-constexpr int kDParts = 2;     // softmax threads per query row, in different warps (2 or 4; measured equal)
-constexpr int kDSoftWarps = 4 * kDParts;
-constexpr int kDThreads = 128 + 32 * kDSoftWarps;
-constexpr int kDHalf = kDK / kDParts;  // keys of a tile one softmax thread looks after
-constexpr int kDCpt = kDHD / kDParts;  // output channels one softmax thread accumulates
-constexpr int kDOutPitch = kDRowB + 16;  // bytes between rows of the output staging tile (skewed across banks)
-constexpr int kDSub = 32;       // keys a softmax thread takes at a time
-constexpr int kDSBuf = 2;      // S tiles in tensor memory: the scores run one tile ahead of the softmax
-constexpr int kTmemCols = 512; // S: 2 x 128 columns, O_part: 2 x 32, O_acc: 32, P: 64 + 64 of rounding residuals
-constexpr int kTmemS = 0, kTmemO = 256, kTmemOAcc = 320, kTmemP = 352;
+constexpr int kDTileB = kDK * kDRowB;
+constexpr int kDMaxKT = 11;    // key tiles in shared memory at most (1024 keys)
+constexpr int kDStreams = 2;   // query tiles in flight, each with its own softmax warps, scores and sums
+constexpr int kDProd = 6;      // producer warps (with four groups of eight rows each they gather the k and v of a key tile at once)
+constexpr int kDParts = 2;     // softmax threads per query row, in different warps: sixteens of a tile's keys in turn
+constexpr int kDSoftWarps = 4 * kDParts;  // softmax warps of a stream
+constexpr int kDFirstSoft = kDStreams + kDProd;   // a multiple of 4: warp % 4 selects the tensor-memory lanes
+constexpr int kDThreads = 32 * (kDFirstSoft + kDStreams * kDSoftWarps);
+constexpr int kDSub = 16;      // keys a softmax thread takes at a time = K of an MMA
+constexpr int kTmemCols = 512; // per stream: two tiles of scores, which P takes over, and the sums O
+constexpr int kTmemStream = 256, kTmemO = 2 * kDK;
+static_assert(kDK % (2 * kDSub) == 0 && kTmemO + kDHD <= kTmemStream && kDFirstSoft % 4 == 0 && kDTileB % 1024 == 0 &&
+                  kDProd * 4 * 8 >= 2 * kDK,
+              "");
 // Scores (log2 domain, less kRef) up to which probabilities are formed without a maximum: exp2 of it times 1024 keys times
 // a v below 2^60 stays far inside fp32, and inside the 16-bit type of P.  The bias slices of the units are stored less
 // kRef.  fp16: with q and k of unit variance and 32 channels the bound of a tile is 16 or 17, above 15; where no score of a row
@@ -91,6 +96,30 @@ struct DenseFast<__half> {
   static constexpr uint32_t kMaxV = 0x7c00u;
 };
 
+// The bias slice in shared memory.  A warp's lanes are consecutive rows of a window, in a full one consecutive positions, and a look-up of the
+// warp reads the slice at their codes.  With rows of x a multiple of 32 plus Wx words apart, and planes of y plus Wx Wy,
+// consecutive positions lie in consecutive banks; with the table's own strides nearly every look-up takes two passes (51.8 M shared-memory wavefronts
+// against 33.6 M over 172 full windows of 9^3 and six heads).  The padded slice takes the room of two plain ones, so it is staged for one head
+// (see the units).  A million voxels, half of the 9^3 windows full, six heads of bf16, plain / padded: 2.27 / 2.33 ms (144 blocks for 148),
+// the same shifted by four 2.18 / 2.02.  Where the padded slice does not fit, the table's strides stay.
+struct BiasShape {
+  int wy2, wx2;        // 2 Wy - 1, 2 Wx - 1: the table's own strides are wx2 and wx2 wy2
+  int py, pz;          // words between rows of x / planes of y
+  int off;             // padded code of the last position
+  int floats;
+};
+inline BiasShape bias_shape(const int32_t w[3], bool padded) {
+  BiasShape b;
+  b.wy2 = 2 * w[1] - 1;
+  b.wx2 = 2 * w[2] - 1;
+  b.py = b.wx2 + (padded ? ((w[2] - b.wx2) % 32 + 32) % 32 : 0);
+  b.pz = b.wy2 * b.py;
+  if (padded) b.pz += ((w[1] * w[2] - b.pz) % 32 + 32) % 32;
+  b.off = (w[0] - 1) * b.pz + (w[1] - 1) * b.py + (w[2] - 1);
+  b.floats = (2 * b.off + 4) & ~3;
+  return b;
+}
+
 struct DenseParams {
   const void* qkv;
   OutSet outs;
@@ -105,34 +134,49 @@ struct DenseParams {
   int rel_off, H, C, tile, n_per_window, table_rows;
   int n_vox, w_cap;
   int c_cap;                  // rows the shared-memory buffers are sized for (a multiple of kDK)
+  int kv_slots, q_bufs;       // key tiles in shared memory; query tiles per stream
+  BiasShape bias;
   float scale;
   int use_mask;
 };
 
 // Shared memory (byte offsets from a 1024-byte aligned base):
-//   [0, 1024)        mbarriers and the tensor-memory address
-//   [1024, 1024 + 2 * kDParts * 512)  partial row maxima / sums the softmax threads of a row exchange
-//   K  c_cap x 64    V  c_cap x 64    (64-byte swizzle; key tile j = rows [128 j, 128 j + 128))
-//   Q  2 x 128 x 64  (64-byte swizzle)
-//   per unit (double buffered): the bias slice of its head, (2Wz-1)(2Wy-1)(2Wx-1) floats
-//   pre-multiplied by log2 e; per row of its window the voxel id, 4 x relative-position code, region
+//   [0, 2048)        mbarriers, the tensor-memory address, largest norms of the tiles
+//   [2048, 8192)     partial row maxima / sums the softmax threads of a row exchange
+//   K, V  kv_slots x 96 x 64 each   (64-byte swizzle), a ring over the key tiles of all units: the next unit's come in
+//                    while this one's are in use
+//   Q  2 streams x q_bufs x 128 x 64  (64-byte swizzle)
+//   the bias slice of the head, pre-multiplied by log2 e
+//   per unit (double buffered), per row of its window: the voxel id, 4 x padded relative-position code, region
 struct DenseSmem {
-  uint32_t k, v, q, bias, bias_floats, vox, rel4, reg, ostage, total;
+  uint32_t k, v, q, bias, vox, rel4, reg, total;
 };
-__host__ __device__ inline DenseSmem dense_smem(int c_cap, int table_rows) {
+__host__ __device__ inline DenseSmem dense_smem(int c_cap, int bias_floats, int kv_slots, int q_bufs) {
   DenseSmem s;
-  uint32_t o = 1024u + 2u * kDParts * 512u;
-  s.k = o; o += (uint32_t)c_cap * kDRowB;
-  s.v = o; o += (uint32_t)c_cap * kDRowB;
-  s.q = o; o += 2u * kDQ * kDRowB;
-  s.bias_floats = ((uint32_t)table_rows + 3u) & ~3u;
-  s.bias = o; o += 2u * s.bias_floats * 4u;
+  uint32_t o = 8192u;
+  s.k = o; o += (uint32_t)kv_slots * kDTileB;
+  s.v = o; o += (uint32_t)kv_slots * kDTileB;
+  s.q = o; o += (uint32_t)(kDStreams * q_bufs) * kDQ * kDRowB;
+  s.bias = o; o += (uint32_t)bias_floats * 4u;
   s.vox = o; o += 2u * (uint32_t)c_cap * 4u;
   s.rel4 = o; o += 2u * (uint32_t)c_cap * 4u;
   s.reg = o; o += 2u * (uint32_t)c_cap * 4u;
-  s.ostage = o; o += (uint32_t)kDQ * kDOutPitch;
   s.total = o;
   return s;
+}
+// Key tiles and query buffers to keep in shared memory: twice a full window's key tiles (at most 8) where they fit, at least one
+// window's; two query tiles a stream where they fit, else one; the padded bias slice where it fits.  False: nothing fits.
+inline bool dense_buffers(int n_per_window, const int32_t w[3], int& c_cap, int& kv_slots, int& q_bufs, BiasShape& bias) {
+  const int need = (n_per_window + kDK - 1) / kDK;
+  c_cap = need * kDK;
+  if (need > kDMaxKT) return false;
+  for (q_bufs = 2; q_bufs > 0; --q_bufs)
+    for (int padded = 1; padded >= 0; --padded) {
+      bias = bias_shape(w, padded != 0);
+      for (kv_slots = 2 * need > 8 ? (need > 8 ? need : 8) : 2 * need; kv_slots >= need; --kv_slots)
+        if ((size_t)dense_smem(c_cap, bias.floats, kv_slots, q_bufs).total + 1024 <= 227 * 1024) return true;
+    }
+  return false;
 }
 
 template <typename T, bool kMask>
@@ -140,65 +184,67 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // the operand layouts want 1024-byte aligned tiles: align the base by hand
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
-  const DenseSmem L = dense_smem(p.c_cap, p.table_rows);
+  const DenseSmem L = dense_smem(p.c_cap, p.bias.floats, p.kv_slots, p.q_bufs);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-  uint64_t* kv_full = bars;                    // [kDMaxKT] key tile j of the unit is in shared memory
-  uint64_t* kv_empty = bars + kDMaxKT;         // [kDMaxKT] the unit's last MMA on key tile j is done
-  uint64_t* q_full = bars + 2 * kDMaxKT;       // [2]
-  uint64_t* q_empty = q_full + 2;              // [2]
-  uint64_t* s_full = q_empty + 2;              // [kDSBuf] S tile in tensor memory
-  uint64_t* s_empty = s_full + kDSBuf;         // [kDSBuf] S tile read out
-  uint64_t* p_full = s_empty + kDSBuf;         // [2] P tile in tensor memory
-  uint64_t* pv_done = p_full + 2;              // [2] P V of the tile done: O_part ready, P buffer free
-  uint64_t* o_empty = pv_done + 2;             // [2] O_part read out
-  uint64_t* meta_full = o_empty + 2;           // [2] a unit's header: voxel ids, metadata, bias slice of its head
+  uint64_t* kv_full = bars;                    // [kDMaxKT] a key tile is in shared memory
+  uint64_t* kv_empty = kv_full + kDMaxKT;      // [kDMaxKT] both streams are done with it
+  uint64_t* meta_full = kv_empty + kDMaxKT;    // [2] a unit's header: voxel ids, metadata, bias slice of its head
   uint64_t* meta_empty = meta_full + 2;        // [2]
   uint64_t* drain_bar = meta_empty + 2;        // [1]
-  uint64_t* xbar = drain_bar + 1;              // [4] the two warps of a row quarter have posted their partial values
-  uint64_t* obar = xbar + 4;                   // [1] output staging tile: written by all / read by all
-  uint64_t* oacc_empty = obar + 1;             // [1] a query tile's O_acc has been read (one phase per query tile)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(oacc_empty + 1);
+  uint64_t* q_full = drain_bar + 1;            // [stream][2]
+  uint64_t* q_empty = q_full + 4;              // [stream][2]
+  uint64_t* s_full = q_empty + 4;              // [stream][2] scores of a tile in tensor memory
+  uint64_t* p_full = s_full + 4;               // [stream][2] P in their place
+  uint64_t* pv_done = p_full + 4;              // [stream][2] P V of the tile done: added to O, the tile's columns free
+  uint64_t* o_empty = pv_done + 4;             // [stream] a query tile's O has been read (one phase per query tile)
+  uint64_t* xbar = o_empty + kDStreams;        // [stream][4] both threads of a quarter's rows have posted their maximum
+  uint64_t* lbar = xbar + 4 * kDStreams;       // [stream][4] a query tile's partial row sums have been posted
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(lbar + 4 * kDStreams);
   int* unit_c = reinterpret_cast<int*>(tmem_slot + 1);      // [2] voxels of the unit's window, with its metadata
-  int* fast_flag = unit_c + 2;                              // [2] the P tile is within the bound: P V goes to O_acc
-  // largest squared norms of a tile's rows, one word per producer warp (the fourth unused)
-  float4* k_norm = reinterpret_cast<float4*>(smem + 512);   // [kDMaxKT]; infinite where a v is too large for O_acc
-  float4* q_norm = k_norm + kDMaxKT;                        // [4] by query tile number
-  float4* b_max = q_norm + 4;                               // [2] largest entry (or 0) of the unit's bias slice
-  float* xch = reinterpret_cast<float*>(smem + 1024);  // [2 buffers][kDParts][128 rows] partial maxima / sums
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // largest squared norms of a tile's rows, one word per producer warp (two of the eight unused)
+  float* k_norm = reinterpret_cast<float*>(smem + 768);     // [kDMaxKT][8]; infinite where a v is too large for O
+  float* q_norm = k_norm + kDMaxKT * 8;                     // [stream][4][8] by query tile of the stream
+  float* b_max = q_norm + kDStreams * 4 * 8;                // [8] largest entry (or 0) of the bias slice
+  float* xmax = reinterpret_cast<float*>(smem + 2048);      // [stream][2][kDParts][128] partial row maxima
+  float* xsum = xmax + kDStreams * 2 * kDParts * 128;       // [stream][2][128] partial row sums
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int H = p.H, C = p.C;
 
   // Whether there is any window beyond a pack is a device-side count: a launch that finds none
   // (the usual case on surface-sparse scenes) leaves before it sets anything up.
   grid_dependency_wait();
-  {
-    BinTables bins0(const_cast<int32_t*>(p.bins), p.n_per_window);
-    const int W0 = min(max(p.header[SSW_H_W], 0), p.w_cap);
-    const int first = p.tile + 1 <= p.n_per_window + 1 ? min(max(bins0.wstart[p.tile + 1], 0), W0) : W0;
-    if (first >= W0) return;
-  }
+  // the windows beyond a pack, heaviest first: window slots [ws0, W) of the plan's pack order
+  BinTables bins(const_cast<int32_t*>(p.bins), p.n_per_window);
+  const int W = min(max(p.header[SSW_H_W], 0), p.w_cap);
+  const int ws0 = p.tile + 1 <= p.n_per_window + 1 ? min(max(bins.wstart[p.tile + 1], 0), W) : W;
+  const int n_units = (W - ws0) * H;
+  // A block's units are u = blockIdx.x, + step, + 2 step, ..., window by window, and the bias slice in shared memory is that of one head: a
+  // multiple of the heads of blocks, where that leaves out one block in sixteen at most, never changes heads.  (Head by head over all
+  // blocks: 2.39 ms against 2.33 on a million voxels of full windows, six heads; a window's heads then find its rows in L2 no more.)
+  const int odd = (int)gridDim.x % H, step = odd * 16 <= (int)gridDim.x ? gridDim.x - odd : gridDim.x;
+  if ((int)blockIdx.x >= min(n_units, step)) return;
   if (threadIdx.x == 0) {
     for (int j = 0; j < kDMaxKT; ++j) {
       mbar_init(kv_full + j, kDProd);
-      mbar_init(kv_empty + j, 1);
+      mbar_init(kv_empty + j, kDStreams);
     }
     for (int b = 0; b < 2; ++b) {
+      mbar_init(meta_full + b, kDProd);
+      mbar_init(meta_empty + b, kDStreams * (kDSoftWarps + 1));
+    }
+    for (int b = 0; b < 2 * kDStreams; ++b) {
       mbar_init(q_full + b, kDProd);
       mbar_init(q_empty + b, 1);
+      mbar_init(s_full + b, 1);
       mbar_init(p_full + b, kDSoftWarps);
       mbar_init(pv_done + b, 1);
-      mbar_init(o_empty + b, kDSoftWarps);
-      mbar_init(meta_full + b, kDProd);
-      mbar_init(meta_empty + b, kDSoftWarps);
     }
-    for (int b = 0; b < kDSBuf; ++b) {
-      mbar_init(s_full + b, 1);
-      mbar_init(s_empty + b, kDSoftWarps);
+    for (int s = 0; s < kDStreams; ++s) mbar_init(o_empty + s, 4);
+    for (int x = 0; x < 4 * kDStreams; ++x) {
+      mbar_init(xbar + x, kDParts);
+      mbar_init(lbar + x, 1);
     }
-    for (int x = 0; x < 4; ++x) mbar_init(xbar + x, kDParts);
-    mbar_init(obar, kDSoftWarps);
-    mbar_init(oacc_empty, kDSoftWarps);
-    mbar_init(drain_bar, 1);
+    mbar_init(drain_bar, kDStreams);
     mbar_fence_init();
   }
   if (warp == 0) tmem_alloc(tmem_slot, kTmemCols);
@@ -207,529 +253,545 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // the windows beyond a pack, heaviest first: window slots [ws0, W) of the plan's pack order
-  BinTables bins(const_cast<int32_t*>(p.bins), p.n_per_window);
-  const int W = min(max(p.header[SSW_H_W], 0), p.w_cap);
-  const int ws0 = p.tile + 1 <= p.n_per_window + 1 ? min(max(bins.wstart[p.tile + 1], 0), W) : W;
-  const int n_units = (W - ws0) * H;
   bool timed_out = false;
-  // every role walks the same unit list; window geometry is read from the plan by each
-  auto unit_window = [&](int u, int& first, int& c, int& h) {
-    const int ws = W - 1 - u / H;
-    h = u % H;
-    const int k = min(max(__ldg(p.pack_win + ws), 0), p.w_cap - 1);
-    first = __ldg(p.win_pstart + k);
-    c = __ldg(p.win_start + k + 1) - __ldg(p.win_start + k);
-    const bool ok = c > p.tile && c <= p.c_cap && first >= 0 && first <= p.n_vox - c;
-    if (!ok) {
-      atomicOr(reinterpret_cast<unsigned*>(p.header + SSW_H_ERROR), SSW_DEV_BAD_PLAN);
-      first = 0;   // a one-row window instead: the result is flagged, and every role still finds work
-      c = 1;
-    }
-  };
   constexpr float kRef = DenseFast<T>::kRef;
   const int a_fmt_qk = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
+  // Every role walks the same units; a unit's query tiles go to the two streams in
+  // turn, counted over all units, so a unit of one tile leaves one stream without work in it.
 
-  if (warp == 0) {
-    // =========================================== MMA issuer ===================================
+  if (warp < kDStreams) {
+    // =========================================== MMA issuer of a stream =======================
     // One lane, two positions in the same sequence of key tiles: `sp`, the next tile whose scores are formed, runs up to
-    // kDSBuf - 1 tiles ahead of `pp`, the next one whose P V is (also across query tiles and units).  It takes whichever
-    // can go: if the scores waited in turn for the P V before them, the softmax would wait for both.
+    // two tiles ahead of `pp`, the next one whose P V is (also across query tiles and units).  Within a unit the two go in turn and
+    // a wait may suspend the thread.  Scores of the next unit may have to wait for key tiles that come in only after the P V behind
+    // them: there the lane takes whichever can go, and sleeps in between (asking without a pause took half of all issue slots
+    // of two schedulers, and the softmax warps there were what the others waited for).
+    // All lanes walk along, on values that the compiler can see are the same in each (vote and shuffle results, parameters),
+    // and one issues: an MMA takes its operands from uniform registers, and from a branch of one lane every operand is first
+    // looked for among the lanes, some hundred instructions an MMA.
+    const int s = warp;
+    const bool leader = elect_one();
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0) + s * kTmemStream;
+    const int units = __shfl_sync(0xffffffffu, n_units, 0), stride = __shfl_sync(0xffffffffu, step, 0);
     struct Pos {
-      uint32_t g, qn;              // key tiles / query tiles before it
-      int u, un, t, j, c;          // unit, units before it, query tile, key tile, the window's voxels (0: not yet read)
-      uint32_t kv;                 // bit j: parity of the uses of key tile j by earlier units
+      uint32_t g, qn;              // key tiles / query tiles of the stream before it
+      uint32_t slot, par;          // ring slot of the unit's first key tile, parity of that slot's use
+      int u, un, qodd;             // unit, units before it, query tiles of all units before it modulo 2
+      int t, j, c;                 // query tile, key tile, the window's voxels (0: not yet read)
     };
-    auto advance = [&](Pos& x) {
-      ++x.g;
-      if (++x.j * kDK < x.c) return;
-      x.j = 0;
-      ++x.qn;
-      if (++x.t * kDQ < x.c) return;
-      x.t = 0;
-      x.kv ^= (1u << ((x.c + kDK - 1) / kDK)) - 1u;
+    auto ring = [&](uint32_t& slot, uint32_t& par, int n) {
+      slot += n;
+      if (slot >= (uint32_t)p.kv_slots) {
+        slot -= p.kv_slots;
+        par ^= 1;
+      }
+    };
+    auto next_unit = [&](Pos& x) {
+      ring(x.slot, x.par, (x.c + kDK - 1) / kDK);
+      x.qodd ^= ((x.c + kDQ - 1) / kDQ) & 1;
       x.c = 0;
       ++x.un;
-      x.u += gridDim.x;
+      x.u += stride;
     };
-    if (lane == 0) {
-      const uint32_t sK = smem_u32(smem + L.k), sV = smem_u32(smem + L.v), sQ = smem_u32(smem + L.q);
-      Pos sp = {0, 0, (int)blockIdx.x, 0, 0, 0, 0, 0u}, pp = sp;
-      uint32_t idle = 0;
-      while (pp.u < n_units) {
-        bool moved = false;
-        // ---- scores of the next tile
-        if (sp.u < n_units && sp.g - pp.g < (uint32_t)kDSBuf) {
-          if (sp.c == 0 && mbar_test(meta_full + (sp.un & 1), (sp.un >> 1) & 1)) {
-            sp.c = *reinterpret_cast<volatile int*>(unit_c + (sp.un & 1));
-          }
-          const uint32_t b = sp.g % kDSBuf, qb = sp.qn & 1;
-          if (sp.c > 0 && (sp.j > 0 || mbar_test(q_full + qb, (sp.qn >> 1) & 1)) &&
-              (sp.t > 0 || mbar_test(kv_full + sp.j, (sp.kv >> sp.j) & 1)) &&
-              (sp.g < (uint32_t)kDSBuf || mbar_test(s_empty + b, (sp.g / kDSBuf - 1) & 1))) {
+    auto advance = [&](Pos& x) {  // true: the unit's last tile of this stream
+      ++x.g;
+      if (++x.j * kDK < x.c) return false;
+      x.j = 0;
+      ++x.qn;
+      x.t += kDStreams;
+      return x.t * kDQ >= x.c;
+    };
+    auto ready = [&](uint64_t* bar, uint32_t parity, bool wait) -> bool {
+      const bool ok = __all_sync(0xffffffffu, wait ? mbar_wait_bounded(bar, parity) : mbar_test(bar, parity));
+      timed_out = timed_out || (wait && !ok);
+      return ok;
+    };
+    auto window_of = [&](int un) { return __shfl_sync(0xffffffffu, *reinterpret_cast<volatile int*>(unit_c + (un & 1)), 0); };
+    const uint64_t q_desc = smem_desc(smem_u32(smem + L.q) + (uint32_t)(s * p.q_bufs) * (kDQ * kDRowB), 512, 4);
+    const uint64_t k_desc = smem_desc(smem_u32(smem + L.k), 512, 4), v_desc = smem_desc(smem_u32(smem + L.v), 512, 4);
+    const uint32_t idesc_s = instr_desc(a_fmt_qk, a_fmt_qk, 0, 0);     // (N is added: a window's last key tile has fewer keys)
+    const uint32_t idesc_o = instr_desc(a_fmt_qk, a_fmt_qk, 1, kDHD);  // A = P, B = V (MN-major)
+    Pos sp = {0, 0, 0, 0, (int)blockIdx.x, 0, 0, 0, 0, 0}, pp = sp;
+    uint32_t idle = 0;
+    while (pp.u < units && !timed_out) {
+      bool moved = false;
+      const uint32_t ahead = sp.g - pp.g;
+      const bool in_turn = sp.un == pp.un;
+      // ---- scores of the next tile
+      if (sp.u < units && ahead < 2) {
+        if (sp.c == 0 && ready(meta_full + (sp.un & 1), (sp.un >> 1) & 1, in_turn)) {
+          sp.c = window_of(sp.un);
+          sp.t = (s - sp.qodd) & 1;
+          if (sp.t * kDQ >= sp.c) next_unit(sp);   // nothing here for this stream
+          moved = true;
+        }
+        if (sp.c > 0) {
+          const uint32_t b = sp.g & 1, qb = p.q_bufs == 2 ? sp.qn & 1 : 0, qpar = p.q_bufs == 2 ? (sp.qn >> 1) & 1 : sp.qn & 1;
+          uint32_t slot = sp.slot, par = sp.par;
+          ring(slot, par, sp.j);
+          // the scores go where the tile two before had its P
+          if ((sp.j > 0 || ready(q_full + 2 * s + qb, qpar, in_turn)) && (sp.t >= kDStreams || ready(kv_full + slot, par, in_turn)) &&
+              (sp.g < 2 || ready(pv_done + 2 * s + b, ((sp.g >> 1) - 1) & 1, in_turn))) {
             tc_fence_after();
             const int nk16 = (min(kDK, sp.c - sp.j * kDK) + 15) & ~15;
-            const uint32_t idesc = instr_desc(a_fmt_qk, a_fmt_qk, 0, nk16);
+            const uint32_t idesc = idesc_s + ((uint32_t)(nk16 >> 3) << 17);
+            const uint64_t qd = q_desc + qb * (kDQ * kDRowB >> 4), kd = k_desc + slot * (kDTileB >> 4);
+            const bool q_end = (sp.j + 1) * kDK >= sp.c;  // every S of this query tile has been issued
+            if (leader) {
 #pragma unroll
-            for (int ks = 0; ks < kDHD / 16; ++ks)
-              umma_ss(tmem + kTmemS + b * kDK, smem_desc(sQ + qb * (kDQ * kDRowB) + ks * 32, 512, 4),
-                      smem_desc(sK + sp.j * (kDK * kDRowB) + ks * 32, 512, 4), idesc, ks > 0);
-            umma_commit(s_full + b);
-            if ((sp.j + 1) * kDK >= sp.c) umma_commit(q_empty + qb);  // every S of this query tile has been issued
-            advance(sp);
+              for (int ks = 0; ks < kDHD / 16; ++ks) umma_ss(tm + b * kDK, qd + ks * 2, kd + ks * 2, idesc, ks > 0);
+              umma_commit(s_full + 2 * s + b);
+              if (q_end) umma_commit(q_empty + 2 * s + qb);
+            }
+            __syncwarp();
+            if (advance(sp)) next_unit(sp);
             moved = true;
           }
         }
-        // ---- P V of the oldest tile whose scores have been formed
-        if (pp.g != sp.g) {
-          if (pp.c == 0) pp.c = *reinterpret_cast<volatile int*>(unit_c + (pp.un & 1));  // (sp has seen its meta_full)
+      }
+      // ---- P V of the oldest tile whose scores have been formed; a unit without tiles of this stream is left behind
+      if (pp.un != sp.un || pp.g != sp.g) {
+        if (pp.c == 0) {
+          pp.c = window_of(pp.un);  // (sp has seen its meta_full)
+          pp.t = (s - pp.qodd) & 1;
+          pp.j = 0;
+        }
+        uint32_t slot = pp.slot, par = pp.par;
+        ring(slot, par, pp.j);
+        if (pp.t * kDQ >= pp.c) {
+          // (each phase of kv_empty wants one arrival of each stream: the phase before has completed once the tile is full)
+          if (ready(kv_full + slot, par, false)) {
+            if (leader) mbar_arrive(kv_empty + slot);
+            if (++pp.j * kDK >= pp.c) {
+              pp.j = 0;
+              if (leader) mbar_arrive(meta_empty + (pp.un & 1));
+              next_unit(pp);
+            }
+            moved = true;
+          }
+        } else if (pp.g != sp.g) {
           const uint32_t b = pp.g & 1;
-          if (mbar_test(p_full + b, (pp.g >> 1) & 1)) {
-            const bool fast = *reinterpret_cast<volatile int*>(fast_flag + b) != 0;
-            // O_acc starts over with the query tile: the one before must have been read.  O_part: the tile two before.
-            const bool go = fast ? pp.j > 0 || pp.qn == 0 || mbar_test(oacc_empty, (pp.qn - 1) & 1)
-                                 : pp.g < 2 || mbar_test(o_empty + b, ((pp.g >> 1) - 1) & 1);
-            if (go) {
-              tc_fence_after();
-              const int nk16 = (min(kDK, pp.c - pp.j * kDK) + 15) & ~15;
-              const uint32_t idesc = instr_desc(a_fmt_qk, a_fmt_qk, 1, kDHD);  // A = P, B = V (MN-major)
-              const uint32_t dst = fast ? tmem + kTmemOAcc : tmem + kTmemO + b * kDHD;
-              for (int part = 0; part < 2; ++part)   // P, then its rounding residual
-                for (int ks = 0; ks < nk16 / 16; ++ks)
-                  umma_ts(dst, tmem + kTmemP + part * (kDK / 2) + ks * 8,
-                          smem_desc(sV + pp.j * (kDK * kDRowB) + ks * (16 * kDRowB), 512, 4), idesc,
-                          (part | ks) > 0 || (fast && pp.j > 0));
-              umma_commit(pv_done + b);
-              if ((pp.t + 1) * kDQ >= pp.c) umma_commit(kv_empty + pp.j);  // the window's last use of the key tile
-              advance(pp);
-              moved = true;
+          // nothing else can go while the scores are two tiles ahead; O starts over with the query tile
+          if (ready(p_full + 2 * s + b, (pp.g >> 1) & 1, ahead >= 2) &&
+              (pp.j > 0 || pp.qn == 0 || ready(o_empty + s, (pp.qn - 1) & 1, ahead >= 2))) {
+            tc_fence_after();
+            const int n16 = (min(kDK, pp.c - pp.j * kDK) + 15) >> 4;
+            const uint32_t a = tm + b * kDK;
+            const uint64_t vd = v_desc + slot * (kDTileB >> 4);
+            const bool kv_end = (pp.t + kDStreams) * kDQ >= pp.c;  // this stream's last use of the key tile
+            if (leader) {
+#pragma unroll
+              for (int ks = 0; ks < kDK / 16; ++ks) {   // P, and its rounding residual beside it
+                if (ks < n16) {
+                  umma_ts(tm + kTmemO, a + ks * kDSub, vd + ks * (16 * kDRowB >> 4), idesc_o, ks > 0 || pp.j > 0);
+                  umma_ts(tm + kTmemO, a + ks * kDSub + kDSub / 2, vd + ks * (16 * kDRowB >> 4), idesc_o, 1);
+                }
+              }
+              umma_commit(pv_done + 2 * s + b);
+              if (kv_end) umma_commit(kv_empty + slot);
+            }
+            __syncwarp();
+            if (advance(pp)) {
+              if (leader) mbar_arrive(meta_empty + (pp.un & 1));
+              next_unit(pp);
+            }
+            moved = true;
+          }
+        }
+      }
+      if (!moved) __nanosleep(100);
+      idle = moved ? 0 : idle + 1;
+      if (idle > (1u << 20)) timed_out = true;
+    }
+    // let the tensor cores finish whatever was issued before the tensor memory is given back
+    if (leader) umma_commit(drain_bar);
+    __syncwarp();
+    mbar_wait_bounded(drain_bar, 0);
+  } else if (warp < kDFirstSoft) {
+    // =========================================== producers ====================================
+    const int pw = warp - kDStreams;
+    const int chunk = lane & 3, rsub = lane >> 2;
+    const T* qkv = reinterpret_cast<const T*>(p.qkv);
+    // Four groups of eight 64-byte row pieces at a time: group g is rows [8 g, 8 g + 8) of `part` (0 q, 1 k, 2 v) from row r0 of the
+    // window on, zero from row c on, stored with the 64-byte swizzle.  Returns the largest squared norm of this warp's rows (q, k; infinite
+    // if one is not finite), or 0 / infinity (v: within kMaxV or not).
+    auto gather = [&](const int* wvox, int c, int h, int n_groups, auto place) -> float {
+      float top = 0.f;
+      uint4 val[4];
+      for (int g0 = pw; g0 < n_groups; g0 += kDProd * 4) {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int gi = g0 + x * kDProd;
+          int part, r0, rl;
+          unsigned char* dst;
+          val[x] = make_uint4(0, 0, 0, 0);
+          if (gi < n_groups) {
+            place(gi, part, r0, rl, dst);
+            const int r = r0 + rl + rsub;
+            if (r < c) val[x] = __ldg(reinterpret_cast<const uint4*>(qkv + (int64_t)wvox[r] * 3 * C + part * C + h * kDHD) + chunk);
+          }
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+          const int gi = g0 + x * kDProd;
+          int part, r0, rl;
+          unsigned char* dst;
+          if (gi < n_groups) {
+            place(gi, part, r0, rl, dst);
+            rl += rsub;
+            *reinterpret_cast<uint4*>(dst + (size_t)rl * kDRowB + ((chunk ^ ((rl >> 1) & 3)) << 4)) = val[x];
+            if (part == 2) {
+              const uint32_t vm = __vmaxu2(__vmaxu2(val[x].x & 0x7fff7fffu, val[x].y & 0x7fff7fffu),
+                                           __vmaxu2(val[x].z & 0x7fff7fffu, val[x].w & 0x7fff7fffu));
+              if (max(vm & 0xffffu, vm >> 16) >= DenseFast<T>::kMaxV) top = INFINITY;
+            } else {
+              float4 a, b;
+              widen8<T>(val[x], a, b);
+              float n2 = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, a.w * a.w))) + fmaf(b.x, b.x, fmaf(b.y, b.y, fmaf(b.z, b.z, b.w * b.w)));
+              n2 += __shfl_xor_sync(0xffffffffu, n2, 1);  // the four lanes of a row
+              n2 += __shfl_xor_sync(0xffffffffu, n2, 2);
+              top = n2 <= 3.0e38f ? fmaxf(top, n2) : INFINITY;  // (NaN as well)
             }
           }
         }
-        idle = moved ? 0 : idle + 1;
-        if (idle > (1u << 24)) {
-          timed_out = true;
-          break;
-        }
-      }
-    }
-    __syncwarp();
-    // let the tensor cores finish whatever was issued before the tensor memory is given back
-    if (lane == 0) umma_commit(drain_bar);
-    __syncwarp();
-    mbar_wait_bounded(drain_bar, 0);
-  } else if (warp <= kDProd) {
-    // =========================================== producers ====================================
-    const int pw = warp - 1;
-    const int chunk = lane & 3, rsub = lane >> 2;
-    const T* qkv = reinterpret_cast<const T*>(p.qkv);
-    // rows [r0, r0 + n_rows) of the window -> tile at `dst` (64-byte rows, 64-byte swizzle); rows
-    // from `c` on are zero.  `part`: 0 q, 1 k, 2 v.  Row groups of eight are dealt to the warps.  Returns the largest
-    // squared norm of this warp's rows (q, k; infinite if one is not finite), or 0 / infinity (v: within kMaxV or not).
-    auto gather = [&](unsigned char* dst, const int* wvox, int r0, int n_rows, int c, int part, int h) -> float {
-      float top = 0.f;
-      uint32_t vm = 0;
-      const int n_groups = (n_rows + 7) >> 3;
-      for (int g0 = pw; g0 < n_groups; g0 += kDProd * 4) {
-        uint4 val[4];
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const int gi = g0 + x * kDProd, rl = gi * 8 + rsub, r = r0 + rl;
-          val[x] = make_uint4(0, 0, 0, 0);
-          if (gi < n_groups && rl < n_rows && r < c) {
-            const int vx = wvox[r];
-            val[x] = __ldg(reinterpret_cast<const uint4*>(qkv + (int64_t)vx * 3 * C + part * C + h * kDHD) + chunk);
-          }
-        }
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-          const int gi = g0 + x * kDProd, rl = gi * 8 + rsub;
-          if (gi < n_groups && rl < n_rows)
-            *reinterpret_cast<uint4*>(dst + (size_t)rl * kDRowB + ((chunk ^ ((rl >> 1) & 3)) << 4)) = val[x];
-          if (part == 2) {
-            vm = __vmaxu2(__vmaxu2(vm, __vmaxu2(val[x].x & 0x7fff7fffu, val[x].y & 0x7fff7fffu)),
-                          __vmaxu2(val[x].z & 0x7fff7fffu, val[x].w & 0x7fff7fffu));
-          } else {
-            float4 a, b;
-            widen8<T>(val[x], a, b);
-            float n2 = fmaf(a.x, a.x, fmaf(a.y, a.y, fmaf(a.z, a.z, a.w * a.w))) + fmaf(b.x, b.x, fmaf(b.y, b.y, fmaf(b.z, b.z, b.w * b.w)));
-            n2 += __shfl_xor_sync(0xffffffffu, n2, 1);  // the four lanes of a row
-            n2 += __shfl_xor_sync(0xffffffffu, n2, 2);
-            top = n2 <= 3.0e38f ? fmaxf(top, n2) : INFINITY;  // (NaN as well)
-          }
-        }
-      }
-      if (part == 2) {
-        const uint32_t m16 = __reduce_max_sync(0xffffffffu, max(vm & 0xffffu, vm >> 16));
-        return m16 < DenseFast<T>::kMaxV ? 0.f : INFINITY;
       }
       return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(top)));  // not negative: ordered as integers
     };
-    uint32_t qn = 0;
-    uint32_t kv_used = 0, kv_par = 0;   // bit j: key tile j has been filled before / how often, modulo two
-    int un = 0;
-    for (int u = blockIdx.x; u < n_units && !timed_out; u += gridDim.x, ++un) {
-      int first, c, h;
-      unit_window(u, first, c, h);
+    // the window of a unit: a few dependent loads, asked for one unit ahead
+    auto unit_window = [&](int u, int& first, int& c) {
+      const int ws = W - 1 - u / H;
+      const int k = min(max(__ldg(p.pack_win + ws), 0), p.w_cap - 1);
+      first = __ldg(p.win_pstart + k);
+      c = __ldg(p.win_start + k + 1) - __ldg(p.win_start + k);
+    };
+    uint32_t qn[kDStreams] = {0, 0};   // query tiles handed to each stream
+    uint32_t slot = 0, use = 0;        // ring slot of the next key tile, how often the ring has been gone through
+    int un = 0, qodd = 0, first_n = 0, c_n = 0, h_staged = -1;
+    float* const bs = reinterpret_cast<float*>(smem + L.bias);
+    unit_window(blockIdx.x, first_n, c_n);
+    for (int u = blockIdx.x; u < n_units && !timed_out; u += step, ++un) {
+      int first = first_n, c = c_n;
+      const int h = u % H;
+      if (!(c > p.tile && c <= p.c_cap && first >= 0 && first <= p.n_vox - c)) {
+        atomicOr(reinterpret_cast<unsigned*>(p.header + SSW_H_ERROR), SSW_DEV_BAD_PLAN);
+        first = 0;   // a one-row window instead: the result is flagged, and every role still finds work
+        c = 1;
+      }
+      if (u + step < n_units) unit_window(u + step, first_n, c_n);
       const int nkt = (c + kDK - 1) / kDK, nqt = (c + kDQ - 1) / kDQ;
       const int mb = un & 1;
       int* wvox = reinterpret_cast<int*>(smem + L.vox) + mb * p.c_cap;
       int* wrel4 = reinterpret_cast<int*>(smem + L.rel4) + mb * p.c_cap;
       int* wreg = reinterpret_cast<int*>(smem + L.reg) + mb * p.c_cap;
       // ---- the window's voxel ids and metadata
-      if (un >= 2 && !mbar_wait_bounded(meta_empty + mb, ((un >> 1) - 1) & 1)) { timed_out = true; break; }
+      if (un >= 2 && !mbar_wait_asleep(meta_empty + mb, ((un >> 1) - 1) & 1)) { timed_out = true; break; }
       if (pw == 0 && lane == 0) unit_c[mb] = c;
+      const int wyx2 = p.bias.wy2 * p.bias.wx2;
       for (int r = pw * 32 + lane; r < nkt * kDK; r += kDProd * 32) {  // (rows from c on: neutral entries)
         int vx = 0, m = 0;
         if (r < c) {
           vx = __ldg(p.pack_perm + first + r);
           m = __ldg(p.pack_meta + first + r);
         }
-        const bool ok = (unsigned)vx < (unsigned)p.n_vox && meta_rel(m) <= p.rel_off;
+        const int code = meta_rel(m), z = code / wyx2, y = (code - z * wyx2) / p.bias.wx2;
+        const int at = z * p.bias.pz + y * p.bias.py + (code - z * wyx2 - y * p.bias.wx2);
+        const bool ok = (unsigned)vx < (unsigned)p.n_vox && code <= p.rel_off && at <= p.bias.off;
         if (!ok) atomicOr(reinterpret_cast<unsigned*>(p.header + SSW_H_ERROR), SSW_DEV_BAD_PLAN);
         wvox[r] = ok ? vx : 0;
-        wrel4[r] = ok ? meta_rel(m) * 4 : 0;
+        wrel4[r] = ok ? at * 4 : 0;
         wreg[r] = ok ? meta_region(m) : 0;
       }
-      // ---- the head's bias slice (rows of the table are [code][head])
-      {
-        float* bs = reinterpret_cast<float*>(smem + L.bias) + (size_t)mb * L.bias_floats;
+      // ---- the head's bias slice (rows of the table are [code][head]), eight loads in flight
+      if (h != h_staged) {
+        // (the unit before is of another head: both streams must be done with it)
+        if (un >= 1 && !mbar_wait_asleep(meta_empty + (mb ^ 1), ((un - 1) >> 1) & 1)) { timed_out = true; break; }
+        h_staged = h;
         float bm = 0.f;
-        for (int i = pw * 32 + lane; i < p.table_rows; i += kDProd * 32) {
-          const float b = __ldg(p.table + (int64_t)i * H + h) * kLog2e;
-          bs[i] = b - DenseFast<T>::kRef;
-          bm = b <= 3.0e38f ? fmaxf(bm, b) : INFINITY;
+        for (int i0 = pw * 32 + lane; i0 < p.table_rows; i0 += kDProd * 32 * 8) {
+          float v[8];
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            const int i = i0 + x * kDProd * 32;
+            v[x] = i < p.table_rows ? __ldg(p.table + (int64_t)i * H + h) * kLog2e : 0.f;
+          }
+#pragma unroll
+          for (int x = 0; x < 8; ++x) {
+            const int i = i0 + x * kDProd * 32, z = i / wyx2, y = (i - z * wyx2) / p.bias.wx2;
+            if (i < p.table_rows) bs[z * p.bias.pz + y * p.bias.py + (i - z * wyx2 - y * p.bias.wx2)] = v[x] - kRef;
+            bm = v[x] <= 3.0e38f ? fmaxf(bm, v[x]) : INFINITY;
+          }
         }
         const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bm)));
-        if (lane == 0) reinterpret_cast<float*>(b_max + mb)[pw] = top;
+        if (lane == 0) b_max[pw] = top;
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(meta_full + mb);
       // the other producer warps' ids are needed for the gathers below
-      if (!mbar_wait_bounded(meta_full + mb, (un >> 1) & 1)) { timed_out = true; break; }
-      // ---- key tiles (k and v), the first query tile in between so that the MMAs can start early
-      for (int j = 0; j < nkt && !timed_out; ++j) {
-        if ((kv_used >> j & 1) && !mbar_wait_bounded(kv_empty + j, (kv_par >> j & 1) ^ 1)) { timed_out = true; break; }
-        const int n_rows = (min(kDK, c - j * kDK) + 15) & ~15;
-        const float kn = gather(smem + L.k + (size_t)j * kDK * kDRowB, wvox, j * kDK, n_rows, c, 1, h);
-        const float vn = gather(smem + L.v + (size_t)j * kDK * kDRowB, wvox, j * kDK, n_rows, c, 2, h);
-        if (lane == 0) reinterpret_cast<float*>(k_norm + j)[pw] = fmaxf(kn, vn);
+      if (!mbar_wait_asleep(meta_full + mb, (un >> 1) & 1)) { timed_out = true; break; }
+      // ---- key tiles; the first query tile of each stream after the first of them so that the MMAs can start early, the
+      // others once all keys are in.  Whatever a wait here is for is work whose tiles have all been handed out before.
+      auto query_tile = [&](int t) {
+        const int s = (qodd + t) & 1;
+        const uint32_t qi = qn[s]++, nb = (uint32_t)p.q_bufs, qb = nb == 2 ? qi & 1 : 0, uses = nb == 2 ? qi >> 1 : qi;
+        if (uses >= 1 && !mbar_wait_asleep(q_empty + 2 * s + qb, (uses - 1) & 1)) {
+          timed_out = true;
+          return;
+        }
+        unsigned char* dq = smem + L.q + (size_t)(s * p.q_bufs + qb) * (kDQ * kDRowB);
+        const float qm = gather(wvox, c, h, kDQ / 8, [&](int gi, int& part, int& r0, int& rl, unsigned char*& dst) {
+          part = 0;
+          r0 = t * kDQ;
+          rl = gi * 8;
+          dst = dq;
+        });
+        if (lane == 0) q_norm[(s * 4 + (qi & 3)) * 8 + pw] = qm;
         fence_async_smem();  // the tensor cores read shared memory through the async proxy
         __syncwarp();
-        if (lane == 0) mbar_arrive(kv_full + j);
-        if (j == 0 || j == nkt - 1) {
-          // query tiles: the first right after key tile 0, the others once all keys are in
-          const int t_lo = j == 0 ? 0 : 1, t_hi = j == 0 ? 1 : nqt;
-          for (int t = (nkt == 1 ? 0 : t_lo); t < (nkt == 1 ? nqt : t_hi) && !timed_out; ++t) {
-            const uint32_t qi = qn + t, qb = qi & 1;
-            if (qi >= 2 && !mbar_wait_bounded(q_empty + qb, ((qi >> 1) - 1) & 1)) { timed_out = true; break; }
-            const float qm = gather(smem + L.q + (size_t)qb * kDQ * kDRowB, wvox, t * kDQ, kDQ, c, 0, h);
-            if (lane == 0) reinterpret_cast<float*>(q_norm + (qi & 3))[pw] = qm;
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(q_full + qb);
-          }
+        if (lane == 0) mbar_arrive(q_full + 2 * s + qb);
+      };
+      for (int j = 0; j < nkt && !timed_out; ++j) {
+        if (use > 0 && !mbar_wait_asleep(kv_empty + slot, (use - 1) & 1)) { timed_out = true; break; }
+        const int ng = ((min(kDK, c - j * kDK) + 15) & ~15) >> 3;
+        unsigned char *dk = smem + L.k + (size_t)slot * kDTileB, *dv = smem + L.v + (size_t)slot * kDTileB;
+        const float kn = gather(wvox, c, h, 2 * ng, [&](int gi, int& part, int& r0, int& rl, unsigned char*& dst) {
+          part = gi < ng ? 1 : 2;
+          r0 = j * kDK;
+          rl = (gi < ng ? gi : gi - ng) * 8;
+          dst = gi < ng ? dk : dv;
+        });
+        if (lane == 0) k_norm[slot * 8 + pw] = kn;
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(kv_full + slot);
+        if (++slot == (uint32_t)p.kv_slots) {
+          slot = 0;
+          ++use;
+        }
+        if (j == 0) {
+          for (int t = 0; t < min(nqt, kDStreams) && !timed_out; ++t) query_tile(t);
         }
       }
-      kv_used |= (1u << nkt) - 1u;
-      kv_par ^= (1u << nkt) - 1u;
-      qn += nqt;
+      for (int t = kDStreams; t < nqt && !timed_out; ++t) query_tile(t);
+      qodd ^= nqt & 1;
     }
   } else {
     // =========================================== softmax rows =================================
-    const int half = (warp - 4) >> 2;          // which part of a tile's keys / of the output channels (0 .. kDParts-1)
+    const int s = (warp - kDFirstSoft) / kDSoftWarps;
+    const int part = ((warp - kDFirstSoft) >> 2) & (kDParts - 1);
     const int sw = warp & 3;                   // tensor-memory lanes [32 sw, 32 sw + 32)
     const int row_in_tile = sw * 32 + lane;
-    const uint32_t t_lane = (uint32_t)(sw * 32) << 16;
+    const uint32_t tm = tmem + ((uint32_t)(sw * 32) << 16) + s * kTmemStream;
     const float qscale = p.scale * kLog2e;
-    uint32_t g = 0;    // key tiles so far
-    uint32_t xn = 0;   // exchanges with the partner warp so far
-    int un = 0;
-    // post a value for the other threads of the row (same row, other key parts) and combine theirs:
-    // the maximum of the others' values, or their sum
-    auto exchange = [&](float mine, float& theirs, bool take_max) -> bool {
-      float* slot = xch + (xn & 1) * (kDParts * 128);
-      slot[half * 128 + row_in_tile] = mine;
-      __syncwarp();
-      if (lane == 0) mbar_arrive(xbar + sw);
-      const bool ok = mbar_wait_bounded(xbar + sw, xn & 1);
-      float acc = take_max ? -INFINITY : 0.f;
-#pragma unroll
-      for (int o2 = 1; o2 < kDParts; ++o2) {
-        const float v = slot[((half + o2) % kDParts) * 128 + row_in_tile];
-        acc = take_max ? fmaxf(acc, v) : acc + v;
-      }
-      theirs = acc;
-      ++xn;
-      return ok;
-    };
-    uint32_t on = 0;  // query tiles this thread has put through the output staging tile
-    uint32_t qt = 0;  // query tiles begun
-    for (int u = blockIdx.x; u < n_units && !timed_out; u += gridDim.x, ++un) {
-      int first, c, h;
-      unit_window(u, first, c, h);
-      const int nkt = (c + kDK - 1) / kDK, nqt = (c + kDQ - 1) / kDQ;
+    uint32_t g = 0;    // key tiles of the stream so far
+    uint32_t qt = 0;   // query tiles of the stream begun
+    uint32_t xn = 0;   // exchanges of maxima so far
+    uint32_t slot0 = 0;  // ring slot of the unit's first key tile
+    int un = 0, qodd = 0;
+    for (int u = blockIdx.x; u < n_units && !timed_out; u += step, ++un) {
       const int mb = un & 1;
+      if (!mbar_wait_bounded(meta_full + mb, (un >> 1) & 1)) { timed_out = true; break; }
+      const int c = *reinterpret_cast<volatile int*>(unit_c + mb), h = u % H;
+      const int nkt = (c + kDK - 1) / kDK, nqt = (c + kDQ - 1) / kDQ;
       const int* wvox = reinterpret_cast<const int*>(smem + L.vox) + mb * p.c_cap;
       const int* wrel4 = reinterpret_cast<const int*>(smem + L.rel4) + mb * p.c_cap;
       const int* wreg = reinterpret_cast<const int*>(smem + L.reg) + mb * p.c_cap;
-      const uint32_t bias_a = smem_u32(smem + L.bias) + (uint32_t)mb * L.bias_floats * 4u;
-      const uint32_t rel4_a = smem_u32(wrel4) + half * kDHalf * 4, reg_a = smem_u32(wreg) + half * kDHalf * 4;
-      if (!mbar_wait_bounded(meta_full + mb, (un >> 1) & 1)) { timed_out = true; break; }
-      for (int t = 0; t < nqt && !timed_out; ++t) {
+      const uint32_t bias_a = smem_u32(smem + L.bias);
+      const uint32_t rel4_a = smem_u32(wrel4), reg_a = smem_u32(wreg);
+      float k_max = 0.f;   // largest squared key norm of the unit, known after the stream's first query tile in it
+      for (int t = (s - qodd) & 1; t < nqt && !timed_out; t += kDStreams) {
         const int qrow = t * kDQ + row_in_tile;
         const bool live = qrow < c;
-        // bias of (me, key j) = slice[(code_me + rel_off) - code_j]: my row's base, minus 4 * code_j
-        const uint32_t my_bias = bias_a + (uint32_t)(live ? wrel4[qrow] : 0) + (uint32_t)p.rel_off * 4u;
+        // bias of (me, key j) = slice[(code_me + off) - code_j] in padded codes: my row's base, minus 4 * code_j
+        const uint32_t my_bias = bias_a + (uint32_t)(live ? wrel4[qrow] : 0) + (uint32_t)p.bias.off * 4u;
         const int my_region = live ? wreg[qrow] : 0;
-        float m = 0.f, l = 0.f, corr_prev = 1.f;   // scores less kRef: the maximum starts from -kRef (0: ops.cu:137)
-        bool fast = true;       // every key tile so far was within the bound
-        float k_limit = 0.f;    // largest squared key norm the bound allows for this query tile
-        float o[kDCpt];
-#pragma unroll
-        for (int e = 0; e < kDCpt; ++e) o[e] = 0.f;
-        for (int j = 0; j <= nkt && !timed_out; ++j) {
-          const uint32_t gp = g - 1, bp = gp & 1;
-          if (j < nkt) {
-            const uint32_t b = g & 1;
-            const int nk = min(kDK, c - j * kDK) - half * kDHalf;  // valid keys among this thread's 64
-            const uint32_t sb = g % kDSBuf;
-            if (!mbar_wait_bounded(s_full + sb, (g / kDSBuf) & 1)) { timed_out = true; break; }
-            tc_fence_after();
-            const uint32_t s_src = tmem + t_lane + kTmemS + sb * kDK + half * kDHalf;
-            const uint32_t p_dst = tmem + t_lane + kTmemP + half * (kDHalf / 2);  // two keys a column
-            if (j == 0) {
-              const float4 q4 = q_norm[qt & 3], b4 = b_max[mb];
-              const float top = fmaxf(fmaxf(b4.x, b4.y), b4.z), q2 = fmaxf(fmaxf(q4.x, q4.y), q4.z);
-              const float lim = (DenseFast<T>::kLimit + kRef - top) / fabsf(qscale);
-              k_limit = lim > 0.f && q2 <= 3.0e38f ? lim * lim / fmaxf(q2, 1e-30f) : -1.f;
+        float m = 0.f, l = 0.f;  // scores less kRef: the maximum starts from -kRef (0: ops.cu:137)
+        bool fast = true;        // every key tile so far was within the bound
+        float k_limit = 0.f;     // largest squared key norm the bound allows for this query tile
+        uint32_t slot = slot0;
+        for (int j = 0; j < nkt; ++j, ++g) {
+          const uint32_t b = g & 1, src = tm + b * kDK;
+          const int nk = min(kDK, c - j * kDK);  // valid keys
+          if (!mbar_wait_bounded(s_full + 2 * s + b, (g >> 1) & 1)) { timed_out = true; break; }
+          tc_fence_after();
+          if (j == 0) {
+            const float4 q4 = *reinterpret_cast<const float4*>(q_norm + (s * 4 + (qt & 3)) * 8);
+            const float2 q2 = *reinterpret_cast<const float2*>(q_norm + (s * 4 + (qt & 3)) * 8 + 4);
+            const float4 b4 = *reinterpret_cast<const float4*>(b_max);
+            const float2 b2 = *reinterpret_cast<const float2*>(b_max + 4);
+            const float top = fmaxf(fmaxf(fmaxf(b4.x, b4.y), fmaxf(b4.z, b4.w)), fmaxf(b2.x, b2.y));
+            const float qq = fmaxf(fmaxf(fmaxf(q4.x, q4.y), fmaxf(q4.z, q4.w)), fmaxf(q2.x, q2.y));
+            const float lim = (DenseFast<T>::kLimit + kRef - top) / fabsf(qscale);
+            k_limit = lim > 0.f && qq <= 3.0e38f ? lim * lim / fmaxf(qq, 1e-30f) : -1.f;
+          }
+          if (t < kDStreams) {
+            const float4 k4 = *reinterpret_cast<const float4*>(k_norm + slot * 8);
+            const float2 k2 = *reinterpret_cast<const float2*>(k_norm + slot * 8 + 4);
+            const float top = fmaxf(fmaxf(fmaxf(k4.x, k4.y), fmaxf(k4.z, k4.w)), fmaxf(k2.x, k2.y));
+            k_max = fmaxf(k_max, top);
+            fast = fast && top <= k_limit;  // the same in every softmax thread
+          } else if (j == 0) {
+            fast = k_max <= k_limit;
+          }
+          if (++slot == (uint32_t)p.kv_slots) slot = 0;
+          // scores of four keys in the log2 domain: bias from the head's slice, -100 across regions
+          auto score4 = [&](const uint32_t* sr, uint32_t key4, float2& lo2, float2& hi2) {
+            const int4 kr = lds_v4(rel4_a + key4);
+            float2 b0 = make_float2(lds_f32(my_bias - (uint32_t)kr.x), lds_f32(my_bias - (uint32_t)kr.y));
+            float2 b1 = make_float2(lds_f32(my_bias - (uint32_t)kr.z), lds_f32(my_bias - (uint32_t)kr.w));
+            if constexpr (kMask) {
+              const int4 kg = lds_v4(reg_a + key4);
+              if (kg.x != my_region) b0.x += -100.0f * kLog2e;
+              if (kg.y != my_region) b0.y += -100.0f * kLog2e;
+              if (kg.z != my_region) b1.x += -100.0f * kLog2e;
+              if (kg.w != my_region) b1.y += -100.0f * kLog2e;
             }
-            const float4 k4 = k_norm[j];
-            const bool was_fast = fast;
-            fast = fast && fmaxf(fmaxf(k4.x, k4.y), k4.z) <= k_limit;   // the same in every softmax thread
-            if (j == 0) m = fast ? 0.f : -kRef;
-            if (fast) {
-              // Packed arithmetic, two keys at a time; nothing here depends on the tile before until P is stored.
-              float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-              const float2 qs2 = make_float2(qscale, qscale), neg = make_float2(-1.f, -1.f);
-#pragma unroll
-              for (int sub = 0; sub < kDHalf / kDSub; ++sub) {
-                uint32_t sr[kDSub], hi[kDSub / 2], lo[kDSub / 2];
-                tmem_ldn(s_src + sub * kDSub, sr);
-                tmem_ld_wait();
-                if (sub == kDHalf / kDSub - 1) {
-                  tc_fence_before();
-                  __syncwarp();
-                  if (lane == 0) mbar_arrive(s_empty + sb);
-                }
-                const int nks = nk - sub * kDSub;
-#pragma unroll
-                for (int q4 = 0; q4 < kDSub / 4; ++q4) {
-                  const uint32_t key4 = (uint32_t)(j * kDK + sub * kDSub + q4 * 4) * 4u;
-                  const int4 kr = lds_v4(rel4_a + key4);
-                  float2 bias[2] = {make_float2(lds_f32(my_bias - (uint32_t)kr.x), lds_f32(my_bias - (uint32_t)kr.y)),
-                                    make_float2(lds_f32(my_bias - (uint32_t)kr.z), lds_f32(my_bias - (uint32_t)kr.w))};
-                  if constexpr (kMask) {
-                    const int4 kg = lds_v4(reg_a + key4);
-                    if (kg.x != my_region) bias[0].x += -100.0f * kLog2e;
-                    if (kg.y != my_region) bias[0].y += -100.0f * kLog2e;
-                    if (kg.z != my_region) bias[1].x += -100.0f * kLog2e;
-                    if (kg.w != my_region) bias[1].y += -100.0f * kLog2e;
-                  }
-#pragma unroll
-                  for (int x = 0; x < 2; ++x) {
-                    const int jj = q4 * 4 + x * 2;
-                    const float2 v = __ffma2_rn(make_float2(__uint_as_float(sr[jj]), __uint_as_float(sr[jj + 1])), qs2, bias[x]);
-                    float2 pv = make_float2(fast_exp2(v.x), fast_exp2(v.y));
-                    if (nks < kDSub) {  // the window's last key tile: nothing beyond its last voxel
-                      if (jj >= nks) pv.x = 0.f;
-                      if (jj + 1 >= nks) pv.y = 0.f;
-                    }
-                    sum2[x] = __fadd2_rn(sum2[x], pv);
-                    hi[jj / 2] = pack2<T>(pv.x, pv.y);
-                    const float2 res = __ffma2_rn(widen2<T>(hi[jj / 2]), neg, pv);
-                    lo[jj / 2] = pack2<T>(res.x, res.y);
-                  }
-                }
-                // the P buffer is free once the P V of the tile before is done
-                if (sub == 0 && g >= 1) {
-                  if (!mbar_wait_bounded(pv_done + bp, (gp >> 1) & 1)) timed_out = true;
-                  tc_fence_after();  // the MMAs read P from tensor memory: the stores below come after them
-                }
-                tmem_stn(p_dst + sub * (kDSub / 2), hi);
-                tmem_stn(p_dst + kDK / 2 + sub * (kDSub / 2), lo);
-              }
-              if (timed_out) break;
-              l += (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y);
-              if (threadIdx.x == 128) fast_flag[b] = 1;
-              tmem_st_wait();
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) {
-                mbar_arrive(p_full + b);
-                if (j > 0) mbar_arrive(o_empty + bp);  // O_part of the tile before was not used: its phase goes on
-              }
-              ++g;
-              continue;
-            }
-            if (was_fast && j > 0) {  // from here on with a running maximum, which starts from the reference of what has been added up
-              if (!mbar_wait_bounded(pv_done + bp, (gp >> 1) & 1)) { timed_out = true; break; }
-              tc_fence_after();
-              uint32_t orr[kDCpt];
-              tmem_ldn(tmem + t_lane + kTmemOAcc + half * kDCpt, orr);
-              tmem_ld_wait();
-              tc_fence_before();
-#pragma unroll
-              for (int e = 0; e < kDCpt; ++e) o[e] = __uint_as_float(orr[e]);
-            }
-            // scores in the log2 domain: bias from the head's slice, -100 across regions, -inf beyond c
-            float s[kDHalf];
-#pragma unroll
-            for (int sub = 0; sub < kDHalf / kDSub; ++sub) {
+            const float2 qs2 = make_float2(qscale, qscale);
+            lo2 = __ffma2_rn(make_float2(__uint_as_float(sr[0]), __uint_as_float(sr[1])), qs2, b0);
+            hi2 = __ffma2_rn(make_float2(__uint_as_float(sr[2]), __uint_as_float(sr[3])), qs2, b1);
+          };
+          float corr = 1.f;
+          if (!fast) {
+            if (j == 0) m = -kRef;
+            float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll 1
+            for (int k = part * kDSub; k < nk; k += kDParts * kDSub) {
               uint32_t sr[kDSub];
-              tmem_ldn(s_src + sub * kDSub, sr);
+              tmem_ldn(src + k, sr);
               tmem_ld_wait();
 #pragma unroll
               for (int q4 = 0; q4 < kDSub / 4; ++q4) {
-                const uint32_t key4 = (uint32_t)(j * kDK + sub * kDSub + q4 * 4) * 4u;
-                const int4 kr = lds_v4(rel4_a + key4);
-                const int krv[4] = {kr.x, kr.y, kr.z, kr.w};
-                int kgv[4] = {0, 0, 0, 0};
-                if constexpr (kMask) {
-                  const int4 kg = lds_v4(reg_a + key4);
-                  kgv[0] = kg.x; kgv[1] = kg.y; kgv[2] = kg.z; kgv[3] = kg.w;
-                }
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                  float v = fmaf(__uint_as_float(sr[q4 * 4 + x]), qscale, lds_f32(my_bias - (uint32_t)krv[x]));
-                  if (kMask && kgv[x] != my_region) v += -100.0f * kLog2e;
-                  s[sub * kDSub + q4 * 4 + x] = v;
-                }
+                float2 v0, v1;
+                score4(sr + q4 * 4, (uint32_t)(j * kDK + k + q4 * 4) * 4u, v0, v1);
+                if (k + q4 * 4 < nk) mx[0] = fmaxf(mx[0], v0.x);   // nothing beyond the window's last voxel
+                if (k + q4 * 4 + 1 < nk) mx[1] = fmaxf(mx[1], v0.y);
+                if (k + q4 * 4 + 2 < nk) mx[2] = fmaxf(mx[2], v1.x);
+                if (k + q4 * 4 + 3 < nk) mx[3] = fmaxf(mx[3], v1.y);
               }
             }
-            tc_fence_before();
+            float mine = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+            float* slots = xmax + (s * 2 + (xn & 1)) * (kDParts * 128);
+            slots[part * 128 + row_in_tile] = mine;
             __syncwarp();
-            if (lane == 0) mbar_arrive(s_empty + sb);
-            if (nk < kDHalf) {  // the window's last key tile: nothing beyond its last voxel
-#pragma unroll
-              for (int jj = 0; jj < kDHalf; ++jj) s[jj] = jj < nk ? s[jj] : -INFINITY;
-            }
-            float mx;
-            {  // four interleaved partial maxima keep the dependency chain short
-              float m4[4] = {s[0], s[1], s[2], s[3]};
-#pragma unroll
-              for (int jj = 4; jj < kDHalf; ++jj) m4[jj & 3] = fmaxf(m4[jj & 3], s[jj]);
-              mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3]));
-            }
-            float mx_other;
-            if (!exchange(mx, mx_other, true)) { timed_out = true; break; }
-            const float m_new = fmaxf(m, fmaxf(mx, mx_other));
-            const float corr = fast_exp2(m - m_new);
+            if (lane == 0) mbar_arrive(xbar + s * 4 + sw);
+            if (!mbar_wait_bounded(xbar + s * 4 + sw, xn & 1)) { timed_out = true; break; }
+            ++xn;
+            const float m_new = fmaxf(m, fmaxf(mine, slots[(part ^ 1) * 128 + row_in_tile]));
+            corr = fast_exp2(m - m_new);
+            const bool grown = m_new != m;
             m = m_new;
-            // the P V of the tile before is done: its O_part is in tensor memory, and the one P buffer, which it read, is free
-            if (g >= 1) {
-              if (!mbar_wait_bounded(pv_done + bp, (gp >> 1) & 1)) { timed_out = true; break; }
-              tc_fence_after();  // before the stores of P below, and the load of O_part
-            }
-            float sum4[4] = {0.f, 0.f, 0.f, 0.f};  // partial row sums, one per pair position
+            if (j > 0 && __any_sync(0xffffffffu, grown)) {  // what has been added up is relative to the old maximum
+              if (!mbar_wait_bounded(pv_done + 2 * s + (b ^ 1), ((g - 1) >> 1) & 1)) { timed_out = true; break; }
+              tc_fence_after();
+              uint32_t orr[kDHD / kDParts];
+              tmem_ldn(tm + kTmemO + part * (kDHD / kDParts), orr);
+              tmem_ld_wait();
 #pragma unroll
-            for (int sub = 0; sub < kDHalf / kDSub; ++sub) {
-              uint32_t hi[kDSub / 2], lo[kDSub / 2];
-#pragma unroll
-              for (int x = 0; x < kDSub / 2; ++x) {
-                const float p0 = fast_exp2(s[sub * kDSub + 2 * x] - m), p1 = fast_exp2(s[sub * kDSub + 2 * x + 1] - m);
-                sum4[x & 3] += p0 + p1;
-                hi[x] = pack2<T>(p0, p1);
-                const float2 h = widen2<T>(hi[x]);
-                lo[x] = pack2<T>(p0 - h.x, p1 - h.y);
-              }
-              tmem_stn(p_dst + sub * (kDSub / 2), hi);
-              tmem_stn(p_dst + kDK / 2 + sub * (kDSub / 2), lo);
+              for (int e = 0; e < kDHD / kDParts; ++e) orr[e] = __float_as_uint(__uint_as_float(orr[e]) * corr);
+              tmem_stn(tm + kTmemO + part * (kDHD / kDParts), orr);
             }
-            l = l * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
-            if (threadIdx.x == 128) fast_flag[b] = 0;
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(p_full + b);
-            // fold the previous tile's O_part in with the factor its maximum update gave
-            if (j > 0) {
-              if (was_fast) {
-                // O_acc was taken over above; it is scaled like a previous O_part whose own factor is 1
-                __syncwarp();
-                if (lane == 0) mbar_arrive(o_empty + bp);
-              } else {
-                uint32_t orr[kDCpt];
-                tmem_ldn(tmem + t_lane + kTmemO + bp * kDHD + half * kDCpt, orr);
-                tmem_ld_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(o_empty + bp);
-#pragma unroll
-                for (int e = 0; e < kDCpt; ++e) o[e] = fmaf(o[e], corr_prev, __uint_as_float(orr[e]));
-              }
-            }
-            corr_prev = corr;
-            ++g;
-          } else {
-            if (!mbar_wait_bounded(pv_done + bp, (gp >> 1) & 1)) { timed_out = true; break; }
-            tc_fence_after();
-            uint32_t orr[kDCpt];
-            tmem_ldn(tmem + t_lane + (fast ? kTmemOAcc : kTmemO + bp * kDHD) + half * kDCpt, orr);
-            tmem_ld_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-              mbar_arrive(o_empty + bp);
-              mbar_arrive(oacc_empty);
-            }
-#pragma unroll
-            for (int e = 0; e < kDCpt; ++e) o[e] = fast ? __uint_as_float(orr[e]) : fmaf(o[e], corr_prev, __uint_as_float(orr[e]));
           }
+          // P = exp2(s - m) and its rounding residual, written over the scores they come from; packed arithmetic, two keys at a time
+          float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+          const float2 neg_m = make_float2(-m, -m);
+          auto probabilities = [&](const uint32_t (&sr)[kDSub], int k, auto less_m, auto last) {
+            uint32_t hi[kDSub / 2], lo[kDSub / 2];
+#pragma unroll
+            for (int q4 = 0; q4 < kDSub / 4; ++q4) {
+              float2 v2[2];
+              score4(sr + q4 * 4, (uint32_t)(j * kDK + k + q4 * 4) * 4u, v2[0], v2[1]);
+#pragma unroll
+              for (int x = 0; x < 2; ++x) {
+                const int jj = q4 * 4 + x * 2;
+                const float2 v = decltype(less_m)::value ? __fadd2_rn(v2[x], neg_m) : v2[x];
+                float2 pv = make_float2(fast_exp2(v.x), fast_exp2(v.y));
+                if (decltype(last)::value) {  // nothing beyond the window's last voxel
+                  if (k + jj >= nk) pv.x = 0.f;
+                  if (k + jj + 1 >= nk) pv.y = 0.f;
+                }
+                sum2[x] = __fadd2_rn(sum2[x], pv);
+                hi[jj / 2] = pack2<T>(pv.x, pv.y);
+                lo[jj / 2] = pack2<T>(residual<T>(pv.x, hi[jj / 2] & 0xffffu), residual<T>(pv.y, hi[jj / 2] >> 16));
+              }
+            }
+            tmem_stn(src + k, hi);
+            tmem_stn(src + k + kDSub / 2, lo);
+          };
+          auto tile = [&](auto less_m) {
+#pragma unroll 1
+            for (int k = part * kDSub; k < nk; k += kDParts * kDSub) {
+              uint32_t sr[kDSub];
+              tmem_ldn(src + k, sr);
+              tmem_ld_wait();
+              if (k + kDSub <= nk) probabilities(sr, k, less_m, std::false_type{});
+              else probabilities(sr, k, less_m, std::true_type{});
+            }
+          };
+          if (fast) tile(std::false_type{});
+          else tile(std::true_type{});
+          l = fmaf(l, corr, (sum2[0].x + sum2[0].y) + (sum2[1].x + sum2[1].y));
+          tmem_st_wait();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(p_full + 2 * s + b);
         }
-        // the row's sum is the two halves' sums (both were kept relative to the same running maximum)
-        float l_other = 0.f;
-        if (!timed_out && !exchange(l, l_other, false)) timed_out = true;
-        // The tile's output goes out through a staging tile in shared memory, so that the four lanes
-        // that write one row's 64-byte head slice sit side by side in one store instruction (a thread
-        // owns only half a slice, and its partner is in another warp).  Whole 64-byte segments matter
-        // for the destinations on peer GPUs, where every store instruction's segments cross NVLink as
-        // packets of their own.  The staging tile is guarded by one barrier of the eight softmax warps
-        // with two phases per query tile: all have written / all have read.
         if (timed_out) break;
-        if (on > 0 && !mbar_wait_bounded(obar, 1)) { timed_out = true; break; }
-        if (live) {
-          // + 1e-8 beside a sum relative to the maximum or 0 (ops.cu:164); one begun within the bound is relative to kRef
-          const float eps = m < 0.f ? 1e-8f : 1e-8f * DenseFast<T>::kExpMinusRef;
-          const float inv = __frcp_rn(l + l_other + eps);
-          const uint32_t dst = smem_u32(smem + L.ostage) + (uint32_t)row_in_tile * kDOutPitch + (uint32_t)half * (kDRowB / kDParts);
+        // ---- the query tile's output, by the one of a row's threads whose turn it is (so that the posted sums of two tiles before have
+        // been read: the other thread's own tile lies in between)
+        float* sums = xsum + (s * 2 + (qt & 1)) * 128;
+        if ((int)(qt & 1) != part) {
+          sums[row_in_tile] = l;
+          __syncwarp();
+          if (lane == 0) mbar_arrive(lbar + s * 4 + sw);
+          ++qt;
+          continue;
+        }
+        if (!mbar_wait_bounded(lbar + s * 4 + sw, qt & 1)) { timed_out = true; break; }
+        l += sums[row_in_tile];
+        uint32_t o[kDHD];
+        if (!mbar_wait_bounded(pv_done + 2 * s + ((g - 1) & 1), ((g - 1) >> 1) & 1)) { timed_out = true; break; }
+        tc_fence_after();
+        tmem_ldn(tm + kTmemO, o);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(o_empty + s);
+        // + 1e-8 beside a sum relative to the maximum or 0 (ops.cu:164); one begun within the bound is relative to kRef
+        const float eps = m < 0.f ? 1e-8f : 1e-8f * DenseFast<T>::kExpMinusRef;
+        const float inv = __frcp_rn(l + eps);
+        // A thread holds the four 16-byte pieces of its own row's head slice.  The four lanes of a group trade pieces, so that each store
+        // instruction writes whole 64-byte segments, a row's slice from four lanes side by side: on a peer GPU every segment
+        // crosses NVLink as a packet of its own.
+        uint32_t w[4][4];
 #pragma unroll
-          for (int e = 0; e < kDCpt / 8; ++e) {
-            uint32_t ww[4];
+        for (int e = 0; e < kDHD / 2; ++e)
+          w[e >> 2][e & 3] = pack2<T>(__uint_as_float(o[2 * e]) * inv, __uint_as_float(o[2 * e + 1]) * inv);
 #pragma unroll
-            for (int x = 0; x < 4; ++x) ww[x] = pack2<T>(o[8 * e + 2 * x] * inv, o[8 * e + 2 * x + 1] * inv);
-            sts_v4(dst + 16u * e, ww[0], ww[1], ww[2], ww[3]);
+        for (int bit = 1; bit <= 2; bit <<= 1) {
+          const bool up = (lane & bit) != 0;
+#pragma unroll
+          for (int x = 0; x < 4; ++x) {
+            if (x & bit) continue;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? w[x][e] : w[x | bit][e], bit);
+              if (up) w[x][e] = got;
+              else w[x | bit][e] = got;
+            }
           }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(obar);
-        if (!mbar_wait_bounded(obar, 0)) { timed_out = true; break; }
 #pragma unroll
-        for (int k2 = 0; k2 < (kDQ * kDRowB / 16) / (32 * kDSoftWarps); ++k2) {
-          const int id = (int)threadIdx.x - 128 + 32 * kDSoftWarps * k2;  // softmax threads are threads 128 and up
-          const int orow = id >> 2, piece = id & 3;
-          if (t * kDQ + orow < c) {
-            const int4 w = lds_v4(smem_u32(smem + L.ostage) + (uint32_t)orow * kDOutPitch + 16u * piece);
-            const int64_t off = (int64_t)wvox[t * kDQ + orow] * C + h * kDHD + piece * 8;
+        for (int x = 0; x < 4; ++x) {
+          const int r = t * kDQ + (row_in_tile & ~3) + x;
+          if (r < c) {
+            const int64_t off = (int64_t)wvox[r] * C + h * kDHD + (lane & 3) * 8;
             for (int d = 0; d < p.outs.n; ++d)
-              *reinterpret_cast<int4*>(reinterpret_cast<T*>(p.outs.base[d]) + off) = w;
+              *reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.outs.base[d]) + off) = make_uint4(w[x][0], w[x][1], w[x][2], w[x][3]);
           }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(obar);
-        ++on;
         ++qt;
       }
+      slot0 = (slot0 + nkt) % (uint32_t)p.kv_slots;
+      qodd ^= nqt & 1;
       __syncwarp();
       if (lane == 0) mbar_arrive(meta_empty + mb);
     }
@@ -761,13 +823,11 @@ int run_attn_dense(const AttnParams& a, const int32_t* bins, const int32_t* win_
   p.table_rows = (2 * rpb_window[0] - 1) * (2 * rpb_window[1] - 1) * (2 * rpb_window[2] - 1);
   p.n_vox = a.n_vox;
   p.w_cap = a.w_cap;
-  p.c_cap = (n_per_window + kDK - 1) / kDK * kDK;
   p.scale = a.scale;
   p.use_mask = a.use_mask;
-  if (p.c_cap > kDMaxKT * kDK) return SSW_E_UNSUPPORTED;
-  const DenseSmem L = dense_smem(p.c_cap, p.table_rows);
+  if (!dense_buffers(n_per_window, rpb_window, p.c_cap, p.kv_slots, p.q_bufs, p.bias)) return SSW_E_UNSUPPORTED;
+  const DenseSmem L = dense_smem(p.c_cap, p.bias.floats, p.kv_slots, p.q_bufs);
   const size_t smem = (size_t)L.total + 1024;  // slack for the 1024-byte alignment of the base
-  if (smem > 227 * 1024) return SSW_E_UNSUPPORTED;
   int dev = 0, sms = 0;
   SSW_CUDA_TRY(cudaGetDevice(&dev));
   SSW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -784,10 +844,9 @@ int run_attn_dense(const AttnParams& a, const int32_t* bins, const int32_t* win_
 // the second phase of the mma.sync kernel).
 bool attn_dense_supported(int head_dim, int n_per_window, const int32_t rpb_window[3]) {
   if (head_dim != kDHD) return false;
-  const int c_cap = (n_per_window + kDK - 1) / kDK * kDK;
-  if (c_cap > kDMaxKT * kDK) return false;
-  const int rows = (2 * rpb_window[0] - 1) * (2 * rpb_window[1] - 1) * (2 * rpb_window[2] - 1);
-  return (size_t)dense_smem(c_cap, rows).total + 1024 <= 227 * 1024;
+  int c_cap, kv_slots, q_bufs;
+  BiasShape bias;
+  return dense_buffers(n_per_window, rpb_window, c_cap, kv_slots, q_bufs, bias);
 }
 
 }  // namespace ssw

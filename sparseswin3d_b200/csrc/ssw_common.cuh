@@ -166,6 +166,17 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
   return false;
 }
+// The same for waits that are long beside the work of the other warps: the warp sleeps between polls, where a loop of try_wait
+// takes issue slots from the others all along.  Bounded in time (about two seconds).
+__device__ __forceinline__ bool mbar_wait_asleep(uint64_t* bar, uint32_t parity, uint32_t ns = 64) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_test(bar, parity)) {
+    if (clock64() - t0 > 4000000000ll) return false;
+    __nanosleep(ns);
+  }
+  return true;
+}
 // global -> shared bulk copy; addresses 16-byte aligned, bytes a multiple of 16.
 __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
   asm volatile(
