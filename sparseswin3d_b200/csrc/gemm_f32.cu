@@ -120,7 +120,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
   uint64_t* drain_bar = lo_empty + 2;        // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   const uint32_t stage0 = smem_u32(smem + 1024);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // (TN: its MMAs are not what it waits for, and with warp-uniform roles it spills: 138 us without for 157 at 150 000 rows, 288 x 96)
+  const int warp = TN ? threadIdx.x >> 5 : __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kGStages; ++s) {
       mbar_init(full + s, kGProd);
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
     // =========================================== producers ====================================
     const uint32_t raw = smem_u32(smem + kGRawOff) + threadIdx.x * 16u;   // this thread's pieces: [kGRaw][8], 4 KB apart
     const int my_tiles = p.tiles > (int)blockIdx.x ? (p.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-    const int64_t total = (int64_t)my_tiles * n_stages;
+    const int total = my_tiles * n_stages;   // (operands that fit the device keep this far below 2^31)
     int lt = blockIdx.x, ls = 0;   // tile and stage the next load belongs to
     // NT: a thread looks after 16-byte piece f4 of rows r0, r0 + 32, ... of both operands (eight lanes read one row's
     // 128 bytes).  TN: warps 0-3 take g, 4-7 take x; a thread, columns 4 quad .. 4 quad + 3 of rows 8 oct .. 8 oct + 7 of
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
     open_tile();
     const int64_t step_rows = TN ? (is_w ? (int64_t)p.N : p.M) : (int64_t)p.K * 32;
     int lslot = 0;
-    int64_t loaded = 0;
+    int loaded = 0;
     auto load = [&]() {   // one commit group per stage, empty beyond the last one
       if (loaded < total) {
         const uint32_t dst = raw + (uint32_t)lslot * kGRawB;
@@ -215,7 +216,8 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
     for (int x = 0; x < kGRaw; ++x) load();
     const uint32_t off = (uint32_t)(r0 * kGRowB + (((f4 >> 1) ^ ((r0 >> 1) & 3)) << 4) + (f4 & 1) * 8);
     int slot = 0;
-    auto step = [&](int64_t i) -> bool {
+    uint32_t s = 0, spar = 1;   // stage, parity of the use of it before this one
+    auto step = [&](int i) -> bool {
       cp_async_wait<kGRaw - 1>();   // this stage's pieces have landed; each thread reads its own
       const uint32_t src = raw + (uint32_t)slot * kGRawB;
       slot = slot + 1 == kGRaw ? 0 : slot + 1;
@@ -225,11 +227,9 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
         const int4 u = lds_v4(src + x * 4096u);
         v[x] = make_float4(__int_as_float(u.x), __int_as_float(u.y), __int_as_float(u.z), __int_as_float(u.w));
       }
-      const int s = (int)(i % kGStages);
-      const int64_t use = i / kGStages;
-      if (use > 0 && !mbar_wait_bounded(empty + s, (uint32_t)(use - 1) & 1)) return false;
+      if (i >= kGStages && !mbar_wait_bounded(empty + s, spar)) return false;
       if constexpr (TN) {
-        const uint32_t base = stage0 + (uint32_t)s * kGStageB + (is_w ? 3u * kGOpB : 0u);
+        const uint32_t base = stage0 + s * kGStageB + (is_w ? 3u * kGOpB : 0u);
         if (!is_w || quad * 4 < bn) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
           }
         }
       } else {
-        const uint32_t base = stage0 + (uint32_t)s * kGStageB + off;
+        const uint32_t base = stage0 + s * kGStageB + off;
 #pragma unroll
         for (int x = 0; x < 8; ++x) {
           if (x >= 4 && r0 + 32 * (x - 4) >= bn) continue;
@@ -263,10 +263,14 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
       fence_async_smem();  // the tensor cores read shared memory through the async proxy
       __syncwarp();
       if (lane == 0) mbar_arrive(full + s);
+      if (++s == kGStages) {
+        s = 0;
+        spar ^= 1;
+      }
       load();   // into the slot just read
       return true;
     };
-    for (int64_t i = 0; i < total && !timed_out; ++i) {
+    for (int i = 0; i < total && !timed_out; ++i) {
       if (!step(i)) {
         timed_out = true;
         break;
@@ -275,34 +279,40 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
     cp_async_wait<0>();   // nothing of this block's may still be on its way into shared memory
   } else if (warp == kGProd) {
     // =========================================== MMA issuer ===================================
-    const uint32_t idesc = instr_desc(1, 1, 0, bn);
-    uint32_t st = 0, ch = 0, tn = 0;   // stages, chunks, tiles so far
+    // All lanes walk along and one issues, on operands that the compiler can see are the same in each: an MMA takes them from
+    // uniform registers, and from a branch of one lane each is first looked for among the lanes (some hundred instructions an
+    // MMA).
+    const uint32_t idesc = instr_desc(1, 1, 0, bn), tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint64_t d0 = smem_desc(stage0, 512, 4);
+    const bool leader = elect_one();
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+      timed_out = !__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+      return !timed_out;
+    };
+    timed_out = __any_sync(0xffffffffu, timed_out);
+    uint32_t s = 0, spar = 0, ch = 0, tn = 0;   // stage and parity of its use, chunks, tiles so far
     for (int t = blockIdx.x; t < p.tiles && !timed_out; t += gridDim.x, ++tn) {
       const uint32_t lb = tn & 1;
-      if (tn >= 2 && !mbar_wait_bounded(lo_empty + lb, ((tn >> 1) - 1) & 1)) { timed_out = true; break; }
-      for (int ks = 0; ks < n_stages; ++ks, ++st) {
-        const uint32_t s = st % kGStages, hb = ch & 1;
+      if (tn >= 2 && !wait(lo_empty + lb, ((tn >> 1) - 1) & 1)) break;
+      for (int ks = 0; ks < n_stages; ++ks) {
+        const uint32_t hb = ch & 1;
         const bool first = ks % kChunk == 0, last = ks % kChunk == kChunk - 1 || ks == n_stages - 1;
-        if (first && ch >= 2 && !mbar_wait_bounded(hh_empty + hb, ((ch >> 1) - 1) & 1)) { timed_out = true; break; }
-        if (!mbar_wait_bounded(full + s, (st / kGStages) & 1)) { timed_out = true; break; }
+        if (first && ch >= 2 && !wait(hh_empty + hb, ((ch >> 1) - 1) & 1)) break;
+        if (!wait(full + s, spar)) break;
         tc_fence_after();
-        if (lane == 0) {
-          const uint32_t A = stage0 + s * kGStageB, B = A + 3 * kGOpB;
+        const uint64_t da = d0 + s * (kGStageB >> 4), db = da + (3 * kGOpB >> 4);
+        const uint32_t hh = tm + hb * kGNMax, lo = tm + kGTmemLow + lb * kGNMax;
+        if (leader) {
+          constexpr int oa = kGOpB >> 4, ob = kGOpWB >> 4;
 #pragma unroll
           for (int k16 = 0; k16 < kGK / 16; ++k16) {
-            uint64_t da[3], db[3];
-#pragma unroll
-            for (int x = 0; x < 3; ++x) {
-              da[x] = smem_desc(A + x * kGOpB + k16 * 32, 512, 4);
-              db[x] = smem_desc(B + x * kGOpWB + k16 * 32, 512, 4);
-            }
-            const uint32_t hh = tmem + hb * kGNMax, lo = tmem + kGTmemLow + lb * kGNMax;
-            umma_ss(hh, da[0], db[0], idesc, !(first && k16 == 0));
-            umma_ss(lo, da[0], db[2], idesc, ks > 0 || k16 > 0);   // smallest first
-            umma_ss(lo, da[2], db[0], idesc, 1);
-            umma_ss(lo, da[1], db[1], idesc, 1);
-            umma_ss(lo, da[0], db[1], idesc, 1);
-            umma_ss(lo, da[1], db[0], idesc, 1);
+            const uint64_t a = da + k16 * 2, b = db + k16 * 2;
+            umma_ss(hh, a, b, idesc, !(first && k16 == 0));
+            umma_ss(lo, a, b + 2 * ob, idesc, ks > 0 || k16 > 0);   // smallest first
+            umma_ss(lo, a + 2 * oa, b, idesc, 1);
+            umma_ss(lo, a + oa, b + ob, idesc, 1);
+            umma_ss(lo, a, b + ob, idesc, 1);
+            umma_ss(lo, a + oa, b, idesc, 1);
           }
           umma_commit(empty + s);
           if (last) umma_commit(hh_full + hb);
@@ -310,10 +320,14 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
         }
         __syncwarp();
         if (last) ++ch;
+        if (++s == kGStages) {
+          s = 0;
+          spar ^= 1;
+        }
       }
     }
     // let the tensor cores finish whatever was issued before the tensor memory is given back
-    if (lane == 0) umma_commit(drain_bar);
+    if (leader) umma_commit(drain_bar);
     __syncwarp();
     mbar_wait_bounded(drain_bar, 0);
   } else {

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kHThreads, 1) k_gemm_gelu(HalfGemmParams p) {
   uint64_t* drain_bar = acc_empty + 2;    // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
   const uint32_t stage0 = smem_u32(smem + 1024);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kHStages; ++s) {
       mbar_init(full + s, kHProd);
@@ -159,27 +159,37 @@ __global__ void __launch_bounds__(kHThreads, 1) k_gemm_gelu(HalfGemmParams p) {
     cp_async_wait<0>();
   } else if (warp == kHProd) {
     const int fmt = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
-    const uint32_t idesc = instr_desc(fmt, fmt, 0, bn);
-    uint32_t st = 0, tn = 0;
+    // (operands in uniform registers: see the issuer of gemm_f32.cu)
+    const uint32_t idesc = instr_desc(fmt, fmt, 0, bn), tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint64_t d0 = smem_desc(stage0, 512, 4);
+    const bool leader = elect_one();
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+      timed_out = !__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+      return !timed_out;
+    };
+    timed_out = __any_sync(0xffffffffu, timed_out);
+    uint32_t s = 0, spar = 0, tn = 0;
     for (int t = blockIdx.x; t < p.tiles && !timed_out; t += gridDim.x, ++tn) {
       const uint32_t ab = tn & 1;
-      if (tn >= 2 && !mbar_wait_bounded(acc_empty + ab, ((tn >> 1) - 1) & 1)) { timed_out = true; break; }
-      for (int ks = 0; ks < n_stages; ++ks, ++st) {
-        const uint32_t s = st % kHStages;
-        if (!mbar_wait_bounded(full + s, (st / kHStages) & 1)) { timed_out = true; break; }
+      if (tn >= 2 && !wait(acc_empty + ab, ((tn >> 1) - 1) & 1)) break;
+      for (int ks = 0; ks < n_stages; ++ks) {
+        if (!wait(full + s, spar)) break;
         tc_fence_after();
-        if (lane == 0) {
-          const uint32_t A = stage0 + s * kHStageB;
+        const uint64_t da = d0 + s * (kHStageB >> 4), db = da + (kHOpB >> 4);
+        if (leader) {
 #pragma unroll
-          for (int k16 = 0; k16 < kHK / 16; ++k16)
-            umma_ss(tmem + ab * kHN, smem_desc(A + k16 * 32, 512, 4), smem_desc(A + kHOpB + k16 * 32, 512, 4), idesc, ks > 0 || k16 > 0);
+          for (int k16 = 0; k16 < kHK / 16; ++k16) umma_ss(tm + ab * kHN, da + k16 * 2, db + k16 * 2, idesc, ks > 0 || k16 > 0);
           umma_commit(empty + s);
           if (ks == n_stages - 1) umma_commit(acc_full + ab);
         }
         __syncwarp();
+        if (++s == kHStages) {
+          s = 0;
+          spar ^= 1;
+        }
       }
     }
-    if (lane == 0) umma_commit(drain_bar);
+    if (leader) umma_commit(drain_bar);
     __syncwarp();
     mbar_wait_bounded(drain_bar, 0);
   } else {
