@@ -22,15 +22,17 @@
 // result is not finite.  150 000 x 288 x 96: one row of Inf 99 -> 110 us, all NaN 920 (library 441); its weight gradient with
 // one row of NaN 138 us, of Inf 520 (353).  Walked to the end, and over all rows by one thread, it was 6060 and 19 300.
 //
-// Persistent, one block per SM, 17 warps: eight bring fp32 pieces in two stages ahead, split them and store the
-// six 64-byte-swizzled operand tiles of a stage (32 of K); one issues the MMAs; eight drain accumulators (a warp
-// may read the 32 tensor-memory lanes warp_id % 4 selects; two warps share them, half the columns each).
-// What bounds it: the issue slots of the split (4.5 instructions per element of both operands) about level with
-// the six MMAs per product.  Against the library's fp32 GEMM with bias:
-// 150 000 x 288 x 96 448 -> 101 us, 150 000 x 96 x 288 270 -> 76, 10 000 x 768 x 192 98 -> 37, 10 000 x 192 x 768
-// 75 -> 46, 128 x 96 x 96 22 -> 12.  Weight gradients: 150 000 rows 288 x 96 358 -> 146, 96 x 96 208 -> 72, 10 000 rows
-// 576 x 192 111 -> 45.  With the raw pieces in registers the latter took 226, 97 and 49: they wait for memory, not for
-// the split.  Two split and three raw stages instead of three and two: 103, 79, 39 and 150.
+// out = a w^T: persistent, one block per SM, 21 warps: eight bring fp32 pieces in three stages (32 of K) ahead, split them and store the terms
+// of a in tensor memory (a thread is a row there) and those of w as 64-byte-swizzled tiles in shared memory; one issues the MMAs; twelve drain
+// accumulators (a warp may read the 32 tensor-memory lanes warp_id % 4 selects; three warps share them, 32 columns each).  Up to K = 192 a block keeps
+// to one tile of columns, whose w it splits once.  What bounds it: the latency of a producer warp's chain per stage (copies, split,
+// stores: 0.95 us a stage, 40 % of the issue slots).  Steps, us at 150 000 x 288 x 96 with bias: 102; MMAs from uniform registers (see the issuer)
+// 96; w kept 91 (shared memory was 84 % busy, a third of it the tensor cores' reads of a); a in tensor memory 79; twelve drain warps for
+// eight 72; loads before the split 71.  The same sizes: 150 000 x 96 x 288 76 -> 70, 150 000 x 96 x 96 41 -> 31, 10 000 x 768 x 192 39 -> 31,
+// 10 000 x 192 x 768 49 -> 39, 10 000 x 192 x 192 20 -> 16, 128 x 576 x 192 14 -> 10; the library's fp32 GEMM 447, 271, 153, 99, 81, 34, 15.
+//
+// Weight gradients: 17 warps, both operands split into shared memory, eight warps drain.  150 000 rows 288 x 96 138 us (library 358), 96 x 96 65 (208),
+// 10 000 rows 576 x 192 44 (111).  With the raw pieces in registers they took 226, 97 and 49: they wait for memory, not for the split.
 #include <math.h>
 
 #include "attn_common.cuh"
@@ -53,15 +55,24 @@ constexpr int kGOpB = kGM * kGRowB;      // bytes of one split tile
 constexpr int kGOpWB = kGNMax * kGRowB;  // ... of w
 constexpr int kGStageB = 3 * kGOpB + 3 * kGOpWB;   // A: h, m, l; B: h, m, l
 constexpr int kGTmemLow = 2 * kGNMax;    // two h h accumulators, then two of small products
-constexpr int kGOutCols = 16, kGOutPitch = kGOutCols + 4;   // a warp's output piece, skewed across the banks
 constexpr int kGRawB = kGProd * 32 * 8 * 16;                  // bytes of one raw stage
-constexpr int kGPiece = 1024 + kGStages * kGStageB, kGRawOff = kGPiece + kGEpi * 32 * kGOutPitch * 4;
+constexpr int kGBiasOff = 1024, kGBiasB = kGEpi * (kGNMax / 2) * 4, kGFirst = 3072;   // the first operand tile: 1024-byte aligned
+static_assert(kGBiasOff + kGBiasB <= kGFirst, "");
+constexpr int kGRawOff = kGFirst + kGStages * kGStageB;
 constexpr int kGSmem = kGRawOff + kGRaw * kGRawB + 1024;
+
+// out = a w^T: a in tensor memory, behind the accumulators, in two stages (h, m, l: 16 columns each); raw pieces of a warp and stage 2 KB.
+constexpr int kNEpi = 12, kNThreads = 32 * (kGProd + 1 + kNEpi);
+constexpr int kNRing = 2, kNTmemA = 4 * kGNMax, kNStageCols = 48;
+constexpr int kNRaws = 4, kNRawWarp = 32 * 64, kNRawStage = kGProd * kNRawWarp, kNRawW = 3 * 4096;
+static_assert(kNTmemA + kNRing * kNStageCols <= 512 && kGNMax <= 96, "");
+struct GemmBars { uint64_t *hh_full, *hh_empty, *lo_full, *lo_empty; };
 
 struct GemmParams {
   const float *a, *w, *bias;
   float* out;
   int gelu;               // the results go through GELU (erf form)
+  int wide;               // rows of out start on 32-byte boundaries
   int64_t M;
   int N, K;
   int bn, n_tiles;        // columns of a tile (a multiple of 16), tiles across N
@@ -69,6 +80,7 @@ struct GemmParams {
   // TN: a is g [rows, M], w is x [rows, N]; out holds `splits` partial results [M, N] of rows_per_split rows each
   int64_t rows;
   int rows_per_split, mn_tiles;
+  int raw_off;            // out = a w^T: where the raw stages lie
   int give_up;           // for tests: as if the first wait had run out (asked at each wait, it costs 2 %)
   int32_t* error;        // SSW_DEV_TIMEOUT goes here, or null
 };
@@ -100,14 +112,347 @@ __device__ __forceinline__ void split8(const float (&x)[8], uint4& h, uint4& m, 
 __device__ __forceinline__ void sts_u4(uint32_t a, const uint4& v) {
   asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
+__device__ __forceinline__ void stg_v8(float* dst, const float2 (&v)[4]) {
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(dst), "r"(__float_as_uint(v[0].x)), "r"(__float_as_uint(v[0].y)),
+               "r"(__float_as_uint(v[1].x)), "r"(__float_as_uint(v[1].y)), "r"(__float_as_uint(v[2].x)), "r"(__float_as_uint(v[2].y)),
+               "r"(__float_as_uint(v[3].x)), "r"(__float_as_uint(v[3].y))
+               : "memory");
+}
 __device__ __forceinline__ float gelu_erf(float x) { return x * 0.5f * (1.0f + erff(x * 0.70710678118654752f)); }
 __device__ __forceinline__ bool not_finite(float v) { return !(fabsf(v) <= 3.402823466e38f); }
 __device__ __forceinline__ void sts_v2(uint32_t a, uint2 v) {
   asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(v.x), "r"(v.y) : "memory");
 }
 
-template <bool TN>
-__global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
+// The warps that drain accumulators: number `ew`, tensor-memory lanes 32 `sub` and up, part number `ew` / 4 of a tile's columns.  This is work in
+// step with the MMAs (a read of the accumulator for every 64 of K, then the stores): with eight warps of half a tile each, 4700 clocks a tile of 96
+// columns at K = 96, it was what 150 000 x 288 x 96 took 79 us for.
+template <bool TN, int PARTS>
+__device__ __forceinline__ void gemm_drain(const GemmParams& p, unsigned char* smem, uint32_t tmem, int ew, int sub, int n_stages, const GemmBars& b,
+                                           bool& timed_out) {
+  constexpr int kChunk = GemmChunk<TN>::kStages, kCols = kGNMax / PARTS;
+  const int lane = threadIdx.x & 31, bn = p.bn, part = ew >> 2;
+  // this thread's columns [c0, c0 + hc) of a tile: 32 of them or what is left (none, where a tile is narrow); TN: half of them
+  const int c0 = PARTS == 3 ? part * kCols : part * (bn / 2), hc = PARTS == 3 ? min(kCols, bn - c0) : bn / 2;
+  const uint32_t t_acc = tmem + ((uint32_t)(sub * 32) << 16) + c0;
+  const int n_chunks = (n_stages + kChunk - 1) / kChunk;
+  float* const bias = reinterpret_cast<float*>(smem + kGBiasOff) + ew * kCols;   // of this warp's columns
+  uint32_t ch = 0, tn = 0;
+  // (after a time-out every tile that is left is stored as NaN: never a plausible result)
+  for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, ++tn) {
+    float2 acc[kCols / 2];
+#pragma unroll
+    for (int e = 0; e < kCols / 2; ++e) acc[e] = make_float2(0.f, 0.f);
+    const int sp = TN ? t / p.mn_tiles : 0, mn = t - sp * (TN ? p.mn_tiles : 0), mt = mn / p.n_tiles;
+    const int n0 = (mn - mt * p.n_tiles) * bn + c0, cols = min(hc, p.N - n0);   // (cols a multiple of four)
+    if (!TN && p.bias) {   // on its way while the products are formed
+      __syncwarp();
+      for (int e = lane; e < cols; e += 32) bias[e] = __ldg(p.bias + n0 + e);
+      __syncwarp();
+    }
+    auto add_columns = [&](uint32_t col) {   // (columns beyond hc of the last sixteen: read, not used)
+      constexpr int kLoads = PARTS == 3 ? 2 : 1;   // at a time
+#pragma unroll
+      for (int e0 = 0; e0 < kCols; e0 += 16 * kLoads) {
+        if (e0 >= hc) continue;
+        uint32_t r[kLoads][16];
+#pragma unroll
+        for (int x = 0; x < kLoads; ++x) tmem_ldn(t_acc + col + e0 + 16 * x, r[x]);
+        tmem_ld_wait();
+#pragma unroll
+        for (int x = 0; x < 16 * kLoads; x += 2)
+          acc[(e0 + x) / 2] = __fadd2_rn(acc[(e0 + x) / 2], make_float2(__uint_as_float(r[x / 16][x % 16]), __uint_as_float(r[x / 16][x % 16 + 1])));
+      }
+    };
+    for (int c = 0; c < n_chunks && !timed_out; ++c, ++ch) {
+      const uint32_t hb = ch & 1;
+      if (!mbar_wait_bounded(b.hh_full + hb, (ch >> 1) & 1)) { timed_out = true; break; }
+      tc_fence_after();
+      add_columns(hb * kGNMax);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(b.hh_empty + hb);
+    }
+    const uint32_t lb = tn & 1;
+    if (!timed_out && !mbar_wait_bounded(b.lo_full + lb, (tn >> 1) & 1)) timed_out = true;
+    if (!timed_out) {
+      tc_fence_after();
+      add_columns(kGTmemLow + lb * kGNMax);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(b.lo_empty + lb);
+    }
+    // A thread stores its own row's columns, 32 bytes (a whole sector) at a time where they start on such a boundary.
+    const int64_t m = (int64_t)mt * kGM + sub * 32 + lane;
+    float* row = p.out + (TN ? (int64_t)sp * p.M * p.N : 0) + m * p.N + n0;
+    const bool wide = p.wide && (n0 & 7) == 0;
+    float2 check = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int e = 0; e < kCols; e += 8) {
+      if (e >= cols) continue;
+      const bool two = e + 4 < cols;
+      float2 v[4] = {acc[e / 2], acc[e / 2 + 1], acc[e / 2 + 2], acc[e / 2 + 3]};
+      if (!TN && p.bias) {
+        const float4 b0 = *reinterpret_cast<const float4*>(bias + e), b1 = *reinterpret_cast<const float4*>(bias + e + 4);
+        v[0] = __fadd2_rn(v[0], make_float2(b0.x, b0.y));
+        v[1] = __fadd2_rn(v[1], make_float2(b0.z, b0.w));
+        v[2] = __fadd2_rn(v[2], make_float2(b1.x, b1.y));
+        v[3] = __fadd2_rn(v[3], make_float2(b1.z, b1.w));
+      }
+      if (timed_out) v[0] = v[1] = v[2] = v[3] = make_float2(NAN, NAN);
+      check = __fadd2_rn(check, __fadd2_rn(v[0], v[1]));
+      if (two) check = __fadd2_rn(check, __fadd2_rn(v[2], v[3]));
+      if (!TN && p.gelu) {
+#pragma unroll
+        for (int x = 0; x < 4; ++x) v[x] = make_float2(gelu_erf(v[x].x), gelu_erf(v[x].y));
+      }
+      if (m < p.M) {
+        if (two && wide) {
+          stg_v8(row + e, v);
+        } else {
+          *reinterpret_cast<float4*>(row + e) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+          if (two) *reinterpret_cast<float4*>(row + e + 4) = make_float4(v[2].x, v[2].y, v[3].x, v[3].y);
+        }
+      }
+    }
+    // a result that is not finite (or a sum of them that is not: looked at once more in vain): once more, from the operands
+    if (!TN && !timed_out && m < p.M && not_finite(check.x + check.y)) {
+      for (int e = 0; e < cols; ++e) {
+        if (!not_finite(row[e])) continue;
+        float v = 0.f;
+        for (int k = 0; k < p.K && v == v; ++k) v = fmaf(__ldg(p.a + m * p.K + k), __ldg(p.w + (int64_t)(n0 + e) * p.K + k), v);
+        if (p.bias) v += __ldg(p.bias + n0 + e);
+        row[e] = p.gelu ? gelu_erf(v) : v;
+      }
+    }
+  }
+}
+
+// out[M, N] = a[M, K] w[N, K]^T.  The rows of a go to tensor memory, where the tensor cores read them beside w in shared memory: a producer thread
+// looks after sixteen columns of one row of a stage, brings them in with its warp through a private piece of shared memory, splits them
+// and stores the three terms with tcgen05.st.  KEPT: a block's columns of w are split once, for all its row tiles.
+template <bool KEPT>
+__global__ void __launch_bounds__(kNThreads, 1) k_gemm_f32(GemmParams p) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
+  uint64_t* full = bars;                     // [kNRing] operands of a stage are in place
+  uint64_t* empty = full + kNRing;           // [kNRing] the stage's MMAs are done
+  uint64_t* hh_full = empty + kNRing;        // [2] a chunk's h h accumulator is complete
+  uint64_t* hh_empty = hh_full + 2;          // [2] ... has been read
+  uint64_t* lo_full = hh_empty + 2;          // [2] a tile's small-product accumulator is complete
+  uint64_t* lo_empty = lo_full + 2;          // [2]
+  uint64_t* drain_bar = lo_empty + 2;        // [1]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kNRing; ++s) {
+      mbar_init(full + s, kGProd);
+      mbar_init(empty + s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(hh_full + b, 1);
+      mbar_init(hh_empty + b, kNEpi);
+      mbar_init(lo_full + b, 1);
+      mbar_init(lo_empty + b, kNEpi);
+    }
+    mbar_init(drain_bar, 1);
+    mbar_fence_init();
+  }
+  if (warp == kGProd) tmem_alloc(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  grid_dependency_wait();
+  const int n_stages = (p.K + kGK - 1) / kGK;       // of one tile
+  const int bn = p.bn;
+  constexpr int kChunk = GemmChunk<false>::kStages;
+  bool timed_out = p.give_up != 0;
+  const uint32_t w_smem = smem_u32(smem + kGFirst);   // [stage][3][bn rows of 64 bytes]: all of K, or the ring's stages
+
+  if (warp < kGProd) {
+    // =========================================== producers ====================================
+    // A warp brings in 32 rows (the tensor-memory lanes warp % 4 selects) of 16 columns: 64 bytes a row by four lanes, into 2 KB of its own
+    // for each stage under way, chunks swapped so that a thread then reads its row without bank conflicts.
+    const int sub = warp & 3, kh = warp >> 2, lc = lane & 3, lr = lane >> 2;
+    const uint32_t mine = smem_u32(smem + p.raw_off) + (uint32_t)warp * kNRawWarp;
+    const int my_tiles = p.tiles > (int)blockIdx.x ? (p.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
+    const int total = my_tiles * n_stages;   // (operands that fit the device keep this far below 2^31)
+    int lt = blockIdx.x, ls = 0;             // tile and stage the next load belongs to
+    const float *pa, *pw = nullptr;
+    int rows_a, rows_w = 0;
+    // w (KEPT: of the first tile): piece f4 of rows wr, wr + 32 and wr + 64 of a stage, each read by the thread that asked for it
+    const int f4 = threadIdx.x & 7, wr = threadIdx.x >> 3;
+    const uint32_t w_mine = smem_u32(smem + p.raw_off) + kNRaws * kNRawStage + threadIdx.x * 16u;
+    auto open_tile = [&]() {
+      const int mt = lt / p.n_tiles, n0 = (lt - mt * p.n_tiles) * bn;
+      const int64_t m0 = (int64_t)mt * kGM + sub * 32;
+      rows_a = (int)max((int64_t)0, min((int64_t)32, p.M - m0));
+      pa = p.a + (m0 + lr) * p.K + kh * 16 + lc * 4;
+      rows_w = min(bn, p.N - n0) - wr;
+      pw = p.w + (int64_t)(n0 + wr) * p.K + f4 * 4;
+    };
+    open_tile();
+    const int64_t k8 = (int64_t)p.K * 8, k32 = (int64_t)p.K * 32;
+    int lslot = 0, loaded = 0;
+    auto load = [&]() {   // one commit group per stage, empty beyond the last one
+      if (loaded < total) {
+        const bool kin = ls * kGK + kh * 16 + lc * 4 < p.K;   // K is a multiple of four
+        const uint32_t dst = mine + (uint32_t)lslot * kNRawStage;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int r = lr + 8 * i;
+          const bool on = kin && r < rows_a;
+          cp_async16_or_zero(dst + r * 64 + ((lc ^ ((r >> 1) & 3)) << 4), on ? pa + i * k8 : p.a, on);
+        }
+        pa += kGK;
+        if (!KEPT || loaded < n_stages) {
+          const bool win = ls * kGK + f4 * 4 < p.K;
+          const uint32_t wd = w_mine + (uint32_t)lslot * kNRawW;
+#pragma unroll
+          for (int i = 0; i < 3; ++i) {
+            const bool on = win && 32 * i < rows_w;
+            cp_async16_or_zero(wd + i * 4096u, on ? pw + i * k32 : p.a, on);
+          }
+          pw += kGK;
+        }
+        lslot = lslot + 1 == kNRaws ? 0 : lslot + 1;
+        ++loaded;
+        if (++ls == n_stages) {
+          ls = 0;
+          lt += gridDim.x;
+          if (lt < p.tiles) open_tile();
+        }
+      }
+      cp_async_commit();
+    };
+    for (int x = 0; x < kNRaws - 1; ++x) load();
+    auto store_w = [&](uint32_t stage, int r, int f, const float4& v) {
+      uint2 h, m, l;
+      split4(v, h, m, l);
+      const uint32_t d = stage + (uint32_t)(r * kGRowB + (((f >> 1) ^ ((r >> 1) & 3)) << 4) + (f & 1) * 8);
+      sts_v2(d, h);
+      sts_v2(d + kGOpWB, m);
+      sts_v2(d + 2 * kGOpWB, l);
+    };
+    int slot = 0;
+    uint32_t s = 0, spar = 1;   // stage, parity of the use of it before this one
+    for (int i = 0; i < total && !timed_out; ++i) {
+      // this stage's pieces have landed, those of the warp's other lanes as well
+      cp_async_wait<kNRaws - 2>();
+      __syncwarp();
+      const uint32_t src = mine + (uint32_t)slot * kNRawStage + lane * 64;
+      int4 raw4[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) raw4[x] = lds_v4(src + ((x ^ ((lane >> 1) & 3)) << 4));
+      load();   // into the slot of the stage before, which all lanes have read
+      uint32_t h[8], m[8], l[8];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int4 u = raw4[x];
+        uint2 h2, m2, l2;
+        split4(make_float4(__int_as_float(u.x), __int_as_float(u.y), __int_as_float(u.z), __int_as_float(u.w)), h2, m2, l2);
+        h[2 * x] = h2.x; h[2 * x + 1] = h2.y;
+        m[2 * x] = m2.x; m[2 * x + 1] = m2.y;
+        l[2 * x] = l2.x; l[2 * x + 1] = l2.y;
+      }
+      if (i >= kNRing && !mbar_wait_bounded(empty + s, spar)) {
+        timed_out = true;
+        break;
+      }
+      tc_fence_after();   // the MMAs that read the stage before come before the stores below
+      const uint32_t ta = tmem + ((uint32_t)(sub * 32) << 16) + kNTmemA + s * kNStageCols + kh * 8;
+      tmem_stn(ta, h);
+      tmem_stn(ta + 16, m);
+      tmem_stn(ta + 32, l);
+      if (!KEPT || i < n_stages) {   // (kept: with the first tile)
+        const uint32_t wsrc = w_mine + (uint32_t)slot * kNRawW;
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+          if (wr + 32 * x >= bn) continue;
+          const int4 u = lds_v4(wsrc + x * 4096u);
+          store_w(w_smem + (KEPT ? (uint32_t)i : s) * 3 * kGOpWB, wr + 32 * x, f4,
+                  make_float4(__int_as_float(u.x), __int_as_float(u.y), __int_as_float(u.z), __int_as_float(u.w)));
+        }
+        fence_async_smem();  // the tensor cores read shared memory through the async proxy
+      }
+      slot = slot + 1 == kNRaws ? 0 : slot + 1;
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(full + s);
+      if (++s == kNRing) {
+        s = 0;
+        spar ^= 1;
+      }
+    }
+    cp_async_wait<0>();   // nothing of this block's may still be on its way into shared memory
+  } else if (warp == kGProd) {
+    // =========================================== MMA issuer ===================================
+    // All lanes walk along and one issues, on operands that the compiler can see are the same in each: an MMA takes them from
+    // uniform registers, and from a branch of one lane each is first looked for among the lanes (some hundred instructions an
+    // MMA: 150 000 x 288 x 96 102 us for 96, 10 000 x 192 x 768 49 for 41).
+    const uint32_t idesc = instr_desc(1, 1, 0, bn), tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint64_t w0 = smem_desc(w_smem, 512, 4);
+    const bool leader = elect_one();
+    auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
+      timed_out = !__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
+      return !timed_out;
+    };
+    timed_out = __any_sync(0xffffffffu, timed_out);
+    uint32_t s = 0, spar = 0, ch = 0, tn = 0;   // stage and parity of its use, chunks, tiles so far
+    for (int t = blockIdx.x; t < p.tiles && !timed_out; t += gridDim.x, ++tn) {
+      const uint32_t lb = tn & 1;
+      if (tn >= 2 && !wait(lo_empty + lb, ((tn >> 1) - 1) & 1)) break;
+      for (int ks = 0; ks < n_stages; ++ks) {
+        const uint32_t hb = ch & 1;
+        const bool first = ks % kChunk == 0, last = ks % kChunk == kChunk - 1 || ks == n_stages - 1;
+        if (first && ch >= 2 && !wait(hh_empty + hb, ((ch >> 1) - 1) & 1)) break;
+        if (!wait(full + s, spar)) break;
+        tc_fence_after();
+        const uint32_t ta = tm + kNTmemA + s * kNStageCols, hh = tm + hb * kGNMax, lo = tm + kGTmemLow + lb * kGNMax;
+        const uint64_t db = w0 + (KEPT ? ks : (int)s) * (3 * kGOpWB >> 4);
+        if (leader) {
+          constexpr int ob = kGOpWB >> 4;
+#pragma unroll
+          for (int k16 = 0; k16 < kGK / 16; ++k16) {
+            const uint32_t a = ta + k16 * 8;
+            const uint64_t b = db + k16 * 2;
+            umma_ts(hh, a, b, idesc, !(first && k16 == 0));
+            umma_ts(lo, a, b + 2 * ob, idesc, ks > 0 || k16 > 0);   // smallest first
+            umma_ts(lo, a + 32, b, idesc, 1);
+            umma_ts(lo, a + 16, b + ob, idesc, 1);
+            umma_ts(lo, a, b + ob, idesc, 1);
+            umma_ts(lo, a + 16, b, idesc, 1);
+          }
+          umma_commit(empty + s);
+          if (last) umma_commit(hh_full + hb);
+          if (ks == n_stages - 1) umma_commit(lo_full + lb);
+        }
+        __syncwarp();
+        if (last) ++ch;
+        if (++s == kNRing) {
+          s = 0;
+          spar ^= 1;
+        }
+      }
+    }
+    // let the tensor cores finish whatever was issued before the tensor memory is given back
+    if (leader) umma_commit(drain_bar);
+    __syncwarp();
+    mbar_wait_bounded(drain_bar, 0);
+  } else {
+    gemm_drain<false, 3>(p, smem, tmem, warp - kGProd - 1, warp & 3, n_stages, {hh_full, hh_empty, lo_full, lo_empty}, timed_out);
+  }
+  if (timed_out && p.error) atomicOr(reinterpret_cast<unsigned*>(p.error), SSW_DEV_TIMEOUT);
+  tc_fence_before();
+  __syncthreads();
+  if (warp == kGProd) tmem_dealloc(tmem, 512);
+}
+
+// out[N, K] = g[M, N]^T x[M, K] over a range of rows: both operands in shared memory.
+__global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32_tn(GemmParams p) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
@@ -119,9 +464,9 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
   uint64_t* lo_empty = lo_full + 2;          // [2]
   uint64_t* drain_bar = lo_empty + 2;        // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
-  const uint32_t stage0 = smem_u32(smem + 1024);
-  // (TN: its MMAs are not what it waits for, and with warp-uniform roles it spills: 138 us without for 157 at 150 000 rows, 288 x 96)
-  const int warp = TN ? threadIdx.x >> 5 : __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t stage0 = smem_u32(smem + kGFirst);
+  // (with roles the compiler knows to be uniform, as k_gemm_f32 has them, this kernel spills: 157 us for 138 at 150 000 rows, 288 x 96)
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < kGStages; ++s) {
       mbar_init(full + s, kGProd);
@@ -142,9 +487,9 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   grid_dependency_wait();
-  const int n_stages = ((TN ? p.rows_per_split : p.K) + kGK - 1) / kGK;       // of one tile
+  const int n_stages = (p.rows_per_split + kGK - 1) / kGK;       // of one tile
   const int bn = p.bn;
-  constexpr int kChunk = GemmChunk<TN>::kStages;
+  constexpr int kChunk = GemmChunk<true>::kStages;
   bool timed_out = p.give_up != 0;
 
   if (warp < kGProd) {
@@ -153,56 +498,33 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
     const int my_tiles = p.tiles > (int)blockIdx.x ? (p.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const int total = my_tiles * n_stages;   // (operands that fit the device keep this far below 2^31)
     int lt = blockIdx.x, ls = 0;   // tile and stage the next load belongs to
-    // NT: a thread looks after 16-byte piece f4 of rows r0, r0 + 32, ... of both operands (eight lanes read one row's
-    // 128 bytes).  TN: warps 0-3 take g, 4-7 take x; a thread, columns 4 quad .. 4 quad + 3 of rows 8 oct .. 8 oct + 7 of
-    // a stage (eight lanes read 128 bytes of one row).
-    const int f4 = threadIdx.x & 7, r0 = threadIdx.x >> 3;
+    // Warps 0-3 take g, 4-7 take x; a thread, columns 4 quad .. 4 quad + 3 of rows 8 oct .. 8 oct + 7 of a stage (eight lanes read 128 bytes
+    // of one row).
     const bool is_w = threadIdx.x >= 128;
     const int oct = threadIdx.x & 3, quad = (threadIdx.x & 127) >> 2;
-    const float *pa, *pw = nullptr;   // this thread's piece of the tile's next stage
-    int rows_a, rows_w = 0;           // NT: rows of the tile from r0 on that exist; TN: rows of the split from oct on, and whether the columns do
+    const float* pa;   // this thread's piece of the tile's next stage
+    int rows_a;        // rows of the split from oct on, and whether the columns exist
     auto open_tile = [&]() {
-      if constexpr (TN) {
-        const int sp = lt / p.mn_tiles, mn = lt - sp * p.mn_tiles, mt = mn / p.n_tiles;
-        const int col = (is_w ? (mn - mt * p.n_tiles) * bn : mt * kGM) + quad * 4, ld = is_w ? p.N : (int)p.M;
-        const int64_t k0 = (int64_t)sp * p.rows_per_split + oct * 8;
-        rows_a = (int)max((int64_t)0, min((int64_t)p.rows_per_split - oct * 8, p.rows - k0));
-        if (col >= ld || (is_w && quad * 4 >= bn)) rows_a = 0;   // M and N are multiples of four
-        pa = (is_w ? p.w : p.a) + k0 * ld + col;
-      } else {
-        const int mt = lt / p.n_tiles, n0 = (lt - mt * p.n_tiles) * bn;
-        const int64_t m0 = (int64_t)mt * kGM;
-        rows_a = (int)min((int64_t)kGM, p.M - m0) - r0;
-        rows_w = min(bn, p.N - n0) - r0;
-        pa = p.a + (m0 + r0) * p.K + f4 * 4;
-        pw = p.w + (int64_t)(n0 + r0) * p.K + f4 * 4;
-      }
+      const int sp = lt / p.mn_tiles, mn = lt - sp * p.mn_tiles, mt = mn / p.n_tiles;
+      const int col = (is_w ? (mn - mt * p.n_tiles) * bn : mt * kGM) + quad * 4, ld = is_w ? p.N : (int)p.M;
+      const int64_t k0 = (int64_t)sp * p.rows_per_split + oct * 8;
+      rows_a = (int)max((int64_t)0, min((int64_t)p.rows_per_split - oct * 8, p.rows - k0));
+      if (col >= ld || (is_w && quad * 4 >= bn)) rows_a = 0;   // M and N are multiples of four
+      pa = (is_w ? p.w : p.a) + k0 * ld + col;
     };
     open_tile();
-    const int64_t step_rows = TN ? (is_w ? (int64_t)p.N : p.M) : (int64_t)p.K * 32;
+    const int64_t step_rows = is_w ? (int64_t)p.N : p.M;
     int lslot = 0;
     int loaded = 0;
     auto load = [&]() {   // one commit group per stage, empty beyond the last one
       if (loaded < total) {
         const uint32_t dst = raw + (uint32_t)lslot * kGRawB;
-        if constexpr (TN) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const bool on = ls * kGK + i < rows_a;
-            cp_async16_or_zero(dst + i * 4096u, on ? pa + i * step_rows : p.a, on);
-          }
-          pa += kGK * step_rows;
-        } else {
-          const bool kin = ls * kGK + f4 * 4 < p.K;   // K is a multiple of four
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const bool ona = kin && 32 * i < rows_a, onw = kin && 32 * i < rows_w;
-            cp_async16_or_zero(dst + i * 4096u, ona ? pa + i * step_rows : p.a, ona);
-            cp_async16_or_zero(dst + (4 + i) * 4096u, onw ? pw + i * step_rows : p.a, onw);
-          }
-          pa += kGK;
-          pw += kGK;
-        }
+        #pragma unroll
+                  for (int i = 0; i < 8; ++i) {
+                    const bool on = ls * kGK + i < rows_a;
+                    cp_async16_or_zero(dst + i * 4096u, on ? pa + i * step_rows : p.a, on);
+                  }
+                  pa += kGK * step_rows;
         lslot = lslot + 1 == kGRaw ? 0 : lslot + 1;
         ++loaded;
         if (++ls == n_stages) {
@@ -214,7 +536,6 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
       cp_async_commit();
     };
     for (int x = 0; x < kGRaw; ++x) load();
-    const uint32_t off = (uint32_t)(r0 * kGRowB + (((f4 >> 1) ^ ((r0 >> 1) & 3)) << 4) + (f4 & 1) * 8);
     int slot = 0;
     uint32_t s = 0, spar = 1;   // stage, parity of the use of it before this one
     auto step = [&](int i) -> bool {
@@ -228,38 +549,23 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
         v[x] = make_float4(__int_as_float(u.x), __int_as_float(u.y), __int_as_float(u.z), __int_as_float(u.w));
       }
       if (i >= kGStages && !mbar_wait_bounded(empty + s, spar)) return false;
-      if constexpr (TN) {
-        const uint32_t base = stage0 + s * kGStageB + (is_w ? 3u * kGOpB : 0u);
-        if (!is_w || quad * 4 < bn) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float x[8];
-#pragma unroll
-            for (int i8 = 0; i8 < 8; ++i8) x[i8] = j == 0 ? v[i8].x : j == 1 ? v[i8].y : j == 2 ? v[i8].z : v[i8].w;
-            uint4 h, m, l;
-            split8(x, h, m, l);
-            const int row = quad * 4 + j;
-            const uint32_t d = base + (uint32_t)(row * kGRowB + ((oct ^ ((row >> 1) & 3)) << 4));
-            const uint32_t op = is_w ? kGOpWB : kGOpB;
-            sts_u4(d, h);
-            sts_u4(d + op, m);
-            sts_u4(d + 2 * op, l);
-          }
-        }
-      } else {
-        const uint32_t base = stage0 + s * kGStageB + off;
-#pragma unroll
-        for (int x = 0; x < 8; ++x) {
-          if (x >= 4 && r0 + 32 * (x - 4) >= bn) continue;
-          uint2 h, m, l;
-          split4(v[x], h, m, l);
-          const uint32_t d = base + (x >= 4 ? 3u * kGOpB : 0u) + (uint32_t)(x & 3) * (32u * kGRowB);
-          const uint32_t op = x >= 4 ? kGOpWB : kGOpB;
-          sts_v2(d, h);
-          sts_v2(d + op, m);
-          sts_v2(d + 2 * op, l);
-        }
-      }
+              const uint32_t base = stage0 + s * kGStageB + (is_w ? 3u * kGOpB : 0u);
+              if (!is_w || quad * 4 < bn) {
+      #pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  float x[8];
+      #pragma unroll
+                  for (int i8 = 0; i8 < 8; ++i8) x[i8] = j == 0 ? v[i8].x : j == 1 ? v[i8].y : j == 2 ? v[i8].z : v[i8].w;
+                  uint4 h, m, l;
+                  split8(x, h, m, l);
+                  const int row = quad * 4 + j;
+                  const uint32_t d = base + (uint32_t)(row * kGRowB + ((oct ^ ((row >> 1) & 3)) << 4));
+                  const uint32_t op = is_w ? kGOpWB : kGOpB;
+                  sts_u4(d, h);
+                  sts_u4(d + op, m);
+                  sts_u4(d + 2 * op, l);
+                }
+              }
       fence_async_smem();  // the tensor cores read shared memory through the async proxy
       __syncwarp();
       if (lane == 0) mbar_arrive(full + s);
@@ -331,99 +637,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32(GemmParams p) {
     __syncwarp();
     mbar_wait_bounded(drain_bar, 0);
   } else {
-    // =========================================== epilogue =====================================
-    const int ew = warp - kGProd - 1, half = ew >> 2, sub = warp & 3;
-    const uint32_t t_lane = (uint32_t)(sub * 32) << 16;
-    const int hc = bn / 2, c0 = half * hc;   // this thread's columns [c0, c0 + hc), hc a multiple of eight
-    const int n_chunks = (n_stages + kChunk - 1) / kChunk;
-    uint32_t ch = 0, tn = 0;
-    // (after a time-out every tile that is left is stored as NaN: never a plausible result)
-    for (int t = blockIdx.x; t < p.tiles; t += gridDim.x, ++tn) {
-      float acc[kGNMax / 2];
-#pragma unroll
-      for (int e = 0; e < kGNMax / 2; ++e) acc[e] = 0.f;
-      auto add_columns = [&](uint32_t col) {
-#pragma unroll
-        for (int e = 0; e < kGNMax / 2; e += 16) {
-          if (e < hc) {   // (the last eight columns of an odd multiple of eight: read, not used)
-            uint32_t r[16];
-            tmem_ld16(tmem + t_lane + col + c0 + e, r);
-            tmem_ld_wait();
-#pragma unroll
-            for (int x = 0; x < 16; ++x) acc[e + x] += __uint_as_float(r[x]);
-          }
-        }
-      };
-      for (int c = 0; c < n_chunks && !timed_out; ++c, ++ch) {
-        const uint32_t hb = ch & 1;
-        if (!mbar_wait_bounded(hh_full + hb, (ch >> 1) & 1)) { timed_out = true; break; }
-        tc_fence_after();
-        add_columns(hb * kGNMax);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(hh_empty + hb);
-      }
-      const uint32_t lb = tn & 1;
-      if (!timed_out && !mbar_wait_bounded(lo_full + lb, (tn >> 1) & 1)) timed_out = true;
-      if (!timed_out) {
-        tc_fence_after();
-        add_columns(kGTmemLow + lb * kGNMax);
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(lo_empty + lb);
-      }
-      // Out through shared memory, 16 columns at a time, so that four lanes store 64 bytes of one row.
-      const int sp = TN ? t / p.mn_tiles : 0, mn = t - sp * (TN ? p.mn_tiles : 0), mt = mn / p.n_tiles;
-      const int64_t m0 = (int64_t)mt * kGM + sub * 32;
-      const int n0 = (mn - mt * p.n_tiles) * bn + c0;
-      float* out = p.out + (TN ? (int64_t)sp * p.M * p.N : 0);
-      float* piece = reinterpret_cast<float*>(smem + kGPiece) + ew * 32 * kGOutPitch;
-      const int pr = lane >> 2, pc = (lane & 3) * 4;
-      bool odd = false;   // a result that is not finite (or a sum of four that is not: looked at once more in vain)
-#pragma unroll
-      for (int e = 0; e < kGNMax / 2; e += kGOutCols) {
-        if (e < hc) {
-          __syncwarp();
-#pragma unroll
-          for (int x = 0; x < kGOutCols; x += 4)
-            *reinterpret_cast<float4*>(piece + lane * kGOutPitch + x) = make_float4(acc[e + x], acc[e + x + 1], acc[e + x + 2], acc[e + x + 3]);
-          __syncwarp();
-          const int n = n0 + e + pc;
-          const bool on = e + pc < hc && n < p.N;   // hc and N are multiples of four
-          float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (on && p.bias) b = __ldg(reinterpret_cast<const float4*>(p.bias + n));
-#pragma unroll
-          for (int x = 0; x < 4; ++x) {
-            const int64_t m = m0 + pr + 8 * x;
-            float4 v = *reinterpret_cast<const float4*>(piece + (pr + 8 * x) * kGOutPitch + pc);
-            v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
-            if (timed_out) v = make_float4(NAN, NAN, NAN, NAN);
-            if (on && m < p.M) {
-              odd = odd || not_finite((v.x + v.y) + (v.z + v.w));
-              if (!TN && p.gelu) v = make_float4(gelu_erf(v.x), gelu_erf(v.y), gelu_erf(v.z), gelu_erf(v.w));
-              *reinterpret_cast<float4*>(out + m * p.N + n) = v;
-            }
-          }
-        }
-      }
-      if (!TN && odd && !timed_out) {  // this lane's results once more, those that are not finite from the operands
-        for (int e = 0; e < hc; e += kGOutCols) {
-          const int n = n0 + e + pc;
-          if (e + pc >= hc || n >= p.N) continue;
-          for (int x = 0; x < 4; ++x) {
-            const int64_t m = m0 + pr + 8 * x;
-            if (m >= p.M) continue;
-            for (int c = 0; c < 4; ++c) {
-              if (!not_finite(out[m * p.N + n + c])) continue;
-              float v = 0.f;
-              for (int k = 0; k < p.K && v == v; ++k) v = fmaf(__ldg(p.a + m * p.K + k), __ldg(p.w + (int64_t)(n + c) * p.K + k), v);
-              if (p.bias) v += __ldg(p.bias + n + c);
-              out[m * p.N + n + c] = p.gelu ? gelu_erf(v) : v;
-            }
-          }
-        }
-      }
-    }
+    gemm_drain<true, 2>(p, smem, tmem, warp - kGProd - 1, warp & 3, n_stages, {hh_full, hh_empty, lo_full, lo_empty}, timed_out);
   }
   if (timed_out && p.error) atomicOr(reinterpret_cast<unsigned*>(p.error), SSW_DEV_TIMEOUT);
   tc_fence_before();
@@ -497,6 +711,10 @@ static int gemm_columns(int64_t m_tiles, int N, int sms, int* n_tiles) {
   return best;
 }
 
+// K up to which a block's columns of w are kept: six stages of 18 KB beside four of 28 KB of raw rows.
+constexpr int kGKeptK = 6 * kGK;
+static_assert(kGFirst + kGKeptK / kGK * 3 * kGOpWB + kNRaws * (kNRawStage + kNRawW) + 1024 <= 227 * 1024, "");
+
 static int gemm_nt(const float* a, const float* w, const float* bias, float* out, int64_t M, int32_t N, int32_t K, int gelu, int32_t* error,
             int give_up, void* stream_) {
   if (M < 0 || N <= 0 || K <= 0) return SSW_E_INVALID;
@@ -512,13 +730,20 @@ static int gemm_nt(const float* a, const float* w, const float* bias, float* out
   GemmParams p = {};
   p.a = a; p.w = w; p.bias = bias; p.out = out; p.M = M; p.N = N; p.K = K; p.gelu = gelu;
   p.error = error; p.give_up = give_up;
+  p.wide = N % 8 == 0 && (reinterpret_cast<uintptr_t>(out) & 31) == 0;
   const int64_t m_tiles = ceil_div64(M, kGM);
   p.bn = gemm_columns(m_tiles, N, sms, &p.n_tiles);
   if (m_tiles * p.n_tiles >= ((int64_t)1 << 30)) return SSW_E_RANGE;
   p.tiles = (int)(m_tiles * p.n_tiles);
-  SSW_CUDA_TRY(cudaFuncSetAttribute(k_gemm_f32<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
-  SSW_CUDA_TRY(launch_chained(k_gemm_f32<false>, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kGThreads), kGSmem,
-                              (cudaStream_t)stream_, p));
+  const int n_stages = (K + kGK - 1) / kGK, groups = sms / p.n_tiles;   // blocks a column tile
+  const bool kept = K <= kGKeptK && groups * p.n_tiles * 16 >= sms * 15;
+  p.raw_off = kGFirst + (kept ? n_stages : kNRing) * 3 * kGOpWB;
+  const int smem = p.raw_off + kNRaws * (kNRawStage + kNRawW) + 1024;
+  auto kern = kept ? k_gemm_f32<true> : k_gemm_f32<false>;
+  // kept: tile t, t + grid, ... of a block are of the same columns
+  const int64_t grid = kept ? (m_tiles < groups ? m_tiles : groups) * p.n_tiles : p.tiles < sms ? p.tiles : sms;
+  SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SSW_CUDA_TRY(launch_chained(kern, dim3((unsigned)grid), dim3(kNThreads), (size_t)smem, (cudaStream_t)stream_, p));
   SSW_LAUNCH_CHECK("k_gemm_f32");
   return SSW_OK;
 }
@@ -581,11 +806,12 @@ static int gemm_tn(const float* g, const float* x, float* out, int64_t M, int32_
   if (rc != SSW_OK) return rc;
   wgrad_shape(M, N, K, sms, p, splits);
   p.a = g; p.w = x; p.out = workspace; p.M = N; p.N = K; p.rows = M;
+  p.wide = K % 8 == 0 && (reinterpret_cast<uintptr_t>(workspace) & 31) == 0;
   p.error = error; p.give_up = give_up;
   if ((int64_t)p.mn_tiles * splits >= ((int64_t)1 << 30)) return SSW_E_RANGE;
   p.tiles = p.mn_tiles * splits;
-  SSW_CUDA_TRY(cudaFuncSetAttribute(k_gemm_f32<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
-  SSW_CUDA_TRY(launch_chained(k_gemm_f32<true>, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kGThreads), kGSmem,
+  SSW_CUDA_TRY(cudaFuncSetAttribute(k_gemm_f32_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
+  SSW_CUDA_TRY(launch_chained(k_gemm_f32_tn, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kGThreads), kGSmem,
                               (cudaStream_t)stream_, p));
   SSW_CUDA_TRY(launch_chained(k_gemm_reduce, dim3((unsigned)ceil_div64((int64_t)N * K, 256)), dim3(256), 0, (cudaStream_t)stream_,
                               (const float*)workspace, splits, p.rows_per_split, g, x, M, (int)N, (int)K, out));

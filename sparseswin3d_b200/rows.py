@@ -163,9 +163,10 @@ def _gemm_ready(x: torch.Tensor, weight: torch.Tensor, first: int = 0) -> bool:
 
 def _gemm_pays(m: int, n: int, k: int) -> bool:
     """Results enough for the fp32 GEMM to be no slower than the library's, which splits K where few tiles of results leave
-    the chip idle; a tile here takes 4 us and 0.8 us for every 32 of K.  With / without bias, (N, K): rows library / own in us.
-    (96, 96): 128 rows 6 / 6, 2500 7 / 6; (576, 192): 128 7 / 8, 512 9 / 8; (96, 384): 2500 12 / 13, 5000 18 / 13;
-    (192, 768): 512 17 / 22, 2500 26 / 23; (384, 1536): 512 32 / 41, 1000 44 / 42; (768, 3072): 1 row 4 / 79, 512 81 / 81."""
+    the chip idle.  With bias, (N, K): rows library / own in us.
+    (96, 96): 128 rows 5.5 / 4.4, 2500 7.1 / 4.4; (576, 192): 128 7.6 / 6.3, 512 9.0 / 6.4; (96, 384): 2500 12 / 9, 5000 18 / 10;
+    (192, 768): 512 17 / 15, 2500 26 / 17; (384, 1536): 512 32 / 27, 1000 44 / 29; (768, 3072): 1 row 5 / 51, 512 80 / 55.  (The line was drawn
+    when a tile took 1.5 times as long; it gives up a us or two below, and keeps few rows of long sums with the library.)"""
     return m * n >= 1024 * min(k, 384)
 
 
