@@ -23,6 +23,10 @@ _DTYPES = (torch.float32, torch.bfloat16, torch.float16)
 ADD_NORM_ROWS = 32768
 # Linear, fp32 (the GEMM): 12 000 rows 1128 / 1056 us, 25 000 rows 1178 / 1368, 40 000 rows 1205 / 1922.
 LINEAR_ROWS_F32 = 16384
+# With wider Linears from as much work (rows times the square of the narrower side).  A stage of two blocks, with / without: 192 channels, 3000 rows
+# 2018 / 1881 us, 5000 2036 / 2066, 10 000 2077 / 3177, 16 000 2556 / 4492; 384 channels, 2500 rows 2036 / 2233, 8000 3160 / 5610; 96 channels, 10 000
+# rows 2051 / 1924.
+LINEAR_WORK_F32 = LINEAR_ROWS_F32 * 96 ** 2
 # Linear, 16 bits (the bias gradient alone), rows at 96 channels: 40 000 rows 1143 / 1125.  A stage of two blocks: 66 000 rows of 96 channels
 # 2245 / 2010, 100 000 2141 / 2170, 150 000 2464 / 2814; 150 000 of 48 2111 / 2065.
 LINEAR_ROWS_16 = 100000
@@ -248,6 +252,13 @@ def _own_linear(module: nn.Module, x: torch.Tensor):
     return w, b
 
 
+def _few_for_training(m: int, narrow: int, dtype: torch.dtype) -> bool:
+    """Too few rows for the passes to pay while autograd records (`narrow`: the narrower side of the Linear)."""
+    if dtype == torch.float32:
+        return m < LINEAR_ROWS_F32 and m * narrow ** 2 < LINEAR_WORK_F32
+    return m * narrow < 96 * LINEAR_ROWS_16
+
+
 def linear(module: nn.Module, x: torch.Tensor, plan=None) -> torch.Tensor:
     """module(x), through the passes above where they apply; time-outs go to the plan's error word."""
     own = _own_linear(module, x)
@@ -258,8 +269,7 @@ def linear(module: nn.Module, x: torch.Tensor, plan=None) -> torch.Tensor:
         plan = _plan.get()
     if not torch.is_grad_enabled() or not (x.requires_grad or w.requires_grad or (b is not None and b.requires_grad)):
         return _affine(x, w, b, plan)
-    few = x.shape[0] < LINEAR_ROWS_F32 if x.dtype == torch.float32 else x.shape[0] * min(w.shape) < 96 * LINEAR_ROWS_16
-    if few or not (b is None or b.shape == w.shape[:1]):
+    if _few_for_training(x.shape[0], min(w.shape), x.dtype) or not (b is None or b.shape == w.shape[:1]):
         return module(x)  # (the backward sums the gradient of a bias [N])
     return _Linear.apply(x, w, b, plan)
 
