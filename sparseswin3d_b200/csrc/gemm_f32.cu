@@ -13,9 +13,8 @@
 // the library's 1.5e-7 at 96 x 96, hence one stage a chunk there).
 //
 //
-// The same kernel forms weight gradients, out[N, K] = g[M, N]^T x[M, K] (TN): the operands' rows are then the steps of the
-// sum, so a producer thread takes four columns of eight consecutive rows and turns them in registers, and the sum
-// over M is split over blocks (partial results, added up in order by k_gemm_reduce).
+// Weight gradients, out[N, K] = g[M, N]^T x[M, K] (TN): the operands' rows are then the steps of the sum, and the sum over M is split
+// over blocks (partial results, added up in order by k_gemm_reduce).
 //
 // An Inf operand has no finite remainder (Inf - Inf), so a result that is not finite is formed again from the
 // operands as they are, by plain fp32 multiply-adds, up to the first NaN; of a weight gradient only the row ranges whose partial
@@ -31,8 +30,9 @@
 // eight 72; loads before the split 71.  The same sizes: 150 000 x 96 x 288 76 -> 70, 150 000 x 96 x 96 41 -> 31, 10 000 x 768 x 192 39 -> 31,
 // 10 000 x 192 x 768 49 -> 39, 10 000 x 192 x 192 20 -> 16, 128 x 576 x 192 14 -> 10; the library's fp32 GEMM 447, 271, 153, 99, 81, 34, 15.
 //
-// Weight gradients: 17 warps, both operands split into shared memory, eight warps drain.  150 000 rows 288 x 96 138 us (library 358), 96 x 96 65 (208),
-// 10 000 rows 576 x 192 44 (111).  With the raw pieces in registers they took 226, 97 and 49: they wait for memory, not for the split.
+// Weight gradients the same way (a producer thread is a column of g; see k_gemm_f32_tn), 20 warps, with the partial results added up 150 000 rows 288 x 96
+// 91 us (library 358), 96 x 96 56 (208), 10 000 rows 576 x 192 32 (111), 192 x 768 42.  With both operands in shared memory, split by eight warps,
+// 138, 65, 44 and 58.
 #include <math.h>
 
 #include "attn_common.cuh"
@@ -41,31 +41,27 @@
 namespace ssw {
 
 constexpr int kGM = 128;                 // rows of a tile
-constexpr int kGNMax = 96;              // columns of a tile at most (48 sums a drain thread: with 64 they spill)
+constexpr int kGNMax = 96;              // columns of a tile at most (tensor memory holds four accumulators and the stages of a)
 constexpr int kGK = 32;                  // K of a stage
 constexpr int kGRowB = kGK * 2;          // bytes of an operand row: one 64-byte swizzle row
 // Stages whose h h products share an accumulator: two, and one for the long sums of a weight gradient.
 template <bool TN>
 struct GemmChunk { static constexpr int kStages = TN ? 1 : 2; };
-constexpr int kGStages = 3;              // of split operands
-constexpr int kGRaw = 2;                 // of fp32 pieces on their way, each read by the thread that asked for it
 constexpr int kGProd = 8, kGEpi = 8;     // warps
-constexpr int kGThreads = 32 * (kGProd + 1 + kGEpi);
-constexpr int kGOpB = kGM * kGRowB;      // bytes of one split tile
 constexpr int kGOpWB = kGNMax * kGRowB;  // ... of w
-constexpr int kGStageB = 3 * kGOpB + 3 * kGOpWB;   // A: h, m, l; B: h, m, l
 constexpr int kGTmemLow = 2 * kGNMax;    // two h h accumulators, then two of small products
-constexpr int kGRawB = kGProd * 32 * 8 * 16;                  // bytes of one raw stage
 constexpr int kGBiasOff = 1024, kGBiasB = kGEpi * (kGNMax / 2) * 4, kGFirst = 3072;   // the first operand tile: 1024-byte aligned
 static_assert(kGBiasOff + kGBiasB <= kGFirst, "");
-constexpr int kGRawOff = kGFirst + kGStages * kGStageB;
-constexpr int kGSmem = kGRawOff + kGRaw * kGRawB + 1024;
 
 // out = a w^T: a in tensor memory, behind the accumulators, in two stages (h, m, l: 16 columns each); raw pieces of a warp and stage 2 KB.
 constexpr int kNEpi = 12, kNThreads = 32 * (kGProd + 1 + kNEpi);
 constexpr int kNRing = 2, kNTmemA = 4 * kGNMax, kNStageCols = 48;
 constexpr int kNRaws = 4, kNRawWarp = 32 * 64, kNRawStage = kGProd * kNRawWarp, kNRawW = 3 * 4096;
 static_assert(kNTmemA + kNRing * kNStageCols <= 512 && kGNMax <= 96, "");
+// Weight gradients: eight warps for g, three for x (its 96 columns by fours and 32 rows by eights; 20 warps in all leave 96 registers a thread).
+constexpr int kTProd = kGProd + 3, kTThreads = 32 * (kTProd + 1 + kGEpi);
+constexpr int kTRawRow = 96 * 16, kTRawX = 8 * kTRawRow, kTRawOff = kGFirst + 4 * 3 * kGOpWB, kTSmem = kTRawOff + kNRaws * (kNRawStage + kTRawX) + 1024;
+static_assert(kTSmem <= 227 * 1024, "");
 struct GemmBars { uint64_t *hh_full, *hh_empty, *lo_full, *lo_empty; };
 
 struct GemmParams {
@@ -124,10 +120,10 @@ __device__ __forceinline__ void sts_v2(uint32_t a, uint2 v) {
   asm volatile("st.shared.v2.b32 [%0], {%1,%2};" ::"r"(a), "r"(v.x), "r"(v.y) : "memory");
 }
 
-// The warps that drain accumulators: number `ew`, tensor-memory lanes 32 `sub` and up, part number `ew` / 4 of a tile's columns.  This is work in
+// The warps that drain accumulators: number `ew`, tensor-memory lanes 32 `sub` and up, part number `ew` / 4 of a tile's columns; LOW accumulators of small products.  This is work in
 // step with the MMAs (a read of the accumulator for every 64 of K, then the stores): with eight warps of half a tile each, 4700 clocks a tile of 96
 // columns at K = 96, it was what 150 000 x 288 x 96 took 79 us for.
-template <bool TN, int PARTS>
+template <bool TN, int PARTS, int LOW>
 __device__ __forceinline__ void gemm_drain(const GemmParams& p, unsigned char* smem, uint32_t tmem, int ew, int sub, int n_stages, const GemmBars& b,
                                            bool& timed_out) {
   constexpr int kChunk = GemmChunk<TN>::kStages, kCols = kGNMax / PARTS;
@@ -173,8 +169,8 @@ __device__ __forceinline__ void gemm_drain(const GemmParams& p, unsigned char* s
       __syncwarp();
       if (lane == 0) mbar_arrive(b.hh_empty + hb);
     }
-    const uint32_t lb = tn & 1;
-    if (!timed_out && !mbar_wait_bounded(b.lo_full + lb, (tn >> 1) & 1)) timed_out = true;
+    const uint32_t lb = tn % LOW;
+    if (!timed_out && !mbar_wait_bounded(b.lo_full + lb, (tn / LOW) & 1)) timed_out = true;
     if (!timed_out) {
       tc_fence_after();
       add_columns(kGTmemLow + lb * kGNMax);
@@ -443,7 +439,7 @@ __global__ void __launch_bounds__(kNThreads, 1) k_gemm_f32(GemmParams p) {
     __syncwarp();
     mbar_wait_bounded(drain_bar, 0);
   } else {
-    gemm_drain<false, 3>(p, smem, tmem, warp - kGProd - 1, warp & 3, n_stages, {hh_full, hh_empty, lo_full, lo_empty}, timed_out);
+    gemm_drain<false, 3, 2>(p, smem, tmem, warp - kGProd - 1, warp & 3, n_stages, {hh_full, hh_empty, lo_full, lo_empty}, timed_out);
   }
   if (timed_out && p.error) atomicOr(reinterpret_cast<unsigned*>(p.error), SSW_DEV_TIMEOUT);
   tc_fence_before();
@@ -451,25 +447,26 @@ __global__ void __launch_bounds__(kNThreads, 1) k_gemm_f32(GemmParams p) {
   if (warp == kGProd) tmem_dealloc(tmem, 512);
 }
 
-// out[N, K] = g[M, N]^T x[M, K] over a range of rows: both operands in shared memory.
-__global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32_tn(GemmParams p) {
+// out[N, K] = g[M, N]^T x[M, K] over a range of rows (p.M and p.N are the N and K of it, the rows the steps of the sum): the columns of g go to tensor memory, where a
+// producer thread is a column.  Its warp brings in 16 rows of 32 columns, 128 bytes a row, and the thread reads its column down them.  x goes to
+// shared memory: a thread of three more warps takes four columns of eight consecutive rows and turns them in registers.
+__global__ void __launch_bounds__(kTThreads, 1) k_gemm_f32_tn(GemmParams p) {
+  constexpr int kRing = 4, kTmemA = 3 * kGNMax;   // one accumulator of small products: the sums are long
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-  uint64_t* full = bars;                     // [kGStages] operands of a stage are in shared memory
-  uint64_t* empty = full + kGStages;         // [kGStages] the stage's MMAs are done
-  uint64_t* hh_full = empty + kGStages;      // [2] a chunk's h h accumulator is complete
+  uint64_t* full = bars;                     // [kRing] operands of a stage are in place
+  uint64_t* empty = full + kRing;            // [kRing] the stage's MMAs are done
+  uint64_t* hh_full = empty + kRing;         // [2] a chunk's h h accumulator is complete
   uint64_t* hh_empty = hh_full + 2;          // [2] ... has been read
   uint64_t* lo_full = hh_empty + 2;          // [2] a tile's small-product accumulator is complete
   uint64_t* lo_empty = lo_full + 2;          // [2]
   uint64_t* drain_bar = lo_empty + 2;        // [1]
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain_bar + 1);
-  const uint32_t stage0 = smem_u32(smem + kGFirst);
-  // (with roles the compiler knows to be uniform, as k_gemm_f32 has them, this kernel spills: 157 us for 138 at 150 000 rows, 288 x 96)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kGStages; ++s) {
-      mbar_init(full + s, kGProd);
+    for (int s = 0; s < kRing; ++s) {
+      mbar_init(full + s, kTProd);
       mbar_init(empty + s, 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -481,7 +478,7 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32_tn(GemmParams p) {
     mbar_init(drain_bar, 1);
     mbar_fence_init();
   }
-  if (warp == kGProd) tmem_alloc(tmem_slot, 512);
+  if (warp == kTProd) tmem_alloc(tmem_slot, 512);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -489,43 +486,50 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32_tn(GemmParams p) {
   grid_dependency_wait();
   const int n_stages = (p.rows_per_split + kGK - 1) / kGK;       // of one tile
   const int bn = p.bn;
-  constexpr int kChunk = GemmChunk<true>::kStages;
   bool timed_out = p.give_up != 0;
+  const uint32_t x_smem = smem_u32(smem + kGFirst);   // [kRing][3][bn rows of 64 bytes]
 
-  if (warp < kGProd) {
+  if (warp < kTProd) {
     // =========================================== producers ====================================
-    const uint32_t raw = smem_u32(smem + kGRawOff) + threadIdx.x * 16u;   // this thread's pieces: [kGRaw][8], 4 KB apart
     const int my_tiles = p.tiles > (int)blockIdx.x ? (p.tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
     const int total = my_tiles * n_stages;   // (operands that fit the device keep this far below 2^31)
-    int lt = blockIdx.x, ls = 0;   // tile and stage the next load belongs to
-    // Warps 0-3 take g, 4-7 take x; a thread, columns 4 quad .. 4 quad + 3 of rows 8 oct .. 8 oct + 7 of a stage (eight lanes read 128 bytes
-    // of one row).
-    const bool is_w = threadIdx.x >= 128;
-    const int oct = threadIdx.x & 3, quad = (threadIdx.x & 127) >> 2;
-    const float* pa;   // this thread's piece of the tile's next stage
-    int rows_a;        // rows of the split from oct on, and whether the columns exist
+    int lt = blockIdx.x, ls = 0;             // tile and stage the next load belongs to
+    const bool is_x = warp >= kGProd;
+    const int sub = warp & 3, kh = warp >> 2, lc = lane & 7, lr = lane >> 3;   // g
+    const int tx = threadIdx.x - kGProd * 32, oct = tx & 3, quad = tx >> 2;    // x
+    const uint32_t raw = smem_u32(smem + kTRawOff) + (is_x ? kNRaws * kNRawStage + tx * 16u : warp * kNRawWarp);
+    const uint32_t raw_b = is_x ? kTRawX : kNRawStage;
+    const int ld = is_x ? p.N : (int)p.M;
+    const float* src = nullptr;
+    int rows = 0;   // of the split, from this thread's first row of a stage on; 0 where its columns do not exist
     auto open_tile = [&]() {
       const int sp = lt / p.mn_tiles, mn = lt - sp * p.mn_tiles, mt = mn / p.n_tiles;
-      const int col = (is_w ? (mn - mt * p.n_tiles) * bn : mt * kGM) + quad * 4, ld = is_w ? p.N : (int)p.M;
-      const int64_t k0 = (int64_t)sp * p.rows_per_split + oct * 8;
-      rows_a = (int)max((int64_t)0, min((int64_t)p.rows_per_split - oct * 8, p.rows - k0));
-      if (col >= ld || (is_w && quad * 4 >= bn)) rows_a = 0;   // M and N are multiples of four
-      pa = (is_w ? p.w : p.a) + k0 * ld + col;
+      const int at = is_x ? quad * 4 : sub * 32 + lc * 4, col = (is_x ? (mn - mt * p.n_tiles) * bn : mt * kGM) + at, r0 = is_x ? oct * 8 : kh * 16 + lr;
+      const int64_t k0 = (int64_t)sp * p.rows_per_split + r0;
+      rows = (int)max((int64_t)0, min((int64_t)p.rows_per_split - r0, p.rows - k0));
+      if (col >= ld || (is_x && at >= bn)) rows = 0;   // M and N are multiples of four
+      src = (is_x ? p.w : p.a) + k0 * ld + col;
     };
     open_tile();
-    const int64_t step_rows = is_w ? (int64_t)p.N : p.M;
-    int lslot = 0;
-    int loaded = 0;
+    int lslot = 0, loaded = 0;
     auto load = [&]() {   // one commit group per stage, empty beyond the last one
       if (loaded < total) {
-        const uint32_t dst = raw + (uint32_t)lslot * kGRawB;
-        #pragma unroll
-                  for (int i = 0; i < 8; ++i) {
-                    const bool on = ls * kGK + i < rows_a;
-                    cp_async16_or_zero(dst + i * 4096u, on ? pa + i * step_rows : p.a, on);
-                  }
-                  pa += kGK * step_rows;
-        lslot = lslot + 1 == kGRaw ? 0 : lslot + 1;
+        const uint32_t dst = raw + (uint32_t)lslot * raw_b;
+        if (is_x) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const bool on = ls * kGK + i < rows;
+            cp_async16_or_zero(dst + i * kTRawRow, on ? src + (int64_t)i * ld : p.a, on);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const bool on = ls * kGK + 4 * i < rows;
+            cp_async16_or_zero(dst + (lr + 4 * i) * 128 + lc * 16, on ? src + (int64_t)(4 * i) * ld : p.a, on);
+          }
+        }
+        src += (int64_t)kGK * ld;
+        lslot = lslot + 1 == kNRaws ? 0 : lslot + 1;
         ++loaded;
         if (++ls == n_stages) {
           ls = 0;
@@ -535,98 +539,118 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32_tn(GemmParams p) {
       }
       cp_async_commit();
     };
-    for (int x = 0; x < kGRaw; ++x) load();
+    for (int x = 0; x < kNRaws - 1; ++x) load();
     int slot = 0;
     uint32_t s = 0, spar = 1;   // stage, parity of the use of it before this one
-    auto step = [&](int i) -> bool {
-      cp_async_wait<kGRaw - 1>();   // this stage's pieces have landed; each thread reads its own
-      const uint32_t src = raw + (uint32_t)slot * kGRawB;
-      slot = slot + 1 == kGRaw ? 0 : slot + 1;
-      float4 v[8];
+    for (int i = 0; i < total && !timed_out; ++i) {
+      // this stage's pieces have landed, those of the warp's other lanes as well
+      cp_async_wait<kNRaws - 2>();
+      __syncwarp();
+      const uint32_t at = raw + (uint32_t)slot * raw_b;
+      slot = slot + 1 == kNRaws ? 0 : slot + 1;
+      if (is_x) {
+        float4 v[8];
 #pragma unroll
-      for (int x = 0; x < 8; ++x) {
-        const int4 u = lds_v4(src + x * 4096u);
-        v[x] = make_float4(__int_as_float(u.x), __int_as_float(u.y), __int_as_float(u.z), __int_as_float(u.w));
+        for (int x = 0; x < 8; ++x) {
+          const int4 u = lds_v4(at + x * kTRawRow);
+          v[x] = make_float4(__int_as_float(u.x), __int_as_float(u.y), __int_as_float(u.z), __int_as_float(u.w));
+        }
+        load();   // into the slot of the stage before, which all lanes have read
+        if (i >= kRing && !mbar_wait_bounded(empty + s, spar)) {
+          timed_out = true;
+          break;
+        }
+        if (quad * 4 < bn) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            float x[8];
+#pragma unroll
+            for (int i8 = 0; i8 < 8; ++i8) x[i8] = j == 0 ? v[i8].x : j == 1 ? v[i8].y : j == 2 ? v[i8].z : v[i8].w;
+            uint4 h, m, l;
+            split8(x, h, m, l);
+            const int row = quad * 4 + j;
+            const uint32_t d = x_smem + s * 3 * kGOpWB + (uint32_t)(row * kGRowB + ((oct ^ ((row >> 1) & 3)) << 4));
+            sts_u4(d, h);
+            sts_u4(d + kGOpWB, m);
+            sts_u4(d + 2 * kGOpWB, l);
+          }
+        }
+        fence_async_smem();  // the tensor cores read shared memory through the async proxy
+      } else {
+        float x[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) x[r] = lds_f32(at + r * 128 + lane * 4);
+        load();
+        uint32_t h[8], m[8], l[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          uint2 h2, m2, l2;
+          split4(make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]), h2, m2, l2);
+          h[2 * q] = h2.x; h[2 * q + 1] = h2.y;
+          m[2 * q] = m2.x; m[2 * q + 1] = m2.y;
+          l[2 * q] = l2.x; l[2 * q + 1] = l2.y;
+        }
+        if (i >= kRing && !mbar_wait_bounded(empty + s, spar)) {
+          timed_out = true;
+          break;
+        }
+        tc_fence_after();   // the MMAs that read the stage before come before the stores below
+        const uint32_t ta = tmem + ((uint32_t)(sub * 32) << 16) + kTmemA + s * kNStageCols + kh * 8;
+        tmem_stn(ta, h);
+        tmem_stn(ta + 16, m);
+        tmem_stn(ta + 32, l);
+        tmem_st_wait();
+        tc_fence_before();
       }
-      if (i >= kGStages && !mbar_wait_bounded(empty + s, spar)) return false;
-              const uint32_t base = stage0 + s * kGStageB + (is_w ? 3u * kGOpB : 0u);
-              if (!is_w || quad * 4 < bn) {
-      #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  float x[8];
-      #pragma unroll
-                  for (int i8 = 0; i8 < 8; ++i8) x[i8] = j == 0 ? v[i8].x : j == 1 ? v[i8].y : j == 2 ? v[i8].z : v[i8].w;
-                  uint4 h, m, l;
-                  split8(x, h, m, l);
-                  const int row = quad * 4 + j;
-                  const uint32_t d = base + (uint32_t)(row * kGRowB + ((oct ^ ((row >> 1) & 3)) << 4));
-                  const uint32_t op = is_w ? kGOpWB : kGOpB;
-                  sts_u4(d, h);
-                  sts_u4(d + op, m);
-                  sts_u4(d + 2 * op, l);
-                }
-              }
-      fence_async_smem();  // the tensor cores read shared memory through the async proxy
       __syncwarp();
       if (lane == 0) mbar_arrive(full + s);
-      if (++s == kGStages) {
+      if (++s == kRing) {
         s = 0;
         spar ^= 1;
       }
-      load();   // into the slot just read
-      return true;
-    };
-    for (int i = 0; i < total && !timed_out; ++i) {
-      if (!step(i)) {
-        timed_out = true;
-        break;
-      }
     }
     cp_async_wait<0>();   // nothing of this block's may still be on its way into shared memory
-  } else if (warp == kGProd) {
+  } else if (warp == kTProd) {
     // =========================================== MMA issuer ===================================
-    // All lanes walk along and one issues, on operands that the compiler can see are the same in each: an MMA takes them from
-    // uniform registers, and from a branch of one lane each is first looked for among the lanes (some hundred instructions an
-    // MMA).
+    // (all lanes walk along: see k_gemm_f32)
     const uint32_t idesc = instr_desc(1, 1, 0, bn), tm = __shfl_sync(0xffffffffu, tmem, 0);
-    const uint64_t d0 = smem_desc(stage0, 512, 4);
+    const uint64_t x0 = smem_desc(x_smem, 512, 4);
     const bool leader = elect_one();
     auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
       timed_out = !__all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
       return !timed_out;
     };
     timed_out = __any_sync(0xffffffffu, timed_out);
-    uint32_t s = 0, spar = 0, ch = 0, tn = 0;   // stage and parity of its use, chunks, tiles so far
+    static_assert(GemmChunk<true>::kStages == 1, "");
+    uint32_t s = 0, spar = 0, ch = 0, tn = 0;   // stage and parity of its use, chunks (stages), tiles so far
     for (int t = blockIdx.x; t < p.tiles && !timed_out; t += gridDim.x, ++tn) {
-      const uint32_t lb = tn & 1;
-      if (tn >= 2 && !wait(lo_empty + lb, ((tn >> 1) - 1) & 1)) break;
-      for (int ks = 0; ks < n_stages; ++ks) {
+      if (tn >= 1 && !wait(lo_empty, (tn - 1) & 1)) break;
+      for (int ks = 0; ks < n_stages; ++ks, ++ch) {
         const uint32_t hb = ch & 1;
-        const bool first = ks % kChunk == 0, last = ks % kChunk == kChunk - 1 || ks == n_stages - 1;
-        if (first && ch >= 2 && !wait(hh_empty + hb, ((ch >> 1) - 1) & 1)) break;
+        if (ch >= 2 && !wait(hh_empty + hb, ((ch >> 1) - 1) & 1)) break;
         if (!wait(full + s, spar)) break;
         tc_fence_after();
-        const uint64_t da = d0 + s * (kGStageB >> 4), db = da + (3 * kGOpB >> 4);
-        const uint32_t hh = tm + hb * kGNMax, lo = tm + kGTmemLow + lb * kGNMax;
+        const uint32_t ta = tm + kTmemA + s * kNStageCols, hh = tm + hb * kGNMax, lo = tm + kGTmemLow;
+        const uint64_t db = x0 + s * (3 * kGOpWB >> 4);
         if (leader) {
-          constexpr int oa = kGOpB >> 4, ob = kGOpWB >> 4;
+          constexpr int ob = kGOpWB >> 4;
 #pragma unroll
           for (int k16 = 0; k16 < kGK / 16; ++k16) {
-            const uint64_t a = da + k16 * 2, b = db + k16 * 2;
-            umma_ss(hh, a, b, idesc, !(first && k16 == 0));
-            umma_ss(lo, a, b + 2 * ob, idesc, ks > 0 || k16 > 0);   // smallest first
-            umma_ss(lo, a + 2 * oa, b, idesc, 1);
-            umma_ss(lo, a + oa, b + ob, idesc, 1);
-            umma_ss(lo, a, b + ob, idesc, 1);
-            umma_ss(lo, a + oa, b, idesc, 1);
+            const uint32_t a = ta + k16 * 8;
+            const uint64_t b = db + k16 * 2;
+            umma_ts(hh, a, b, idesc, k16 > 0);
+            umma_ts(lo, a, b + 2 * ob, idesc, ks > 0 || k16 > 0);   // smallest first
+            umma_ts(lo, a + 32, b, idesc, 1);
+            umma_ts(lo, a + 16, b + ob, idesc, 1);
+            umma_ts(lo, a, b + ob, idesc, 1);
+            umma_ts(lo, a + 16, b, idesc, 1);
           }
           umma_commit(empty + s);
-          if (last) umma_commit(hh_full + hb);
-          if (ks == n_stages - 1) umma_commit(lo_full + lb);
+          umma_commit(hh_full + hb);
+          if (ks == n_stages - 1) umma_commit(lo_full);
         }
         __syncwarp();
-        if (last) ++ch;
-        if (++s == kGStages) {
+        if (++s == kRing) {
           s = 0;
           spar ^= 1;
         }
@@ -637,12 +661,12 @@ __global__ void __launch_bounds__(kGThreads, 1) k_gemm_f32_tn(GemmParams p) {
     __syncwarp();
     mbar_wait_bounded(drain_bar, 0);
   } else {
-    gemm_drain<true, 2>(p, smem, tmem, warp - kGProd - 1, warp & 3, n_stages, {hh_full, hh_empty, lo_full, lo_empty}, timed_out);
+    gemm_drain<true, 2, 1>(p, smem, tmem, warp - kTProd - 1, warp & 3, n_stages, {hh_full, hh_empty, lo_full, lo_empty}, timed_out);
   }
   if (timed_out && p.error) atomicOr(reinterpret_cast<unsigned*>(p.error), SSW_DEV_TIMEOUT);
   tc_fence_before();
   __syncthreads();
-  if (warp == kGProd) tmem_dealloc(tmem, 512);
+  if (warp == kTProd) tmem_dealloc(tmem, 512);
 }
 
 // Partial results of a weight gradient added up in order.  If that is not finite, the partial results that are not are
@@ -810,8 +834,8 @@ static int gemm_tn(const float* g, const float* x, float* out, int64_t M, int32_
   p.error = error; p.give_up = give_up;
   if ((int64_t)p.mn_tiles * splits >= ((int64_t)1 << 30)) return SSW_E_RANGE;
   p.tiles = p.mn_tiles * splits;
-  SSW_CUDA_TRY(cudaFuncSetAttribute(k_gemm_f32_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem));
-  SSW_CUDA_TRY(launch_chained(k_gemm_f32_tn, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kGThreads), kGSmem,
+  SSW_CUDA_TRY(cudaFuncSetAttribute(k_gemm_f32_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmem));
+  SSW_CUDA_TRY(launch_chained(k_gemm_f32_tn, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kTThreads), kTSmem,
                               (cudaStream_t)stream_, p));
   SSW_CUDA_TRY(launch_chained(k_gemm_reduce, dim3((unsigned)ceil_div64((int64_t)N * K, 256)), dim3(256), 0, (cudaStream_t)stream_,
                               (const float*)workspace, splits, p.rows_per_split, g, x, M, (int)N, (int)K, out));
