@@ -33,7 +33,8 @@
 // ties them to one another.  A million voxels, half of the 9^3 windows full, six heads of bf16, in ms: 4.53 with one stream, 128-key tiles and
 // MMAs issued from a branch of one lane (there every operand is looked for among the lanes: see the issuer); 2.99 two streams of four
 // softmax warps; 2.82 eight softmax warps each (two threads a row); 2.30 MMAs issued from uniform registers; 2.27 the residual
-// of P in one mixed-precision instruction.  Bound by issue slots and their latencies: 66 % of them used (13 warp instructions a key, 7.5 of them
+// of P in one mixed-precision instruction; 2.26 the bias slice padded (see there) and staged by the softmax warps (10 000 voxels, 3 heads: 13.6 us
+// by the producers ahead of the first rows, 11.5 so).  Bound by issue slots and their latencies: 66 % of them used (13 warp instructions a key, 7.5 of them
 // the look-up of the bias, the exponential and the split of P), exponential unit 46 %, shared memory 35 to 60 %; without exponentials
 // the time is the same within 3 %.  Floor of the exponential unit: 0.97 ms.
 //
@@ -100,7 +101,7 @@ struct DenseFast<__half> {
 // warp reads the slice at their codes.  With rows of x a multiple of 32 plus Wx words apart, and planes of y plus Wx Wy,
 // consecutive positions lie in consecutive banks; with the table's own strides nearly every look-up takes two passes (51.8 M shared-memory wavefronts
 // against 33.6 M over 172 full windows of 9^3 and six heads).  The padded slice takes the room of two plain ones, so it is staged for one head
-// (see the units).  A million voxels, half of the 9^3 windows full, six heads of bf16, plain / padded: 2.27 / 2.33 ms (144 blocks for 148),
+// (see the units).  A million voxels, half of the 9^3 windows full, six heads of bf16, plain / padded: 2.27 / 2.26 ms (144 blocks for 148),
 // the same shifted by four 2.18 / 2.02.  Where the padded slice does not fit, the table's strides stay.
 struct BiasShape {
   int wy2, wx2;        // 2 Wy - 1, 2 Wx - 1: the table's own strides are wx2 and wx2 wy2
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
   // largest squared norms of a tile's rows, one word per producer warp (two of the eight unused)
   float* k_norm = reinterpret_cast<float*>(smem + 768);     // [kDMaxKT][8]; infinite where a v is too large for O
   float* q_norm = k_norm + kDMaxKT * 8;                     // [stream][4][8] by query tile of the stream
-  float* b_max = q_norm + kDStreams * 4 * 8;                // [8] largest entry (or 0) of the bias slice
+  float* b_max = q_norm + kDStreams * 4 * 8;                // [16] largest entry (or 0) of the bias slice, by the warps that staged it
   float* xmax = reinterpret_cast<float*>(smem + 2048);      // [stream][2][kDParts][128] partial row maxima
   float* xsum = xmax + kDStreams * 2 * kDParts * 128;       // [stream][2][128] partial row sums
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
@@ -247,12 +248,35 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
     mbar_init(drain_bar, kDStreams);
     mbar_fence_init();
   }
+  if (threadIdx.x < kDStreams * kDSoftWarps) b_max[threadIdx.x] = 0.f;
   if (warp == 0) tmem_alloc(tmem_slot, kTmemCols);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
+  // A head's bias slice (rows of the table are [code][head]) by `n` threads, eight loads in flight; the largest entry (or 0) of a warp's share.
+  const int wyx2 = p.bias.wy2 * p.bias.wx2;
+  const bool one_head = step % H == 0;   // the softmax warps stage it before their first unit; else the producers, unit by unit
+  auto stage_bias = [&](int h, int t, int n) -> float {
+    float* const bs = reinterpret_cast<float*>(smem + L.bias);
+    float bm = 0.f;
+    for (int i0 = t; i0 < p.table_rows; i0 += n * 8) {
+      float v[8];
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const int i = i0 + x * n;
+        v[x] = i < p.table_rows ? __ldg(p.table + (int64_t)i * H + h) * kLog2e : 0.f;
+      }
+#pragma unroll
+      for (int x = 0; x < 8; ++x) {
+        const int i = i0 + x * n, z = i / wyx2, y = (i - z * wyx2) / p.bias.wx2;
+        if (i < p.table_rows) bs[z * p.bias.pz + y * p.bias.py + (i - z * wyx2 - y * p.bias.wx2)] = v[x] - DenseFast<T>::kRef;
+        bm = v[x] <= 3.0e38f ? fmaxf(bm, v[x]) : INFINITY;
+      }
+    }
+    return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bm)));
+  };
   bool timed_out = false;
   constexpr float kRef = DenseFast<T>::kRef;
   const int a_fmt_qk = std::is_same<T, __nv_bfloat16>::value ? 1 : 0;
@@ -467,7 +491,7 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
     uint32_t qn[kDStreams] = {0, 0};   // query tiles handed to each stream
     uint32_t slot = 0, use = 0;        // ring slot of the next key tile, how often the ring has been gone through
     int un = 0, qodd = 0, first_n = 0, c_n = 0, h_staged = -1;
-    float* const bs = reinterpret_cast<float*>(smem + L.bias);
+
     unit_window(blockIdx.x, first_n, c_n);
     for (int u = blockIdx.x; u < n_units && !timed_out; u += step, ++un) {
       int first = first_n, c = c_n;
@@ -486,7 +510,6 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
       // ---- the window's voxel ids and metadata
       if (un >= 2 && !mbar_wait_asleep(meta_empty + mb, ((un >> 1) - 1) & 1)) { timed_out = true; break; }
       if (pw == 0 && lane == 0) unit_c[mb] = c;
-      const int wyx2 = p.bias.wy2 * p.bias.wx2;
       for (int r = pw * 32 + lane; r < nkt * kDK; r += kDProd * 32) {  // (rows from c on: neutral entries)
         int vx = 0, m = 0;
         if (r < c) {
@@ -502,26 +525,11 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
         wreg[r] = ok ? meta_region(m) : 0;
       }
       // ---- the head's bias slice (rows of the table are [code][head]), eight loads in flight
-      if (h != h_staged) {
+      if (!one_head && h != h_staged) {
         // (the unit before is of another head: both streams must be done with it)
         if (un >= 1 && !mbar_wait_asleep(meta_empty + (mb ^ 1), ((un - 1) >> 1) & 1)) { timed_out = true; break; }
         h_staged = h;
-        float bm = 0.f;
-        for (int i0 = pw * 32 + lane; i0 < p.table_rows; i0 += kDProd * 32 * 8) {
-          float v[8];
-#pragma unroll
-          for (int x = 0; x < 8; ++x) {
-            const int i = i0 + x * kDProd * 32;
-            v[x] = i < p.table_rows ? __ldg(p.table + (int64_t)i * H + h) * kLog2e : 0.f;
-          }
-#pragma unroll
-          for (int x = 0; x < 8; ++x) {
-            const int i = i0 + x * kDProd * 32, z = i / wyx2, y = (i - z * wyx2) / p.bias.wx2;
-            if (i < p.table_rows) bs[z * p.bias.pz + y * p.bias.py + (i - z * wyx2 - y * p.bias.wx2)] = v[x] - kRef;
-            bm = v[x] <= 3.0e38f ? fmaxf(bm, v[x]) : INFINITY;
-          }
-        }
-        const float top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(bm)));
+        const float top = stage_bias(h, pw * 32 + lane, kDProd * 32);
         if (lane == 0) b_max[pw] = top;
       }
       __syncwarp();
@@ -587,6 +595,11 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
     uint32_t xn = 0;   // exchanges of maxima so far
     uint32_t slot0 = 0;  // ring slot of the unit's first key tile
     int un = 0, qodd = 0;
+    if (one_head) {
+      const float top = stage_bias(blockIdx.x % H, threadIdx.x - kDFirstSoft * 32, kDStreams * kDSoftWarps * 32);
+      if (lane == 0) b_max[warp - kDFirstSoft] = top;
+      asm volatile("bar.sync 1, %0;" ::"n"(kDStreams * kDSoftWarps * 32) : "memory");   // the softmax warps
+    }
     for (int u = blockIdx.x; u < n_units && !timed_out; u += step, ++un) {
       const int mb = un & 1;
       if (!mbar_wait_bounded(meta_full + mb, (un >> 1) & 1)) { timed_out = true; break; }
@@ -616,9 +629,8 @@ __global__ void __launch_bounds__(kDThreads, 1) k_attn_dense(DenseParams p) {
           if (j == 0) {
             const float4 q4 = *reinterpret_cast<const float4*>(q_norm + (s * 4 + (qt & 3)) * 8);
             const float2 q2 = *reinterpret_cast<const float2*>(q_norm + (s * 4 + (qt & 3)) * 8 + 4);
-            const float4 b4 = *reinterpret_cast<const float4*>(b_max);
-            const float2 b2 = *reinterpret_cast<const float2*>(b_max + 4);
-            const float top = fmaxf(fmaxf(fmaxf(b4.x, b4.y), fmaxf(b4.z, b4.w)), fmaxf(b2.x, b2.y));
+            float top = b_max[lane & 15];   // (all of them: a warp's lanes hold every entry twice)
+            top = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(top)));
             const float qq = fmaxf(fmaxf(fmaxf(q4.x, q4.y), fmaxf(q4.z, q4.w)), fmaxf(q2.x, q2.y));
             const float lim = (DenseFast<T>::kLimit + kRef - top) / fabsf(qscale);
             k_limit = lim > 0.f && qq <= 3.0e38f ? lim * lim / fmaxf(qq, 1e-30f) : -1.f;
