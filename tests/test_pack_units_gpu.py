@@ -1,0 +1,39 @@
+"""16-bit packs, sixteen slots a warp, and the windows beyond a pack that the tcgen05 kernel does not serve, against the dense restatement in float64."""
+import pytest
+import torch
+
+from oracle import ssw_oracle as O
+from tests.cases import rel_err
+from tests.test_dense_streams_gpu import _boxes
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("w,heads,hd,counts", [
+    ((7, 7, 7), 3, 32, [1, 2, 3, 4, 5, 8, 9, 15, 16, 17, 31, 32, 33, 47, 48, 49, 63, 64] * 2),
+    ((7, 7, 7), 2, 16, [64, 65, 79, 80, 81, 343, 16, 1] * 2),   # beyond a pack: remainders of query and key blocks
+    ((7, 7, 7), 12, 32, [16, 17, 12, 3] * 30),                  # packs of 32 slots; the table in global memory
+    ((5, 6, 7), 1, 16, [9] * 1500),                             # more units than warps
+    ((9, 9, 9), 6, 16, [729, 200, 40]),
+])
+def test_units(dtype, w, heads, hd, counts):
+    from sparseswin3d_b200 import attention, window
+
+    coords, dims = _boxes(counts, w, seed=heads)
+    n = len(coords)
+    g = torch.Generator().manual_seed(6)
+    qkv = torch.randn(n, 3, heads, hd, generator=g).to(dtype)
+    table = torch.randn((2 * w[0] - 1) * (2 * w[1] - 1) * (2 * w[2] - 1), heads, generator=g) * 0.5
+    for shift in ((0, 0, 0), (w[0] // 2, 0, 0)):
+        geom = window.resolve_geometry(1, dims, w, shift)
+        plan = window.bucket_windows(coords=coords.cuda(), geom=geom, **attention.plan_params(heads, hd, dtype, w))
+        out = attention.window_attention_fused(qkv.cuda(), plan, table.cuda(), hd ** -0.5, use_mask=bool(geom.shifted))
+        plan.raise_on_error()
+        idx = O.window_keys(coords, 1, dims, w, shift)[0]
+        mask = O.compute_mask(tuple(geom.dims_p), tuple(geom.ws), tuple(geom.ss)) if geom.shifted else None
+        ref = O.dense_window_attention(qkv.double(), idx, hd ** -0.5, table.double(), O.relative_position_index(w), mask)
+        # one rounding of the output and that of the probabilities (bf16 keeps the rounding residual as well), which weigh values up to max |v|
+        p_bits, o_bits = (2.0 ** -17, 2.0 ** -8) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -11)
+        bound = o_bits + p_bits * float(qkv[:, 2].double().abs().max() / ref.pow(2).mean().sqrt())
+        assert rel_err(out.double().cpu(), ref) <= bound
