@@ -136,9 +136,9 @@ typedef struct ssw_plan_layout {
  * from ssw_default_tile_rows / ssw_default_padded for the configuration. */
 int ssw_plan_layout_init(ssw_plan_layout* L, int64_t n_vox, int32_t n_windows, int32_t n_per_window,
                          int32_t tile_rows, int32_t padded);
-/* The default tile_rows for a configuration (host only): the largest tile that leaves three
- * (fp32, CUDA-core kernel) or four (16-bit, tensor-core kernel) pipeline stages in one SM's shared
- * memory next to the bias table, when that is small enough to be staged there. */
+/* The default tile_rows for a configuration (host only): the largest tile of whose rows three (fp32)
+ * or four (16-bit) stages fit one SM's shared memory next to the bias table, when that is small
+ * enough to be staged there. */
 int32_t ssw_default_tile_rows(int32_t heads, int32_t head_dim, int dtype, const int32_t rpb_window[3]);
 /* 1 when ssw_attn_fused serves this dtype with the tensor-core kernel (bf16, fp16), else 0. */
 int32_t ssw_default_padded(int dtype);

@@ -1,5 +1,5 @@
-// Device helpers shared by the fused attention kernels: fast exp2, mbarrier arrive, bulk (TMA)
-// stores, proxy fence, mbarrier-based group barrier, 16-bit widening and packing.
+// Device helpers shared by the fused attention kernels: checks of plan entries, fast exp2, mbarrier arrive, proxy fence,
+// mbarrier-based group barrier, 16-bit widening and packing.
 #pragma once
 
 #include <type_traits>
@@ -12,7 +12,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 constexpr int kMaxStages = 6;
 constexpr int kMaxGroups = 4;
-constexpr int kMaxTile = 64, kMaxProducerWarps = kMaxStages;
+constexpr int kMaxTile = 64;
 
 // Destinations of the output rows: the caller's buffer and, when one scene is split over several
 // GPUs, the same [N, C] buffer on every peer (mapped into this process): a finished row is stored
@@ -46,12 +46,9 @@ struct AttnParams {
   int use_mask;
   int row_stride;     // bytes between fp32 rows in a stage
   int stage_bytes;    // bytes of one pipeline stage
-  int out_off;        // byte offset of the 16-bit output staging area inside a stage (0 for fp32)
   int table_floats;   // > 0: the bias table is staged in shared memory (that many floats)
   int skip_big;       // windows beyond a pack are left to k_attn_tiles
 };
-
-
 
 // The attention kernels turn plan entries into addresses.  A plan that is stale or was overwritten
 // must not become a wild access: entries are held to their bounds, violations set SSW_DEV_BAD_PLAN
@@ -119,20 +116,9 @@ __device__ __forceinline__ float fast_exp2(float x) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
-// shared -> global bulk (TMA) store of `bytes` (multiple of 16, both addresses 16-byte aligned)
-__device__ __forceinline__ void bulk_s2g(void* gmem_dst, const void* smem_src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(smem_u32(smem_src)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-// make generic-proxy writes to shared memory visible to the async proxy (bulk stores)
+// make generic-proxy writes to shared memory visible to the async proxy (bulk copies)
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// Stage the relative-position bias table in shared memory, pre-multiplied by log2(e).  Loads are
-// issued eight at a time so that the loop is bound by bandwidth, not by one L2 round trip per value.
 // Stage the bias table in shared memory, pre-multiplied by log2 e.  Called by the first `step`
 // threads of the CTA (tid = 0..step-1).  When the table starts on a 16-byte boundary its bulk
 // comes in with one bulk (TMA) copy completing on `bar` (initialised with count 1) and is scaled
@@ -164,28 +150,13 @@ __device__ __forceinline__ bool stage_table(float* dst, const float* __restrict_
 }
 
 // ---- producer-side plan prefetch ------------------------------------------------------------
-// Work items are dealt to the producer warps whole, and every pipeline stage has exactly one
-// producer warp: warp w owns the stages w, w + PW, ... and gathers the items that fall into them.  (What an item costs its producer is mostly
-// fixed - a few hundred dependent instructions of one warp, about a microsecond - so the warps must
-// not all pay it for every item.  And a stage must have a single producer: a parity wait on the
-// stage's `empty` barrier tells two consecutive phases apart and no more, so the waiter has to see
-// every phase, which a warp that skipped uses of the stage would not.)  Per item a warp needs the
-// item's descriptor and then, at addresses the descriptor gives, the voxel id and metadata word of
-// each row slot.  Both come from the plan in global memory and are requested a few of the warp's own
-// items ahead with asynchronous 4/16-byte copies into small shared-memory rings;
-// cp.async.wait_group keeps exactly the wanted number of requests in flight.
-constexpr int kDescRing = 8, kDescAhead = 4;  // descriptor of the warp's item t + 4 is requested while item t is issued
-constexpr int kVoxRing = 4, kVoxAhead = 2;    // voxel ids / metadata of its item t + 2
+// Per item a producer warp needs the item's descriptor and then, at addresses the descriptor gives, the voxel id and metadata word of
+// each of its rows.  Both come from the plan in global memory and are requested a few items ahead with asynchronous 4/16-byte
+// copies into small shared-memory rings; cp.async.wait_group keeps exactly the wanted number of requests in flight.
+constexpr int kDescRing = 8, kDescAhead = 4;  // descriptor of item t + 4 is requested while item t is issued
+constexpr int kVoxRing = 4, kVoxAhead = 2;    // voxel ids / metadata of item t + 2
 // bytes of plan-prefetch rings one producer warp owns: descriptors, then (voxel id, metadata) pairs
 __host__ __device__ inline int producer_scratch_bytes(int tile) { return kDescRing * 16 + kVoxRing * tile * 8; }
-// Before a timed-out CTA retires: wait (bounded) for the row copies this producer warp submitted
-// and nobody will consume.  The warp owns stages pw, pw + PW, ... (K = S / PW of them) and has
-// submitted `issued` items, the t-th into stage pw + (t % K) * PW as that stage's use t / K; only
-// the latest use of each stage can still be in flight.
-__device__ __forceinline__ void drain_producer(uint64_t* full, int pw, int PW, int S, int issued) {
-  const int K = S / PW;
-  for (int t = issued - 1; t >= 0 && t >= issued - K; --t) mbar_wait_bounded(full + pw + (t % K) * PW, (t / K) & 1);
-}
 __device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
 }
@@ -255,6 +226,5 @@ __device__ __forceinline__ uint32_t pack2(float a, float b) {
     return *reinterpret_cast<uint32_t*>(&v);
   }
 }
-
 
 }  // namespace ssw

@@ -731,7 +731,7 @@ __global__ void __maxnreg__(regs_for_threads(MAXT)) k_attn_fused(AttnParams p) {
 constexpr int kTableSmemMax = 40 * 1024;
 constexpr size_t kSmemBudget = 226 * 1024;
 struct KernelShape {
-  int hg, group_threads, groups, stages, prod_warps, row_stride, stage_bytes, out_off, table_floats;
+  int hg, group_threads, groups, stages, prod_warps, row_stride, stage_bytes, table_floats;
   size_t smem;
 };
 static int table_entries(const int32_t w[3], int heads) {
@@ -748,7 +748,6 @@ static KernelShape kernel_shape(int tile, int heads, int head_dim, int elt, cons
   const int C = heads * head_dim;
   s.row_stride = 3 * C * 4 + 16;  // +16 B skews rows across shared-memory banks
   const int rows_bytes = kStageRowsOff + tile * s.row_stride;
-  s.out_off = 0;
   s.stage_bytes = rows_bytes;
   (void)elt;
   const int tf = table_entries(rpb_window, heads);
@@ -910,7 +909,6 @@ extern "C" int ssw_attn_fused_multi(const void* qkv, int dtype, int32_t heads, i
   p.prod_warps = s.prod_warps;
   p.row_stride = s.row_stride;
   p.stage_bytes = s.stage_bytes;
-  p.out_off = s.out_off;
   p.table_floats = s.table_floats;
   switch (dtype) {
     case SSW_F32: {

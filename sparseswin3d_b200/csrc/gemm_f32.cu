@@ -12,7 +12,6 @@
 // gradients of 150 000 rows: 2.0e-7 against 1.3e-6, all-positive 6e-8 against 2.1e-7 (with 64 steps a chunk 2.0e-7 against
 // the library's 1.5e-7 at 96 x 96, hence one stage a chunk there).
 //
-//
 // Weight gradients, out[N, K] = g[M, N]^T x[M, K] (TN): the operands' rows are then the steps of the sum, and the sum over M is split
 // over blocks (partial results, added up in order by k_gemm_reduce).
 //
