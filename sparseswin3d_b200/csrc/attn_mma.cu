@@ -9,9 +9,12 @@
 // (16 channels a head, or a bias table too large): 16 query rows and a head at a time, key blocks in turn.
 //
 // The queries of 16 slots against their own window's keys, 16 at a time, are m16n8k16 products, and the fragments are loaded from the voxel
-// rows themselves: the sum over channels does not depend on their order, so lane t of a row's four takes channels [8 t, 8 t + 8) of the
-// head (16 bytes; 8 for 16 channels) for both operands of Q K^T, where the instruction's own order would have it read 4 bytes in
-// four places.  A row of v, loaded the same way, becomes the other operand of P V by transposing its 8 x 8 blocks (movmatrix), which
+// rows themselves.  Lane t of a row's four takes channels [4 t, 4 t + 4) and [16 + 4 t, 16 + 4 t + 4) of the head for both operands of Q K^T,
+// 8 bytes each, where the instruction's own order would have it read 4 bytes in four places: a product sums sixteen consecutive channels all the
+// same, whichever of them a lane brings.  (16 bytes a lane, channels [8 t, 8 t + 8), would put other channels into the two sums, and with that
+// other roundings: the 16-bit output of a stage of two blocks moves by 2e-4.  It is no
+// faster: 47.5 us at 150 000 voxels, 3 heads, 43.8 shifted, for 47.6 and 43.5.)  A row of v is loaded 16 bytes a lane (8 for
+// 16 channels) and becomes the other operand of P V by transposing its 8 x 8 blocks (movmatrix), which
 // leaves a lane with the same eight channels of the output: one 16-byte store a row, four lanes side by side.
 //
 // us, with whole rows copied to shared memory by one bulk copy each and read from there by ldmatrix / so (rooms, windows of 7^3, shifted): 150 000 voxels,
@@ -77,6 +80,18 @@ __device__ __forceinline__ RowPart<HD> load_part(const T* row) {
   } else {
     const uint2 v = __ldg(reinterpret_cast<const uint2*>(row));
     r.x[0] = v.x; r.x[1] = v.y;
+  }
+  return r;
+}
+
+// The same of q or k: a product of sixteen channels takes consecutive ones, four from each lane of a row.
+template <typename T, int HD>
+__device__ __forceinline__ RowPart<HD> load_operand(const T* row) {
+  RowPart<HD> r;
+#pragma unroll
+  for (int ks = 0; ks < HD / 16; ++ks) {
+    const uint2 v = __ldg(reinterpret_cast<const uint2*>(row + 16 * ks));
+    r.x[2 * ks] = v.x; r.x[2 * ks + 1] = v.y;
   }
   return r;
 }
@@ -175,7 +190,8 @@ __global__ void __launch_bounds__(kPackThreads, 1) k_attn_mma(AttnParams p) {
   const int tile = p.tile, C = p.C, H = p.H;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, qr = lane >> 2, qt = lane & 3;
   const float qscale = p.scale * kLog2e;
-  const T* qkv = reinterpret_cast<const T*>(p.qkv) + qt * (HD / 4);
+  const T* qkv = reinterpret_cast<const T*>(p.qkv) + qt * 4;
+  const int v_off = 2 * C + qt * (HD / 4 - 4);   // from a lane's first channels of q to those of v
   if (threadIdx.x == 0) {
     mbar_init(&tbar, 1);
     mbar_fence_init();
@@ -325,16 +341,16 @@ __global__ void __launch_bounds__(kPackThreads, 1) k_attn_mma(AttnParams p) {
     const int row_lo = ((me_lo >> 16) + p.rel_off) * row_b + h * 4, row_hi = ((me_hi >> 16) + p.rel_off) * row_b + h * 4;
     const int64_t row_e = (int64_t)3 * C;
     PackRows<HD> r;
-    r.q_lo = load_part<T, HD>(qkv + (q_lo < 0 ? some : q_lo) * row_e + h * HD);
-    r.q_hi = load_part<T, HD>(qkv + (q_hi < 0 ? some : q_hi) * row_e + h * HD);
+    r.q_lo = load_operand<T, HD>(qkv + (q_lo < 0 ? some : q_lo) * row_e + h * HD);
+    r.q_hi = load_operand<T, HD>(qkv + (q_hi < 0 ? some : q_hi) * row_e + h * HD);
     begin(r);
     for (int k0 = 0; k0 < c; k0 += 16) {
       const int vox = k_vox, info = k_info;
       row_of(k0 + 16 + lane, k0 + 16 + lane < c, k_vox, k_info);
       const int n_lo = __shfl_sync(0xffffffffu, vox, qr), n_hi = __shfl_sync(0xffffffffu, vox, qr + 8);
-      const T *klo = qkv + (n_lo < 0 ? some : n_lo) * row_e + C + h * HD, *khi = qkv + (n_hi < 0 ? some : n_hi) * row_e + C + h * HD;
-      const RowPart<HD> k_lo = load_part<T, HD>(klo), k_hi = load_part<T, HD>(khi);
-      const RowPart<HD> v_lo = load_part<T, HD>(klo + C), v_hi = load_part<T, HD>(khi + C);
+      const T *klo = qkv + (n_lo < 0 ? some : n_lo) * row_e + h * HD, *khi = qkv + (n_hi < 0 ? some : n_hi) * row_e + h * HD;
+      const RowPart<HD> k_lo = load_operand<T, HD>(klo + C), k_hi = load_operand<T, HD>(khi + C);
+      const RowPart<HD> v_lo = load_part<T, HD>(klo + v_off), v_hi = load_part<T, HD>(khi + v_off);
       float add_lo[4], add_hi[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -375,10 +391,10 @@ __global__ void __launch_bounds__(kPackThreads, 1) k_attn_mma(AttnParams p) {
       }
       for (int h = cur.h0; h < H; h += parts, lo += parts * HD, hi += parts * HD) {
         PackRows<HD> r;
-        r.q_lo = load_part<T, HD>(lo);
-        r.q_hi = load_part<T, HD>(hi);
-        const RowPart<HD> k_lo = load_part<T, HD>(lo + C), k_hi = load_part<T, HD>(hi + C);
-        const RowPart<HD> v_lo = load_part<T, HD>(lo + 2 * C), v_hi = load_part<T, HD>(hi + 2 * C);
+        r.q_lo = load_operand<T, HD>(lo);
+        r.q_hi = load_operand<T, HD>(hi);
+        const RowPart<HD> k_lo = load_operand<T, HD>(lo + C), k_hi = load_operand<T, HD>(hi + C);
+        const RowPart<HD> v_lo = load_part<T, HD>(lo + v_off), v_hi = load_part<T, HD>(hi + v_off);
         float add_lo[4], add_hi[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
@@ -394,14 +410,14 @@ __global__ void __launch_bounds__(kPackThreads, 1) k_attn_mma(AttnParams p) {
       const int kbase = slot0 / cpad * cpad, blocks = cpad >> 4;
       for (int h = cur.h0; h < H; h += parts, lo += parts * HD, hi += parts * HD) {
         PackRows<HD> r;
-        r.q_lo = load_part<T, HD>(lo);
-        r.q_hi = load_part<T, HD>(hi);
+        r.q_lo = load_operand<T, HD>(lo);
+        r.q_hi = load_operand<T, HD>(hi);
         begin(r);
         for (int kb = 0; kb < blocks; ++kb) {
           const int block = kbase + kb * 16, n_lo = of_slot(cur.vox, block, qr), n_hi = of_slot(cur.vox, block, qr + 8);
-          const T *klo = qkv + (n_lo < 0 ? some : n_lo) * row_e + C + h * HD, *khi = qkv + (n_hi < 0 ? some : n_hi) * row_e + C + h * HD;
-          const RowPart<HD> k_lo = load_part<T, HD>(klo), k_hi = load_part<T, HD>(khi);
-          const RowPart<HD> v_lo = load_part<T, HD>(klo + C), v_hi = load_part<T, HD>(khi + C);
+          const T *klo = qkv + (n_lo < 0 ? some : n_lo) * row_e + h * HD, *khi = qkv + (n_hi < 0 ? some : n_hi) * row_e + h * HD;
+          const RowPart<HD> k_lo = load_operand<T, HD>(klo + C), k_hi = load_operand<T, HD>(khi + C);
+          const RowPart<HD> v_lo = load_part<T, HD>(klo + v_off), v_hi = load_part<T, HD>(khi + v_off);
           float add_lo[4], add_hi[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {

@@ -37,3 +37,29 @@ def test_units(dtype, w, heads, hd, counts):
         p_bits, o_bits = (2.0 ** -17, 2.0 ** -8) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -11)
         bound = o_bits + p_bits * float(qkv[:, 2].double().abs().max() / ref.pow(2).mean().sqrt())
         assert rel_err(out.double().cpu(), ref) <= bound
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("c", [8, 40])   # one block of keys, several
+def test_channels_are_added_up_in_order(dtype, c):
+    """Sixteen consecutive channels a product: 2^24 + 1 is 2^24 in fp32, less 2^24 from channel 16 is 0, as a sum channel by channel gives it."""
+    from sparseswin3d_b200 import attention, window
+
+    w, hd = (7, 7, 7), 32
+    coords, dims = _boxes([c] * 3, w, seed=1)
+    n = len(coords)
+    qkv = torch.zeros(n, 3, 1, hd)
+    qkv[:, 0, 0, 0] = qkv[:, 0, 0, 16] = qkv[:, 1, 0, 0] = 4096.0
+    qkv[:, 1, 0, 16] = -4096.0
+    qkv[:, 0, 0, 1] = 1.0
+    qkv[::2, 1, 0, 1] = 1.0   # every second key: with the 1 its score is 1
+    qkv[::2, 2] = 1.0
+    geom = window.resolve_geometry(1, dims, w, (0, 0, 0))
+    plan = window.bucket_windows(coords=coords.cuda(), geom=geom, **attention.plan_params(1, hd, dtype, w))
+    out = attention.window_attention_fused(qkv.to(dtype).cuda(), plan, torch.zeros(13 ** 3, 1).cuda(), 1.0, use_mask=False)
+    plan.raise_on_error()
+    win = O.window_keys(coords, 1, dims, w, (0, 0, 0))[0][:, 0]
+    for x in win.unique():
+        here = win == x
+        # all scores 0: the mean of v, rounded to 16 bits
+        assert (out.float().cpu()[here] - qkv[here, 2].mean(0)).abs().max() <= 2.0 ** -8
