@@ -53,3 +53,32 @@ def test_window_mixes(dtype, w, heads, counts):
     p_bits, o_bits = (2.0 ** -17, 2.0 ** -8) if dtype == torch.bfloat16 else (2.0 ** -11, 2.0 ** -11)
     bound = o_bits + p_bits * float(qkv[:, 2].double().abs().max() / ref.pow(2).mean().sqrt())
     assert rel_err(out.double().cpu(), ref) <= bound
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_key_tiles_beyond_the_bound_are_added_up_rounding_to_nearest(dtype):
+    """All weights 1, a value of 2^14 in the first key tile and of -2^14 in the last, 2^-14 in those between: a tile's 96 of these are
+    three units in the last place of 2^14 together, which fp32 adds keep and sums that are cut off product by product lose."""
+    from sparseswin3d_b200 import attention, window
+
+    w, heads, hd = (9, 9, 9), 2, 32
+    coords, dims = _boxes([729, 729], w, seed=2)
+    n = len(coords)
+    geom = window.resolve_geometry(1, dims, w, (0, 0, 0))
+    plan = window.bucket_windows(coords=coords.cuda(), geom=geom, **attention.plan_params(heads, hd, dtype, w))
+    at = O.window_keys(coords, 1, dims, w, (0, 0, 0))[0][:, 1].long()   # full windows: keys come by position
+    v = torch.zeros(729)
+    v[96:672] = 2.0 ** -14
+    v[3], v[700] = 2.0 ** 14, -(2.0 ** 14)
+    qkv = torch.zeros(n, 3, heads, hd, dtype=dtype)
+    qkv[:, 2] = v[at].to(dtype)[:, None, None]
+    # a bias beyond the bound for one pair of the window, the query in one corner and the key in the other
+    table = torch.zeros(17 ** 3, heads)
+    table[-1] = 100.0
+    out = attention.window_attention_fused(qkv.cuda(), plan, table.cuda(), hd ** -0.5, use_mask=False).float().cpu()
+    plan.raise_on_error()
+    exact = 576 * 2.0 ** -14 / 729
+    rest = at != 728
+    # one rounding of the output; fp16: of a subnormal
+    bound = exact * 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -24
+    assert (out[rest] - exact).abs().max() <= bound
