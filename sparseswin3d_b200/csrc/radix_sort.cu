@@ -13,13 +13,13 @@ namespace ssw {
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
 constexpr int kSortThreads = 256;
-constexpr int kManyRounds = 8, kFewRounds = 4, kManyTiles = 3 * 148;
+constexpr int kManyRounds = 8, kFewRounds = 4;
+constexpr int64_t kManyKeys = (int64_t)3 * 148 * kManyRounds * kSortThreads;
 // Keys a thread takes: a larger tile has longer runs to write and a smaller table to scan, a smaller one has its blocks done sooner.
 // The whole sort with 4 / 8 / 16 keys: 82 / 94 / 111 us for 100 000, 113 / 119 / - for 700 000, 141 / 135 / 158 for 1.3 M,
-// 232 / 221 / 223 for 3.4 M, 448 / 387 / 446 for 8 M; the line lies at three tiles of 2048 a multiprocessor.
-static int sort_rounds(int64_t n) {
-  return n >= (int64_t)kManyRounds * kSortThreads * kManyTiles ? kManyRounds : kFewRounds;
-}
+// 232 / 221 / 223 for 3.4 M, 448 / 387 / 446 for 8 M; the line lies at three tiles of 2048 for each of a B200's 148
+// multiprocessors.  (A constant, not the present device's count: the size of a workspace is asked for without a device.)
+static int sort_rounds(int64_t n) { return n >= kManyKeys ? kManyRounds : kFewRounds; }
 
 __device__ __forceinline__ uint32_t digit_of(int32_t key, int shift) {
   return (((uint32_t)key ^ 0x80000000u) >> shift) & (kRadix - 1);
@@ -126,12 +126,17 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const int32_t* _
 
 using namespace ssw;
 
+// Two key buffers, one value buffer, digit table, scan workspace.
+static int64_t sort_bytes(int64_t n, int rounds) {
+  const int64_t table = (int64_t)kRadix * ceil_div64(n, kSortThreads * rounds);
+  return 4 * (3 * n + table) + 8 * scan_workspace_i64(table) + 64;
+}
+// Small tiles want a larger table: at the line and for some 4 % beyond it, what the largest sort with small tiles wants, so that a workspace for
+// n keys serves fewer as well as they can be served.
 extern "C" int64_t ssw_argsort_workspace_bytes(int64_t n) {
   if (n <= 0) return 64;
-  const int64_t tiles = ceil_div64(n, kSortThreads * sort_rounds(n));
-  const int64_t table = (int64_t)kRadix * tiles;
-  // two key buffers, one value buffer, digit table, scan workspace
-  return 4 * (3 * n + table) + 8 * scan_workspace_i64(table) + 64;
+  const int64_t here = sort_bytes(n, sort_rounds(n)), below = sort_bytes(kManyKeys - 1, kFewRounds);
+  return n >= kManyKeys && here < below ? below : here;
 }
 
 extern "C" int ssw_argsort_i32(const int32_t* keys, int64_t n, int32_t* perm_out, void* workspace,
@@ -140,10 +145,11 @@ extern "C" int ssw_argsort_i32(const int32_t* keys, int64_t n, int32_t* perm_out
   if (n == 0) return SSW_OK;
   if (n >= (int64_t(1) << 31)) return SSW_E_RANGE;
   if (!keys || !perm_out || !workspace) return SSW_E_INVALID;
-  if (workspace_bytes < ssw_argsort_workspace_bytes(n)) return SSW_E_WORKSPACE;
+  if (workspace_bytes < sort_bytes(n, kManyRounds)) return SSW_E_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
-  const bool many = sort_rounds(n) == kManyRounds;
-  const int tiles = (int)ceil_div64(n, kSortThreads * sort_rounds(n));
+  // a workspace that holds the table of large tiles alone gets these: the same order, in a little more time
+  const bool many = sort_rounds(n) == kManyRounds || workspace_bytes < sort_bytes(n, kFewRounds);
+  const int tiles = (int)ceil_div64(n, kSortThreads * (many ? kManyRounds : kFewRounds));
   const int64_t table = (int64_t)kRadix * tiles;
   long long* ws = (long long*)workspace;
   const int64_t ws_i64 = scan_workspace_i64(table);

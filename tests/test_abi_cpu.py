@@ -103,3 +103,14 @@ def test_submanifold_rulebook_sizes():
     invalid, out_of_range = -1, -2
     assert status(100, (64, 64, 64), 3) == invalid and status(7_000_000, (400, 400, 400), 7) == invalid
     assert status(2 ** 31, (400, 400, 400), 1) == out_of_range and status(100, (2048, 1024, 1024), 3) == out_of_range
+
+
+def test_argsort_workspace_for_more_keys_serves_fewer():
+    from sparseswin3d_b200 import _lib
+
+    b = _lib.lib.ssw_argsort_workspace_bytes
+    line = 444 * 2048   # tiles of 1024 keys below, of 2048 from here on
+    sizes = sorted({*range(1, 5000, 7), *range(line - 3000, line + 3000, 11), line - 1, line, line + 1, *range(line, line + 60000, 1023), 10 ** 7, 2 ** 31 - 1})
+    got = [b(n) for n in sizes]
+    assert all(x <= y for x, y in zip(got, got[1:]))
+    assert b(0) == 64 and b(10 ** 7) < 13 * 10 ** 7

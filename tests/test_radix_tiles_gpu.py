@@ -18,3 +18,19 @@ def test_stable_order(n, keys):
          "signed": torch.randint(-2 ** 31, 2 ** 31, (n,), generator=g),
          "descending": -torch.arange(n)}[keys].to(torch.int32)
     assert torch.equal(ops.sort_indices(k.cuda()).cpu(), O.sort_indices(k))
+
+
+@pytest.mark.parametrize("n, room", [(909311, 909312), (3000, 3000), (908000, 908000)])
+def test_workspaces_of_large_tiles_are_taken(n, room):
+    """The size without the longer table of small tiles: 12 bytes a key, 1024 for each 2048 keys, the scan's and 64."""
+    from sparseswin3d_b200 import _lib
+
+    tiles = -(-room // 2048)
+    k = torch.randint(-2 ** 31, 2 ** 31, (n,), generator=torch.Generator().manual_seed(n)).to(torch.int32)
+    size = 12 * room + 1024 * tiles + 8 * (2 + -(-256 * tiles // 2048)) + 64
+    keys, out = k.cuda(), torch.empty(n, dtype=torch.int32, device="cuda")
+    ws = torch.empty(size, dtype=torch.uint8, device="cuda")
+    args = keys.data_ptr(), n, out.data_ptr(), ws.data_ptr()
+    assert _lib.lib.ssw_argsort_i32(*args, size - 4 * (room - n) * 3 - 8192, _lib.stream_ptr(out.device)) == -5   # (nothing is launched)
+    assert _lib.lib.ssw_argsort_i32(*args, size, _lib.stream_ptr(out.device)) == 0
+    assert torch.equal(out.cpu(), O.sort_indices(k))
