@@ -711,7 +711,7 @@ static int launch_bwd(const BwdParams& p, cudaStream_t stream) {
   // two blocks per SM, every block on one head throughout (it keeps that head's table column)
   const unsigned grid = (unsigned)(p.H * (2 * sms > p.H ? 2 * sms / p.H : 1));
   for (int k = 0; k < (p.n_per_window > kBwdRows ? 3 : 1); ++k) {
-    SSW_CUDA_TRY(cudaFuncSetAttribute(kerns[k], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SSW_CUDA_TRY(allow_smem(kerns[k]));
     SSW_CUDA_TRY(launch_chained(kerns[k], dim3(grid), dim3(kBwdThreads), smem, stream, p));
   }
   return SSW_OK;

@@ -873,7 +873,7 @@ int run_attn_dense(const AttnParams& a, const int32_t* bins, const int32_t* win_
   void (*kern)(DenseParams) =
       dtype == SSW_BF16 ? (p.use_mask ? k_attn_dense<__nv_bfloat16, true> : k_attn_dense<__nv_bfloat16, false>)
                         : (p.use_mask ? k_attn_dense<__half, true> : k_attn_dense<__half, false>);
-  SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SSW_CUDA_TRY(allow_smem(kern));
   SSW_CUDA_TRY(launch_chained(kern, dim3(sms), dim3(kDThreads), smem, stream, p));
   SSW_LAUNCH_CHECK("k_attn_dense");
   return SSW_OK;

@@ -780,7 +780,7 @@ static int launch_attn(const AttnParams& p, int threads, size_t smem, cudaStream
     if (p.split) {
       if (threads > 640) return SSW_E_UNSUPPORTED;
       void (*kern)(AttnParams) = k_attn_fused<T, HD, kTableSmem, 640, true>;
-      SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      SSW_CUDA_TRY(allow_smem(kern));
       SSW_CUDA_TRY(launch_chained(kern, dim3(sms), dim3(threads), smem, stream, p));
       SSW_LAUNCH_CHECK("k_attn_fused");
       return SSW_OK;
@@ -788,15 +788,15 @@ static int launch_attn(const AttnParams& p, int threads, size_t smem, cudaStream
   }
   if (threads <= 384) {
     auto kern = k_attn_fused<T, HD, kTableSmem, 384, false>;
-    SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SSW_CUDA_TRY(allow_smem(kern));
     SSW_CUDA_TRY(launch_chained(kern, dim3(sms), dim3(threads), smem, stream, p));
   } else if (threads <= 512) {
     auto kern = k_attn_fused<T, HD, kTableSmem, 512, false>;
-    SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SSW_CUDA_TRY(allow_smem(kern));
     SSW_CUDA_TRY(launch_chained(kern, dim3(sms), dim3(threads), smem, stream, p));
   } else {
     auto kern = k_attn_fused<T, HD, kTableSmem, 1024, false>;
-    SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SSW_CUDA_TRY(allow_smem(kern));
     SSW_CUDA_TRY(launch_chained(kern, dim3(sms), dim3(threads), smem, stream, p));
   }
   SSW_LAUNCH_CHECK("k_attn_fused");

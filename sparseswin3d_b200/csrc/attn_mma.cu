@@ -27,6 +27,7 @@
 
 namespace ssw {
 
+constexpr int kTableMost = 160 * 1024;   // bytes of a bias table in shared memory
 constexpr int kPackThreads = 640;        // one block per SM: 96 registers a thread, one copy of the bias table
 constexpr int kPackWindow = 127;         // window number of unused slots (bits 5..11 of a slot's word)
 constexpr int kPackWindowBits = 127 << 5;
@@ -439,7 +440,7 @@ static int launch_packs(AttnParams p, bool big, const int32_t rpb_window[3], cud
   SSW_CUDA_TRY(cudaGetDevice(&dev));
   SSW_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int64_t entries = (int64_t)(2 * rpb_window[0] - 1) * (2 * rpb_window[1] - 1) * (2 * rpb_window[2] - 1) * p.H;
-  const bool in_smem = entries * 4 <= 160 * 1024;   // the rest of the SM's 256 KB is L1, for the rows
+  const bool in_smem = entries * 4 <= kTableMost;   // the rest of the SM's 256 KB is L1, for the rows
   p.table_floats = in_smem ? (int)entries : 0;
   const size_t smem = in_smem ? ((size_t)entries * 4 + 15) & ~(size_t)15 : 0;
   void (*kern)(AttnParams);
@@ -449,7 +450,7 @@ static int launch_packs(AttnParams p, bool big, const int32_t rpb_window[3], cud
   auto pick2 = [&](auto table_smem, auto mask) { big ? pick(table_smem, mask, std::true_type{}) : pick(table_smem, mask, std::false_type{}); };
   auto pick1 = [&](auto table_smem) { p.use_mask ? pick2(table_smem, std::true_type{}) : pick2(table_smem, std::false_type{}); };
   in_smem ? pick1(std::true_type{}) : pick1(std::false_type{});
-  SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SSW_CUDA_TRY(allow_smem(kern, kTableMost));
   SSW_CUDA_TRY(launch_chained(kern, dim3(sms), dim3(kPackThreads), smem, stream, p));
   SSW_LAUNCH_CHECK("k_attn_mma");
   return SSW_OK;

@@ -22,6 +22,7 @@ constexpr int kTRows = 64;       // query rows of a unit at most, keys of a stag
 constexpr int kTThreads = 2 * kTRows;
 constexpr int kTBlocks = 4;      // blocks per SM the registers are kept to
 constexpr int kTLevels = 16;     // units per (window, head): up to 1023 rows
+constexpr int kTSmemMost = 113 * 1024;   // two blocks an SM at least
 
 struct TileParams {
   const float* qkv;
@@ -283,7 +284,7 @@ static int tiles_table(const int32_t w[3]) { return (2 * w[0] - 1) * (2 * w[1] -
 // voxels, 3 heads) it took 93 + 18 us where k_attn_fused alone takes 105, at 10 66 + 94 for 225.
 bool attn_tiles_pays(const AttnParams& a, int n_per_window, int64_t n_windows, int head_dim, const int32_t rpb_window[3]) {
   if (n_per_window <= a.tile || (head_dim != 16 && head_dim != 32)) return false;
-  if (tiles_smem<32>(tiles_table(rpb_window)) > 113 * 1024) return false;   // (two blocks an SM at least)
+  if (tiles_smem<32>(tiles_table(rpb_window)) > kTSmemMost) return false;
   return a.tile < 48 || a.n_vox >= 6 * n_windows;
 }
 
@@ -296,7 +297,7 @@ static int launch_tiles(const TileParams& p, cudaStream_t stream) {
   int per_sm = (int)((227 * 1024) / (smem + 1024 + 64));
   if (per_sm > kTBlocks) per_sm = kTBlocks;
   const int all = sms * per_sm, grid = all >= p.H ? all / p.H * p.H : all;
-  SSW_CUDA_TRY(cudaFuncSetAttribute(k_attn_tiles<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SSW_CUDA_TRY(allow_smem(k_attn_tiles<HD>, kTSmemMost));
   k_attn_tiles<HD><<<grid, kTThreads, smem, stream>>>(p);
   SSW_LAUNCH_CHECK("k_attn_tiles");
   return SSW_OK;

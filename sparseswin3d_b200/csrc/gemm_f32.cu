@@ -765,7 +765,7 @@ static int gemm_nt(const float* a, const float* w, const float* bias, float* out
   auto kern = kept ? k_gemm_f32<true> : k_gemm_f32<false>;
   // kept: tile t, t + grid, ... of a block are of the same columns
   const int64_t grid = kept ? (m_tiles < groups ? m_tiles : groups) * p.n_tiles : p.tiles < sms ? p.tiles : sms;
-  SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  SSW_CUDA_TRY(allow_smem(kern));
   SSW_CUDA_TRY(launch_chained(kern, dim3((unsigned)grid), dim3(kNThreads), (size_t)smem, (cudaStream_t)stream_, p));
   SSW_LAUNCH_CHECK("k_gemm_f32");
   return SSW_OK;
@@ -833,7 +833,7 @@ static int gemm_tn(const float* g, const float* x, float* out, int64_t M, int32_
   p.error = error; p.give_up = give_up;
   if ((int64_t)p.mn_tiles * splits >= ((int64_t)1 << 30)) return SSW_E_RANGE;
   p.tiles = p.mn_tiles * splits;
-  SSW_CUDA_TRY(cudaFuncSetAttribute(k_gemm_f32_tn, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmem));
+  SSW_CUDA_TRY(allow_smem(k_gemm_f32_tn));
   SSW_CUDA_TRY(launch_chained(k_gemm_f32_tn, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kTThreads), kTSmem,
                               (cudaStream_t)stream_, p));
   SSW_CUDA_TRY(launch_chained(k_gemm_reduce, dim3((unsigned)ceil_div64((int64_t)N * K, 256)), dim3(256), 0, (cudaStream_t)stream_,

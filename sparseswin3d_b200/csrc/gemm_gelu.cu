@@ -283,7 +283,7 @@ int ssw::gemm_gelu(const void* a, const void* w, const void* bias, int dtype, vo
   if (m_tiles * p.n_tiles >= ((int64_t)1 << 30)) return SSW_E_RANGE;
   p.tiles = (int)(m_tiles * p.n_tiles);
   auto kern = dtype == SSW_BF16 ? k_gemm_gelu<__nv_bfloat16> : k_gemm_gelu<__half>;
-  SSW_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kHSmem));
+  SSW_CUDA_TRY(allow_smem(kern));
   SSW_CUDA_TRY(launch_chained(kern, dim3((unsigned)(p.tiles < sms ? p.tiles : sms)), dim3(kHThreads), kHSmem, (cudaStream_t)stream_, p));
   return SSW_OK;
 }

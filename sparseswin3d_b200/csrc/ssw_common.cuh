@@ -95,6 +95,14 @@ __host__ __device__ inline int packs_of_bin(int c, int cnt, int tile, int padded
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The dynamic shared memory a launch may ask for is state of the function on its device, not of a launch: every caller sets the same value, the
+// most a kernel is given.  With the size of the call at hand, a caller on another thread could lower it between this one's call and its launch.
+constexpr int kSmemMost = 227 * 1024;   // of a block (a kernel's static shared memory counts)
+template <typename... KArgs>
+static inline cudaError_t allow_smem(void (*kern)(KArgs...), int most = kSmemMost) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 template <typename... KArgs, typename... Args>
 static inline cudaError_t launch_chained(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                          Args... args) {
