@@ -23,10 +23,12 @@ _DTYPES = (torch.float32, torch.bfloat16, torch.float16)
 ADD_NORM_ROWS = 32768
 # Linear, fp32 (the GEMM): 12 000 rows 1128 / 1056 us, 25 000 rows 1178 / 1368, 40 000 rows 1205 / 1922.
 LINEAR_ROWS_F32 = 16384
-# With wider Linears from as much work (rows times the square of the narrower side).  A stage of two blocks, with / without: 192 channels, 3000 rows
-# 2018 / 1881 us, 5000 2036 / 2066, 10 000 2077 / 3177, 16 000 2556 / 4492; 384 channels, 2500 rows 2036 / 2233, 8000 3160 / 5610; 96 channels, 10 000
-# rows 2051 / 1924.
-LINEAR_WORK_F32 = LINEAR_ROWS_F32 * 96 ** 2
+# Wider Linears: (their narrower side, rows).  A stage of two blocks, with / without, on two hosts (what it takes at least is the host's time, 1950 to
+# 2300 us with, 1910 to 2050 without): 192 channels, 4096 rows 2016 / 1921 and 1996 / 1927 us, 5000 2108 / 2115 and 1964 / 2109, 7000 2210 / 2674; 384 channels,
+# 1500 rows 2233 / 2105, 2000 2287 / 2135 and 1946 / 2131, 2500 2501 / 2606 and 1932 / 2314; 768 channels, 512 rows 2378 / 2101 and 1972 / 1913, 850
+# 1983 / 2758, 1024 2164 / 2949 and 1958 / 2875.  96 channels, 12 000 rows 2431 / 2319, 16 384 2141 / 2613.  From these rows on the three products of such a
+# Linear are ones that pay (see _gemm_pays).
+LINEAR_ROWS_F32_WIDE = ((768, 1024), (384, 2500), (192, 5000))
 # Linear, 16 bits (the bias gradient alone), rows at 96 channels: 40 000 rows 1143 / 1125.  A stage of two blocks: 66 000 rows of 96 channels
 # 2245 / 2010, 100 000 2141 / 2170, 150 000 2464 / 2814; 150 000 of 48 2111 / 2065.
 LINEAR_ROWS_16 = 100000
@@ -223,6 +225,8 @@ class _Linear(torch.autograd.Function):
         g = _rows(g)
         gx = gw = gb = None
         if need[0]:
+            # (no question of _gemm_pays: with 16 384 rows the own product is the faster one too where few input channels say otherwise, 16 of them
+            # and 384 outputs 11 us for 14, 20 and 3072 59 for 98; and with fewer rows the lines above are ones from which it pays)
             wt = weight.t()
             if g.dtype == torch.float32 and weight.shape[1] % 4 == 0:
                 wt = wt.contiguous()
@@ -255,7 +259,7 @@ def _own_linear(module: nn.Module, x: torch.Tensor):
 def _few_for_training(m: int, narrow: int, dtype: torch.dtype) -> bool:
     """Too few rows for the passes to pay while autograd records (`narrow`: the narrower side of the Linear)."""
     if dtype == torch.float32:
-        return m < LINEAR_ROWS_F32 and m * narrow ** 2 < LINEAR_WORK_F32
+        return m < LINEAR_ROWS_F32 and not any(narrow >= channels and m >= rows for channels, rows in LINEAR_ROWS_F32_WIDE)
     return m * narrow < 96 * LINEAR_ROWS_16
 
 
