@@ -47,7 +47,9 @@ struct AttnParams {
   int row_stride;     // bytes between fp32 rows in a stage
   int stage_bytes;    // bytes of one pipeline stage
   int table_floats;   // > 0: the bias table is staged in shared memory (that many floats)
-  int skip_big;       // windows beyond a pack are left to k_attn_tiles
+  // windows beyond a pack are left to k_attn_tiles, if they hold so many rows on average (see tiles_take)
+  int skip_big, beyond_rows, n_per_window;
+  const int32_t* bins;
 };
 
 // The attention kernels turn plan entries into addresses.  A plan that is stale or was overwritten
@@ -106,6 +108,15 @@ __device__ __forceinline__ int64_t checked_coo_block(int slot, int c, const Attn
   }
   flag_bad_plan(p);
   return -1;
+}
+
+// Whether the windows beyond a pack are k_attn_tiles' or k_attn_fused's: both ask the same of the plan's tables, so one of them takes each.
+template <typename P>
+__device__ __forceinline__ bool tiles_take(const P& p) {
+  if (p.beyond_rows == 0) return true;
+  const BinTables bins(const_cast<int32_t*>(p.bins), p.n_per_window);
+  const int first = p.tile + 1, end = p.n_per_window + 1;   // (tile <= n_per_window where there are such windows)
+  return bins.rowstart[end] - bins.rowstart[first] >= (int64_t)p.beyond_rows * (bins.wstart[end] - bins.wstart[first]);
 }
 
 __device__ __forceinline__ float fast_exp2(float x) {

@@ -612,7 +612,7 @@ __global__ void __maxnreg__(regs_for_threads(MAXT)) k_attn_fused(AttnParams p) {
   // ------------------------------------------------------------------------------------------
   // Phase B: windows with c > tile; one query tile per item, key tiles through stage 0 (unless k_attn_tiles takes them)
   // ------------------------------------------------------------------------------------------
-  if (p.skip_big) return;
+  if (p.skip_big && tiles_take(p)) return;
   // Key tiles alternate between stages 0 and 1: the copy of the next tile is in flight while the
   // current one is used.  In the lane-pair form two adjacent threads share a (row, head).
   constexpr int HB = kSplit ? HD / 2 : HD;  // channels per thread
@@ -813,9 +813,9 @@ static int dispatch(const AttnParams& p, int hd, int threads, size_t smem, cudaS
   return SSW_E_UNSUPPORTED;
 }
 
-bool attn_tiles_pays(const AttnParams& a, int n_per_window, int64_t n_windows, int head_dim, const int32_t rpb_window[3]);
-int run_attn_tiles(const AttnParams& a, const int32_t* bins, const int32_t* win_start, const int32_t* win_pstart, int n_per_window,
-                   int head_dim, const int32_t rpb_window[3], cudaStream_t stream);
+bool attn_tiles_pays(const AttnParams& a, int64_t n_windows, int head_dim, const int32_t rpb_window[3], int* beyond_rows);
+int run_attn_tiles(const AttnParams& a, const int32_t* win_start, const int32_t* win_pstart, int head_dim, const int32_t rpb_window[3],
+                   cudaStream_t stream);
 int mma_default_tile(int heads, int head_dim, const int32_t rpb_window[3]);
 int run_attn_mma(AttnParams p, int dtype, int head_dim, const int32_t rpb_window[3], const int32_t* bins,
                  const int32_t* win_start, const int32_t* win_pstart, int n_per_window, cudaStream_t stream);
@@ -912,11 +912,12 @@ extern "C" int ssw_attn_fused_multi(const void* qkv, int dtype, int32_t heads, i
   p.table_floats = s.table_floats;
   switch (dtype) {
     case SSW_F32: {
-      p.skip_big = split && attn_tiles_pays(p, (int)L->n_per_window, L->n_windows, head_dim, rpb_window);
+      p.bins = plan + L->off_bins;
+      p.n_per_window = (int)L->n_per_window;
+      p.skip_big = split && attn_tiles_pays(p, L->n_windows, head_dim, rpb_window, &p.beyond_rows);
       const int st = dispatch<float>(p, head_dim, threads, s.smem, stream);
       if (st != SSW_OK || !p.skip_big) return st;
-      return run_attn_tiles(p, plan + L->off_bins, plan + L->off_win_start, plan + L->off_win_pstart, (int)L->n_per_window, head_dim,
-                            rpb_window, stream);
+      return run_attn_tiles(p, plan + L->off_win_start, plan + L->off_win_pstart, head_dim, rpb_window, stream);
     }
     case SSW_BF16: return dispatch<__nv_bfloat16>(p, head_dim, threads, s.smem, stream);
     case SSW_F16: return dispatch<__half>(p, head_dim, threads, s.smem, stream);

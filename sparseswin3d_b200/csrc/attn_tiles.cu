@@ -30,7 +30,7 @@ struct TileParams {
   int32_t* header;
   const int32_t *bins, *pack_win, *win_start, *win_pstart, *pack_perm, *pack_meta;
   const float* table;
-  int rel_off, H, C, tile, n_per_window, table_rows, n_vox, w_cap;
+  int rel_off, H, C, tile, n_per_window, beyond_rows, table_rows, n_vox, w_cap;
   float scale;
   int use_mask;
 };
@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(kTThreads, kTBlocks) k_attn_tiles(TileParams p
   __shared__ int level_units[kTLevels];
   float* bias = reinterpret_cast<float*>(smem + 2 * kTRows * RB);
   const int H = p.H, C = p.C, tid = threadIdx.x, x = tid & 1, kh = tid / kTRows;   // half of the channels, which of the keys
+  if (!tiles_take(p)) return;
   const int r0 = (tid & 32) + (tid >> 1 & 15);   // this thread's query rows of the unit: r0 and r0 + 16
   const float qscale = p.scale * kLog2e;
   // Windows come in pack order by occupancy, so those with more than 64 k rows are the last ones.  Level k holds the units of their query rows
@@ -188,9 +189,8 @@ __global__ void __launch_bounds__(kTThreads, kTBlocks) k_attn_tiles(TileParams p
     const int c = cur.c, h = cur.h;
     const bool more = u + (int)gridDim.x < n_units;
     if (more) next = find(u + gridDim.x);
-    // the window's query rows in equal shares of whole warps
-    const int nb = (c + kTRows - 1) / kTRows, share = ((c + nb - 1) / nb + 31) & ~31;
-    const int q0 = cur.qb * share, q_rows = min(share, c - q0);
+    const int nb = (c + kTRows - 1) / kTRows;   // key tiles
+    const int q0 = cur.qb * kTRows, q_rows = min(kTRows, c - q0);
     const bool active = (tid & 32) < q_rows;   // of the warp
     RowPair<HH> st;
     st.reset();
@@ -279,13 +279,26 @@ template <int HD>
 static size_t tiles_smem(int table_rows) { return 2 * kTRows * TileRow<HD>::kBytes + (((size_t)table_rows * 4 + 15) & ~(size_t)15); }
 static int tiles_table(const int32_t w[3]) { return (2 * w[0] - 1) * (2 * w[1] - 1) * (2 * w[2] - 1); }
 
-// Whether a launch of its own for the windows beyond a pack pays.  Where packs hold 48 rows, raw scans have none or a few (a window in 13 000 at
-// 150 000 voxels: two voxels for each window of the dense grid), and the launch costs 3 us: it is made from six voxels a window on.  At 4.5 (150 000
-// voxels, 3 heads) it took 93 + 18 us where k_attn_fused alone takes 105, at 10 66 + 94 for 225.
-bool attn_tiles_pays(const AttnParams& a, int n_per_window, int64_t n_windows, int head_dim, const int32_t rpb_window[3]) {
-  if (n_per_window <= a.tile || (head_dim != 16 && head_dim != 32)) return false;
+// Whether a launch of its own for the windows beyond a pack pays.  The host knows how many voxels there are for each window of the dense grid, not how
+// many windows are beyond a pack: a launch that finds none costs 2 us.  us, k_attn_fused alone / both kernels, by voxels for each window (7^3, room
+// scenes where nothing is said):
+// packs of 48 rows (3 heads of 32): 40 000 voxels at 4.0 37 / 37, at 8.4 41 / 43; 150 000 at 4.6 112 / 101, at 10 230 / 162; 10 000 at 7.4 26 / 24; cells drawn
+//   evenly, no window beyond a pack, 20 000 at 20 20 / 22, 100 000 at 15 49 / 51;
+// 32 (6 of 32): 2000 at 2.0 8.3 / 10.2, 10 000 at 2.6 28 / 24, 40 000 at 4.0 63 / 67, 150 000 at 2.0 161 / 165, at 4.6 308 / 267;
+// 24 (8 of 32): 2000 at 2.0 8.0 / 9.4, 10 000 at 2.6 30 / 27, 40 000 at 4.0 94 / 88, 150 000 at 0.7 150 / 152, at 2.0 242 / 233;
+// 16 (24 of 16): 2000 at 2.0 22 / 16, 10 000 at 1.0 20 / 22, 40 000 at 4.0 217 / 226, at 8.4 396 / 347, 150 000 at 4.6 1257 / 1322.
+// Few voxels leave SMs idle in k_attn_fused's second phase, so the line lies lower there.  With packs of 16 rows, many windows of little more than
+// that are better left to the second phase, whose tiles are as small: a unit of 64 rows does a third of its work on 20 (cells drawn evenly, 100 000
+// voxels, windows beyond a pack of 19.7 rows on average: 636 / 748; rooms, 23.2 rows 217 / 226, 26.7 396 / 347; both kernels ask the plan: see tiles_take).
+bool attn_tiles_pays(const AttnParams& a, int64_t n_windows, int head_dim, const int32_t rpb_window[3], int* beyond_rows) {
+  *beyond_rows = 0;
+  if (a.n_per_window <= a.tile || (head_dim != 16 && head_dim != 32)) return false;
   if (tiles_smem<32>(tiles_table(rpb_window)) > kTSmemMost) return false;
-  return a.tile < 48 || a.n_vox >= 6 * n_windows;
+  const bool few = a.n_vox <= 16384;
+  if (a.tile < 24 && !few) *beyond_rows = 26;
+  // voxels for four windows
+  const int line = a.tile >= 48 ? 24 : a.tile >= 32 ? (few ? 10 : 17) : a.tile >= 24 ? (few ? 10 : 16) : few ? 8 : 28;
+  return 4 * (int64_t)a.n_vox >= line * n_windows;
 }
 
 template <int HD>
@@ -303,13 +316,13 @@ static int launch_tiles(const TileParams& p, cudaStream_t stream) {
   return SSW_OK;
 }
 
-int run_attn_tiles(const AttnParams& a, const int32_t* bins, const int32_t* win_start, const int32_t* win_pstart, int n_per_window,
-                   int head_dim, const int32_t rpb_window[3], cudaStream_t stream) {
+int run_attn_tiles(const AttnParams& a, const int32_t* win_start, const int32_t* win_pstart, int head_dim, const int32_t rpb_window[3],
+                   cudaStream_t stream) {
   TileParams p = {};
   p.qkv = reinterpret_cast<const float*>(a.qkv);
   p.outs = a.outs;
   p.header = a.header;
-  p.bins = bins;
+  p.bins = a.bins;
   p.pack_win = a.pack_win;
   p.win_start = win_start;
   p.win_pstart = win_pstart;
@@ -320,7 +333,8 @@ int run_attn_tiles(const AttnParams& a, const int32_t* bins, const int32_t* win_
   p.H = a.H;
   p.C = a.C;
   p.tile = a.tile;
-  p.n_per_window = n_per_window;
+  p.n_per_window = a.n_per_window;
+  p.beyond_rows = a.beyond_rows;
   p.table_rows = tiles_table(rpb_window);
   p.n_vox = a.n_vox;
   p.w_cap = a.w_cap;

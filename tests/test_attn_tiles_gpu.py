@@ -15,6 +15,8 @@ pytestmark = pytest.mark.gpu
     ((7, 7, 7), 3, 32, [49, 48, 47, 65, 200] * 2),     # packs of 48 rows
     ((10, 10, 10), 6, 16, [1000, 961, 40]),            # sixteen shares
     ((7, 7, 7), 24, 16, [50] * 60),                    # more units than blocks
+    ((7, 7, 7), 12, 32, [20] * 850 + [3] * 10),        # packs of 16 rows, and windows beyond them too small on average
+    ((7, 7, 7), 12, 32, [20] * 200 + [40] * 330),      # ... and not
 ])
 def test_windows_beyond_a_pack(w, heads, hd, counts):
     from sparseswin3d_b200 import attention, window
