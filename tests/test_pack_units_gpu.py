@@ -63,3 +63,27 @@ def test_channels_are_added_up_in_order(dtype, c):
         here = win == x
         # all scores 0: the mean of v, rounded to 16 bits
         assert (out.float().cpu()[here] - qkv[here, 2].mean(0)).abs().max() <= 2.0 ** -8
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("c, spoilt", [(16, 1), (20, 1), (4, 4)])   # a window a tile of sixteen slots, tiles of its own, four windows a tile
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("part", [1, 2])   # k, v
+def test_rows_that_are_not_finite_spoil_their_tile_at_most(dtype, c, spoilt, value, part):
+    from sparseswin3d_b200 import attention, window
+
+    w, heads, hd = (7, 7, 7), 2, 32
+    coords, dims = _boxes([c] * 40, w, seed=8)
+    n = len(coords)
+    qkv = torch.randn(n, 3, heads, hd, generator=torch.Generator().manual_seed(9)).to(dtype)
+    table = torch.zeros(13 ** 3, heads, device="cuda")
+    geom = window.resolve_geometry(1, dims, w, (0, 0, 0))
+    plan = window.bucket_windows(coords=coords.cuda(), geom=geom, **attention.plan_params(heads, hd, dtype, w))
+    whole = attention.window_attention_fused(qkv.cuda(), plan, table, hd ** -0.5, use_mask=False).cpu()
+    qkv[17, part, 0] = value
+    out = attention.window_attention_fused(qkv.cuda(), plan, table, hd ** -0.5, use_mask=False).cpu()
+    plan.raise_on_error()
+    win = O.window_keys(coords, 1, dims, w, (0, 0, 0))[0][:, 0]
+    other = ~torch.isclose(out, whole, rtol=0, atol=0, equal_nan=True).view(n, -1).all(1)
+    assert win[17] in win[other] and len(win[other].unique()) <= spoilt
+    assert torch.equal(out.view(n, heads, hd)[:, 1], whole.view(n, heads, hd)[:, 1])   # (the other head is untouched)
