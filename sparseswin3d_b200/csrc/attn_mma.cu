@@ -1,11 +1,12 @@
 // Fused window attention for 16-bit inputs (bf16 / fp16) on packs of sparse windows (mma.sync): a unit of work is 16 row slots of a pack, by one
-// warp and in its registers.
+// warp and in its registers.  (With 32 channels a head not quite: 20 warps leave 96, and 80 to 120 bytes a thread are spilled, 170 with windows beyond
+// a pack; with 16 none.)
 //
 // The plan is *padded*: inside a pack every window gets a run of row slots rounded up to 1, 2, 4, 8, 16, 32, 48 or 64, so 16 slots hold whole windows
 // (several when c < 16) or a 16-row slice of one window.  Softmax keeps upstream's semantics: the maximum starts at 0, the denominator gets
 // +1e-8 (ops.cu:137, 164); bias from a copy of the table in shared memory (pre-multiplied by log2 e), -100 shift mask.  Values that are not finite:
-// upstream confines them to their own window; here a v row that holds Inf or NaN also spoils the other windows that share its 16
-// slots (p = 0 for those keys, and 0 * Inf is NaN).  Windows beyond a pack come here as well where the tcgen05 kernel does not serve them
+// upstream confines them to their own window; here a k or v row that holds Inf or NaN also spoils the other windows that share its 16
+// slots (the mask is added to the score, p is multiplied with v, and neither Inf - Inf nor 0 * Inf is 0).  Windows beyond a pack come here as well where the tcgen05 kernel does not serve them
 // (16 channels a head, or a bias table too large): 16 query rows and a head at a time, key blocks in turn.
 //
 // The queries of 16 slots against their own window's keys, 16 at a time, are m16n8k16 products, and the fragments are loaded from the voxel
@@ -20,7 +21,7 @@
 // us, with whole rows copied to shared memory by one bulk copy each and read from there by ldmatrix / so (rooms, windows of 7^3, shifted): 150 000 voxels,
 // 3 heads of 32 bf16 48.8 / 45.5, 6 heads 82.7 / 65.8, 12 heads of 16 143 / 97, 3 of 16 40 / 35; 150 000 voxels of 23 a window 71 / 66; 4 x 33 333, 6 heads
 // of 16 fp16 with the windows beyond a pack 37 / 32; 2 000 10.3 / 8.3; 100 000, windows of 5^3, fp16 30.6 / 26.  Bound by instructions and their
-// latencies: 17.5 M warp instructions at 150 000 x 3 heads (22.4 M before), 43 % of the issue slots with 20 warps an SM.  16 warps of 128 registers
+// latencies: 18 M warp instructions at 150 000 x 3 heads (22.4 M before), 44 % of the issue slots with 20 warps an SM.  16 warps of 128 registers
 // 46 us (4 x 33 333: 44), 24 of 80 49 us; the rows of the next head asked for ahead in registers 45, the next unit's rows brought into L2 46.
 #include "attn_common.cuh"
 #include "tcgen05.cuh"
@@ -457,8 +458,8 @@ static int launch_packs(AttnParams p, bool big, const int32_t rpb_window[3], cud
 }
 
 // What the default tile and the widest rows follow: the room that five, or three, stages of whole rows would take in one SM's shared memory
-// beside the bias table.  The kernel above keeps no rows there, but plans are built, sized and saved with these tiles, and rows wider than
-// that have always been refused.
+// beside the bias table.  No kernel keeps rows there any more, and nothing else asks for the smaller tile of wide rows (32 slots at 12 heads of 32): it stays
+// because plans are built, sized and saved with it, and which windows are beyond a pack follows from it.  Rows wider than that have always been refused.
 static int row_stages(int tile, int heads, int head_dim, const int32_t rpb_window[3]) {
   const int64_t stride = (int64_t)3 * heads * head_dim * 2 + 16;
   const int64_t per_stage = 16 + kMaxTile * 4 + tile * stride + producer_scratch_bytes(tile);

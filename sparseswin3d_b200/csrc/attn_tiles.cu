@@ -12,7 +12,7 @@
 // us, with k_attn_fused alone / this kernel and k_attn_fused for the packs (room scenes, windows of 7^3): 10 000 voxels of 34-49 a window, 6 heads 86 /
 // 41 + 12; 2 500, 12 heads 74 / 35 + 7; 40 000, 6 heads 180 / 99 + 36; 40 000, 3 heads 93 / 36 + 30; 150 000, 3 heads 225 / 66 + 94; full 9^3 windows,
 // 45 700 voxels, 6 heads 1731 / 924 + 13.  Bound by the latency of a row's chain (dot product, maximum, exponential, sum) at 15 warps an
-// SM: issue slots 51 %, shared memory 54 %.  One row on two lanes, 18 warps: 41 and 1096 us (shared memory 77 %: a 16-byte load returns
+// SM (128 registers; 32 channels spill 40 bytes a thread): issue slots 51 %, shared memory 54 %.  One row on two lanes, 18 warps: 41 and 1096 us (shared memory 77 %: a 16-byte load returns
 // 512 bytes a warp however few addresses it names); one row a thread: 55 and 1289; two rows, keys shared among four lanes: 42 and 1073.
 #include "attn_common.cuh"
 

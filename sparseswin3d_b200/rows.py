@@ -168,11 +168,11 @@ def _gemm_ready(x: torch.Tensor, weight: torch.Tensor, first: int = 0) -> bool:
 
 
 def _gemm_pays(m: int, n: int, k: int) -> bool:
-    """Results enough for the fp32 GEMM to be no slower than the library's, which splits K where few tiles of results leave
-    the chip idle.  With bias, (N, K): rows library / own in us.
-    (96, 96): 128 rows 5.5 / 4.4, 2500 7.1 / 4.4; (576, 192): 128 7.6 / 6.3, 512 9.0 / 6.4; (96, 384): 2500 12 / 9, 5000 18 / 10;
-    (192, 768): 512 17 / 15, 2500 26 / 17; (384, 1536): 512 32 / 27, 1000 44 / 29; (768, 3072): 1 row 5 / 51, 512 80 / 55.  (The line was drawn
-    when a tile took 1.5 times as long; it gives up a us or two below, and keeps few rows of long sums with the library.)"""
+    """From where the fp32 GEMM is taken for a product.  The library's splits K where few tiles of results leave the chip idle; the line lies where the two met
+    while a tile here took 1.5 times as long as it does now.  Above it this one is faster at every pair measured; below it so too from 128 rows on, by up to
+    1.7 times, and slower with a few rows of a long sum.  With bias, (N, K): rows library / own in us, * below the line.  (96, 96): *128 5.9 / 4.3,
+    *1000 6.1 / 4.3, 2500 7.1 / 4.5; (576, 192): *128 7.5 / 6.1, 512 9.0 / 6.2; (96, 384): *2500 12 / 9, 5000 18 / 10; (192, 768): *64 15 / 14, *1500 19 / 15,
+    2500 26 / 16; (384, 1536): *64 19 / 26, *512 32 / 27, *1000 44 / 29, 1500 45 / 29; (768, 3072): *1 5 / 50, *256 59 / 50, 512 81 / 55."""
     return m * n >= 1024 * min(k, 384)
 
 
