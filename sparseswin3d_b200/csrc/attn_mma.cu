@@ -20,7 +20,10 @@
 //
 // us, with whole rows copied to shared memory by one bulk copy each and read from there by ldmatrix / so (rooms, windows of 7^3, shifted): 150 000 voxels,
 // 3 heads of 32 bf16 48.8 / 45.5, 6 heads 82.7 / 65.8, 12 heads of 16 143 / 97, 3 of 16 40 / 35; 150 000 voxels of 23 a window 71 / 66; 4 x 33 333, 6 heads
-// of 16 fp16 with the windows beyond a pack 37 / 32; 2 000 10.3 / 8.3; 100 000, windows of 5^3, fp16 30.6 / 26.  Bound by instructions and their
+// of 16 fp16 with the windows beyond a pack 37 / 32; 2 000 10.3 / 8.3; 100 000, windows of 5^3, fp16 30.6 / 26.  Windows beyond a pack alone, 79 000
+// voxels in half-full 9^3 windows, heads of 16, bf16: 6 heads 675 / 553, 12 1373 / 1287, shifted 919 / 726; not so 3 heads 289 / 300 and 12 of fp16 1170 / 1257,
+// where the rows of a window that all warps read from shared memory at a time had been the better form (with the next keys' rows asked for ahead 296 and
+// 1229, but 12 heads shifted 774; with a window's query rows on neighbouring warps 309 and 1298).  Bound by instructions and their
 // latencies: 18 M warp instructions at 150 000 x 3 heads (22.4 M before), 44 % of the issue slots with 20 warps an SM.  16 warps of 128 registers
 // 46 us (4 x 33 333: 44), 24 of 80 49 us; the rows of the next head asked for ahead in registers 45, the next unit's rows brought into L2 46.
 #include "attn_common.cuh"
